@@ -510,13 +510,12 @@ def cell_phases(w, dtype_name):
     t = buf.cpu().numpy().reshape(-1, 8)
     t = t[t[:, 0] > 0]
     if len(t) == 0:
-        return dict(error="no stamps: this shape does not run the split-K tensor-core cell")
+        return dict(error="no stamps: this shape does not run the tcgen05 cell kernel")
     rel = (t - t[:, 0].min()) / 1e3
-    names = ["start", "setup_done", "accumulators_complete", "partial_tile_pushed", "cluster_barrier_passed",
-             "slots_read", "gate_math_done", "stores_issued"]
+    names = {0: "start", 1: "setup_done", 2: "accumulators_complete", 6: "outputs_written", 7: "end"}
     return dict(kernel="lstm_cell", H=H, B=B, dtype=dtype_name, ctas=int(len(t)), unit="us",
                 phases={n: dict(min=round(float(rel[:, i].min()), 2), mean=round(float(rel[:, i].mean()), 2),
-                                max=round(float(rel[:, i].max()), 2)) for i, n in enumerate(names)})
+                                max=round(float(rel[:, i].max()), 2)) for i, n in names.items()})
 
 
 def main():

@@ -9,11 +9,10 @@
 extern "C" {
 #endif
 
-/* Device-side phase stamps of the split-K tensor-core launches.
- * zrnn_debug_tc_profile(d_buf): while d_buf is set, every CTA of every split-K tensor-core launch writes 8
- * %globaltimer values (ns) to d_buf[cta * 8 ..]: start, set-up done, accumulators complete, partial tile pushed,
- * cluster barrier passed, exchange slots read, gate math done, stores issued.  d_buf must hold 8 values per CTA of
- * the largest launch; NULL switches it off.
+/* Device-side phase stamps of the tensor-core launches of the recurrent chain (LSTM cells).
+ * zrnn_debug_tc_profile(d_buf): while d_buf is set, every CTA of every such launch writes %globaltimer values (ns) to
+ * d_buf[cta * 8 ..]: [0] start, [1] set-up done, [2] accumulators complete, [6] outputs written, [7] end.  d_buf must hold 8
+ * values per CTA of the largest launch; NULL switches it off.
  * zrnn_debug_tc_timeline(d_buf, slots): launch i (counted from the call) writes the same 8 stamps of its CTA (0,0,0)
  * to d_buf[i * 8 ..] for i < slots. */
 int zrnn_debug_tc_profile(long long* d_buf);

@@ -1,0 +1,81 @@
+"""LSTM cells and attention steps at the sizes where the launch rule changes kernels or a kernel has a ragged edge: one column,
+whole and broken groups of 8 and 128 columns, hidden sizes that fill no k-block, few and many row tiles, with and without the
+feed-input operand; against a float64 cell / the CPU oracle's tolerances."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# dtype id -> (relative, absolute) tolerance: 3xTF32, fp16 split, bf16, tf32
+TOL = {4: (2e-5, 2e-5), 5: (2e-5, 2e-5), 1: (3e-2, 3e-2), 2: (1e-2, 1e-2)}
+
+
+def sigmoid(x):
+    return 1.0 / (1.0 + np.exp(-x))
+
+
+@pytest.mark.parametrize("dtype", sorted(TOL))
+@pytest.mark.parametrize("H,B", [(64, 1), (68, 3), (104, 9), (264, 16), (500, 17), (504, 33), (520, 64), (1000, 8), (1000, 24),
+                                 (1000, 65), (1000, 127), (1000, 129), (2048, 40), (1024, 700)])
+@pytest.mark.parametrize("feed", [0, 1])
+def test_cell_edges(dtype, H, B, feed):
+    import torch
+    from zoph_rnn_b200 import api
+    if dtype == 1 and H % 8:
+        pytest.skip("bf16 needs a multiple of 8")
+    rng = np.random.default_rng(H * 1000 + B)
+    V = 50
+    t = []
+    for _ in range(4):
+        t += [(rng.standard_normal(H * H) / np.sqrt(H)).astype(np.float32), (rng.standard_normal(H) * 0.1).astype(np.float32)]
+    t.append(rng.uniform(-1, 1, H * V).astype(np.float32))
+    t += [(rng.standard_normal(H * H) / np.sqrt(H)).astype(np.float32) for _ in range(8 if feed else 4)]
+    layer = api.Input_To_Hidden_Layer(H, V, feed_input=bool(feed), dtype=dtype)
+    layer.load_weights(t)
+    ids = rng.integers(0, V, B).astype(np.int32)
+    mask = (rng.random(B) > 0.2).astype(np.int32)
+    h, c, q = (rng.uniform(-1, 1, (B, H)).astype(np.float32) for _ in range(3))
+
+    def dev(a):
+        return torch.as_tensor(np.ascontiguousarray(a)).cuda()
+    got_h, got_c = layer.forward_prop(dev(ids), dev(mask), dev(h.reshape(-1)), dev(c.reshape(-1)), dev(q.reshape(-1)) if feed else None)
+    mat = [np.asarray(x, dtype=np.float64).reshape(-1, H).T for x in t]  # column-major H x H
+    Wh, b, emb, M = [mat[2 * g] for g in range(4)], [t[2 * g + 1].astype(np.float64) for g in range(4)], mat[8], mat[9:13]
+    x = emb[:, ids].T
+    pre = []
+    for g in range(4):  # i, f, g (c), o; the input matrices come as i, f, o, c
+        k = (0, 1, 3, 2)[g]
+        z = x @ M[k].T + h.astype(np.float64) @ Wh[g].T + b[g]
+        if feed:
+            z = z + q.astype(np.float64) @ mat[13 + k].T
+        pre.append(z)
+    cn = sigmoid(pre[1]) * c + sigmoid(pre[0]) * np.tanh(pre[2])
+    hn = sigmoid(pre[3]) * np.tanh(cn)
+    r, a = TOL[dtype]
+    np.testing.assert_allclose(got_h.cpu().numpy().reshape(B, H), hn * mask[:, None], rtol=r, atol=a)
+    np.testing.assert_allclose(got_c.cpu().numpy().reshape(B, H), cn * mask[:, None], rtol=r, atol=a)
+
+
+@pytest.mark.parametrize("dtype", [5, 1, 4])
+@pytest.mark.parametrize("H,B", [(72, 1), (200, 12), (504, 40), (1000, 64), (1000, 130)])
+@pytest.mark.parametrize("att", [1, 2])
+def test_attention_step_edges(oracle, dtype, H, B, att):
+    """The attention step in the tensor-core engines against the exact engine on the same inputs."""
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(H + B)
+    S = 7
+    w = [(rng.standard_normal(H * H) / np.sqrt(H)).astype(np.float32) for _ in range(2)]
+    w += [(rng.standard_normal(H) * 0.05).astype(np.float32), (rng.standard_normal(H) * 0.1).astype(np.float32)]
+    w += [(rng.standard_normal(H * H) / np.sqrt(H)).astype(np.float32) for _ in range(2)]
+    lens = rng.integers(1, S + 1, B).astype(np.int32)
+    hs, h = (torch.as_tensor(rng.uniform(-0.3, 0.3, n).astype(np.float32)).cuda() for n in (S * B * H, B * H))
+    mask = torch.ones(B, dtype=torch.int32, device="cuda")
+    out = {}
+    for dt in (3, dtype):
+        layer = api.attention_layer(H, 3, att_type=att, dtype=dt)
+        layer.load_weights(w)
+        layer.prep_minibatch_info(hs, S, B, torch.as_tensor(lens).cuda(), torch.as_tensor(S - lens).cuda())
+        out[dt] = layer.forward_prop(h, mask).cpu().numpy()
+    r, a = TOL[dtype]
+    np.testing.assert_allclose(out[dtype], out[3], rtol=r, atol=a)

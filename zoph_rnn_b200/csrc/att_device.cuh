@@ -34,6 +34,10 @@ __device__ __forceinline__ void att_store_op(const AttArgs& a, int b, int i, flo
   }
 }
 
+// zeros in the padding of operand row b (the next product reads whole 128-byte blocks), by threads tid, tid + nt, ...
+__device__ __forceinline__ void att_zero_pad(const AttArgs& a, int b, int tid, int nt) {
+  for (int i = a.H + tid; i < a.ld_op; i += nt) att_store_op(a, b, i, 0.f);
+}
 #define ZR_ATT_MAXW 64
 struct SyncCta {  // the team is a whole CTA
   __device__ __forceinline__ void operator()() const { __syncthreads(); }
@@ -78,6 +82,7 @@ __device__ __forceinline__ void att_local_fast_body(const AttArgs& a, const int 
   const int lane = tid & 31, w = tid >> 5;
   const int H = a.H, H4 = H >> 2, Wn = 2 * a.D + 1, sb = b / a.cols_per_sent;
   float* c = a.c_t + (size_t)b * H;
+  att_zero_pad(a, b, tid, kAttTeam);
   if (a.mask && a.mask[b] != 1) {
     for (int i = tid; i < H; i += kAttTeam) { c[i] = 0.f; att_store_op(a, b, i, 0.f); }
     if (a.align_out) {
@@ -267,6 +272,7 @@ __device__ __forceinline__ void att_global_fast_body(const AttArgs& a, const int
   const int lane = tid & 31, w = tid >> 5;
   const int H = a.H, H4 = H >> 2, sb = b / a.cols_per_sent;
   float* c = a.c_t + (size_t)b * H;
+  att_zero_pad(a, b, tid, kAttTeam);
   if (a.mask && a.mask[b] != 1) {
     for (int i = tid; i < H; i += kAttTeam) { c[i] = 0.f; att_store_op(a, b, i, 0.f); }
     if (a.align_out)

@@ -208,16 +208,16 @@ cudaError_t launch_pack_weights(const PackArgs& a, cudaStream_t st) {
 }
 __global__ void convert_rows_kernel(const float* __restrict__ src, long long rows, int K, long long ld_src, int mode,
                                     void* dst_hi, float* dst_lo, long long ld_dst) {
-  const long long total = rows * K;
+  const long long total = rows * ld_dst;  // the padding up to ld_dst is set to zero
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long r = e / K;
-    const int k = (int)(e % K);
-    store_op(dst_hi, dst_lo, mode, (size_t)(r * ld_dst + k), src[r * ld_src + k]);
+    const long long r = e / ld_dst;
+    const int k = (int)(e % ld_dst);
+    store_op(dst_hi, dst_lo, mode, (size_t)e, k < K ? src[r * ld_src + k] : 0.f);
   }
 }
 cudaError_t launch_convert_rows(const float* src, long long rows, int K, long long ld_src, int op_mode, void* dst_hi,
                                 float* dst_lo, long long ld_dst, cudaStream_t st) {
-  const long long total = rows * K;
+  const long long total = rows * ld_dst;
   if (total <= 0) return cudaSuccess;
   long long blocks = (total + 255) / 256;
   convert_rows_kernel<<<(unsigned)(blocks > 148 * 32 ? 148 * 32 : blocks), 256, 0, st>>>(src, rows, K, ld_src, op_mode,
@@ -1007,6 +1007,7 @@ __global__ void __launch_bounds__(256) att_local_kernel(const AttArgs a) {
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int H = a.H, Wn = 2 * a.D + 1, sb = b / a.cols_per_sent;
   float* c = a.c_t + (size_t)b * H;
+  att_zero_pad(a, b, tid, blockDim.x);
   if (a.mask && a.mask[b] != 1) {  // create_indicies_kernel: every window slot is -1 -> context 0
     for (int i = tid; i < H; i += blockDim.x) { c[i] = 0.f; att_store_op(a, b, i, 0.f); }
     if (a.align_out) {
@@ -1113,6 +1114,7 @@ __global__ void __launch_bounds__(256) att_global_kernel(const AttArgs a) {
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int H = a.H, sb = b / a.cols_per_sent;
   float* c = a.c_t + (size_t)b * H;
+  att_zero_pad(a, b, tid, blockDim.x);
   if (a.align_out)
     for (int s = tid; s < a.S_max; s += blockDim.x) a.align_out[(size_t)s * a.B + b] = 0.f;
   if (a.mask && a.mask[b] != 1) {
@@ -1280,6 +1282,15 @@ __device__ __forceinline__ void seq_store_op(const SeqArgs& a, size_t n, int i, 
   }
 }
 
+// zeros in the padding of the operand rows (a later product reads whole 128-byte blocks), after the last step, by all CTAs
+__device__ __forceinline__ void seq_zero_pads(const SeqArgs& a, unsigned rank, unsigned csize) {
+  const int pad = a.ld_op - a.H;
+  if (!a.zero_pad || pad <= 0) return;
+  const size_t total = (size_t)a.S * a.B * pad;
+  for (size_t e = rank * blockDim.x + threadIdx.x; e < total; e += (size_t)csize * blockDim.x)
+    seq_store_op(a, e / pad, a.H + (int)(e % pad), 0.f);
+}
+
 // One cluster of C CTAs per launch.  CTA r keeps Wt[k][jl] = (Wh_i, Wh_f, Wh_g, Wh_o)[j0 + jl, k] for its Hc hidden
 // units in shared memory; thread (jl, cg) owns the cell of unit j0 + jl for CPT consecutive columns.  h_{t-1} lives in
 // every CTA's shared memory (hb[buf][k][column], double-buffered); after a step each thread sends its new h values
@@ -1445,6 +1456,7 @@ __global__ void __launch_bounds__(CPT >= 4 ? 256 : 1024, 1) lstm_seq_resident_ke
       }
     }
   }
+  seq_zero_pads(a, rank, csize);
   // no CTA leaves while a peer may still write into its shared memory or wait for its bytes
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (active)
@@ -1626,6 +1638,9 @@ __global__ void __launch_bounds__(512, 1) lstm_seq_reg_kernel(const SeqArgs a, i
       }
     }
   }
+  unsigned csize;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+  seq_zero_pads(a, rank, csize);
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (col) a.c_out[(size_t)s * H + j] = cst;
 }

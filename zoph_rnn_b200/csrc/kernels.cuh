@@ -121,6 +121,7 @@ struct SeqArgs {
   void* op_h_hi;
   void* op_h_lo;
   int ld_op;
+  int zero_pad;          // keep elements H .. ld_op of the operand rows at zero (attention reads whole 128-byte blocks)
 };
 // false when the shape does not fit (H > 320, B > 32, ...): the caller keeps its per-step path
 bool lstm_seq_resident_supported(int H, int B);

@@ -1,0 +1,70 @@
+// Tensor-core products on the chain between two time steps: LSTM cells, the attention layer's projections and the tanh
+// combiner.  One launch is one link of a chain of dependent launches, so what counts is its latency.  See tc_chain.cu.
+#pragma once
+#include "tc_gemm.cuh"
+
+namespace zrnn {
+
+// acc[M x N] = sum_s A_s[M x K] * W[N x Kcat]^T as in tc_gemm.cuh; M: batch columns, N: weight rows
+struct ChainParams {
+  CUtensorMap a[3];           // activation rows: make_rows_map with a_rows rows, all parts, kbs k-blocks
+  CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units (BN == 256: 32 units,
+                              // one part and one k-block per box)
+  int w_kbtot, w_tiles;       // LSTM: k-blocks per packed tile, packed tiles
+  int nsrc, kb;               // sources, k-blocks per source
+  int kbs;                    // k-blocks per box: chain_kbs(mode, BN, a_rows)
+  int wkb0[3];                // first k-block of each source on the weights' K axis
+  int a_row0[3];              // first row of each source's map that belongs to this problem
+  int a_rows;                 // rows per activation box: a multiple of 8, at most 128
+  int M, N;                   // N: STORE output rows; LSTM hidden size
+  const float* bias;          // STORE [N] or null; LSTM [4][N] gate-major (i,f,g,o)
+  const int* mask;            // [M] or null
+  float* C;                   // fp32 out, row m at C + m * ldc
+  int ldc;
+  int act, act_rows;          // STORE: tanh for n < act_rows (0 = all) when act == 1
+  __nv_bfloat16* op_b16;      // operand-form copies of the output (row m at + m * ld_op), as TcParams
+  float* op_hi;
+  float* op_lo;
+  __half* op_h_hi;
+  __half* op_h_lo;
+  int ld_op;
+  const float* c_prev;        // LSTM
+  float* c_out;
+  int* err;
+  long long* prof;            // developer stamps, as TcParams
+  int prof_slot;
+};
+struct ChainBatch {
+  enum { MAX = 8 };
+  ChainParams p[MAX];
+};
+// n independent problems (same BN, mode, epilogue, N; M <= 128 each when n > 1) in one launch.
+// BN: 32, 64, 128, 256 for LSTM (256: tiles of two packed 128-row tiles); 16, 32, 64, 128, 256 for STORE.
+// split == 2 (n == 1; LSTM BN 32, 64; STORE BN 16, 32): two CTAs per tile, each over half of the K axis.
+cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st);
+// k-blocks per ring stage: as many as leave the ring four stages
+constexpr int kChainRingBytes = 224 * 1024;
+inline int chain_kbs(int mode, int BN, int a_rows) {
+  const int parts = (mode == TC_TF32X3 || mode == TC_F16X2) ? 2 : 1;
+  int k = 4;
+  while (k > 1 && 4 * parts * k * (a_rows + BN) * 128 > kChainRingBytes - (128 - a_rows) * 128 - 1024) k /= 2;
+  return k;
+}
+// Tile width and K split of a launch, and about how long it takes.
+struct ChainPlan {
+  int BN, split;
+  float us;
+};
+// rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks over all sources; M: columns
+ChainPlan plan_chain(int mode, int epi, int rows, int cells, int kb, int M);
+
+// K-major rows as 4-D boxes (k within a 128-byte block, row, part, k-block): box_rows rows of all parts of box_kb k-blocks.
+// parts == 2: the lo rows lie part_bytes behind the hi rows.
+bool make_rows_map(CUtensorMap* out, const void* base, int elem_bytes, long long row_bytes, long long rows, int parts,
+                   long long part_bytes, int kblocks, int box_rows, int box_kb);
+// Weights of an LSTM layer, packed in tiles of 32 hidden units x 4 gates, every (tile, 128-byte k-block) one 16 KB chunk:
+// 5-D boxes (k within a block, hidden unit, gate, part, tile * k-blocks per tile + k-block)
+bool make_gate_map(CUtensorMap* out, const void* base, int elem_bytes, int parts, long long part_bytes, int chunks, int box_units,
+                   int box_parts, int box_kb);
+
+}  // namespace zrnn

@@ -19,6 +19,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
@@ -217,6 +220,72 @@ __device__ __forceinline__ void store4_operand(const P& p, size_t idx, const flo
     if (p.op_lo) store4_f32(p.op_lo, idx, lo, nvalid);
   }
 }
+// W consecutive outputs of one row (W = 2 or a multiple of 4), nvalid of them to be written
+template <int W>
+__device__ __forceinline__ void store_f32(float* base, size_t idx, const float* v, int nvalid) {
+  if constexpr (W == 2) {
+    if (nvalid == 2 && (idx & 1) == 0) *reinterpret_cast<float2*>(base + idx) = make_float2(v[0], v[1]);
+    else
+      for (int u = 0; u < nvalid; ++u) base[idx + u] = v[u];
+  } else {
+#pragma unroll
+    for (int u = 0; u < W; u += 4)
+      if (u < nvalid) store4_f32(base, idx + u, v + u, nvalid - u >= 4 ? 4 : nvalid - u);
+  }
+}
+template <int W, class P>
+__device__ __forceinline__ void store_operand(const P& p, size_t idx, const float* v, int nvalid) {
+  if constexpr (W == 2) {
+    const bool vec = nvalid == 2 && (idx & 1) == 0;
+    if (p.op_b16) {
+      if (vec) *reinterpret_cast<__nv_bfloat162*>(p.op_b16 + idx) = __floats2bfloat162_rn(v[0], v[1]);
+      else
+        for (int u = 0; u < nvalid; ++u) p.op_b16[idx + u] = __float2bfloat16(v[u]);
+    }
+    if (p.op_h_hi) {
+      __half hi[2], lo[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        hi[u] = __float2half_rn(v[u]);
+        lo[u] = __float2half_rn((v[u] - __half2float(hi[u])) * 2048.0f);
+      }
+      if (vec) {
+        *reinterpret_cast<__half2*>(p.op_h_hi + idx) = __halves2half2(hi[0], hi[1]);
+        *reinterpret_cast<__half2*>(p.op_h_lo + idx) = __halves2half2(lo[0], lo[1]);
+      } else {
+        for (int u = 0; u < nvalid; ++u) { p.op_h_hi[idx + u] = hi[u]; p.op_h_lo[idx + u] = lo[u]; }
+      }
+    }
+    if (p.op_hi) {
+      float hi[2], lo[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) { hi[u] = tf32_round_dev(v[u]); lo[u] = v[u] - hi[u]; }
+      store_f32<2>(p.op_hi, idx, hi, nvalid);
+      if (p.op_lo) store_f32<2>(p.op_lo, idx, lo, nvalid);
+    }
+  } else if constexpr (W % 8 == 0) {
+#pragma unroll
+    for (int u = 0; u < W; u += 8)
+      if (u < nvalid) store8_operand(p, idx + u, v + u, nvalid - u >= 8 ? 8 : nvalid - u);
+  } else {
+#pragma unroll
+    for (int u = 0; u < W; u += 4)
+      if (u < nvalid) store4_operand(p, idx + u, v + u, nvalid - u >= 4 ? 4 : nvalid - u);
+  }
+}
+// zeros in elements [n, ld) of an operand row (n a multiple of 4)
+template <class P>
+__device__ __forceinline__ void zero_operand_pad(const P& p, size_t base, int n, int ld) {
+  for (int i = n; i < ld; i += 4) {
+    if (p.op_b16) *reinterpret_cast<uint2*>(p.op_b16 + base + i) = make_uint2(0u, 0u);
+    if (p.op_h_hi) {
+      *reinterpret_cast<uint2*>(p.op_h_hi + base + i) = make_uint2(0u, 0u);
+      *reinterpret_cast<uint2*>(p.op_h_lo + base + i) = make_uint2(0u, 0u);
+    }
+    if (p.op_hi) *reinterpret_cast<float4*>(p.op_hi + base + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.op_lo) *reinterpret_cast<float4*>(p.op_lo + base + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
 
 // Mode traits.  "Split" modes keep every operand as a hi part plus a residual lo part and spend three MMAs per
 // k-step (hi*hi into the main accumulators, lo*hi and hi*lo into the cross accumulator):
@@ -247,23 +316,6 @@ __device__ __forceinline__ float act_sigmoid(float x) {
 
 constexpr int kABytes = 128 * 128;  // A tile: 128 rows x 128-byte k-block
 __host__ __device__ constexpr int stage_bytes(int BN, int mode) { return (mode_split(mode) ? 2 : 1) * (kABytes + BN * 128); }
-// bytes of the split-K exchange slots: SPLITK slots of (BN/SPLITK)/4 x 128 rows of float4.  They must not overlap
-// the stage ring: a peer that finishes its main loop early pushes into them while this CTA may still be loading.
-__host__ __device__ constexpr int slot_bytes(int BN, int splitk) {
-  return splitk > 1 ? splitk * 128 * (BN / splitk) * 4 : 0;
-}
-// 3xTF32 stages are twice as large (hi + lo parts), and with exchange slots of their own only two would fit, too few
-// bytes in flight to keep HBM busy.  In that mode the slots alias the ring instead, which costs one more cluster
-// barrier (nobody may push into a peer's ring before that peer's MMAs have consumed it).
-__host__ __device__ constexpr bool slots_alias_ring(int mode, int splitk) { return mode_split(mode) && splitk > 1; }
-__host__ __device__ constexpr int num_stages(int BN, int mode, int splitk = 1) {
-  int s = (225 * 1024 - 1024 - (slots_alias_ring(mode, splitk) ? 0 : slot_bytes(BN, splitk))) / stage_bytes(BN, mode);
-  return s > 8 ? 8 : s;
-}
-__host__ __device__ constexpr int smem_bytes(int BN, int mode, int splitk) {
-  return num_stages(BN, mode, splitk) * stage_bytes(BN, mode) + (slots_alias_ring(mode, splitk) ? 0 : slot_bytes(BN, splitk)) + 1024;
-}
-
 // The split modes keep fp32-level accuracy only if the tensor core's accumulator is not asked to absorb hundreds of
 // additions: its fp32 accumulation truncates toward zero (measured: a relative shrink of ~8e-6 after 375
 // additions).  So in those modes the hi*hi products are spread round-robin over NACC TMEM accumulators (each sees
@@ -306,6 +358,41 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t local_smem_addr, uint32
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
   return r;
 }
+// arrival (release at cluster scope) on the barrier at the same place in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_map(smem_u32(bar), rank)) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// mbar_wait for a barrier that other CTAs of the cluster arrive on
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int code,
+                                                  long long limit = 2000000000LL) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const long long t0 = clock64();
+  int spins = 0;
+  while (!mbar_try_wait_cluster(bar, parity)) {
+    if ((++spins & 63) == 0) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > limit) {
+        *abort_flag = 1;
+        if (err) atomicExch(err, code);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
                : "memory");

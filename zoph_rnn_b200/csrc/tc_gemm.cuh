@@ -1,8 +1,8 @@
 // Blackwell tensor-core GEMM family (tcgen05.mma with TMEM accumulators, TMA-fed shared-memory ring):
 //   acc[M x N] = sum_s A_s[M x K_s] * B[N x Kcat]^T        (both operands K-major)
 // M indexes batch columns (the reference's H x B activations are already "B rows of K contiguous values"),
-// N indexes weight rows, so every epilogue thread owns one batch column and sees all N outputs of its row:
-// the LSTM gate math, the softmax max / sum-exp and the bias + tanh + mask are thread-local.
+// N indexes weight rows, so every epilogue thread owns one batch column and sees all N outputs of its row: the softmax's
+// max / sum-exp and the bias + tanh + mask are thread-local.  The recurrent cells and the attention products are in tc_chain.cuh.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -22,15 +22,9 @@ struct TcParams {
   int nsrc;
   int kblocks[3];  // 128-byte k-blocks per source
   int b_koff[3];   // element offset of each source inside B's K axis
-  // > 0: B is stored tile-contiguously (k-blocks per row tile): the box of (row tile n, k-block kb) is the
-  // rows [(n * b_tiled_kbtot + kb) * BN, + BN) of a 128-byte-wide 2-D array (tc_gemm_kernel only)
-  int b_tiled_kbtot;
-  // > 0 and < BN: B was packed for row tiles of this many rows (LSTM: 4 gates x pack/4 hidden units per tile) and the
-  // launch uses a wider tile made of BN / b_pack_rows consecutive packed tiles (tc_gemm_kernel, SPLITK == 1)
-  int b_pack_rows;
   int M;           // batch columns
-  int N;           // STORE / LSE: output rows; LSTM: hidden size H (B holds 4H packed rows)
-  const float* bias;  // STORE / LSE: [N]; LSTM: [4][H] gate-major (i,f,g,o)
+  int N;           // output rows
+  const float* bias;  // [N]
   const int* mask;    // [M] or null
   // --- STORE: C[n + m*ldc] = act(acc + bias[n]) * mask[m]
   float* C;
@@ -44,9 +38,6 @@ struct TcParams {
   __half* op_h_hi;  // TC_F16X2 consumers: fp16 hi part and scaled fp16 lo part
   __half* op_h_lo;
   int ld_op;
-  // --- LSTM (gates i,f,g,o): c = f*c_prev + i*g ; h = o*tanh(c) ; (h,c) *= mask ; h -> C (ld = ldc), c -> c_out
-  const float* c_prev;
-  float* c_out;
   // --- LSE: per (N tile, m) max and sum exp(z - max) of z = acc + bias, plus the logit of target[m]
   const int* target;
   int target_offset;
@@ -57,19 +48,6 @@ struct TcParams {
   long long* prof;   // optional: 8 globaltimer stamps per CTA (developer profiling)
   int prof_slot;     // >= 0: only CTA (0,0,0) stamps, into prof[prof_slot*8 ..] (timeline of many launches)
 };
-
-// BN = N-tile (LSTM: 4*TH). Returns cudaErrorInvalidValue for unsupported (BN, mode, epi) combinations.
-// splitk > 1 (BN == 128 only: 2, 4, and 8 for the non-LSTM epilogues) splits the K axis over a thread-block cluster;
-// the LSE epilogue then produces n_tiles * splitk partial rows.
-cudaError_t launch_tc_gemm(const TcParams& p, int BN, int mode, int epi, cudaStream_t st, int splitk = 1);
-
-// Up to TcMulti::MAX independent LSTM layer-steps (EPI_LSTM, 128-row weight tiles, M <= 128 columns and the same
-// hidden size each) in one launch: grid (n, row tiles, splitk).  Nothing orders the problems among themselves.
-struct TcMulti {
-  enum { MAX = 8 };
-  TcParams p[MAX];
-};
-cudaError_t launch_tc_lstm_multi(const TcMulti& pm, int n, int mode, cudaStream_t st, int splitk);
 
 // Persistent one-CTA-per-SM variant for large problems (store and log-sum-exp epilogues).  The B tensor map must use
 // 256-row boxes for TC_BF16 / TC_TF32 and 128-row boxes for the split modes.  Two epilogue warps share each output

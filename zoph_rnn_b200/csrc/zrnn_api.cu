@@ -17,6 +17,7 @@
 #include "../../include/zrnn_debug.h"
 #include "kernels.cuh"
 #include "model_file.hpp"
+#include "tc_chain.cuh"
 #include "tc_decoder.cuh"
 #include "tc_gemm.cuh"
 
@@ -219,24 +220,23 @@ int check_f16_range(int eng, const float* p, size_t n, const char* what) {
 struct OpMem {
   void* hi = nullptr;
   float* lo = nullptr;
+  // one allocation, the lo array right behind the hi array: a TMA box can then span both parts
   int alloc(size_t elems, int eng) {
     release();
     ++g_buf_generation;  // a captured graph may still hold the old addresses
-    ZR_CUDA(cudaMalloc(&hi, elems * eng_eb(eng)));
-    ZR_CUDA(cudaMemset(hi, 0, elems * eng_eb(eng)));
-    if (eng_split(eng)) {
-      ZR_CUDA(cudaMalloc((void**)&lo, elems * eng_eb(eng)));
-      ZR_CUDA(cudaMemset(lo, 0, elems * eng_eb(eng)));
-    }
+    const size_t bytes = (elems * eng_eb(eng) + 255) / 256 * 256;
+    ZR_CUDA(cudaMalloc(&hi, bytes * (eng_split(eng) ? 2 : 1)));
+    ZR_CUDA(cudaMemset(hi, 0, bytes * (eng_split(eng) ? 2 : 1)));
+    if (eng_split(eng)) lo = (float*)((char*)hi + bytes);
     return ZRNN_OK;
   }
   void release() {
-    if (hi || lo) ++g_buf_generation;
+    if (hi) ++g_buf_generation;
     cudaFree(hi);
-    cudaFree(lo);
     hi = nullptr;
     lo = nullptr;
   }
+  long long part_bytes() const { return lo ? (char*)lo - (char*)hi : 0; }
 };
 
 // An activation matrix: column-major fp32 (H x cols) and/or its operand-form copy (cols rows of Kpad elements)
@@ -275,11 +275,12 @@ struct zrnn_lstm_layer {
   int kbtot = 0;  // > 0: weights stored tile-contiguously with this many k-blocks per row tile
   OpMem Wcat, emb;
   CUtensorMap wmap, wmap_lo;
-  DevBuf sc_x, sc_h, sc_q, sc_xl, sc_hl, sc_ql;  // operand scratch for the fp32 layer-level entry points
+  CUtensorMap gmap[4][3];  // boxes of 8 / 16 / 32 hidden units x 4 gates (tc_chain.cu)
+  DevBuf sc_x, sc_h, sc_q;  // operand scratch for the fp32 layer-level entry points
   ~zrnn_lstm_layer() {
     cudaFree(W); cudaFree(Wh); cudaFree(Mx); cudaFree(Q); cudaFree(b);
     x.release(); Wcat.release(); emb.release();
-    sc_x.release(); sc_h.release(); sc_q.release(); sc_xl.release(); sc_hl.release(); sc_ql.release();
+    sc_x.release(); sc_h.release(); sc_q.release();
   }
 };
 
@@ -299,11 +300,11 @@ struct zrnn_attention {
   int Kpad = 0, BN = 128;
   OpMem WpWaT_op, Wc_op;  // [2H rows x Kpad], [H rows x 2*Kpad]
   CUtensorMap pmap, pmap_lo, cmap, cmap_lo;
-  DevBuf ctx_hi, ctx_lo, sc_h, sc_hl;
+  DevBuf ctx_op, sc_h;
   ~zrnn_attention() {
     cudaFree(WpWaT); cudaFree(v_p); cudaFree(bias); cudaFree(Wc1); cudaFree(Wc2);
     tq.release(); ctx.release(); WpWaT_op.release(); Wc_op.release();
-    ctx_hi.release(); ctx_lo.release(); sc_h.release(); sc_hl.release();
+    ctx_op.release(); sc_h.release();
   }
 };
 
@@ -317,48 +318,22 @@ struct zrnn_softmax {
   int kbtot = 0;  // > 0: weights stored tile-contiguously with this many k-blocks per row tile
   OpMem D_op;  // [n_tiles*BN rows x Kpad]
   CUtensorMap dmap, dmap_lo;
-  DevBuf sc_h, sc_hl;
+  DevBuf sc_h;
   ~zrnn_softmax() {
     cudaFree(D); cudaFree(b);
-    parts.release(); tgt.release(); logits.release(); D_op.release(); sc_h.release(); sc_hl.release();
+    parts.release(); tgt.release(); logits.release(); D_op.release(); sc_h.release();
   }
 };
 
 namespace {
-
-// Split the K axis over a cluster when that shortens the launch: with one CTA per SM a launch runs in
-// ceil(CTAs / SMs) waves, a split by s multiplies the CTAs by s and divides the work of each by s at the price of the
-// exchange.  Picks the s that minimises waves * (1/s + exchange), e.g. 32 CTAs -> 4 (one wave of quarter-size CTAs),
-// 16 CTAs -> 4, 64 CTAs -> 2, 192 CTAs (768 decode columns) -> 1 (splitting them was measured slightly slower).
-int pick_splitk(int m_cols, int n_rows, int BN, int max_split) {
-  if (BN != 128) return 1;
-  const int ctas = ((m_cols + 127) / 128) * ((n_rows + BN - 1) / BN);
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      sms = 148;
-  }
-  int best = 1;
-  double best_t = 1e30;
-  for (int s = 1; s <= max_split && s <= 8; s *= 2) {
-    // 8-CTA clusters of one CTA per SM: no more than 8 of them are resident at once on this part (measured: 16 such
-    // clusters ran as two waves)
-    if (s == 8 && ctas > 8) break;
-    const int waves = (ctas * s + sms - 1) / sms;
-    const double t = waves * (1.0 / s + (s > 1 ? 0.2 : 0.0));  // exchange ~ 20 % of an unsplit CTA's time (measured)
-    if (t < best_t - 1e-9) { best_t = t; best = s; }
-  }
-  return best;
-}
 
 long long* g_dec_detail = nullptr;  // developer timeline of the persistent decoder kernel (zrnn_debug_decoder_timeline)
 int g_dec_detail_cta = 0;
 long long* g_tc_prof = nullptr;  // developer profiling buffer (see zrnn_debug_tc_profile)
 int g_tc_prof_slot = -1;          // >= 0: timeline mode, one slot per tensor-core launch
 int g_tc_prof_cap = 0;
-void prof_attach(zrnn::TcParams& tp) {
+template <class P>
+void prof_attach(P& tp) {
   tp.prof = g_tc_prof;
   tp.prof_slot = -1;
   if (g_tc_prof && g_tc_prof_slot >= 0) {
@@ -389,13 +364,13 @@ int act_maps(const Act& a, int eng, int H, int Kpad, int rows, CUtensorMap* hi, 
 }
 
 // fp32 activation (H x cols, column-major) -> operand form in scratch buffers
-int to_operand(const float* f32, int H, int Kpad, int cols, int eng, DevBuf& hi, DevBuf& lo, Act* out, cudaStream_t st) {
-  ZR_CUDA(hi.reserve((size_t)cols * Kpad * eng_eb(eng)));
-  if (eng_split(eng)) ZR_CUDA(lo.reserve((size_t)cols * Kpad * eng_eb(eng)));
-  ZR_CUDA(zrnn::launch_convert_rows(f32, cols, H, H, eng_opmode(eng), hi.p, lo.as<float>(), Kpad, st));
+int to_operand(const float* f32, int H, int Kpad, int cols, int eng, DevBuf& buf, Act* out, cudaStream_t st) {
+  const size_t part = aligned((size_t)cols * Kpad * eng_eb(eng));
+  ZR_CUDA(buf.reserve(part * (eng_split(eng) ? 2 : 1)));
   out->f32 = const_cast<float*>(f32);
-  out->hi = hi.p;
-  out->lo = eng_split(eng) ? lo.as<float>() : nullptr;
+  out->hi = buf.p;
+  out->lo = eng_split(eng) ? (float*)(buf.as<char>() + part) : nullptr;
+  ZR_CUDA(zrnn::launch_convert_rows(f32, cols, H, H, eng_opmode(eng), out->hi, out->lo, Kpad, st));
   return ZRNN_OK;
 }
 
@@ -424,8 +399,21 @@ int lstm_cell_simt(zrnn_lstm_layer* L, const float* x, const int* mask, const fl
   return ZRNN_OK;
 }
 
-// where the epilogue leaves the operand-form copy of its output for the next GEMM
-void set_operand_outputs(zrnn::TcParams& tp, int eng, const Act& out, int Kpad) {
+// How a link of the chain is launched
+struct LinkPlan {
+  zrnn::ChainPlan chain;
+};
+LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int H, int cols, int n = 1) {
+  const int epk = 128 / eng_eb(eng);
+  LinkPlan p;
+  p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc * ((H + epk - 1) / epk), cols);
+  return p;
+}
+
+// ---- one link of the recurrent chain on tcgen05 without splitting K (tc_chain.cu)
+int chain_a_rows(int B) { return B >= 128 ? 128 : (B + 7) / 8 * 8; }
+// where the epilogue leaves the operand-form copy of its output for the next product
+void chain_operand_outputs(zrnn::ChainParams& tp, int eng, const Act& out, int Kpad) {
   tp.ld_op = Kpad;
   if (eng == ENG_BF16) {
     tp.op_b16 = (__nv_bfloat16*)out.hi;
@@ -437,48 +425,78 @@ void set_operand_outputs(zrnn::TcParams& tp, int eng, const Act& out, int Kpad) 
     tp.op_lo = eng == ENG_X3 ? out.lo : nullptr;
   }
 }
-
-// One LSTM cell.  x / h_prev / htild and the output are activations in the form the layer's engine needs.
-// kernel parameters of one tensor-core LSTM layer-step
-int cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
-                int B, const Act& out, float* c_out, zrnn::TcParams& tp) {
-  const int H = L->H, Kpad = L->Kpad, eng = L->eng;
-  const int kb = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
-  std::memset(&tp, 0, sizeof(tp));
-  ZR_TRY(act_maps(x, eng, H, Kpad, B, &tp.a[0], &tp.a_lo[0]));
-  ZR_TRY(act_maps(hp, eng, H, Kpad, B, &tp.a[1], &tp.a_lo[1]));
-  tp.nsrc = 2;
-  if (q) {
-    ZR_TRY(act_maps(*q, eng, H, Kpad, B, &tp.a[2], &tp.a_lo[2]));
-    tp.nsrc = 3;
-  }
-  for (int s = 0; s < 3; ++s) { tp.kblocks[s] = kb; tp.b_koff[s] = s * Kpad; }
-  tp.b = L->wmap; tp.b_lo = L->wmap_lo; tp.b_tiled_kbtot = L->kbtot;
-  tp.M = B; tp.N = H; tp.bias = L->b; tp.mask = mask;
-  tp.C = out.f32; tp.ldc = H;
-  set_operand_outputs(tp, eng, out, Kpad);
-  tp.c_prev = c_prev; tp.c_out = c_out; tp.err = tc_error_word(); prof_attach(tp);
+int chain_source(zrnn::ChainParams& p, const Act& a, int eng, int H, int Kpad, int B, int koff) {
+  const int s = p.nsrc++;
+  p.a_row0[s] = 0;
+  p.wkb0[s] = koff / (128 / eng_eb(eng));
+  if (!a.hi) return fail(ZRNN_E_STATE, "internal: activation has no operand-form copy");
+  if (!zrnn::make_rows_map(&p.a[s], a.hi, eng_eb(eng), (long long)Kpad * eng_eb(eng), B, eng_split(eng) ? 2 : 1,
+                           (char*)a.lo - (char*)a.hi, p.kb, p.a_rows, p.kbs))
+    return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for an activation operand");
   return ZRNN_OK;
 }
+int chain_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
+                      int B, const Act& out, float* c_out, int BN, zrnn::ChainParams& p) {
+  const int H = L->H, Kpad = L->Kpad, eng = L->eng, epk = 128 / eng_eb(eng);
+  std::memset(&p, 0, sizeof(p));
+  p.a_rows = chain_a_rows(B);
+  p.kb = (H + epk - 1) / epk;
+  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows);
+  ZR_TRY(chain_source(p, x, eng, H, Kpad, B, 0));
+  ZR_TRY(chain_source(p, hp, eng, H, Kpad, B, Kpad));
+  if (q) ZR_TRY(chain_source(p, *q, eng, H, Kpad, B, 2 * Kpad));
+  p.w = L->gmap[BN == 32 ? 0 : (BN == 64 ? 1 : (BN == 128 ? 2 : 3))][p.kbs == 1 ? 0 : (p.kbs == 2 ? 1 : 2)];
+  p.w_kbtot = L->kbtot; p.w_tiles = L->n_tiles;
+  p.M = B; p.N = H; p.bias = L->b; p.mask = mask;
+  p.C = out.f32; p.ldc = H;
+  chain_operand_outputs(p, eng, out, Kpad);
+  p.c_prev = c_prev; p.c_out = c_out; p.err = tc_error_word();
+  prof_attach(p);
+  return ZRNN_OK;
+}
+// C = act(W [a0 | a1] + bias) with plain K-major weight rows
+int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act* a0, const Act* a1, int H, int Kpad, int B, int BN,
+                       zrnn::ChainParams& p) {
+  const int epk = 128 / eng_eb(eng);
+  std::memset(&p, 0, sizeof(p));
+  p.a_rows = chain_a_rows(B);
+  p.kb = (H + epk - 1) / epk;
+  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows);
+  ZR_TRY(chain_source(p, *a0, eng, H, Kpad, B, 0));
+  if (a1) ZR_TRY(chain_source(p, *a1, eng, H, Kpad, B, Kpad));
+  const long long rows = (N + 127) / 128 * 128;
+  if (!zrnn::make_rows_map(&p.w, w.hi, eng_eb(eng), ldw * eng_eb(eng), rows, eng_split(eng) ? 2 : 1, w.part_bytes(),
+                           (int)(ldw / epk), BN, p.kbs))
+    return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for a weight operand");
+  p.M = B; p.N = N; p.err = tc_error_word();
+  if (g_tc_prof_slot >= 0) prof_attach(p);
+  return ZRNN_OK;
+}
+
+// One LSTM cell.  x / h_prev / htild and the output are activations in the form the layer's engine needs.
 int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
                  int B, const Act& out, float* c_out, cudaStream_t st) {
   if (L->eng == ENG_SIMT)
     return lstm_cell_simt(L, x.f32, mask, hp.f32, c_prev, q ? q->f32 : nullptr, B, out.f32, c_out, st);
   const int H = L->H, eng = L->eng;
-  zrnn::TcParams tp;
-  ZR_TRY(cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, tp));
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, H, B);
   KScope ks(KC_LSTM, st);
-  int bn = L->BN;
-  const int splitk = pick_splitk(B, 4 * H, L->BN, 4);
-  // many columns (beam decoding): 128-row tiles would need more than one wave of CTAs; 256-row tiles built from two
-  // packed tiles halve the CTA count and the activation traffic per flop.  A 256-column tile leaves TMEM room for one
-  // main accumulator only (measured per-token log-prob error at H = 1000: fp16 split 0.8e-6 -> 2.1e-6, 3xTF32
-  // 1.6e-6 -> 3.9e-6), so the 3xTF32 engine, chosen for its accuracy margin, keeps the 128-row tiles.
-  if (splitk == 1 && L->BN == 128 && eng != ENG_X3 && ((B + 127) / 128) * L->n_tiles > 148) {
-    bn = 256;
-    tp.b_pack_rows = 128;
-  }
-  ZR_CUDA(zrnn::launch_tc_gemm(tp, bn, eng_tcmode(eng), zrnn::TC_EPI_LSTM, st, splitk));
+  zrnn::ChainBatch cb;
+  ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain.BN, cb.p[0]));
+  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, st));
+  return ZRNN_OK;
+}
+// out = act(W [a0 | a1] + bias) * mask for plain K-major weight rows, act = tanh on the first act_rows rows (0: all)
+int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, const Act* a1, const float* bias, const int* mask,
+               int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st) {
+  const int nsrc = a1 ? 2 : 1;
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, H, B);
+  zrnn::ChainBatch cb;
+  zrnn::ChainParams& p = cb.p[0];
+  ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain.BN, p));
+  p.bias = bias; p.mask = mask; p.act = 1; p.act_rows = act_rows; p.C = C; p.ldc = ldc;
+  if (op) chain_operand_outputs(p, eng, *op, Kpad);
+  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, plan.chain.split, st));
   return ZRNN_OK;
 }
 
@@ -496,10 +514,10 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   Act ctx;
   ctx.f32 = A->ctx.as<float>();
   if (eng != ENG_SIMT) {
-    ZR_CUDA(A->ctx_hi.reserve((size_t)B * Kpad * eng_eb(eng)));
-    if (eng_split(eng)) ZR_CUDA(A->ctx_lo.reserve((size_t)B * Kpad * eng_eb(eng)));
-    ctx.hi = A->ctx_hi.p;
-    ctx.lo = eng_split(eng) ? A->ctx_lo.as<float>() : nullptr;
+    const size_t part = aligned((size_t)B * Kpad * eng_eb(eng));
+    ZR_CUDA(A->ctx_op.reserve(part * (eng_split(eng) ? 2 : 1)));
+    ctx.hi = A->ctx_op.p;
+    ctx.lo = eng_split(eng) ? (float*)(A->ctx_op.as<char>() + part) : nullptr;
     a.ld_op = Kpad;
     if (eng == ENG_BF16) a.op_b16 = ctx.hi;
     else if (eng == ENG_H2) { a.op_h_hi = ctx.hi; a.op_h_lo = ctx.lo; }
@@ -515,15 +533,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
       g.M = 2 * H; g.N = B; g.C = A->tq.as<float>(); g.ldc = 2 * H; g.act = 1; g.act_rows = H;
       ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, 0, st));
     } else {
-      zrnn::TcParams tp;
-      std::memset(&tp, 0, sizeof(tp));
-      ZR_TRY(act_maps(h_t, eng, H, Kpad, B, &tp.a[0], &tp.a_lo[0]));
-      tp.nsrc = 1; tp.kblocks[0] = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng)); tp.b_koff[0] = 0;
-      tp.b = A->pmap; tp.b_lo = A->pmap_lo;
-      tp.M = B; tp.N = 2 * H; tp.C = A->tq.as<float>(); tp.ldc = 2 * H; tp.act = 1; tp.act_rows = H;
-      tp.err = tc_error_word();
-      if (g_tc_prof_slot >= 0) prof_attach(tp);
-      ZR_CUDA(zrnn::launch_tc_gemm(tp, A->BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, st, pick_splitk(B, 2 * H, A->BN, 8)));
+      ZR_TRY(link_store(eng, A->WpWaT_op, 2 * H, H, Kpad, &h_t, nullptr, nullptr, nullptr, H, B, A->tq.as<float>(), 2 * H, nullptr, st));
     }
     a.tanh1 = A->tq.as<float>(); a.q = A->tq.as<float>() + H; a.ld_tq = 2 * H; a.v_p = A->v_p;
     ZR_CUDA(zrnn::launch_att_local(a, st));
@@ -539,19 +549,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
     g.M = H; g.N = B; g.C = out.f32; g.ldc = H; g.bias[0] = A->bias; g.mask = mask; g.act = 1;
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, 0, st));
   } else {
-    zrnn::TcParams tp;
-    std::memset(&tp, 0, sizeof(tp));
-    const int kb = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
-    ZR_TRY(act_maps(ctx, eng, H, Kpad, B, &tp.a[0], &tp.a_lo[0]));
-    ZR_TRY(act_maps(h_t, eng, H, Kpad, B, &tp.a[1], &tp.a_lo[1]));
-    tp.nsrc = 2; tp.kblocks[0] = tp.kblocks[1] = kb; tp.b_koff[0] = 0; tp.b_koff[1] = Kpad;
-    tp.b = A->cmap; tp.b_lo = A->cmap_lo;
-    tp.M = B; tp.N = H; tp.bias = A->bias; tp.mask = mask; tp.act = 1;
-    tp.C = out.f32; tp.ldc = H;
-    set_operand_outputs(tp, eng, out, Kpad);
-    tp.err = tc_error_word();
-    if (g_tc_prof_slot >= 0) prof_attach(tp);
-    ZR_CUDA(zrnn::launch_tc_gemm(tp, A->BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, st, pick_splitk(B, H, A->BN, 8)));
+    ZR_TRY(link_store(eng, A->Wc_op, H, H, Kpad, &ctx, &h_t, A->bias, mask, 0, B, out.f32, H, &out, st));
   }
   return ZRNN_OK;
 }
@@ -712,7 +710,7 @@ struct zrnn_model {
   DevBuf dec_counter;       // phase counter of the persistent decoder kernel
   DevBuf seq_xp;            // input half of the pre-activations for the resident-weight sequence kernel
   int persist_state = 0;    // 0 untried, 1 works, -1 refused by the runtime (the per-launch path is used)
-  zrnn::TcMulti enc_multi;  // parameter block of the encoder's multi-cell launches (host scratch)
+  zrnn::ChainBatch diag;    // parameter block of the multi-cell launches (host scratch)
   const float* last_top = nullptr;
   int last_top_cols = 0;
   Act last_top_act;  // the same vectors with their operand-form copies
@@ -942,16 +940,20 @@ int zrnn_lstm_load(zrnn_lstm_layer* L, const float* const* t, int n) {
     ZR_TRY(L->Wcat.alloc((size_t)rows * Kcat, L->eng));
     // Tile-contiguous storage: the 128 rows x 128 bytes a CTA fetches per k-block are one 16 KB chunk of memory
     // instead of 128 pieces that lie a whole row (8-12 KB) apart, so the weight stream reads whole DRAM pages.
-    static const bool tiled = std::getenv("ZRNN_WEIGHT_ROWMAJOR") == nullptr;
     const int epk = 128 / eng_eb(L->eng);
-    L->kbtot = tiled ? (int)(Kcat / epk) : 0;
+    L->kbtot = (int)(Kcat / epk);
     const float* srcs[3] = {L->Mx, L->Wh, L->Q};
     for (int s = 0; s < nsrc; ++s) {
       const float* g4[4] = {srcs[s], srcs[s] + HH, srcs[s] + 2 * HH, srcs[s] + 3 * HH};
       ZR_TRY(pack_into(L->Wcat, L->eng, g4, 4, H, H, H, TH, L->n_tiles, (int)Kcat, s * Kpad, L->kbtot));
     }
-    if (tiled) ZR_TRY(weight_maps(L->Wcat, L->eng, epk, rows * L->kbtot, L->BN, &L->wmap, &L->wmap_lo));
-    else ZR_TRY(weight_maps(L->Wcat, L->eng, Kcat, rows, L->BN, &L->wmap, &L->wmap_lo));
+    ZR_TRY(weight_maps(L->Wcat, L->eng, epk, rows * L->kbtot, L->BN, &L->wmap, &L->wmap_lo));
+    const int parts = eng_split(L->eng) ? 2 : 1;
+    for (int i = 0; i < 4; ++i)    // boxes of 8, 16 and 32 units with all parts, and of 32 units of one part
+      for (int k = 0; k < 3; ++k)  // of 1, 2 and 4 k-blocks
+        if (!zrnn::make_gate_map(&L->gmap[i][k], L->Wcat.hi, eng_eb(L->eng), parts, L->Wcat.part_bytes(), L->n_tiles * L->kbtot,
+                                 i < 3 ? 8 << i : 32, i < 3 ? parts : 1, i < 3 ? 1 << k : 1))
+          return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for the gate weights");
     if (L->is_ih) {
       ZR_TRY(L->emb.alloc((size_t)L->V * Kpad, L->eng));
       ZR_CUDA(zrnn::launch_convert_rows(L->W, L->V, H, H, eng_opmode(L->eng), L->emb.hi, L->emb.lo, Kpad, nullptr));
@@ -999,16 +1001,16 @@ static int layer_forward_f32(zrnn_lstm_layer* L, const int* d_ids, const float* 
     q.f32 = const_cast<float*>(d_htild);
   } else {
     if (d_ids) {
-      ZR_CUDA(L->sc_x.reserve((size_t)B * L->Kpad * eng_eb(L->eng)));
-      if (eng_split(L->eng)) ZR_CUDA(L->sc_xl.reserve((size_t)B * L->Kpad * eng_eb(L->eng)));
+      const size_t part = aligned((size_t)B * L->Kpad * eng_eb(L->eng));
+      ZR_CUDA(L->sc_x.reserve(part * (eng_split(L->eng) ? 2 : 1)));
       x.hi = L->sc_x.p;
-      x.lo = eng_split(L->eng) ? L->sc_xl.as<float>() : nullptr;
+      x.lo = eng_split(L->eng) ? (float*)(L->sc_x.as<char>() + part) : nullptr;
       ZR_TRY(gather_act(L, d_ids, B, x, st));
     } else {
-      ZR_TRY(to_operand(d_x, H, L->Kpad, B, L->eng, L->sc_x, L->sc_xl, &x, st));
+      ZR_TRY(to_operand(d_x, H, L->Kpad, B, L->eng, L->sc_x, &x, st));
     }
-    ZR_TRY(to_operand(d_h_prev, H, L->Kpad, B, L->eng, L->sc_h, L->sc_hl, &hp, st));
-    if (d_htild) ZR_TRY(to_operand(d_htild, H, L->Kpad, B, L->eng, L->sc_q, L->sc_ql, &q, st));
+    ZR_TRY(to_operand(d_h_prev, H, L->Kpad, B, L->eng, L->sc_h, &hp, st));
+    if (d_htild) ZR_TRY(to_operand(d_htild, H, L->Kpad, B, L->eng, L->sc_q, &q, st));
   }
   return cell_forward(L, x, hp, d_htild ? &q : nullptr, d_mask, d_c_prev, B, out, d_c_out, st);
 }
@@ -1124,7 +1126,7 @@ int zrnn_att_forward(zrnn_attention* A, const float* d_h_t, const int* d_mask, i
   Act h, out;
   h.f32 = const_cast<float*>(d_h_t);
   out.f32 = d_htild_out;
-  if (A->eng != ENG_SIMT) ZR_TRY(to_operand(d_h_t, A->H, A->Kpad, B, A->eng, A->sc_h, A->sc_hl, &h, st));
+  if (A->eng != ENG_SIMT) ZR_TRY(to_operand(d_h_t, A->H, A->Kpad, B, A->eng, A->sc_h, &h, st));
   return att_forward(A, h, d_mask, B, out, d_align_out, st, g_att_viterbi_out);
 }
 int zrnn_att_forward_viterbi(zrnn_attention* A, const float* d_h_t, const int* d_mask, int B, float* d_htild_out,
@@ -1179,7 +1181,7 @@ int zrnn_softmax_load(zrnn_softmax* S, const float* h_D, const float* h_b_d) {
 }
 static int softmax_input(zrnn_softmax* S, const float* d_h, int N, Act* h, cudaStream_t st) {
   h->f32 = const_cast<float*>(d_h);
-  if (S->eng != ENG_SIMT) ZR_TRY(to_operand(d_h, S->H, S->Kpad, N, S->eng, S->sc_h, S->sc_hl, h, st));
+  if (S->eng != ENG_SIMT) ZR_TRY(to_operand(d_h, S->H, S->Kpad, N, S->eng, S->sc_h, h, st));
   return ZRNN_OK;
 }
 int zrnn_softmax_partials(zrnn_softmax* S, const float* d_h, const int* d_targets, int N, float* d_max, float* d_sum,
@@ -1536,6 +1538,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
       a.h_seq = seq[l].f32;
       a.xp = m->seq_xp.as<float>();
       a.ld_op = g.Kpad;
+      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm;  // the decoder's cells and the attention read these rows as operands
       if (g.eng == ENG_BF16) a.op_b16 = seq[l].hi;
       else if (g.eng == ENG_H2) { a.op_h_hi = seq[l].hi; a.op_h_lo = seq[l].lo; }
       else if (g.eng != ENG_SIMT) { a.op_hi = (float*)seq[l].hi; a.op_lo = g.eng == ENG_X3 ? seq[l].lo : nullptr; }
@@ -1544,29 +1547,15 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
     return ZRNN_OK;
   }
   // Anti-diagonal order: the cells (layer l, step d - l) of diagonal d depend only on diagonal d - 1, so one launch
-  // runs them side by side.  L cells fill the SMs with less (or no) K splitting than one cell alone: each CTA streams a
-  // longer K slice, no partial tiles cross the cluster, and S + L - 1 launches replace S * L.  Needs one column tile
-  // per cell, the tensor-core engine, and all L cells' row tiles resident at once.
+  // runs them side by side: S + L - 1 launches replace S * L.  Needs one column tile per cell.
   static const bool by_layers = [] {
     const char* e = std::getenv("ZRNN_ENCODER_ORDER");
     return e && std::string(e) == "layers";
   }();
   const zrnn_lstm_layer* L0 = layers[0];
-  int dsplit = 0;
-  // Not for 3xTF32: its tf32 MMAs cover 8 k-values each, so an unsplit K = 2H chain puts twice as many truncating
-  // additions into one accumulator as the fp16 split does (measured at H = 1000, 4 layers: per-token log-prob error
-  // 9e-6 against 4e-6), too close to the 1e-5 this engine promises.
-  if (!by_layers && L >= 2 && L <= zrnn::TcMulti::MAX && L0->eng != ENG_SIMT && L0->eng != ENG_X3 && B <= 128 &&
-      L0->BN == 128)
-    for (int k = 4; k >= 1 && !dsplit; k >>= 1)
-      if (L * L0->n_tiles * k <= 148) dsplit = k;
-  if (dsplit && std::getenv("ZRNN_DIAG_SPLITK")) {  // developer knob: 1, 2 or 4 (more CTAs than SMs run in waves)
-    const int k = std::atoi(std::getenv("ZRNN_DIAG_SPLITK"));
-    if (k == 1 || k == 2 || k == 4) dsplit = k;
-  }
-  if (dsplit) {
+  if (!by_layers && L >= 2 && L <= zrnn::ChainBatch::MAX && L0->eng != ENG_SIMT && B <= 128) {
+    const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, g.H, B, L);
     KScope sweep(KC_LSTM, s, S * L, true);
-    zrnn::TcMulti* pm = &m->enc_multi;
     for (int d = 0; d < S + L - 1; ++d) {
       int n = 0;
       for (int l = std::max(0, d - S + 1); l <= std::min(L - 1, d); ++l) {
@@ -1575,11 +1564,12 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         const Act hp = t == 0 ? h0[l] : act_at(seq[l], (size_t)(t - 1) * B, g);
         const Act out = act_at(seq[l], (size_t)t * B, g);
         const int cu = cur[l];
-        ZR_TRY(cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], pm->p[n]));
+        ZR_TRY(chain_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l],
+                                      plan.chain.BN, m->diag.p[n]));
         cur[l] = cu ^ 1;
         ++n;
       }
-      ZR_CUDA(zrnn::launch_tc_lstm_multi(*pm, n, eng_tcmode(L0->eng), s, dsplit));
+      ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, s));
     }
     return ZRNN_OK;
   }
@@ -1653,10 +1643,11 @@ static int run_decoder_persistent(zrnn_model* m, const Geom& g, int S, int T, in
   p.ht_f32 = hts.f32; p.ht_op_hi = hts.hi; p.ht_op_lo = hts.lo;
   // the step's context vectors and (local-p) the stacked projection live in the attention layer's own buffers
   ZR_CUDA(A->ctx.reserve(sizeof(float) * (size_t)H * B));
-  ZR_CUDA(A->ctx_hi.reserve((size_t)B * Kpad * eb));
-  if (eng_split(eng)) ZR_CUDA(A->ctx_lo.reserve((size_t)B * Kpad * eb));
+  const size_t ctx_part = aligned((size_t)B * Kpad * eb);
+  ZR_CUDA(A->ctx_op.reserve(ctx_part * (eng_split(eng) ? 2 : 1)));
   Act ctx;
-  ctx.f32 = A->ctx.as<float>(); ctx.hi = A->ctx_hi.p; ctx.lo = eng_split(eng) ? A->ctx_lo.as<float>() : nullptr;
+  ctx.f32 = A->ctx.as<float>(); ctx.hi = A->ctx_op.p;
+  ctx.lo = eng_split(eng) ? (float*)(A->ctx_op.as<char>() + ctx_part) : nullptr;
   ZR_TRY(act_maps(ctx, eng, H, Kpad, B, &p.ctx_hi, &p.ctx_lo, ar));
   p.ctx_f32 = ctx.f32; p.ctx_op_hi = ctx.hi; p.ctx_op_lo = ctx.lo;
   p.wc_hi = A->cmap; p.wc_lo = A->cmap_lo;
@@ -2765,43 +2756,40 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
   const bool split = mode >= 3;
   const int kb_elems = 128 / eb;
   const int Kpad = (K + 63) / 64 * 64;
-  const int BN = n_rows >= 256 ? 256 : (n_rows >= 128 ? 128 : (n_rows >= 64 ? 64 : 32));
-  const int n_tiles = (n_rows + BN - 1) / BN;
-  const size_t a_elems = (size_t)m_cols * Kpad, b_elems = (size_t)n_tiles * BN * Kpad;
-  DevBuf a_hi, a_lo, b_hi, b_lo;
-  ZR_CUDA(a_hi.reserve(a_elems * eb));
-  ZR_CUDA(b_hi.reserve(b_elems * eb));
-  ZR_CUDA(cudaMemsetAsync(a_hi.p, 0, a_elems * eb, st));
-  ZR_CUDA(cudaMemsetAsync(b_hi.p, 0, b_elems * eb, st));
-  if (split) {
-    ZR_CUDA(a_lo.reserve(a_elems * eb));
-    ZR_CUDA(b_lo.reserve(b_elems * eb));
-    ZR_CUDA(cudaMemsetAsync(a_lo.p, 0, a_elems * eb, st));
-    ZR_CUDA(cudaMemsetAsync(b_lo.p, 0, b_elems * eb, st));
-  }
-  ZR_CUDA(zrnn::launch_convert_rows(d_X, m_cols, K, ldx, op_mode, a_hi.p, a_lo.as<float>(), Kpad, st));
-  zrnn::PackArgs pk;
-  std::memset(&pk, 0, sizeof(pk));
-  pk.src[0] = d_W; pk.G = 1; pk.H = n_rows; pk.K = K; pk.lda = ldw; pk.TH = BN; pk.n_tiles = n_tiles;
-  pk.dst_hi = b_hi.p; pk.dst_lo = b_lo.as<float>(); pk.op_mode = op_mode; pk.ld_dst = Kpad; pk.koff = 0;
-  ZR_CUDA(zrnn::launch_pack_weights(pk, st));
-  zrnn::TcParams tp;
-  std::memset(&tp, 0, sizeof(tp));
-  bool ok = zrnn::make_kmajor_map(&tp.a[0], a_hi.p, eb, Kpad, m_cols, Kpad, 128) &&
-            zrnn::make_kmajor_map(&tp.b, b_hi.p, eb, Kpad, (long long)n_tiles * BN, Kpad, BN);
-  if (split)
-    ok = ok && zrnn::make_kmajor_map(&tp.a_lo[0], a_lo.p, eb, Kpad, m_cols, Kpad, 128) &&
-         zrnn::make_kmajor_map(&tp.b_lo, b_lo.p, eb, Kpad, (long long)n_tiles * BN, Kpad, BN);
-  if (!ok) {
-    a_hi.release(); a_lo.release(); b_hi.release(); b_lo.release();
-    return fail(ZRNN_E_CUDA, "gemm: cannot encode TMA tensor maps");
-  }
-  tp.nsrc = 1; tp.kblocks[0] = (K + kb_elems - 1) / kb_elems; tp.b_koff[0] = 0;
-  tp.M = m_cols; tp.N = n_rows; tp.C = d_C; tp.ldc = ldc; tp.err = tc_error_word();
-  cudaError_t e = zrnn::launch_tc_gemm(tp, BN, tcm, zrnn::TC_EPI_STORE, st);
-  cudaError_t e2 = cudaStreamSynchronize(st);
-  a_hi.release(); a_lo.release(); b_hi.release(); b_lo.release();
-  ZR_CUDA(e);
+  const int n_tiles = (n_rows + 127) / 128;
+  const size_t a_part = aligned((size_t)m_cols * Kpad * eb), b_part = aligned((size_t)n_tiles * 128 * Kpad * eb);
+  DevBuf buf;  // [activations hi | lo][weights hi | lo]
+  const int parts = split ? 2 : 1;
+  ZR_CUDA(buf.reserve((a_part + b_part) * parts));
+  char *a_hi = buf.as<char>(), *b_hi = a_hi + a_part * parts;
+  auto run = [&]() -> int {
+    ZR_CUDA(cudaMemsetAsync(b_hi, 0, b_part * parts, st));
+    ZR_CUDA(zrnn::launch_convert_rows(d_X, m_cols, K, ldx, op_mode, a_hi, (float*)(a_hi + a_part), Kpad, st));
+    zrnn::PackArgs pk;
+    std::memset(&pk, 0, sizeof(pk));
+    pk.src[0] = d_W; pk.G = 1; pk.H = n_rows; pk.K = K; pk.lda = ldw; pk.TH = 128; pk.n_tiles = n_tiles;
+    pk.dst_hi = b_hi; pk.dst_lo = (float*)(b_hi + b_part); pk.op_mode = op_mode; pk.ld_dst = Kpad; pk.koff = 0;
+    ZR_CUDA(zrnn::launch_pack_weights(pk, st));
+    zrnn::ChainBatch cb;
+    zrnn::ChainParams& p = cb.p[0];
+    std::memset(&p, 0, sizeof(p));
+    p.nsrc = 1; p.kb = (K + kb_elems - 1) / kb_elems;
+    const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, p.kb, m_cols);
+    p.a_rows = chain_a_rows(m_cols);
+    p.kbs = zrnn::chain_kbs(tcm, plan.BN, p.a_rows);
+    const int kbs_total = Kpad / kb_elems;
+    if (!zrnn::make_rows_map(&p.a[0], a_hi, eb, (long long)Kpad * eb, m_cols, parts, (long long)a_part, kbs_total, p.a_rows, p.kbs) ||
+        !zrnn::make_rows_map(&p.w, b_hi, eb, (long long)Kpad * eb, (long long)n_tiles * 128, parts, (long long)b_part, kbs_total,
+                             plan.BN, p.kbs))
+      return fail(ZRNN_E_CUDA, "gemm: cannot encode TMA tensor maps");
+    p.M = m_cols; p.N = n_rows; p.C = d_C; p.ldc = ldc; p.err = tc_error_word();
+    ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.BN, tcm, zrnn::TC_EPI_STORE, plan.split, st));
+    return ZRNN_OK;
+  };
+  const int status = run();
+  const cudaError_t e2 = cudaStreamSynchronize(st);
+  buf.release();
+  ZR_TRY(status);
   ZR_CUDA(e2);
   const int code = zrnn_tc_error();
   if (code != 0) return fail(ZRNN_E_TIMEOUT, "gemm: a bounded device wait gave up (role " + std::to_string(code) + ")");
