@@ -17,6 +17,7 @@
 #include "../../include/zrnn_debug.h"
 #include "kernels.cuh"
 #include "model_file.hpp"
+#include "skinny_gemm.cuh"
 #include "tc_chain.cuh"
 #include "tc_decoder.cuh"
 #include "tc_gemm.cuh"
@@ -399,15 +400,48 @@ int lstm_cell_simt(zrnn_lstm_layer* L, const float* x, const int* mask, const fl
   return ZRNN_OK;
 }
 
-// How a link of the chain is launched
+// ---- few columns: the warp-level kernels of skinny_gemm.cu
+bool skinny_engine(int eng) { return eng == ENG_BF16 || eng == ENG_H2; }
+int skinny_mode(int eng) { return eng == ENG_BF16 ? zrnn::SK_BF16 : zrnn::SK_F16X2; }
+// How a link of the chain is launched: the kernel that should take less time (their own estimates)
 struct LinkPlan {
+  bool skinny;
   zrnn::ChainPlan chain;
 };
 LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int H, int cols, int n = 1) {
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
   p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc * ((H + epk - 1) / epk), cols);
+  p.skinny = skinny_engine(eng) && zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) < p.chain.us;
   return p;
+}
+// weights stored in packed 128-row tiles: tile-contiguous k-blocks (kbtot > 0) or plain rows of ld elements
+void skinny_weights(zrnn::SkinnyParams& p, const OpMem& w, int kbtot, long long ld) {
+  p.w_hi = w.hi;
+  p.w_lo = w.lo;
+  if (kbtot > 0) {
+    p.w_tile_bytes = (long long)kbtot * 128 * 128; p.w_row_bytes = 128; p.w_kb_bytes = 128 * 128;
+  } else {
+    p.w_tile_bytes = 128 * ld * 2; p.w_row_bytes = (int)(ld * 2); p.w_kb_bytes = 128;
+  }
+}
+void skinny_source(zrnn::SkinnyParams& p, const Act& a, bool f32, int koff) {
+  p.a_hi[p.nsrc] = f32 ? (const void*)a.f32 : a.hi;
+  p.a_lo[p.nsrc] = f32 ? nullptr : a.lo;
+  p.a_kb0[p.nsrc] = koff / 64;
+  ++p.nsrc;
+}
+void skinny_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
+                        int B, const Act& out, float* c_out, zrnn::SkinnyParams& p, bool f32 = false) {
+  std::memset(&p, 0, sizeof(p));
+  skinny_weights(p, L->Wcat, L->kbtot, (long long)(L->feed ? 3 : 2) * L->Kpad);
+  skinny_source(p, x, f32, 0);
+  skinny_source(p, hp, f32, L->Kpad);
+  if (q) skinny_source(p, *q, f32, 2 * L->Kpad);
+  p.lda = f32 ? L->H : L->Kpad;
+  p.K = L->H; p.M = B; p.N = L->H; p.bias = L->b; p.mask = mask;
+  p.C = out.f32; p.ldc = L->H; p.op_hi = out.hi; p.op_lo = out.lo; p.ld_op = L->Kpad;
+  p.c_prev = c_prev; p.c_out = c_out;
 }
 
 // ---- one link of the recurrent chain on tcgen05 without splitting K (tc_chain.cu)
@@ -481,6 +515,12 @@ int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, 
   const int H = L->H, eng = L->eng;
   const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, H, B);
   KScope ks(KC_LSTM, st);
+  if (plan.skinny) {
+    zrnn::SkinnyBatch sb;
+    skinny_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, sb.p[0]);
+    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_LSTM, false, st));
+    return ZRNN_OK;
+  }
   zrnn::ChainBatch cb;
   ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain.BN, cb.p[0]));
   ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, st));
@@ -491,6 +531,19 @@ int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, c
                int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st) {
   const int nsrc = a1 ? 2 : 1;
   const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, H, B);
+  if (plan.skinny) {
+    zrnn::SkinnyBatch sb;
+    zrnn::SkinnyParams& sp = sb.p[0];
+    std::memset(&sp, 0, sizeof(sp));
+    skinny_weights(sp, w, 0, (long long)nsrc * Kpad);
+    skinny_source(sp, *a0, false, 0);
+    if (a1) skinny_source(sp, *a1, false, Kpad);
+    sp.lda = Kpad; sp.K = H; sp.M = B; sp.N = N; sp.bias = bias; sp.mask = mask; sp.act = 1; sp.act_rows = act_rows;
+    sp.C = C; sp.ldc = ldc;
+    if (op) { sp.op_hi = op->hi; sp.op_lo = op->lo; sp.ld_op = Kpad; }
+    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_STORE, false, st));
+    return ZRNN_OK;
+  }
   zrnn::ChainBatch cb;
   zrnn::ChainParams& p = cb.p[0];
   ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain.BN, p));
@@ -1556,6 +1609,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
   if (!by_layers && L >= 2 && L <= zrnn::ChainBatch::MAX && L0->eng != ENG_SIMT && B <= 128) {
     const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, g.H, B, L);
     KScope sweep(KC_LSTM, s, S * L, true);
+    zrnn::SkinnyBatch sb;
     for (int d = 0; d < S + L - 1; ++d) {
       int n = 0;
       for (int l = std::max(0, d - S + 1); l <= std::min(L - 1, d); ++l) {
@@ -1564,12 +1618,14 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         const Act hp = t == 0 ? h0[l] : act_at(seq[l], (size_t)(t - 1) * B, g);
         const Act out = act_at(seq[l], (size_t)t * B, g);
         const int cu = cur[l];
-        ZR_TRY(chain_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l],
+        if (plan.skinny) skinny_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], sb.p[n]);
+        else ZR_TRY(chain_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l],
                                       plan.chain.BN, m->diag.p[n]));
         cur[l] = cu ^ 1;
         ++n;
       }
-      ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, s));
+      if (plan.skinny) ZR_CUDA(zrnn::launch_skinny(sb, n, skinny_mode(L0->eng), zrnn::SK_EPI_LSTM, false, s));
+      else ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, s));
     }
     return ZRNN_OK;
   }
