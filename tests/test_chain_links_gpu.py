@@ -79,3 +79,22 @@ def test_attention_step_edges(oracle, dtype, H, B, att):
         out[dt] = layer.forward_prop(h, mask).cpu().numpy()
     r, a = TOL[dtype]
     np.testing.assert_allclose(out[dtype], out[3], rtol=r, atol=a)
+
+
+@pytest.mark.parametrize("beam", [1, 2, 15, 16, 32])
+def test_ragged_batch_equals_single_sentences(beam):
+    """A batch whose sentences stop at different steps, in any order: every sentence's hypotheses are those of decoding it alone."""
+    from zoph_rnn_b200 import api, synth
+    cfg = synth.make_cfg(2, 128, 300, 1100, attention=1, feed_input=1, D=3)
+    m = api.neuralMT_model(cfg, dtype=api.F32_SIMT)
+    m.load_weights(synth.make_weights(cfg, seed=11, scale=0.3))
+    rng = np.random.default_rng(beam)
+    srcs = [rng.integers(2, 300, n).astype(np.int32) for n in (3, 11, 1, 7, 11, 2, 5)]
+    kw = dict(beam=beam, k_best=3, min_ratio=0.5, max_ratio=1.5, longest_sent=30, want_align=True)
+    ids, ln, sc, al = m.decode(srcs, **kw)
+    for i, s in enumerate(srcs):
+        i1, l1, s1, a1 = m.decode([s], **kw)
+        np.testing.assert_array_equal(ln[i], l1[0])
+        np.testing.assert_array_equal(ids[i], i1[0])
+        np.testing.assert_array_equal(al[i], a1[0])
+        np.testing.assert_allclose(sc[i], s1[0], rtol=1e-5)

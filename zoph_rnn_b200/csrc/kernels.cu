@@ -66,17 +66,18 @@ __device__ float block_sum(float v, float* red) {
 // ------------------------------------------------------------------------------------------
 // ids: -1 padding -> (id or 0, mask)
 // ------------------------------------------------------------------------------------------
-__global__ void prep_ids_kernel(const int* __restrict__ raw, int n, int* __restrict__ nonm1, int* __restrict__ mask01) {
+__global__ void prep_ids_kernel(const int* __restrict__ raw, int n, int* __restrict__ nonm1, int* __restrict__ mask01,
+                                const int* __restrict__ order, int n_cols) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int v = raw[i];
+    const int v = raw[order ? i - i % n_cols + order[i % n_cols] : i];
     if (nonm1) nonm1[i] = (v == -1) ? 0 : v;
     if (mask01) mask01[i] = (v == -1) ? 0 : 1;
   }
 }
-cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cudaStream_t st) {
+cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cudaStream_t st, const int* order, int n_cols) {
   if (n <= 0) return cudaSuccess;
   const int blocks = (n + 255) / 256;
-  prep_ids_kernel<<<blocks > 1184 ? 1184 : blocks, 256, 0, st>>>(raw, n, nonm1, mask01);
+  prep_ids_kernel<<<blocks > 1184 ? 1184 : blocks, 256, 0, st>>>(raw, n, nonm1, mask01, order, n_cols);
   count_launch();
   return cudaGetLastError();
 }
@@ -285,13 +286,20 @@ cudaError_t launch_gather_rows16(const void* src, size_t row_bytes, int n_src_ro
   return cudaGetLastError();
 }
 
-__global__ void col_gather_kernel(ColGatherArgs a) {
+__global__ void __launch_bounds__(128) col_gather_kernel(const __grid_constant__ ColGatherArgs a) {
+  pdl_enter();
   const int arr = blockIdx.y;
   const float* src = a.src[arr];
   float* dst = a.dst[arr];
   const int H = a.h_arr[arr] > 0 ? a.h_arr[arr] : a.H;
+  const bool table = arr >= a.n_arrays - a.n_table;  // rows of a table picked by a.ids, else columns picked by a.map
   for (int col = blockIdx.x; col < a.n_cols; col += gridDim.x) {
-    const int sc = a.map[col];
+    int sc = table ? a.ids[col] : a.map[col];
+    if (table && sc < 0) sc = 0;  // an invalid beam slot; its column is never consumed
+    if (table && sc >= a.table_rows) {
+      sc = 0;
+      if (a.err && threadIdx.x == 0) atomicExch(a.err, kErrBadTokenId);
+    }
     const float* s = src + (size_t)sc * H;
     float* d = dst + (size_t)col * H;
     if ((H & 3) == 0) {
@@ -304,10 +312,8 @@ __global__ void col_gather_kernel(ColGatherArgs a) {
 }
 cudaError_t launch_col_gather(const ColGatherArgs& a, cudaStream_t st) {
   if (a.n_cols <= 0 || a.n_arrays <= 0) return cudaSuccess;
-  dim3 grid(a.n_cols > 1184 ? 1184 : a.n_cols, a.n_arrays);
-  col_gather_kernel<<<grid, 128, 0, st>>>(a);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(col_gather_kernel, dim3(a.n_cols > 1184 ? 1184 : a.n_cols, a.n_arrays), dim3(128), 0, st, a);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -630,6 +636,52 @@ cudaError_t launch_lse_combine(const float* pm, const float* ps, const float* tg
 // (part_width rows per tile) pass 2 also skips every tile whose maximum is below the bound: it reads about k tiles
 // of the column instead of all of it.
 #define ZR_TOPK_TILES 1024
+// too many candidates (massive ties): raise the bound just above the k-th largest distinct stored value, which is still a
+// lower bound of the column's k-th largest distinct value; the caller collects again.  One warp.
+__device__ void topk_raise_bound(const float* cval, int k, int lane, float thr, float* s_thr, int* s_count) {
+  float best = INFINITY;
+  for (int r = 0; r < k; ++r) {
+    float vmax = -INFINITY;
+    for (int j = lane; j < ZR_TOPK_CAND; j += 32)
+      if (cval[j] < best) vmax = fmaxf(vmax, cval[j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    if (vmax == -INFINITY) break;
+    best = vmax;
+  }
+  if (lane == 0) {
+    *s_thr = (best > thr && best != INFINITY) ? best : nextafterf(thr, INFINITY);
+    *s_count = 0;
+  }
+}
+// the k-th largest of 256 values in shared memory (duplicates count), by one warp: k rounds of a warp-wide argmax over 8 values
+// per lane, the winner's owner dropping it
+__device__ float topk_kth_of_256(const float* tmax, int k, int lane) {
+  float loc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) loc[i] = tmax[lane + 32 * i];
+  const int rounds = k < 256 ? k : 256;
+  float kth = -INFINITY;
+  for (int r = 0; r < rounds; ++r) {
+    float bm = loc[0];
+    int bi = 0;
+#pragma unroll
+    for (int i = 1; i < 8; ++i)
+      if (loc[i] > bm) { bm = loc[i]; bi = i; }
+    float wmax = bm;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+    kth = wmax;
+    if (wmax == -INFINITY) break;
+    const unsigned owners = __ballot_sync(0xffffffffu, bm == wmax);
+    if (lane == __ffs(owners) - 1) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (i == bi) loc[i] = -INFINITY;
+    }
+  }
+  return kth;
+}
 __global__ void __launch_bounds__(256) topk_logp_kernel(const float* __restrict__ z, int V, int N, int k,
                                                          const float* __restrict__ part_max,
                                                          const float* __restrict__ part_sum, int n_parts,
@@ -644,6 +696,7 @@ __global__ void __launch_bounds__(256) topk_logp_kernel(const float* __restrict_
   __shared__ float red_m[8], red_s[8];
   __shared__ float s_M, s_logS, s_thr;
   __shared__ int s_count;
+  pdl_enter();
   const int col = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const float* zc = z + (size_t)col * V;
   float m = -INFINITY, s = 0.f;
@@ -705,32 +758,8 @@ __global__ void __launch_bounds__(256) topk_logp_kernel(const float* __restrict_
       if (lse_out) lse_out[col] = M + s_logS;
     }
   }
-  // the k-th largest of the 256 thread maxima (duplicates count): k rounds of a warp-wide argmax over 8 values per
-  // lane, the winner's owner dropping it
-  if (w == 0) {
-    float loc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) loc[i] = tmax[lane + 32 * i];
-    const int rounds = k < 256 ? k : 256;
-    float kth = -INFINITY;
-    for (int r = 0; r < rounds; ++r) {
-      float bm = loc[0];
-      int bi = 0;
-#pragma unroll
-      for (int i = 1; i < 8; ++i)
-        if (loc[i] > bm) { bm = loc[i]; bi = i; }
-      float wmax = bm;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
-      kth = wmax;
-      if (wmax == -INFINITY) break;
-      const unsigned owners = __ballot_sync(0xffffffffu, bm == wmax);
-      if (lane == __ffs(owners) - 1) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (i == bi) loc[i] = -INFINITY;
-      }
-    }
+  if (w == 0) {  // the selection bound
+    const float kth = topk_kth_of_256(tmax, k, lane);
     if (lane == 0) s_thr = kth;
   }
   __syncthreads();
@@ -816,24 +845,7 @@ __global__ void __launch_bounds__(256) topk_logp_kernel(const float* __restrict_
     }
     __syncthreads();
     if (s_count <= ZR_TOPK_CAND) break;
-    // too many candidates (massive ties): raise the bound just above the k-th largest distinct stored value, which
-    // is still a lower bound of the column's k-th largest distinct value, and collect again
-    if (tid < 32) {
-      float best = INFINITY;
-      for (int r = 0; r < k; ++r) {
-        float vmax = -INFINITY;
-        for (int j = lane; j < ZR_TOPK_CAND; j += 32)
-          if (cval[j] < best) vmax = fmaxf(vmax, cval[j]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-        if (vmax == -INFINITY) break;
-        best = vmax;
-      }
-      if (lane == 0) {
-        s_thr = (best > thr && best != INFINITY) ? best : nextafterf(thr, INFINITY);
-        s_count = 0;
-      }
-    }
+    if (tid < 32) topk_raise_bound(cval, k, lane, thr, &s_thr, &s_count);
     __syncthreads();
     thr = s_thr;
   }
@@ -904,10 +916,9 @@ cudaError_t launch_topk_logp(const float* logits, int V, int N, int k, float* va
                              int part_width, int eos_row, float* lse_out) {
   if (N <= 0) return cudaSuccess;
   if (k < 1 || k > ZR_TOPK_MAX) return cudaErrorInvalidValue;
-  topk_logp_kernel<<<N, 256, 0, st>>>(logits, V, N, k, part_max, part_sum, n_parts, part_width, val_out, idx_out,
-                                      logp_eos, eos_row, lse_out);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(topk_logp_kernel, dim3(N), dim3(256), 0, st, logits, V, N, k, part_max, part_sum, n_parts, part_width, val_out,
+                      idx_out, logp_eos, eos_row, lse_out);
 }
 
 // Merge of G vocabulary shards' candidates.  Shard g reports, per column, its k best rows as log-probabilities under
@@ -1801,6 +1812,124 @@ __global__ void __launch_bounds__(256) ensemble_logmean_kernel(const EnsembleArg
     a.out[col + v] = logf(p);
   }
 }
+// The k best words of the averaged distribution p(v) = mean_k softmax(z_k)(v), one CTA per column.  Writing log p for the whole
+// vocabulary and selecting from that read every logit three times and the result twice (105 + 26 us for two models of 20000
+// words and 72 columns); the partials of the logits products give each model's normaliser, and bounds per tile: p is at least
+// the largest of the models' tile maxima over K and at most their sum, so only tiles whose upper bound reaches the k-th
+// largest lower bound are read.  p sums to 1 by construction, so no renormalisation follows.
+__global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constant__ EnsembleArgs a, int k, float* __restrict__ val_out,
+                                                             int* __restrict__ idx_out, float* __restrict__ logp_eos) {
+  pdl_enter();
+  __shared__ int sel[ZR_TOPK_TILES];
+  __shared__ float tmax[256], cval[ZR_TOPK_CAND];
+  __shared__ int cidx[ZR_TOPK_CAND];
+  __shared__ float red_m[ZR_ENSEMBLE_MAX][8], red_s[ZR_ENSEMBLE_MAX][8], s_M[ZR_ENSEMBLE_MAX], s_inv[ZR_ENSEMBLE_MAX];
+  __shared__ float s_thr;
+  __shared__ int s_count, s_nsel;
+  const int col = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_parts = a.n_parts[0], K = a.K;
+  for (int m = 0; m < K; ++m) {
+    float mx = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = tid + 256 * q;
+      if (j < n_parts) {
+        const float pm = a.part_max[m][(size_t)j * a.N + col], ps = a.part_sum[m][(size_t)j * a.N + col];
+        if (pm > mx) { sum = sum * expf(mx - pm) + ps; mx = pm; }
+        else if (pm != -INFINITY) sum += ps * expf(pm - mx);
+      }
+    }
+    float wm = mx;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, o));
+    const float ws = warp_sum(mx == -INFINITY ? 0.f : sum * expf(mx - wm));
+    if (lane == 0) { red_m[m][w] = wm; red_s[m][w] = ws; }
+  }
+  if (tid == 0) { s_count = 0; s_nsel = 0; }
+  __syncthreads();
+  if (tid < K) {
+    float M = red_m[tid][0];
+    for (int i = 1; i < 8; ++i) M = fmaxf(M, red_m[tid][i]);
+    float S = 0.f;
+    for (int i = 0; i < 8; ++i)
+      if (red_m[tid][i] != -INFINITY) S += red_s[tid][i] * expf(red_m[tid][i] - M);
+    s_M[tid] = M;
+    s_inv[tid] = 1.0f / (S * (float)K);
+  }
+  __syncthreads();
+  float lb = 0.f, ub[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int j = tid + 256 * q;
+    if (j < n_parts)
+      for (int m = 0; m < K; ++m) {
+        const float e = expf(a.part_max[m][(size_t)j * a.N + col] - s_M[m]) * s_inv[m];
+        lb = fmaxf(lb, e);
+        ub[q] += e;
+      }
+  }
+  tmax[tid] = lb;
+  __syncthreads();
+  if (w == 0) {
+    const float kth = topk_kth_of_256(tmax, k, lane);
+    if (lane == 0) s_thr = kth;
+  }
+  if (tid == 32 && logp_eos) {
+    float p = 0.f;
+    for (int m = 0; m < K; ++m) p += expf(a.logits[m][(size_t)col * a.V + 1] - s_M[m]) * s_inv[m];
+    logp_eos[col] = logf(p);
+  }
+  __syncthreads();
+  float thr = s_thr;
+  // (an upper bound and an element are the same sum in the same order, so rounding cannot put an element above its tile's bound)
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (tid + 256 * q < n_parts && ub[q] >= thr && ub[q] > 0.f) sel[atomicAdd(&s_nsel, 1)] = tid + 256 * q;
+  __syncthreads();
+  const int width = a.part_width[0];
+  for (int attempt = 0; attempt < 4; ++attempt) {
+    const int tot = s_nsel * width;
+    for (int e = tid; e < tot; e += 256) {
+      const int i = sel[e / width] * width + e % width;
+      if (i >= a.V) continue;
+      float p = 0.f;
+      for (int m = 0; m < K; ++m) p += expf(a.logits[m][(size_t)col * a.V + i] - s_M[m]) * s_inv[m];
+      if (p >= thr && p > 0.f) {
+        const int at = atomicAdd(&s_count, 1);
+        if (at < ZR_TOPK_CAND) { cval[at] = p; cidx[at] = i; }
+      }
+    }
+    __syncthreads();
+    if (s_count <= ZR_TOPK_CAND) break;
+    if (tid < 32) topk_raise_bound(cval, k, lane, thr, &s_thr, &s_count);
+    __syncthreads();
+    thr = s_thr;
+  }
+  const int nc = s_count < ZR_TOPK_CAND ? s_count : ZR_TOPK_CAND;
+  for (int c = tid; c < nc; c += 256) {  // every candidate counts the ones that beat it
+    const float v = cval[c];
+    const int id = cidx[c];
+    int rank = 0;
+    for (int i = 0; i < nc; ++i) {
+      const float o = cval[i];
+      rank += (o > v || (o == v && cidx[i] < id)) ? 1 : 0;
+    }
+    if (rank < k) {
+      val_out[(size_t)col * k + rank] = logf(v);
+      idx_out[(size_t)col * k + rank] = id;
+    }
+  }
+  if (tid < k && tid >= nc) {  // fewer candidates than k: the tail stays empty
+    val_out[(size_t)col * k + tid] = -INFINITY;
+    idx_out[(size_t)col * k + tid] = -1;
+  }
+}
+bool ensemble_topk_supported(const EnsembleArgs& a) { return a.n_parts[0] >= 1 && a.n_parts[0] <= ZR_TOPK_TILES && a.part_width[0] > 0; }
+cudaError_t launch_ensemble_topk(const EnsembleArgs& a, int k, float* val_out, int* idx_out, float* logp_eos, cudaStream_t st) {
+  if (a.N <= 0) return cudaSuccess;
+  if (a.K < 1 || a.K > ZR_ENSEMBLE_MAX || k < 1 || k > ZR_TOPK_MAX || !ensemble_topk_supported(a)) return cudaErrorInvalidValue;
+  count_launch();
+  return launch_chain(ensemble_topk_kernel, dim3(a.N), dim3(256), 0, st, a, k, val_out, idx_out, logp_eos);
+}
 __global__ void ensemble_viterbi_kernel(const EnsembleVitArgs a) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= a.N) return;
@@ -1835,7 +1964,7 @@ cudaError_t launch_ensemble_logmean(const EnsembleArgs& a, cudaStream_t st) {
 // beam bookkeeping, one CTA per sentence
 // ------------------------------------------------------------------------------------------
 __global__ void beam_init_kernel(const BeamArgs a) {
-  const int s = blockIdx.x, tid = threadIdx.x;
+  const int s = blockIdx.x, tid = threadIdx.x;  // (every sentence's results are cleared: the order does not matter here)
   const size_t rowbase = (size_t)s * a.beam * a.Lmax;
   for (int i = tid; i < a.beam * a.Lmax; i += blockDim.x) { a.top_sent[rowbase + i] = 0; a.top_tmp[rowbase + i] = 0; }
   if (a.vit_rows) {
@@ -1857,34 +1986,40 @@ cudaError_t launch_beam_init(const BeamArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// insert (prefix of `row` up to position last_pos, then <EOF>) with `score` into the sentence's k-best list
+// insert (prefix of `row` up to position last_pos, then <EOF>) with `score` into the sentence's k-best list; one whole warp
 // vrow / last_align: the alignments stored with the prefix and the one of the step that produced <EOF> (tracking on)
 __device__ void beam_insert_hyp(const BeamArgs& a, int s, const int* row, int last_pos, float score, const int* vrow,
-                                int last_align) {
+                                int last_align, int lane) {
   const int len = last_pos + 2;
   const float ratio = ((float)len) / (float)a.src_len[s];
   if (!(ratio > a.min_ratio)) return;
-  int* ids = a.best_ids + (size_t)s * a.k_best * a.Lmax;
-  int* lens = a.best_len + s * a.k_best;
-  float* sc = a.best_score + s * a.k_best;
+  const int o = a.out_index ? a.out_index[s] : s;  // where the caller wants this sentence's results
+  int* ids = a.best_ids + (size_t)o * a.k_best * a.Lmax;
+  int* lens = a.best_len + o * a.k_best;
+  float* sc = a.best_score + o * a.k_best;
   int pos = 0;
   while (pos < a.k_best && lens[pos] != 0 && !(score > sc[pos])) ++pos;
   if (pos >= a.k_best) return;
-  int* al = a.best_align ? a.best_align + (size_t)s * a.k_best * a.Lmax : nullptr;
+  __syncwarp();  // every lane has found the place before anybody moves an entry
+  int* al = a.best_align ? a.best_align + (size_t)o * a.k_best * a.Lmax : nullptr;
   for (int j = a.k_best - 1; j > pos; --j) {
-    if (lens[j - 1] == 0) continue;
-    for (int i = 0; i < a.Lmax; ++i) ids[(size_t)j * a.Lmax + i] = ids[(size_t)(j - 1) * a.Lmax + i];
-    if (al)
-      for (int i = 0; i < a.Lmax; ++i) al[(size_t)j * a.Lmax + i] = al[(size_t)(j - 1) * a.Lmax + i];
-    lens[j] = lens[j - 1];
-    sc[j] = sc[j - 1];
+    const int lj = lens[j - 1];
+    if (lj == 0) continue;
+    const float sj = sc[j - 1];
+    __syncwarp();
+    for (int i = lane; i < a.Lmax; i += 32) {  // (a position always stays with its lane)
+      ids[(size_t)j * a.Lmax + i] = ids[(size_t)(j - 1) * a.Lmax + i];
+      if (al) al[(size_t)j * a.Lmax + i] = al[(size_t)(j - 1) * a.Lmax + i];
+    }
+    if (lane == 0) { lens[j] = lj; sc[j] = sj; }
+    __syncwarp();
   }
-  for (int i = 0; i < a.Lmax; ++i) ids[(size_t)pos * a.Lmax + i] = (i <= last_pos) ? row[i] : (i == last_pos + 1 ? 1 : -1);
-  if (al)
-    for (int i = 0; i < a.Lmax; ++i)
-      al[(size_t)pos * a.Lmax + i] = (i <= last_pos) ? vrow[i] : (i == last_pos + 1 ? last_align : -1);
-  lens[pos] = len;
-  sc[pos] = score;
+  for (int i = lane; i < a.Lmax; i += 32) {
+    ids[(size_t)pos * a.Lmax + i] = (i <= last_pos) ? row[i] : (i == last_pos + 1 ? 1 : -1);
+    if (al) al[(size_t)pos * a.Lmax + i] = (i <= last_pos) ? vrow[i] : (i == last_pos + 1 ? last_align : -1);
+  }
+  if (lane == 0) { lens[pos] = len; sc[pos] = score; }
+  __syncwarp();
 }
 
 // NL: candidates per lane of the selecting warp: 8 covers beam * (beam + 1) <= 256 (beam <= 15), 33 covers beam <= 32
@@ -1892,8 +2027,10 @@ template <int NL>
 __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
   __shared__ float cv[32 * NL];
   __shared__ int ci[32 * NL];
+  __shared__ int order[NL <= 8 ? 256 : 1];
   __shared__ int n_chg[ZR_BEAM_MAX], n_cur[ZR_BEAM_MAX];
   __shared__ float n_sc[ZR_BEAM_MAX];
+  pdl_enter();
   const int s = blockIdx.x, tid = threadIdx.x, beam = a.beam, kc = a.k_cand, t = a.step;
   const int base = s * beam;
   const int max_steps = a.max_steps[s];
@@ -1906,12 +2043,12 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
     return;
   }
   if (t == max_steps) {  // finish_current_hypotheses
-    if (tid == 0)
+    if (tid < 32)
       for (int i = 0; i < beam; ++i) {
         if (a.cur_ids[base + i] == -1) continue;
         const float sc = a.scores[base + i] + (a.logp_eos[base + i] + a.penalty);
         beam_insert_hyp(a, s, rows + (size_t)i * a.Lmax, t, sc, vrows ? vrows + (size_t)i * a.Lmax : nullptr,
-                        vrows ? a.viterbi[base + i] : -1);
+                        vrows ? a.viterbi[base + i] : -1, tid);
       }
     if (tid < beam) a.col_map[base + tid] = base + tid;
     return;
@@ -1938,48 +2075,90 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
     ci[c] = wd;  // its word, kept on chip: the selection below reads one per pick
   }
   __syncthreads();
-  // One warp walks the candidates in descending score (the lower candidate index wins a tie) until the beam is full:
-  // a warp-wide argmax per pick, the winner's owner dropping it.
-  if (tid < 32) {
-    const int lane = tid;
-    float loc[NL];
-#pragma unroll
-    for (int j = 0; j < NL; ++j) loc[j] = cv[lane + 32 * j];
-    int filled = 0;
-    while (filled < beam) {
-      float bv = loc[0];
-      int bj = 0;
-#pragma unroll
-      for (int j = 1; j < NL; ++j)
-        if (loc[j] > bv) { bv = loc[j]; bj = j; }
-      int bidx = lane + 32 * bj;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-        if (ov > bv || (ov == bv && oi < bidx)) { bv = ov; bidx = oi; }
+  if constexpr (NL <= 8) {
+    // At most one candidate per thread: each counts the candidates that beat it (higher score, or the same score and a lower
+    // index) and puts itself at that place; one warp then walks over the sorted list, 32 candidates at a time.  (A warp-wide
+    // argmax per pick, with its shuffles, was a chain of a thousand cycles and more.)
+    const int n_cand = beam * kc;
+    if (tid < n_cand) {
+      const float v = cv[tid];
+      int rank = 0;
+      for (int i = 0; i < n_cand; ++i) {
+        const float o = cv[i];
+        rank += (o > v || (o == v && i < tid)) ? 1 : 0;
       }
-      if (bv == -INFINITY) {  // no candidate left: the remaining slots stay empty
-        if (lane == 0)
-          for (; filled < beam; ++filled) { n_cur[filled] = -1; n_chg[filled] = 0; n_sc[filled] = 0.f; }
-        break;
+      order[rank] = tid;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      const int lane = tid;
+      int filled = 0;
+      for (int p0 = 0; p0 < n_cand && filled < beam; p0 += 32) {
+        const int c = p0 + lane < n_cand ? order[p0 + lane] : -1;
+        const float v = c >= 0 ? cv[c] : -INFINITY;
+        const int wd = c >= 0 ? ci[c] : -1;
+        const bool alive = v != -INFINITY;
+        const bool word = alive && wd != 0 && wd != 1;  // <START> is never extended, <EOF> finishes a hypothesis
+        const unsigned words = __ballot_sync(0xffffffffu, word);
+        const int slot = filled + __popc(words & ((1u << lane) - 1u));  // words taken before this candidate
+        if (word && slot < beam) { n_cur[slot] = wd; n_chg[slot] = c / kc; n_sc[slot] = v + a.penalty; }
+        // finished hypotheses that come before the beam is full, in order; they do not take a slot
+        unsigned ends = __ballot_sync(0xffffffffu, alive && wd == 1 && slot < beam);
+        while (ends) {
+          const int l = __ffs(ends) - 1;
+          ends &= ends - 1;
+          const int i = __shfl_sync(0xffffffffu, c, l) / kc;
+          const float sc = __shfl_sync(0xffffffffu, v, l) + a.penalty;
+          beam_insert_hyp(a, s, rows + (size_t)i * a.Lmax, t, sc, vrows ? vrows + (size_t)i * a.Lmax : nullptr,
+                          vrows ? a.viterbi[base + i] : -1, lane);
+        }
+        filled += __popc(words);
+        if (!__all_sync(0xffffffffu, alive || p0 + lane >= n_cand)) break;  // only empty candidates follow
       }
-      if ((bidx & 31) == lane) {
-#pragma unroll
-        for (int j = 0; j < NL; ++j)
-          if (j == (bidx >> 5)) loc[j] = -INFINITY;
-      }
-      const int i = bidx / kc;
-      const int wd = ci[bidx];
-      if (wd == 0) continue;  // <START> is never extended
-      if (wd == 1) {          // <EOF>: finished hypothesis, does not take a slot
-        if (lane == 0)
+      if (lane >= filled && lane < beam) { n_cur[lane] = -1; n_chg[lane] = 0; n_sc[lane] = 0.f; }
+    }
+  } else {
+    // One warp walks the candidates in descending score (the lower candidate index wins a tie) until the beam is full:
+    // a warp-wide argmax per pick, the winner's owner dropping it.
+    if (tid < 32) {
+      const int lane = tid;
+      float loc[NL];
+  #pragma unroll
+      for (int j = 0; j < NL; ++j) loc[j] = cv[lane + 32 * j];
+      int filled = 0;
+      while (filled < beam) {
+        float bv = loc[0];
+        int bj = 0;
+  #pragma unroll
+        for (int j = 1; j < NL; ++j)
+          if (loc[j] > bv) { bv = loc[j]; bj = j; }
+        int bidx = lane + 32 * bj;
+  #pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+          if (ov > bv || (ov == bv && oi < bidx)) { bv = ov; bidx = oi; }
+        }
+        if (bv == -INFINITY) {  // no candidate left: the remaining slots stay empty
+          if (lane == 0)
+            for (; filled < beam; ++filled) { n_cur[filled] = -1; n_chg[filled] = 0; n_sc[filled] = 0.f; }
+          break;
+        }
+        if ((bidx & 31) == lane) {
+  #pragma unroll
+          for (int j = 0; j < NL; ++j)
+            if (j == (bidx >> 5)) loc[j] = -INFINITY;
+        }
+        const int i = bidx / kc;
+        const int wd = ci[bidx];
+        if (wd == 0) continue;  // <START> is never extended
+        if (wd == 1) {          // <EOF>: finished hypothesis, does not take a slot
           beam_insert_hyp(a, s, rows + (size_t)i * a.Lmax, t, bv + a.penalty, vrows ? vrows + (size_t)i * a.Lmax : nullptr,
-                          vrows ? a.viterbi[base + i] : -1);
-        __syncwarp();
-      } else {
-        if (lane == 0) { n_cur[filled] = wd; n_chg[filled] = i; n_sc[filled] = bv + a.penalty; }
-        ++filled;
+                          vrows ? a.viterbi[base + i] : -1, lane);
+        } else {
+          if (lane == 0) { n_cur[filled] = wd; n_chg[filled] = i; n_sc[filled] = bv + a.penalty; }
+          ++filled;
+        }
       }
     }
   }
@@ -2005,10 +2184,9 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
 cudaError_t launch_beam_step(const BeamArgs& a, cudaStream_t st) {
   if (a.n_sent <= 0) return cudaSuccess;
   if (a.beam < 1 || a.beam > ZR_BEAM_MAX || a.k_cand > ZR_BEAM_MAX + 1 || a.beam * a.k_cand > 32 * 33) return cudaErrorInvalidValue;
-  if (a.beam * a.k_cand <= 256) beam_step_kernel<8><<<a.n_sent, 256, 0, st>>>(a);
-  else beam_step_kernel<33><<<a.n_sent, 256, 0, st>>>(a);
   count_launch();
-  return cudaGetLastError();
+  if (a.beam * a.k_cand <= 256) return launch_chain(beam_step_kernel<8>, dim3(a.n_sent), dim3(256), 0, st, a);
+  return launch_chain(beam_step_kernel<33>, dim3(a.n_sent), dim3(256), 0, st, a);
 }
 
 }  // namespace zrnn

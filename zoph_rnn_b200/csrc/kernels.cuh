@@ -9,7 +9,9 @@ namespace zrnn {
 void count_launch(int n = 1);
 
 // ---- input preparation (replaces vocab_to_01 / vocab_to_nonM1, src/custom_kernels.h:9-32)
-cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cudaStream_t st);
+// order (optional): column c of the n_cols columns (ids time-major) comes from column order[c]
+cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cudaStream_t st, const int* order = nullptr,
+                            int n_cols = 1);
 
 // ---- embedding column gather (replaces sparse_lookup_kernel, src/custom_kernels.h:340-348)
 // V > 0: an id >= V reads column 0 instead of memory past the table and sets *err (if given) to kErrBadTokenId
@@ -25,13 +27,18 @@ cudaError_t launch_gather_rows16(const void* src, size_t row_bytes, int n_src_ro
 // (replaces the per-column cudaMemcpy loops of swap_states_decoding / transfer_decoding_states_GPU,
 // src/Input_To_Hidden_Layer.hpp:1231-1260, src/model.hpp:2715-2719)
 struct ColGatherArgs {
-  enum { MAX_ARRAYS = 40 };  // 8 layers x (h: fp32 + two operand parts, c) + the fed-back attention vector
+  enum { MAX_ARRAYS = 40 };  // 8 layers x (h: fp32 + two operand parts, c) + the fed-back attention vector + the next inputs
   const float* src[MAX_ARRAYS];
   float* dst[MAX_ARRAYS];
   int h_arr[MAX_ARRAYS];  // floats per column of each array; 0 = H
   int n_arrays;
   int H, n_cols;
   const int* map;  // n_cols source column indices
+  // the last n_table arrays are not columns but rows of a table (an embedding): dst[:,c] = src row ids[c] (negative: row 0; an id
+  // >= table_rows reads row 0 and sets *err)
+  int n_table, table_rows;
+  const int* ids;
+  int* err;
 };
 cudaError_t launch_col_gather(const ColGatherArgs& a, cudaStream_t st);
 
@@ -201,8 +208,16 @@ struct EnsembleArgs {
   const float* logits[ZR_ENSEMBLE_MAX];  // each V x N, column-major
   int K, V, N;
   float* out;  // V x N
+  // what the logits products left per row tile and column ([part][N], as launch_topk_logp's): maximum and exp-sum
+  const float* part_max[ZR_ENSEMBLE_MAX];
+  const float* part_sum[ZR_ENSEMBLE_MAX];
+  int n_parts[ZR_ENSEMBLE_MAX], part_width[ZR_ENSEMBLE_MAX];  // the same for all models
 };
 cudaError_t launch_ensemble_logmean(const EnsembleArgs& a, cudaStream_t st);
+// The k largest log-probabilities of the averaged distribution per column straight from the models' logits and partials (the
+// averaged distribution is never written down); needs the same tiling in all models and at most 1024 tiles
+bool ensemble_topk_supported(const EnsembleArgs& a);
+cudaError_t launch_ensemble_topk(const EnsembleArgs& a, int k, float* val_out, int* idx_out, float* logp_eos, cudaStream_t st);
 // Alignment voting of an ensemble (ensembles_models, src/ensemble_factory.hpp:798-834): per column the source position
 // with the largest sum over the models of the attention weight at that position; the running maximum starts at 0,
 // so a column whose weights are all zero reports -1.  align[k] is S_max[k] x N by position.
@@ -224,6 +239,7 @@ struct BeamArgs {
   const float* logp_eos;   // [n_sent*beam]
   const int* src_len;      // [n_sent]
   const int* max_steps;    // [n_sent]
+  const int* out_index;    // [n_sent] sentence number in the best_* arrays (null: the same number)
   int* top_sent;           // [n_sent][beam][Lmax]
   int* top_tmp;            // same size: the step writes the surviving rows here; the caller swaps the two after it
   float* scores;           // [n_sent][beam]

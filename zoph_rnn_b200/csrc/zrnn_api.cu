@@ -5,6 +5,7 @@
 #include <dlfcn.h>
 #include <nccl.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -2149,22 +2150,23 @@ struct BeamModel {
       if (eng_split(g.eng)) add_plain(ga, (const float*)srcA.lo, (float*)dstA.lo, opf);
     }
   }
-  int run_gathers(zrnn::ColGatherArgs* ga, const int* map, cudaStream_t s) const {
+  int run_gathers(zrnn::ColGatherArgs* ga, const int* map, int cols, cudaStream_t s) const {
     if (ga->n_arrays == 0) return ZRNN_OK;
-    ga->H = g.H; ga->n_cols = NB; ga->map = map;
+    ga->H = g.H; ga->n_cols = cols; ga->map = map;
     KScope ks(KC_REORDER, s);
     ZR_CUDA(zrnn::launch_col_gather(*ga, s));
     return ZRNN_OK;
   }
   // forward_prop_source + transfer_decoding_states_GPU (src/model.hpp:2367-2452)
-  int encode(const int* d_src, cudaStream_t s) {
+  // order: column c of the search is sentence order[c] (null: the same)
+  int encode(const int* d_src, const int* order, cudaStream_t s) {
     const zrnn_model_config& c = m->cfg;
     const int L = c.num_layers;
     const size_t HBs = (size_t)c.H * n, nS = (size_t)S_max * n;
     cur.assign(L, 0);
     ZR_TRY(act_zero(zero, g, n, s));
     for (int l = 0; l < L; ++l) ZR_CUDA(cudaMemsetAsync(cst[0][l], 0, sizeof(float) * HBs, s));
-    ZR_CUDA(zrnn::launch_prep_ids(d_src, (int)nS, src_id, src_mk, s));
+    ZR_CUDA(zrnn::launch_prep_ids(d_src, (int)nS, src_id, src_mk, s, order, n));
     ZR_CUDA(zrnn::launch_src_len(src_mk, S_max, n, len, off, s));
     ZR_TRY(run_encoder(m, g, src_id, src_mk, S_max, n, X0, zero, sseq, cst, cur, s));
     if (c.attention) ZR_TRY(zrnn_att_set_source(m->att, sseq[L - 1].f32, S_max, n, len, off, beam));
@@ -2178,27 +2180,27 @@ struct BeamModel {
       add_gather(&ga, act_at(sseq[l], (size_t)(S_max - 1) * n, g), hp[l]);
       add_plain(&ga, cst[cur[l]][l], cp[l], c.H);
     }
-    return run_gathers(&ga, rep_map, s);
+    return run_gathers(&ga, rep_map, NB, s);
   }
-  // forward_prop_target (src/model.hpp:2573-2689) up to the vector handed to the softmax
-  int forward(int t, const int* cur_ids, Act* top, cudaStream_t s) {
+  // forward_prop_target (src/model.hpp:2573-2689) up to the vector handed to the softmax, for the first `cols` columns
+  int forward(int t, const int* cur_ids, int cols, Act* top, cudaStream_t s) {
     const zrnn_model_config& c = m->cfg;
-    ZR_TRY(gather_act(m->tgt[0], cur_ids, NB, x, s));
+    if (t == 0) ZR_TRY(gather_act(m->tgt[0], cur_ids, cols, x, s));  // (later inputs come with the reorder)
     Act xin = x;
     for (int l = 0; l < c.num_layers; ++l) {
       const bool use_feed = (l == 0 && c.feed_input && t > 0);
-      ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], NB, hn[l], cn[l], s));
+      ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], cols, hn[l], cn[l], s));
       xin = hn[l];
     }
     *top = xin;
     if (c.attention) {
-      ZR_TRY(att_forward(m->att, xin, nullptr, NB, htild_new, align_pos, s, vit, 0.f, align_pos != nullptr));
+      ZR_TRY(att_forward(m->att, xin, nullptr, cols, htild_new, align_pos, s, vit, 0.f, align_pos != nullptr));
       *top = htild_new;
     }
     return ZRNN_OK;
   }
-  // swap_decoding_states + target_copy_prev_states (src/model.hpp:2691-2726)
-  int reorder(const int* col_map, cudaStream_t s) {
+  // swap_decoding_states + target_copy_prev_states (src/model.hpp:2691-2726) and the embedding rows of the next words
+  int reorder(const int* col_map, const int* cur_ids, int cols, cudaStream_t s) {
     const zrnn_model_config& c = m->cfg;
     zrnn::ColGatherArgs ga;
     std::memset(&ga, 0, sizeof(ga));
@@ -2207,7 +2209,17 @@ struct BeamModel {
       add_plain(&ga, cn[l], cp[l], c.H);
     }
     if (c.feed_input) add_gather(&ga, htild_new, htild_feed);
-    return run_gathers(&ga, col_map, s);
+    const zrnn_lstm_layer* L0 = m->tgt[0];
+    const int before = ga.n_arrays;
+    if (tc) {
+      const int opf = g.Kpad * eng_eb(g.eng) / 4;
+      add_plain(&ga, (const float*)L0->emb.hi, (float*)x.hi, opf);
+      if (eng_split(g.eng)) add_plain(&ga, (const float*)L0->emb.lo, (float*)x.lo, opf);
+    } else {
+      add_plain(&ga, L0->W, x.f32, c.H);
+    }
+    ga.n_table = ga.n_arrays - before; ga.table_rows = L0->V; ga.ids = cur_ids; ga.err = tc_error_word();
+    return run_gathers(&ga, col_map, cols, s);
   }
 };
 
@@ -2242,16 +2254,25 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
   zrnn_model* m0 = models[0];
 
   // per-sentence step limits (src/ensemble_factory.hpp:637)
-  m0->h_tmp.resize(2 * (size_t)n);
-  int Tmax = 0;
+  auto limit = [&](int i) { return std::min((int)(max_ratio * h_src_len[i]), Lmax - 2); };
   for (int i = 0; i < n; ++i) {
     ZR_CHECK(h_src_len[i] >= 1 && h_src_len[i] <= S_max[0], "beam_decode: source length out of range");
-    int ms = std::min((int)(max_ratio * h_src_len[i]), Lmax - 2);
-    ZR_CHECK(ms >= 1, "beam_decode: max_ratio*source_length must allow at least one step");
-    m0->h_tmp[i] = h_src_len[i];
-    m0->h_tmp[n + i] = ms;
-    Tmax = std::max(Tmax, ms);
+    ZR_CHECK(limit(i) >= 1, "beam_decode: max_ratio*source_length must allow at least one step");
   }
+  // The sentences are worked on in the order of their limits, longest first: at every step the ones that are still running
+  // are the leading columns, and every launch of the step covers just those (64 sentences of 10 .. 50 words: 59 % of the
+  // columns over the whole search).
+  std::vector<int> order(n);
+  for (int i = 0; i < n; ++i) order[i] = i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return limit(x) > limit(y); });
+  const bool sorted = std::is_sorted(order.begin(), order.end());
+  m0->h_tmp.resize(3 * (size_t)n);
+  for (int i = 0; i < n; ++i) {
+    m0->h_tmp[i] = h_src_len[order[i]];
+    m0->h_tmp[n + i] = limit(order[i]);
+    m0->h_tmp[2 * n + i] = order[i];
+  }
+  const int Tmax = m0->h_tmp[n];
   const bool track = d_out_align != nullptr;
   const bool vote = track && K > 1;  // alignment voting over the models of an ensemble
   std::vector<BeamModel> bm(K);
@@ -2263,7 +2284,7 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
     b.S_max = S_max[k]; b.n = n; b.NB = NB; b.beam = beam;
     size_t bytes = b.bytes(track && k == 0, vote);
     if (k == 0) {  // shared bookkeeping lives in model 0's workspace
-      bytes += 2 * aligned(sizeof(int) * n) + 2 * aligned(sizeof(int) * NB) + 2 * aligned(sizeof(int) * (size_t)NB * Lmax);
+      bytes += aligned(sizeof(int) * 3 * n) + 2 * aligned(sizeof(int) * NB) + 2 * aligned(sizeof(int) * (size_t)NB * Lmax);
       bytes += aligned(sizeof(int) * (size_t)NB * kc) + 2 * aligned(sizeof(float) * NB) + aligned(sizeof(float) * (size_t)NB * kc);
       if (track) bytes += 2 * aligned(sizeof(int) * (size_t)NB * Lmax);
       if (K > 1) bytes += aligned(sizeof(float) * (size_t)V * NB);
@@ -2271,8 +2292,8 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
     ZR_CUDA(models[k]->ws.reserve(bytes));
   }
   Carver cv0(m0->ws.p);
-  int* d_len_host = cv0.take<int>(n);
-  int* max_steps = cv0.take<int>(n);
+  int* d_len_host = cv0.take<int>(3 * (size_t)n);  // [source length][step limit][sentence number] in working order
+  const int *max_steps = d_len_host + n, *d_order = d_len_host + 2 * n;
   int* cur_ids = cv0.take<int>(NB);
   int* col_map = cv0.take<int>(NB);
   int* top_sent = cv0.take<int>((size_t)NB * Lmax);
@@ -2290,49 +2311,60 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
     bm[k].carve(cv, false, vote);
   }
 
-  ZR_CUDA(cudaMemcpyAsync(d_len_host, m0->h_tmp.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
-  ZR_CUDA(cudaMemcpyAsync(max_steps, m0->h_tmp.data() + n, sizeof(int) * n, cudaMemcpyHostToDevice, s));
-  for (int k = 0; k < K; ++k) ZR_TRY(bm[k].encode(d_src[k], s));
+  ZR_CUDA(cudaMemcpyAsync(d_len_host, m0->h_tmp.data(), sizeof(int) * 3 * n, cudaMemcpyHostToDevice, s));
+  for (int k = 0; k < K; ++k) ZR_TRY(bm[k].encode(d_src[k], sorted ? nullptr : d_order, s));
 
   zrnn::BeamArgs ba;
   std::memset(&ba, 0, sizeof(ba));
   ba.n_sent = n; ba.beam = beam; ba.k_cand = kc; ba.Lmax = Lmax; ba.k_best = k_best;
   ba.min_ratio = min_ratio; ba.penalty = penalty;
   ba.cand_val = cand_val; ba.cand_idx = cand_idx; ba.logp_eos = logp_eos; ba.src_len = d_len_host; ba.max_steps = max_steps;
+  ba.out_index = d_order;
   ba.top_sent = top_sent; ba.top_tmp = top_tmp; ba.scores = scores; ba.cur_ids = cur_ids; ba.col_map = col_map;
   ba.best_ids = d_out_ids; ba.best_len = d_out_len; ba.best_score = d_out_score;
   ba.viterbi = bm[0].vit; ba.vit_rows = vit_rows; ba.vit_tmp = vit_tmp; ba.best_align = d_out_align;
   ZR_CUDA(zrnn::launch_beam_init(ba, s));
 
+  int n_act = n;  // sentences still running: the leading ones
   for (int t = 0; t <= Tmax; ++t) {
+    while (m0->h_tmp[n + n_act - 1] < t) --n_act;
+    const int cols = n_act * beam;
     if (K == 1) {
       Act top;
-      ZR_TRY(bm[0].forward(t, cur_ids, &top, s));
-      if (comm) ZR_TRY(softmax_topk_sharded_act(m0->sm, comm, top, NB, kc, cand_val, cand_idx, logp_eos, s));
-      else ZR_TRY(softmax_topk_act(m0->sm, top, NB, kc, cand_val, cand_idx, logp_eos, s));
+      ZR_TRY(bm[0].forward(t, cur_ids, cols, &top, s));
+      if (comm) ZR_TRY(softmax_topk_sharded_act(m0->sm, comm, top, cols, kc, cand_val, cand_idx, logp_eos, s));
+      else ZR_TRY(softmax_topk_act(m0->sm, top, cols, kc, cand_val, cand_idx, logp_eos, s));
     } else {
       zrnn::EnsembleArgs ea;
       std::memset(&ea, 0, sizeof(ea));
+      bool partials = true;
       for (int k = 0; k < K; ++k) {
         Act top;
-        ZR_TRY(bm[k].forward(t, cur_ids, &top, s));
-        const float* pm = nullptr;
+        ZR_TRY(bm[k].forward(t, cur_ids, cols, &top, s));
+        const float *pm = nullptr, *ps = nullptr;
         int np = 0;
-        ZR_TRY(softmax_logits_act(models[k]->sm, top, NB, s, &pm, &np));
+        ZR_TRY(softmax_logits_act(models[k]->sm, top, cols, s, &pm, &np, &ps));
         ea.logits[k] = models[k]->sm->logits.as<float>();
+        ea.part_max[k] = pm; ea.part_sum[k] = ps; ea.n_parts[k] = np; ea.part_width[k] = models[k]->sm->BN / zrnn::kPersistentParts;
+        partials = partials && pm && ps && np == ea.n_parts[0] && ea.part_width[k] == ea.part_width[0];
       }
-      ea.K = K; ea.V = V; ea.N = NB; ea.out = mean_logits;
+      ea.K = K; ea.V = V; ea.N = cols; ea.out = mean_logits;
       if (vote) {  // ensembles_models: sum the models' weights per source position, take the largest
         zrnn::EnsembleVitArgs va;
         std::memset(&va, 0, sizeof(va));
         for (int k = 0; k < K; ++k) { va.align[k] = bm[k].align_pos; va.S_max[k] = bm[k].S_max; }
-        va.K = K; va.N = NB; va.viterbi_out = bm[0].vit;
+        va.K = K; va.N = cols; va.viterbi_out = bm[0].vit;
         ZR_CUDA(zrnn::launch_ensemble_viterbi(va, s));
       }
       KScope ks(KC_SOFTMAX_REDUCE, s);
-      ZR_CUDA(zrnn::launch_ensemble_logmean(ea, s));
-      ZR_CUDA(zrnn::launch_topk_logp(mean_logits, V, NB, kc, cand_val, cand_idx, logp_eos, s, nullptr, nullptr, 0));
+      if (partials && zrnn::ensemble_topk_supported(ea)) {
+        ZR_CUDA(zrnn::launch_ensemble_topk(ea, kc, cand_val, cand_idx, logp_eos, s));
+      } else {
+        ZR_CUDA(zrnn::launch_ensemble_logmean(ea, s));
+        ZR_CUDA(zrnn::launch_topk_logp(mean_logits, V, cols, kc, cand_val, cand_idx, logp_eos, s, nullptr, nullptr, 0));
+      }
     }
+    ba.n_sent = n_act;
     ba.step = t;
     {
       KScope ks(KC_BEAM, s);
@@ -2342,7 +2374,7 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
       std::swap(ba.vit_rows, ba.vit_tmp);
     }
     if (t < Tmax)
-      for (int k = 0; k < K; ++k) ZR_TRY(bm[k].reorder(col_map, s));
+      for (int k = 0; k < K; ++k) ZR_TRY(bm[k].reorder(col_map, cur_ids, cols, s));
   }
   return ZRNN_OK;
 }
