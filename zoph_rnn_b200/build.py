@@ -7,7 +7,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libzrnn.so")
 CLI = os.path.join(HERE, "bin", "zoph_rnn")
-SOURCES = ["kernels.cu", "tc_gemm.cu", "tc_decoder.cu", "tc_chain.cu", "skinny_gemm.cu", "zrnn_api.cu"]
+SOURCES = ["kernels.cu", "tc_gemm.cu", "tc_decoder.cu", "tc_chain.cu", "tc_link.cu", "skinny_gemm.cu", "zrnn_api.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "--expt-relaxed-constexpr"]
 
@@ -48,11 +48,15 @@ def build(force=False, verbose=False):
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     objs = []
-    for src in SOURCES:
+    running = []
+    for src in SOURCES:  # side by side: one source takes up to a minute
         obj = os.path.join(CSRC, src.replace(".cu", ".o"))
         cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-c", os.path.join(CSRC, src), "-o", obj]
-        subprocess.check_call(cmd)
+        running.append((cmd, subprocess.Popen(cmd)))
         objs.append(obj)
+    for cmd, proc in running:
+        if proc.wait() != 0:
+            raise subprocess.CalledProcessError(proc.returncode, cmd)
     subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB] + objs + ["-lcudart"])
     build_cli(force=True)
     return LIB

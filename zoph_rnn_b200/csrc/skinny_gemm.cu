@@ -61,40 +61,16 @@ __device__ __forceinline__ void mma_chunk(float* c, const uint4& u, const uint4&
   mma16816<MODE>(c, u.x, v.x, u.y, v.y, b.x, b.y);
   mma16816<MODE>(c, u.z, v.z, u.w, v.w, b.z, b.w);
 }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&t);
-}
-__device__ __forceinline__ uint32_t pack_half(__half a, __half b) {
-  __half2 t = __halves2half2(a, b);
-  return *reinterpret_cast<uint32_t*>(&t);
-}
-// eight fp32 activations -> operand pieces
-template <int MODE>
-__device__ __forceinline__ void split8(const float* x, uint4* hi, uint4* lo) {
-  if (MODE == SK_BF16) {
-    *hi = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
-  } else {
-    __half h[8], l[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      h[i] = __float2half_rn(x[i]);
-      l[i] = __float2half_rn((x[i] - __half2float(h[i])) * 2048.0f);
-    }
-    *hi = make_uint4(pack_half(h[0], h[1]), pack_half(h[2], h[3]), pack_half(h[4], h[5]), pack_half(h[6], h[7]));
-    *lo = make_uint4(pack_half(l[0], l[1]), pack_half(l[2], l[3]), pack_half(l[4], l[5]), pack_half(l[6], l[7]));
-  }
-}
 template <int MODE>
 __device__ __forceinline__ float sk_tanh(float x) {
-  if (MODE == SK_F16X2) return tanhf(x);
+  if (MODE == SK_F16X2) return tanh_f32(x);
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 template <int MODE>
 __device__ __forceinline__ float sk_sigmoid(float x) {
-  if (MODE == SK_F16X2) return 1.0f / (1.0f + expf(-x));
+  if (MODE == SK_F16X2) return sigmoid_f32(x);
   return fmaf(0.5f, sk_tanh<MODE>(0.5f * x), 0.5f);
 }
 template <int MODE>
@@ -123,21 +99,20 @@ __device__ __forceinline__ void sk_zero_pad(const SkinnyParams& p, int row, int 
 // of one gate at a time) both spread over the banks when it is an odd multiple of 8
 __host__ __device__ constexpr int part_ld(int NT) { return (NT & 1) ? 8 * NT : 8 * NT + 8; }
 __host__ __device__ constexpr int parts_of(int mode) { return mode == SK_F16X2 ? 2 : 1; }
-__host__ __device__ constexpr int act_pieces(int mode, bool f32) { return (f32 || mode == SK_F16X2) ? 2 : 1; }
 // bytes of one warp's ring stage: its weight and activation pieces of one chunk
-__host__ __device__ constexpr int warp_stage(int MT, int NT, int mode, bool f32) {
-  return (2 * MT * parts_of(mode) + NT * act_pieces(mode, f32)) * 512;
+__host__ __device__ constexpr int warp_stage(int MT, int NT, int mode) {
+  return (2 * MT + NT) * parts_of(mode) * 512;
 }
 __host__ __device__ constexpr int warp_part_bytes(int MT, int NT) { return MT * 16 * part_ld(NT) * 4; }
 __device__ __forceinline__ void cp16z(uint32_t dst, const void* src, int bytes) {  // the rest of the 16 bytes is zeroed
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
-template <int MT, int NT, int MODE, int EPI, bool F32A>
+template <int MT, int NT, int MODE, int EPI>
 __global__ void __launch_bounds__(kWarps * 32, (MT * NT <= 4) ? 2 : 1)
     skinny_kernel(const __grid_constant__ SkinnyBatch pb, int PD) {
-  constexpr int P = parts_of(MODE), AP = act_pieces(MODE, F32A);
-  constexpr int STAGE = warp_stage(MT, NT, MODE, F32A);
+  constexpr int P = parts_of(MODE);
+  constexpr int STAGE = warp_stage(MT, NT, MODE);
   constexpr int LD = part_ld(NT), NC = 8 * NT;
   extern __shared__ __align__(16) unsigned char sk_smem[];
   const SkinnyParams& p = pb.p[blockIdx.z];
@@ -193,28 +168,33 @@ __global__ void __launch_bounds__(kWarps * 32, (MT * NT <= 4) ? 2 : 1)
     for (int nt = 0; nt < NT; ++nt) {
       const int col = col0 + nt * 8 + g;
       const bool in = col < p.M;  // missing columns are zeros: reading a stand-in would make every SM poll the same few lines
-      if (F32A) {
-        const float* a = (const float*)p.a_hi[s] + (in ? (size_t)col * p.lda : 0);
-        cp16z(d, a + (left >= 4 ? k : 0), in && left >= 4 ? 16 : 0);
-        cp16z(d + 512, a + (left >= 8 ? k + 4 : 0), in && left >= 8 ? 16 : 0);
-      } else {
-        // what an operand row holds beyond K may be anything
-        const int bytes = !in ? 0 : (left >= 8 ? 16 : (left > 0 ? 2 * left : 0));
-        const size_t o = bytes ? ((size_t)col * p.lda + k) * 2 : 0;
-        cp16z(d, (const char*)p.a_hi[s] + o, bytes);
-        if (P == 2) cp16z(d + 512, (const char*)p.a_lo[s] + o, bytes);
-      }
-      d += AP * 512;
+      // what an operand row holds beyond K may be anything
+      const int bytes = !in ? 0 : (left >= 8 ? 16 : (left > 0 ? 2 * left : 0));
+      const size_t o = bytes ? ((size_t)col * p.lda + k) * 2 : 0;
+      cp16z(d, (const char*)p.a_hi[s] + o, bytes);
+      if (P == 2) cp16z(d + 512, (const char*)p.a_lo[s] + o, bytes);
+      d += P * 512;
     }
   };
 
-  // the weights of the first stages do not depend on the predecessor kernel
+  // The weights of the first stages do not depend on the predecessor kernel, and the chunks of the early sources were complete
+  // when it passed its own wait: this warp works on them (its first n_e) until it needs the predecessor's results.  The successor
+  // may start after that, so that what it reads early is complete in its turn.
+  const int early = p.n_early * cps, n_e = early > warp ? (early - warp + kWarps - 1) / kWarps : 0;
+  bool waited = false;
+  auto wait_for = [&](int i) {
+    if (waited || i < n_e) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    waited = true;
+  };
   const int pre = n_my < PD ? n_my : PD;
   for (int i = 0; i < pre; ++i) load_w(i, i);
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int i = 0; i < PD; ++i) {
-    if (i < n_my) load_a(i, i);
+    if (i < n_my) {
+      wait_for(i);
+      load_a(i, i);
+    }
     cp_commit();
   }
   float acc[MT][NT][4];
@@ -246,14 +226,8 @@ __global__ void __launch_bounds__(kWarps * 32, (MT * NT <= 4) ? 2 : 1)
         for (int x = 0; x < P; ++x) w[mt][h][x] = lds128(d + ((mt * 2 + h) * P + x) * 512);
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      const uint32_t da = d + (2 * MT * P + nt * AP) * 512;
-      uint4 b_hi = lds128(da), b_lo = make_uint4(0, 0, 0, 0);
-      if (AP == 2) b_lo = lds128(da + 512);
-      if (F32A) {
-        const float x[8] = {__uint_as_float(b_hi.x), __uint_as_float(b_hi.y), __uint_as_float(b_hi.z), __uint_as_float(b_hi.w),
-                            __uint_as_float(b_lo.x), __uint_as_float(b_lo.y), __uint_as_float(b_lo.z), __uint_as_float(b_lo.w)};
-        split8<MODE>(x, &b_hi, &b_lo);
-      }
+      const uint32_t da = d + (2 * MT + nt) * P * 512;
+      const uint4 b_hi = lds128(da), b_lo = P == 2 ? lds128(da + 512) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         if (MODE == SK_BF16) {
@@ -270,12 +244,14 @@ __global__ void __launch_bounds__(kWarps * 32, (MT * NT <= 4) ? 2 : 1)
     }
     if (i + PD < n_my) {
       load_w(i + PD, slot);
+      wait_for(i + PD);
       load_a(i + PD, slot);
     }
     cp_commit();
     if (++slot == PD) slot = 0;
   }
 
+  wait_for(n_e);
   // the cell's other inputs, requested while the partial tiles are put down
   constexpr int OUT = EPI == SK_EPI_LSTM ? MT * 4 * NC : MT * 16 * NC;
   constexpr int EPT = (OUT + kWarps * 32 - 1) / (kWarps * 32);
@@ -345,9 +321,9 @@ __global__ void __launch_bounds__(kWarps * 32, (MT * NT <= 4) ? 2 : 1)
 
 const bool g_pdl = std::getenv("ZRNN_NO_PDL") == nullptr;
 
-template <int MT, int NT, int MODE, int EPI, bool F32A>
+template <int MT, int NT, int MODE, int EPI>
 cudaError_t launch_t(const SkinnyBatch& b, int n, cudaStream_t st) {
-  constexpr int STAGE = warp_stage(MT, NT, MODE, F32A);
+  constexpr int STAGE = warp_stage(MT, NT, MODE);
   const SkinnyParams& p = b.p[0];
   const int tiles = EPI == SK_EPI_LSTM ? (p.N + 3) / 4 : (p.N + 15) / 16;
   const int chunks = p.nsrc * ((p.K + 31) / 32), per_warp = (chunks + kWarps - 1) / kWarps;
@@ -362,7 +338,7 @@ cudaError_t launch_t(const SkinnyBatch& b, int n, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(skinny_kernel<MT, NT, MODE, EPI, F32A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(skinny_kernel<MT, NT, MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          227 * 1024);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
@@ -379,52 +355,48 @@ cudaError_t launch_t(const SkinnyBatch& b, int n, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = g_pdl ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, skinny_kernel<MT, NT, MODE, EPI, F32A>, b, PD);
+  return cudaLaunchKernelEx(&cfg, skinny_kernel<MT, NT, MODE, EPI>, b, PD);
 }
-template <int NT, int MODE, int EPI, bool F32A>
+template <int NT, int MODE, int EPI>
 cudaError_t launch_mt(const SkinnyBatch& b, int n, int mt, cudaStream_t st) {
-  if (mt <= 1) return launch_t<1, NT, MODE, EPI, F32A>(b, n, st);
-  if (mt == 2) return launch_t<2, NT, MODE, EPI, F32A>(b, n, st);
-  return launch_t<4, NT, MODE, EPI, F32A>(b, n, st);
+  if (mt <= 1) return launch_t<1, NT, MODE, EPI>(b, n, st);
+  if (mt == 2) return launch_t<2, NT, MODE, EPI>(b, n, st);
+  return launch_t<4, NT, MODE, EPI>(b, n, st);
 }
-template <int MODE, int EPI, bool F32A>
+template <int MODE, int EPI>
 cudaError_t launch_nt(const SkinnyBatch& b, int n, int mt, int nt, cudaStream_t st) {
   switch (nt) {
-    case 1: return launch_mt<1, MODE, EPI, F32A>(b, n, mt, st);
-    case 2: return launch_mt<2, MODE, EPI, F32A>(b, n, mt, st);
-    case 3: return launch_mt<3, MODE, EPI, F32A>(b, n, mt, st);
-    case 4: return launch_mt<4, MODE, EPI, F32A>(b, n, mt, st);
-    case 5: case 6: return launch_mt<6, MODE, EPI, F32A>(b, n, mt, st);
+    case 1: return launch_mt<1, MODE, EPI>(b, n, mt, st);
+    case 2: return launch_mt<2, MODE, EPI>(b, n, mt, st);
+    case 3: return launch_mt<3, MODE, EPI>(b, n, mt, st);
+    case 4: return launch_mt<4, MODE, EPI>(b, n, mt, st);
+    case 5: case 6: return launch_mt<6, MODE, EPI>(b, n, mt, st);
   }
-  return launch_mt<8, MODE, EPI, F32A>(b, n, mt, st);
+  return launch_mt<8, MODE, EPI>(b, n, mt, st);
 }
 
 }  // namespace
 
 // Fitted to measurements (us per launch; f32 / bf16): 4 M weights 5.8 / 4.2 at 8 columns, 8.7 / 5.1 at 32; 16 M weights 11 / 7.9 at
-// 8 columns, 17 / 10 at 24.
+// 8 columns, 17 / 10 at 24; 2 M weights at 64 columns 10 / -.  (From two column groups on every weight is read twice: not offered.)
 float skinny_us(int mode, int rows, int K, int cols, int n) {
   const float mw = (float)rows * K * n * 1e-6f, nt = (float)((cols + 7) / 8);
-  return mode == SK_F16X2 ? 4.0f + mw * (0.25f + 0.19f * nt) : 3.2f + mw * (0.22f + 0.07f * nt);
+  return mode == SK_F16X2 ? 4.0f + mw * (0.285f + nt * (0.144f + 0.0114f * nt)) : 3.2f + mw * (0.22f + 0.07f * nt);
 }
 
-cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, bool a_f32, cudaStream_t st) {
+cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st) {
   const SkinnyParams& p = b.p[0];
-  if (n < 1 || n > SkinnyBatch::MAX || p.M < 1 || p.N < 1 || p.nsrc < 1 || p.nsrc > 3 || (p.K & 3)) return cudaErrorInvalidValue;
+  if (n < 1 || n > SkinnyBatch::MAX || p.M < 1 || p.N < 1 || p.nsrc < 1 || p.nsrc > 3 || p.n_early < 0 || p.n_early >= p.nsrc || (p.K & 3)) return cudaErrorInvalidValue;
   for (int i = 1; i < n; ++i)
     if (b.p[i].N != p.N || b.p[i].K != p.K || b.p[i].M != p.M || b.p[i].nsrc != p.nsrc) return cudaErrorInvalidValue;
   const int tiles = n * (epi == SK_EPI_LSTM ? (p.N + 3) / 4 : (p.N + 15) / 16);
   const int groups = (p.M + 63) / 64, nt = (p.M + groups * 8 - 1) / (groups * 8);
   // as few row tiles per CTA as keep the launch at one CTA per SM: the activations are read once per CTA
   const int mt = tiles <= 148 ? 1 : (tiles <= 296 ? 2 : 4);
-  if (mode == SK_F16X2) {
-    if (epi == SK_EPI_LSTM) return a_f32 ? launch_nt<SK_F16X2, SK_EPI_LSTM, true>(b, n, mt, nt, st) : launch_nt<SK_F16X2, SK_EPI_LSTM, false>(b, n, mt, nt, st);
-    return a_f32 ? launch_nt<SK_F16X2, SK_EPI_STORE, true>(b, n, mt, nt, st) : launch_nt<SK_F16X2, SK_EPI_STORE, false>(b, n, mt, nt, st);
-  }
-  if (mode == SK_BF16) {
-    if (epi == SK_EPI_LSTM) return a_f32 ? launch_nt<SK_BF16, SK_EPI_LSTM, true>(b, n, mt, nt, st) : launch_nt<SK_BF16, SK_EPI_LSTM, false>(b, n, mt, nt, st);
-    return a_f32 ? launch_nt<SK_BF16, SK_EPI_STORE, true>(b, n, mt, nt, st) : launch_nt<SK_BF16, SK_EPI_STORE, false>(b, n, mt, nt, st);
-  }
+  if (mode == SK_F16X2)
+    return epi == SK_EPI_LSTM ? launch_nt<SK_F16X2, SK_EPI_LSTM>(b, n, mt, nt, st) : launch_nt<SK_F16X2, SK_EPI_STORE>(b, n, mt, nt, st);
+  if (mode == SK_BF16)
+    return epi == SK_EPI_LSTM ? launch_nt<SK_BF16, SK_EPI_LSTM>(b, n, mt, nt, st) : launch_nt<SK_BF16, SK_EPI_STORE>(b, n, mt, nt, st);
   return cudaErrorInvalidValue;
 }
 

@@ -18,7 +18,8 @@ struct SkinnyParams {
   long long w_tile_bytes;
   int w_row_bytes, w_kb_bytes;
   int nsrc;
-  const void* a_hi[3];  // [cols][lda] operand rows, or fp32 columns (a_f32)
+  int n_early;          // leading sources that were complete when the predecessor kernel passed its own wait
+  const void* a_hi[3];  // [cols][lda] operand rows
   const void* a_lo[3];
   int a_kb0[3];         // first k-block of the source inside the weights' K axis
   int lda;
@@ -42,8 +43,7 @@ struct SkinnyBatch {
 };
 // about how long launch_skinny takes for n problems of `rows` weight rows x K elements (all sources) and `cols` columns
 float skinny_us(int mode, int rows, int K, int cols, int n);
-// n independent problems of the same shape class (mode, epilogue, N, K, M) in one launch; a_f32: the activations are plain
-// fp32 columns (lda = K) that the kernel converts itself
-cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, bool a_f32, cudaStream_t st);
+// n independent problems of the same shape class (mode, epilogue, N, K, M) in one launch
+cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st);
 
 }  // namespace zrnn

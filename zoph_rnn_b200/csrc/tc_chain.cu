@@ -1,15 +1,12 @@
-// tcgen05 kernels for the links of the recurrent chain (LSTM cells, attention projections, combiner).
+// tcgen05 kernel for the links of the recurrent chain with wide tiles (many columns, or several cells in a launch) and the rule
+// that picks a link's tile.  Narrow tiles: tc_link.cu.
 //
-// A CTA computes 128 batch rows x BN weight rows over the WHOLE K axis: no CTA waits for another one's partial tile, so a
-// launch is: activations in (one TMA latency), K loop, epilogue.  BN is chosen so that the tiles of the launch just fill the
-// SMs (H = 1000: 125 tiles of 32 rows = 8 hidden units x 4 gates).  The price is that every CTA reads all activations (the
-// same lines at about the same time, which L2 serves at full rate); splitting K over a cluster instead, with the exchange of
-// partial tiles through distributed shared memory, spent 3 - 4 us of a launch on the exchange alone; only where the K axis is long do two CTAs share a tile (SPLIT below).
+// A CTA computes 128 batch rows x BN = 128 or 256 weight rows over the WHOLE K axis: no CTA waits for another one's partial
+// tile, so a launch is: activations in (one TMA latency), K loop, epilogue.
 //
-// Warps: EW epilogue warps (warp w reads TMEM lane quadrant w % 4 and takes column group w / 4 of the tile), one for the
-// activation loads, one for the weight loads, one that issues the MMAs.  The weights do not depend on the predecessor
-// kernel, so their loads start before griddepcontrol.wait; with tiles of up to 64 rows two CTAs fit an SM (shared memory and
-// TMEM halves), so the successor's set-up and first weights overlap this kernel's last microseconds.
+// Warps: 16 epilogue warps (warp w reads TMEM lane quadrant w % 4 and takes column group w / 4 of the tile), one for the
+// activation loads, one for the weight loads, two that issue MMAs.  The weights do not depend on the predecessor kernel, so
+// their loads start before griddepcontrol.wait.
 #include "tc_chain.cuh"
 
 #include <algorithm>
@@ -18,22 +15,17 @@
 #include <cstring>
 
 #include "kernels.cuh"
-#include "tc_device.cuh"
+#include "tc_chain_device.cuh"
 
 namespace zrnn {
 namespace {
 
-__host__ __device__ constexpr int chain_epi_warps(int BN) { return BN == 16 ? 8 : 16; }
-// An MMA of 128 rows takes 45 cycles up to 32 columns, 48 at 64, 64 at 128 (measured): it is bound by the reads of its A
-// tile.  Narrow tiles of the split modes therefore multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the
-// columns for two products, and A_lo by W_hi: two MMAs per k-step instead of three.
-__host__ __device__ constexpr bool chain_stacked(int BN, int mode) { return mode_split(mode) && BN <= 64; }
+constexpr int kEpiWarps = 16;
 // Two warps issue MMAs, so that the wait for a stage and the commit (300 cycles in one thread, as long as a k-block's MMAs) of
 // one overlap the other's MMAs.  They take alternate stages, each into accumulators of its own; wide tiles of the split modes
 // have no room for that, there one warp issues the hi * hi products of every stage and the other the two cross products.
 constexpr int kMmaWarps = 2;
-__host__ __device__ constexpr bool chain_by_product(int BN, int mode) { return mode_split(mode) && BN > 64; }
-__host__ __device__ constexpr int chain_threads(int BN) { return (chain_epi_warps(BN) + 2 + kMmaWarps) * 32; }
+constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
 // The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb more than kRoundKb k-blocks
 // (16 k-steps) in a row: the K axis is walked in rounds, each into a fresh accumulator set, and the epilogue warps, idle until
 // the end otherwise, add every finished round to sums of their own in registers (round to nearest) while the next round runs.
@@ -41,74 +33,30 @@ __host__ __device__ constexpr int chain_threads(int BN) { return (chain_epi_warp
 // 5.7e-7 and 23e-7).
 constexpr int kRoundKb = 4;
 __host__ __device__ constexpr bool chain_rounds(int BN, int mode) { return mode_split(mode) && BN <= 128; }
-// accumulator sets.  Stacked: a main and a cross accumulator each, two per MMA warp.  Wide split tiles: main accumulators, with
-// one cross accumulator behind them.  Other modes: one per MMA warp.
-__host__ __device__ constexpr int chain_sets(int BN, int mode) {
-  return !mode_split(mode) ? kMmaWarps : (BN <= 64 ? 2 * kMmaWarps : (BN <= 128 ? 3 : 1));
-}
+// accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  Other modes: one per MMA warp.
+__host__ __device__ constexpr int chain_sets(int BN, int mode) { return !mode_split(mode) ? kMmaWarps : (BN <= 128 ? 3 : 1); }
 __host__ __device__ constexpr int chain_tmem(int BN, int mode) {
-  int need = !mode_split(mode) ? chain_sets(BN, mode) * BN
-                               : (chain_stacked(BN, mode) ? 2 * chain_sets(BN, mode) * BN : (chain_sets(BN, mode) + 1) * BN);
+  const int need = (chain_sets(BN, mode) + (mode_split(mode) ? 1 : 0)) * BN;
   int c = 32;
   while (c < need) c *= 2;
   return c;
 }
-constexpr int kMaxStages = 8;
-// rows y.. of k-blocks kb.., all parts (make_rows_map)
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int y, int kb) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3, %5}], [%2];"
-      :
-      : "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(kb)
-      : "memory");
-}
-// hidden units y.. of all gates from part `part` and k-block kb on (make_gate_map)
-__device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int y, int part, int kb) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3, %5, %6}], [%2];"
-      :
-      : "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(part), "r"(kb)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
-  uint32_t r0, r1, r2, r3;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(taddr));
-  v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1); v[2] = __uint_as_float(r2); v[3] = __uint_as_float(r3);
-}
-template <int W>
-__device__ __forceinline__ void tmem_ldw(uint32_t taddr, float* v) {
-  if constexpr (W == 2) {
-    uint32_t r0, r1;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(taddr));
-    v[0] = __uint_as_float(r0); v[1] = __uint_as_float(r1);
-  } else if constexpr (W == 4) tmem_ld4(taddr, v);
-  else tmem_ld8(taddr, v);
-}
+constexpr int kChainRingBytes = 224 * 1024, kMaxStages = 8;
 
-// bytes of the exchange slots of a CTA pair that splits K: the accumulator columns of half a tile
-__host__ __device__ constexpr int chain_slot_bytes(int BN, int split) { return split == 2 ? BN / 2 * 128 * 4 : 0; }
-
-// SPLIT == 2: a cluster of two CTAs (blockIdx.z = rank) shares a tile, each over half of the K axis.  The epilogue warps of the
-// column groups that belong to the other CTA push their sums into that CTA's shared memory and are done; the warps of the same
-// place there add them to their own sums and finish those outputs.
-template <int BN, int MODE, int EPI, int SPLIT>
+template <int BN, int MODE, int EPI>
 __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_block, const int stages) {
-  constexpr int EW = chain_epi_warps(BN), kAWarp = EW, kWWarp = EW + 1, kMmaWarp = EW + 2;
-  constexpr bool BY_PRODUCT = chain_by_product(BN, MODE), ROUNDS = chain_rounds(BN, MODE);
+  constexpr int EW = kEpiWarps, kAWarp = EW, kWWarp = EW + 1, kMmaWarp = EW + 2;
+  constexpr bool BY_PRODUCT = mode_split(MODE), ROUNDS = chain_rounds(BN, MODE);
   constexpr int STEP = BY_PRODUCT ? 1 : kMmaWarps;  // stages from one of an MMA warp to its next
   constexpr int PARTS = mode_split(MODE) ? 2 : 1;
   constexpr int WKB = BN * 128;  // bytes of one k-block of one weight part
-  constexpr bool STACKED = chain_stacked(BN, MODE);
-  constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN), IDESC2 = make_idesc(mode_fmt(MODE), STACKED ? 2 * BN : BN);
-  constexpr int NSET = chain_sets(BN, MODE), SETC = STACKED ? 2 * BN : BN, TMEM_COLS = chain_tmem(BN, MODE);
+  constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN);
+  constexpr int NSET = chain_sets(BN, MODE), TMEM_COLS = chain_tmem(BN, MODE);
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
   __shared__ __align__(8) uint64_t accum_bar;  // everything accumulated (rounds: the cross products of wide tiles)
   __shared__ __align__(8) uint64_t set_full[chain_sets(BN, MODE)], set_empty[chain_sets(BN, MODE)];
-  __shared__ __align__(8) uint64_t xchg_bar[EW];  // SPLIT: the other CTA's share for this warp has arrived
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   __shared__ float s_bias[BN];
@@ -122,14 +70,9 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   const int KBS = p.kbs;
   // KBS x [A hi][A lo], KBS x [W hi][W lo]; every piece is a multiple of 1024 bytes
   const int stage_bytes = PARTS * KBS * (akb + WKB);
-  const int src_it = (p.kb + KBS - 1) / KBS, total_it = p.nsrc * src_it;
+  const int src_it = (p.kb + KBS - 1) / KBS, n_it = p.nsrc * src_it;
   const int round_its = KBS < kRoundKb ? kRoundKb / KBS : 1;  // stages per round
   constexpr int NBUF = BY_PRODUCT ? NSET : NSET / kMmaWarps;  // accumulator sets an MMA warp takes in turn
-  // every row tile walks the K axis from another stage on: the CTAs do not all ask L2 for the same few activation rows at
-  // the same moment
-  const int rank = SPLIT > 1 ? (int)blockIdx.z : 0;
-  const int it_lo = total_it * rank / SPLIT, it_hi = total_it * (rank + 1) / SPLIT, n_it = it_hi - it_lo;
-  const int it_first = it_lo + n_tile % n_it;
   ZR_STAMP(0);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -141,8 +84,6 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       mbar_init(&set_full[i], 1);
       mbar_init(&set_empty[i], EW);
     }
-    if (SPLIT > 1)
-      for (int i = 0; i < EW; ++i) mbar_init(&xchg_bar[i], 1);
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -155,10 +96,8 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (SPLIT > 1) cluster_arrive();  // (the barriers above are ready; waited for before the first remote store)
   const uint32_t tmem_base = tmem_base_s;
   ZR_STAMP(1);
-  pdl_trigger();  // the successor touches nothing of this kernel's before it has waited for its end
 
   if (warp == kWWarp) {
     // ------------------------------------------------------------ weights: nothing here depends on the predecessor
@@ -166,7 +105,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       bool ok = true;
       int it = 0, st = 0;
       uint32_t ph = 0;
-      int s = it_first / src_it, c = it_first % src_it, gi = it_first;
+      int s = 0, c = 0;
       for (; it < n_it; ++it) {
         if (it >= stages && !mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
         uint8_t* w = tiles + (size_t)st * stage_bytes + PARTS * KBS * akb;
@@ -187,13 +126,9 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
           tma_load_4d(w, &p.w, &full_bar[st], n_tile * BN, wkb);
         }
         if (++st == stages) { st = 0; ph ^= 1u; }
-        if (++gi == it_hi) { gi = it_lo; s = gi / src_it; c = gi % src_it; }
-        else if (++c == src_it) { c = 0; ++s; }
+        if (++c == src_it) { c = 0; ++s; }
       }
-      if (!ok) {  // copies in flight land before the CTA may retire
-        const long long t0 = clock64();
-        while (clock64() - t0 < 20000000LL) {}
-      }
+      if (!ok) settle_copies();
     }
     __syncwarp();
     pdl_wait();
@@ -202,23 +137,20 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
     if (warp == kAWarp) {
       // ------------------------------------------------------------ activations
       if (lane == 0) {
+        pdl_trigger();  // after the wait: the successor may read what this kernel's predecessor left (tc_link.cu)
         bool ok = true;
         int it = 0, st = 0;
         uint32_t ph = 0;
-        int s = it_first / src_it, c = it_first % src_it, gi = it_first;
+        int s = 0, c = 0;
         for (; it < n_it; ++it) {
           if (it >= stages && !mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 7)) { ok = false; break; }
           uint8_t* a = tiles + (size_t)st * stage_bytes;
           mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * akb));
           tma_load_4d(a, &p.a[s], &full_bar[st], p.a_row0[s] + m0, c * KBS);
           if (++st == stages) { st = 0; ph ^= 1u; }
-          if (++gi == it_hi) { gi = it_lo; s = gi / src_it; c = gi % src_it; }
-        else if (++c == src_it) { c = 0; ++s; }
+          if (++c == src_it) { c = 0; ++s; }
         }
-        if (!ok) {
-          const long long t0 = clock64();
-          while (clock64() - t0 < 20000000LL) {}
-        }
+        if (!ok) settle_copies();
       }
     } else if (warp >= kMmaWarp) {
       // ------------------------------------------------------------ MMA issuers
@@ -237,7 +169,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
           if (!mbar_wait(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
-          const uint32_t d = tmem_base + (uint32_t)(set * SETC), d_cross = tmem_base + (uint32_t)(NSET * BN);
+          const uint32_t d = tmem_base + (uint32_t)(set * BN), d_cross = tmem_base + (uint32_t)(NSET * BN);
           const bool fresh = rounds ? in_round == 0 : it < STEP;  // the accumulator starts with this stage
           for (int b = 0; b < KBS; ++b) {
             const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
@@ -245,10 +177,8 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const uint32_t acc = (!fresh || b > 0 || k > 0) ? 1u : 0u;
-              if (!BY_PRODUCT || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC2, acc);
-              if (STACKED) {
-                umma<mode_kind_tf32(MODE)>(d + BN, dal + 2 * k, dw + 2 * k, IDESC, 1u);
-              } else if (BY_PRODUCT && mw == 1) {
+              if (!BY_PRODUCT || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC, acc);
+              if (BY_PRODUCT && mw == 1) {
                 umma<mode_kind_tf32(MODE)>(d_cross, dal + 2 * k, dw + 2 * k, IDESC, acc);
                 umma<mode_kind_tf32(MODE)>(d_cross, da + 2 * k, dwl + 2 * k, IDESC, 1u);
               }
@@ -286,16 +216,15 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
     asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
   }
   const int quad = warp & 3, cg = warp >> 2;
-  const bool mine = SPLIT == 1 || cg / (EW / 4 / 2) == rank;  // this CTA finishes the warp's outputs
   const int row = m0 + quad * 32 + lane;
   const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
   constexpr int GROUPS = EW / 4;
   constexpr int PER = EPI == TC_EPI_LSTM ? BN / 4 / GROUPS : BN / GROUPS;  // outputs per row and column group
-  constexpr int W = PER < 4 ? 2 : ((PER < 8 || STACKED) ? 4 : 8);                         // outputs handled at a time (registers)
+  constexpr int W = 8;                                    // outputs handled at a time (registers)
   // the cell's other inputs do not depend on the accumulators: fetch the first ones while the main loop runs
   float pre_c[W];
   float mk = 1.0f;
-  if (epi_warp && mine && row < p.M) {
+  if (epi_warp && row < p.M) {
     if (p.mask) mk = (float)p.mask[row];
     if constexpr (EPI == TC_EPI_LSTM) {
       const int hb = n_tile * (BN / 4) + cg * PER;
@@ -323,17 +252,14 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         ready = __all_sync(0xffffffffu, mbar_wait(&set_full[set], (uint32_t)((r / NBUF) & 1), &abort_s, p.err, 3));
         tc_fence_after();
         if (ready && live) {
-          float t[NCH][W], x[NCH][W];
+          float t[NCH][W];
 #pragma unroll
-          for (int ch = 0; ch < NCH; ++ch) {
-            tmem_ldw<W>(taddr + set * SETC + chunk_col(ch), t[ch]);
-            if (STACKED) tmem_ldw<W>(taddr + set * SETC + BN + chunk_col(ch), x[ch]);
-          }
+          for (int ch = 0; ch < NCH; ++ch) tmem_ldw<W>(taddr + set * BN + chunk_col(ch), t[ch]);
           tmem_wait_ld();
 #pragma unroll
           for (int ch = 0; ch < NCH; ++ch)
 #pragma unroll
-            for (int u = 0; u < W; ++u) sum[ch][u] += STACKED ? fmaf(x[ch][u], mode_cross_scale(MODE), t[ch][u]) : t[ch][u];
+            for (int u = 0; u < W; ++u) sum[ch][u] += t[ch][u];
         }
         tc_fence_before();
         __syncwarp();
@@ -362,7 +288,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       float t[NSET][W], x[W];
 #pragma unroll
       for (int a = 0; a < NSET; ++a)
-        if (a == 0 || a < n_sets) tmem_ldw<W>(taddr + a * SETC + col, t[a]);
+        if (a == 0 || a < n_sets) tmem_ldw<W>(taddr + a * BN + col, t[a]);
       if (PARTS == 2) tmem_ldw<W>(taddr + NSET * BN + col, x);
       tmem_wait_ld();
 #pragma unroll
@@ -379,43 +305,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       }
     }
   };
-  float fin[SPLIT > 1 ? NCH : 1][W];
-  if constexpr (SPLIT > 1) {
-    static_assert(BN <= 64 && (NCH * W) % 4 == 0, "chunks of the exchange");
-    __syncwarp();
-    cluster_wait();
-    if (ready && live) {
-      constexpr int V4 = NCH * W / 4;
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) load_acc(ch, chunk_col(ch), fin[ch]);
-      float* f = &fin[0][0];
-      // float4 units [warp's place among its CTA's finishing warps][V4][lane]
-      float4* slot = reinterpret_cast<float4*>(tiles + (size_t)stages * stage_bytes) + (size_t)((cg % (EW / 4 / 2)) * 4 + quad) * V4 * 32 + lane;
-      if (!mine) {
-        const uint32_t peer = cluster_map(smem_u32(slot), (uint32_t)(rank ^ 1));
-#pragma unroll
-        for (int i = 0; i < V4; ++i) st_cluster_v4(peer + i * 512, f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(&xchg_bar[warp], (uint32_t)(rank ^ 1));  // releases the whole warp's stores
-      } else {
-        ready = __all_sync(0xffffffffu, mbar_wait_cluster(&xchg_bar[warp], 0, &abort_s, p.err, 6));
-#pragma unroll
-        for (int i = 0; i < V4; ++i) {
-          const float4 o = slot[i * 32];
-          f[4 * i] += o.x; f[4 * i + 1] += o.y; f[4 * i + 2] += o.z; f[4 * i + 3] += o.w;
-        }
-      }
-    }
-  }
-  auto finished = [&](int ch, int col, float* v) {
-    if constexpr (SPLIT > 1) {
-#pragma unroll
-      for (int u = 0; u < W; ++u) v[u] = fin[ch][u];
-    } else {
-      load_acc(ch, col, v);
-    }
-  };
-  if (ready && live && mine) {
+  if (ready && live) {
     if constexpr (EPI == TC_EPI_LSTM) {
       constexpr int TH = BN / 4, THP = TH < 32 ? TH : 32;  // hidden units per gate block of the accumulator
       const int H = p.N;
@@ -424,7 +314,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         const int j0 = cg * PER + j8;
         float g[4][W];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) finished(q, (j0 / THP) * (4 * THP) + q * THP + (j0 % THP), g[q]);
+        for (int q = 0; q < 4; ++q) load_acc(q, (j0 / THP) * (4 * THP) + q * THP + (j0 % THP), g[q]);
         const int hb = n_tile * TH + j0;
         if (row < p.M && hb < H) {
           float hv[W], cv[W];
@@ -454,7 +344,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       for (int c8 = 0; c8 < PER; c8 += W) {
         const int c0 = cg * PER + c8, n = n_tile * BN + c0, left = p.N - n;
         float v[W];
-        finished(c8 / W, c0, v);
+        load_acc(c8 / W, c0, v);
         if (row < p.M && left > 0) {
 #pragma unroll
           for (int u = 0; u < W; ++u) {
@@ -470,7 +360,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
     }
   }
   // the operand rows' padding up to a whole k-block is read by the next product: the last row tile keeps it at zero
-  if (epi_warp && n_tile == (int)gridDim.y - 1 && row < p.M && cg == 0 && rank == 0) zero_operand_pad(p, (size_t)row * p.ld_op, p.N, p.ld_op);
+  if (epi_warp && n_tile == (int)gridDim.y - 1 && row < p.M && cg == 0) zero_operand_pad(p, (size_t)row * p.ld_op, p.N, p.ld_op);
   ZR_STAMP(6);
   tc_fence_before();
   __syncthreads();
@@ -482,44 +372,43 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   }
 }
 
-template <int BN, int MODE, int EPI, int SPLIT>
-__global__ void __launch_bounds__(chain_threads(BN), 1)
+template <int BN, int MODE, int EPI>
+__global__ void __launch_bounds__(kThreads, 1)
     tc_chain_kernel(const __grid_constant__ ChainParams p, int stages) {
-  chain_body<BN, MODE, EPI, SPLIT>(p, (int)blockIdx.x, stages);
+  chain_body<BN, MODE, EPI>(p, (int)blockIdx.x, stages);
 }
 // Several independent problems of one row block each (M <= 128): blockIdx.x selects the problem.  The cells of one
 // anti-diagonal of a stack (layer l at step t, layer l - 1 at step t + 1, ...) do not depend on one another.
 template <int BN, int MODE, int EPI>
-__global__ void __launch_bounds__(chain_threads(BN), 1)
+__global__ void __launch_bounds__(kThreads, 1)
     tc_chain_multi_kernel(const __grid_constant__ ChainBatch pb, int stages) {
-  chain_body<BN, MODE, EPI, 1>(pb.p[blockIdx.x], 0, stages);
+  chain_body<BN, MODE, EPI>(pb.p[blockIdx.x], 0, stages);
 }
 
 const bool g_pdl_on = std::getenv("ZRNN_NO_PDL") == nullptr;
 
-template <int BN, int MODE, int EPI, int SPLIT>
+template <int BN, int MODE, int EPI>
 cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   const ChainParams& p = b.p[0];
   constexpr int PARTS = mode_split(MODE) ? 2 : 1;
   const int stage = PARTS * p.kbs * (p.a_rows * 128 + BN * 128);
   // the MMA reads 128 rows of activations, the last stage's reads may run past a narrower box
-  const int slack = 1024 + std::max((128 - p.a_rows) * 128, chain_slot_bytes(BN, SPLIT));
+  const int slack = 1024 + (128 - p.a_rows) * 128;
   int stages = (kChainRingBytes - slack) / stage;
   stages = stages > kMaxStages ? kMaxStages : (stages < 2 ? 2 : stages);
   const int its = p.nsrc * ((p.kb + p.kbs - 1) / p.kbs);
-  if (its < SPLIT) return cudaErrorInvalidValue;
-  if (stages > (its + SPLIT - 1) / SPLIT) stages = (its + SPLIT - 1) / SPLIT;
+  if (stages > its) stages = its;
   // a whole number of stages per MMA warp: each waits on barriers of its own only.  (A barrier shared by two waiters would let
   // one that is a round ahead mistake "the round before last is complete" for its own round.)
-  if (!chain_by_product(BN, MODE)) stages = stages < kMmaWarps ? kMmaWarps : stages / kMmaWarps * kMmaWarps;
+  if (!mode_split(MODE)) stages = stages < kMmaWarps ? kMmaWarps : stages / kMmaWarps * kMmaWarps;
   const size_t smem = (size_t)stages * stage + slack;
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_chain_kernel<BN, MODE, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(tc_chain_kernel<BN, MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
     if (e != cudaSuccess) return e;
-    if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1) {
+    if constexpr (EPI == TC_EPI_LSTM) {
       e = cudaFuncSetAttribute(tc_chain_multi_kernel<BN, MODE, TC_EPI_LSTM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
       if (e != cudaSuccess) return e;
     }
@@ -528,85 +417,64 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   const int rows = EPI == TC_EPI_LSTM ? p.N * 4 : p.N;
-  cfg.gridDim = dim3(n > 1 ? n : (p.M + 127) / 128, (rows + BN - 1) / BN, SPLIT);
-  cfg.blockDim = dim3(chain_threads(BN));
+  cfg.gridDim = dim3(n > 1 ? n : (p.M + 127) / 128, (rows + BN - 1) / BN);
+  cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  int na = 0;
-  if (SPLIT > 1) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = 1;
-    attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = SPLIT;
-    ++na;
-  }
-  if (g_pdl_on) {
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = na;
+  cfg.numAttrs = g_pdl_on ? 1 : 0;
   count_launch();
-  if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1) {
+  if constexpr (EPI == TC_EPI_LSTM) {
     if (n > 1) return cudaLaunchKernelEx(&cfg, tc_chain_multi_kernel<BN, MODE, EPI>, b, stages);
   }
-  return cudaLaunchKernelEx(&cfg, tc_chain_kernel<BN, MODE, EPI, SPLIT>, p, stages);
+  return cudaLaunchKernelEx(&cfg, tc_chain_kernel<BN, MODE, EPI>, p, stages);
 }
 template <int MODE>
-cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, int split, cudaStream_t st) {
-  if (epi == TC_EPI_LSTM && split == 1) {
-    switch (BN) {
-      case 32: return launch_t<32, MODE, TC_EPI_LSTM, 1>(b, n, st);
-      case 64: return launch_t<64, MODE, TC_EPI_LSTM, 1>(b, n, st);
-      case 128: return launch_t<128, MODE, TC_EPI_LSTM, 1>(b, n, st);
-      case 256: return launch_t<256, MODE, TC_EPI_LSTM, 1>(b, n, st);
-    }
-  } else if (epi == TC_EPI_LSTM && split == 2 && n == 1) {
-    if (BN == 32) return launch_t<32, MODE, TC_EPI_LSTM, 2>(b, n, st);
-    if (BN == 64) return launch_t<64, MODE, TC_EPI_LSTM, 2>(b, n, st);
-  } else if (epi == TC_EPI_STORE && split == 1 && n == 1) {
-    switch (BN) {
-      case 16: return launch_t<16, MODE, TC_EPI_STORE, 1>(b, n, st);
-      case 32: return launch_t<32, MODE, TC_EPI_STORE, 1>(b, n, st);
-      case 64: return launch_t<64, MODE, TC_EPI_STORE, 1>(b, n, st);
-      case 128: return launch_t<128, MODE, TC_EPI_STORE, 1>(b, n, st);
-      case 256: return launch_t<256, MODE, TC_EPI_STORE, 1>(b, n, st);
-    }
-  } else if (epi == TC_EPI_STORE && split == 2 && n == 1) {
-    if (BN == 16) return launch_t<16, MODE, TC_EPI_STORE, 2>(b, n, st);
-    if (BN == 32) return launch_t<32, MODE, TC_EPI_STORE, 2>(b, n, st);
-  }
+cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_t st) {
+  if (epi == TC_EPI_LSTM && BN == 128) return launch_t<128, MODE, TC_EPI_LSTM>(b, n, st);
+  if (epi == TC_EPI_LSTM && BN == 256) return launch_t<256, MODE, TC_EPI_LSTM>(b, n, st);
+  if (epi == TC_EPI_STORE && n == 1 && BN == 128) return launch_t<128, MODE, TC_EPI_STORE>(b, n, st);
+  if (epi == TC_EPI_STORE && n == 1 && BN == 256) return launch_t<256, MODE, TC_EPI_STORE>(b, n, st);
   return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-// Which tile: a launch takes, per wave of CTAs, the longest of (a) the bytes a CTA fetches, at the 140 KB/us an SM takes in from
-// L2, (b) the MMAs, (c) the shared-memory traffic of both, 128 bytes per cycle; the K split adds its exchange, the epilogue
-// grows with the outputs per CTA.  Against measurements (us per launch, H = 1000, f32): cell at 128 columns, 32 rows per tile
-// 17.4, 64 rows and two halves of K 14.2; at 64 columns 13.2 and 12.3; bf16 at 64 columns 6.8 and 7.2 (there the split does not
-// pay); combiner of 1000 rows 12 and 8.
-ChainPlan plan_chain(int mode, int epi, int rows, int cells, int kb, int M) {
+// Which tile: a launch takes, per wave of CTAs, the longest of (a) the bytes a CTA fetches, at the 77 KB/us that an SM takes in from
+// L2 while all of them load, (b) the MMAs, (c) the shared-memory traffic of both, 128 bytes per cycle; then a fixed part, the
+// exchange of a K split and an epilogue that grows with the outputs per CTA.  Of a narrow tile's early sources half is counted: the
+// other half runs beside the predecessor.
+ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M) {
   const bool two = mode_split(mode);
   const int parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
   ChainPlan best{0, 1, 1e30f};
   for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 256; BN *= 2) {
     if (BN == 256 && (cells > 1 || mode == TC_TF32X3)) continue;  // (one accumulator over all of K: not for the most exact mode)
     for (int split = 1; split <= 2; ++split) {
-      if (split == 2 && (cells > 1 || BN > (epi == TC_EPI_LSTM ? 64 : 32) || kb < 8)) continue;
+      if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
       const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + 147) / 148;
       const float n_mma = BN <= 64 || !two ? 45.f : 64.f, cyc_n = BN <= 64 ? 48.f : BN / 2.f;
       const float mma = 4.f * (!two ? std::max(45.f, cyc_n) : (BN <= 64 ? std::max(45.f, (float)BN) + n_mma : 3.f * cyc_n));
       const float reads = 4.f * (!two ? 4096.f + 32.f * BN : (BN <= 64 ? 8192.f + 96.f * BN : 3.f * (4096.f + 32.f * BN)));
       const float writes = parts * 128.f * (a_rows + BN);
-      const float kb_us = std::max(writes / 140e3f, std::max(mma, (reads + writes) / 128.f) / 1900.f);
-      const float us = 3.2f + waves * (kb_us * kb / split + (two ? 0.01f : 0.005f) * BN) + (split == 2 ? 1.3f : 0.f);
+      const float kb_us = std::max(writes / 77e3f, std::max(mma, (reads + writes) / 128.f) / 1900.f);
+      const float kbs = kb * (nsrc - (BN <= 64 ? 0.5f * n_early : 0.f)) / split;
+      const float us = 3.2f + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : 0.f);
       if (us < best.us) best = ChainPlan{BN, split, us};
     }
   }
   return best;
+}
+
+int chain_kbs(int mode, int BN, int a_rows, int kb, int split) {
+  if (BN <= 64) return link_kbs(mode, BN, a_rows, kb, split);
+  const int parts = mode_split(mode) ? 2 : 1;
+  int k = 4;  // as many as leave the ring four stages
+  while (k > 1 && 4 * parts * k * (a_rows + BN) * 128 > kChainRingBytes - (128 - a_rows) * 128 - 1024) k /= 2;
+  return k;
 }
 
 cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st) {
@@ -615,14 +483,17 @@ cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int ep
     const ChainParams& p = b.p[i];
     if (p.M < 1 || (n > 1 && p.M > 128) || p.N != b.p[0].N || p.a_rows < 8 || p.a_rows > 128 || (p.a_rows & 7) ||
         p.a_rows != b.p[0].a_rows || (p.M > 128 && p.a_rows != 128) || p.a_rows < (p.M < 128 ? p.M : 128) || p.kb < 1 || p.nsrc < 1 ||
-        p.nsrc * p.kb != b.p[0].nsrc * b.p[0].kb || p.kbs != b.p[0].kbs || p.kbs != chain_kbs(mode, BN, p.a_rows))
+        p.nsrc * p.kb != b.p[0].nsrc * b.p[0].kb || p.kbs != b.p[0].kbs || p.kbs != chain_kbs(mode, BN, p.a_rows, p.kb, split) ||
+        p.n_early < 0 || p.n_early >= p.nsrc)
       return cudaErrorInvalidValue;
   }
+  if (BN <= 64) return launch_tc_link(b, n, BN, mode, epi, split, st);
+  if (split != 1) return cudaErrorInvalidValue;
   switch (mode) {
-    case TC_BF16: return launch_mode<TC_BF16>(b, n, BN, epi, split, st);
-    case TC_TF32: return launch_mode<TC_TF32>(b, n, BN, epi, split, st);
-    case TC_TF32X3: return launch_mode<TC_TF32X3>(b, n, BN, epi, split, st);
-    case TC_F16X2: return launch_mode<TC_F16X2>(b, n, BN, epi, split, st);
+    case TC_BF16: return launch_mode<TC_BF16>(b, n, BN, epi, st);
+    case TC_TF32: return launch_mode<TC_TF32>(b, n, BN, epi, st);
+    case TC_TF32X3: return launch_mode<TC_TF32X3>(b, n, BN, epi, st);
+    case TC_F16X2: return launch_mode<TC_F16X2>(b, n, BN, epi, st);
   }
   return cudaErrorInvalidValue;
 }

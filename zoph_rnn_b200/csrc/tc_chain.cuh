@@ -1,5 +1,6 @@
 // Tensor-core products on the chain between two time steps: LSTM cells, the attention layer's projections and the tanh
-// combiner.  One launch is one link of a chain of dependent launches, so what counts is its latency.  See tc_chain.cu.
+// combiner.  One launch is one link of a chain of dependent launches, so what counts is its latency.  See tc_link.cu (tiles of up
+// to 64 weight rows) and tc_chain.cu (wider ones).
 #pragma once
 #include "tc_gemm.cuh"
 
@@ -12,7 +13,8 @@ struct ChainParams {
                               // one part and one k-block per box)
   int w_kbtot, w_tiles;       // LSTM: k-blocks per packed tile, packed tiles
   int nsrc, kb;               // sources, k-blocks per source
-  int kbs;                    // k-blocks per box: chain_kbs(mode, BN, a_rows)
+  int n_early;                // leading sources that were complete when the predecessor kernel passed its own wait
+  int kbs;                    // k-blocks per box: chain_kbs
   int wkb0[3];                // first k-block of each source on the weights' K axis
   int a_row0[3];              // first row of each source's map that belongs to this problem
   int a_rows;                 // rows per activation box: a multiple of 8, at most 128
@@ -40,23 +42,19 @@ struct ChainBatch {
 };
 // n independent problems (same BN, mode, epilogue, N; M <= 128 each when n > 1) in one launch.
 // BN: 32, 64, 128, 256 for LSTM (256: tiles of two packed 128-row tiles); 16, 32, 64, 128, 256 for STORE.
-// split == 2 (n == 1; LSTM BN 32, 64; STORE BN 16, 32): two CTAs per tile, each over half of the K axis.
+// split == 2 (n == 1, BN <= 64): two CTAs per tile, each over half of the K axis.
 cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st);
-// k-blocks per ring stage: as many as leave the ring four stages
-constexpr int kChainRingBytes = 224 * 1024;
-inline int chain_kbs(int mode, int BN, int a_rows) {
-  const int parts = (mode == TC_TF32X3 || mode == TC_F16X2) ? 2 : 1;
-  int k = 4;
-  while (k > 1 && 4 * parts * k * (a_rows + BN) * 128 > kChainRingBytes - (128 - a_rows) * 128 - 1024) k /= 2;
-  return k;
-}
+cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st);
+// k-blocks per ring stage and TMA box: a TMA instruction costs its issuing thread about 200 cycles and a stage's hand-over 300
+int chain_kbs(int mode, int BN, int a_rows, int kb, int split);
+int link_kbs(int mode, int BN, int a_rows, int kb, int split);
 // Tile width and K split of a launch, and about how long it takes.
 struct ChainPlan {
   int BN, split;
   float us;
 };
-// rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks over all sources; M: columns
-ChainPlan plan_chain(int mode, int epi, int rows, int cells, int kb, int M);
+// rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks per source; M: columns
+ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M);
 
 // K-major rows as 4-D boxes (k within a 128-byte block, row, part, k-block): box_rows rows of all parts of box_kb k-blocks.
 // parts == 2: the lo rows lie part_bytes behind the hi rows.

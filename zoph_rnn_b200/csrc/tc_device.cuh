@@ -8,6 +8,7 @@
 
 #include <cstdint>
 
+#include "att_device.cuh"
 #include "tc_gemm.cuh"
 
 namespace zrnn {
@@ -300,17 +301,17 @@ __host__ __device__ constexpr int mode_epk(int mode) { return mode_kind_tf32(mod
 __host__ __device__ constexpr uint32_t mode_fmt(int mode) { return mode == TC_BF16 ? 1u : (mode == TC_F16X2 ? 0u : 2u); }
 __host__ __device__ constexpr float mode_cross_scale(int mode) { return mode == TC_F16X2 ? (1.0f / 2048.0f) : 1.0f; }
 
-// activations: exact for the fp32-accurate mode, hardware approximations (tanh.approx, ~2^-11) for bf16 / tf32
+// activations: fp32-accurate for the split modes, hardware approximations (tanh.approx, ~2^-11) for bf16 / tf32
 template <int MODE>
 __device__ __forceinline__ float act_tanh(float x) {
-  if (mode_exact_math(MODE)) return tanhf(x);
+  if (mode_exact_math(MODE)) return tanh_f32(x);
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 template <int MODE>
 __device__ __forceinline__ float act_sigmoid(float x) {
-  if (mode_exact_math(MODE)) return 1.0f / (1.0f + expf(-x));
+  if (mode_exact_math(MODE)) return sigmoid_f32(x);
   return fmaf(0.5f, act_tanh<MODE>(0.5f * x), 0.5f);
 }
 

@@ -409,11 +409,11 @@ struct LinkPlan {
   bool skinny;
   zrnn::ChainPlan chain;
 };
-LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int H, int cols, int n = 1) {
+LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int cols, int n = 1) {
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
-  p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc * ((H + epk - 1) / epk), cols);
-  p.skinny = skinny_engine(eng) && zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) < p.chain.us;
+  p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols);
+  p.skinny = skinny_engine(eng) && cols <= 64 && zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) < p.chain.us;
   return p;
 }
 // weights stored in packed 128-row tiles: tile-contiguous k-blocks (kbtot > 0) or plain rows of ld elements
@@ -426,20 +426,23 @@ void skinny_weights(zrnn::SkinnyParams& p, const OpMem& w, int kbtot, long long 
     p.w_tile_bytes = 128 * ld * 2; p.w_row_bytes = (int)(ld * 2); p.w_kb_bytes = 128;
   }
 }
-void skinny_source(zrnn::SkinnyParams& p, const Act& a, bool f32, int koff) {
-  p.a_hi[p.nsrc] = f32 ? (const void*)a.f32 : a.hi;
-  p.a_lo[p.nsrc] = f32 ? nullptr : a.lo;
+void skinny_source(zrnn::SkinnyParams& p, const Act& a, int koff) {
+  p.a_hi[p.nsrc] = a.hi;
+  p.a_lo[p.nsrc] = a.lo;
   p.a_kb0[p.nsrc] = koff / 64;
   ++p.nsrc;
 }
 void skinny_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
-                        int B, const Act& out, float* c_out, zrnn::SkinnyParams& p, bool f32 = false) {
+                        int B, const Act& out, float* c_out, int early, zrnn::SkinnyParams& p) {
   std::memset(&p, 0, sizeof(p));
   skinny_weights(p, L->Wcat, L->kbtot, (long long)(L->feed ? 3 : 2) * L->Kpad);
-  skinny_source(p, x, f32, 0);
-  skinny_source(p, hp, f32, L->Kpad);
-  if (q) skinny_source(p, *q, f32, 2 * L->Kpad);
-  p.lda = f32 ? L->H : L->Kpad;
+  const Act* src[3] = {&x, &hp, q};
+  for (int pass = 0; pass < 2; ++pass) {  // the early sources first
+    for (int i = 0; i < (q ? 3 : 2); ++i)
+      if ((early >> i & 1) == 1 - pass) skinny_source(p, *src[i], i * L->Kpad);
+    if (pass == 0) p.n_early = p.nsrc;
+  }
+  p.lda = L->Kpad;
   p.K = L->H; p.M = B; p.N = L->H; p.bias = L->b; p.mask = mask;
   p.C = out.f32; p.ldc = L->H; p.op_hi = out.hi; p.op_lo = out.lo; p.ld_op = L->Kpad;
   p.c_prev = c_prev; p.c_out = c_out;
@@ -471,15 +474,19 @@ int chain_source(zrnn::ChainParams& p, const Act& a, int eng, int H, int Kpad, i
   return ZRNN_OK;
 }
 int chain_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
-                      int B, const Act& out, float* c_out, int BN, zrnn::ChainParams& p) {
+                      int B, const Act& out, float* c_out, const zrnn::ChainPlan& plan, int early, zrnn::ChainParams& p) {
   const int H = L->H, Kpad = L->Kpad, eng = L->eng, epk = 128 / eng_eb(eng);
   std::memset(&p, 0, sizeof(p));
   p.a_rows = chain_a_rows(B);
   p.kb = (H + epk - 1) / epk;
-  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows);
-  ZR_TRY(chain_source(p, x, eng, H, Kpad, B, 0));
-  ZR_TRY(chain_source(p, hp, eng, H, Kpad, B, Kpad));
-  if (q) ZR_TRY(chain_source(p, *q, eng, H, Kpad, B, 2 * Kpad));
+  const int BN = plan.BN;
+  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows, p.kb, plan.split);
+  const Act* src[3] = {&x, &hp, q};
+  for (int pass = 0; pass < 2; ++pass) {  // the early sources first
+    for (int i = 0; i < (q ? 3 : 2); ++i)
+      if ((early >> i & 1) == 1 - pass) ZR_TRY(chain_source(p, *src[i], eng, H, Kpad, B, i * Kpad));
+    if (pass == 0) p.n_early = p.nsrc;
+  }
   p.w = L->gmap[BN == 32 ? 0 : (BN == 64 ? 1 : (BN == 128 ? 2 : 3))][p.kbs == 1 ? 0 : (p.kbs == 2 ? 1 : 2)];
   p.w_kbtot = L->kbtot; p.w_tiles = L->n_tiles;
   p.M = B; p.N = H; p.bias = L->b; p.mask = mask;
@@ -490,15 +497,18 @@ int chain_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act
   return ZRNN_OK;
 }
 // C = act(W [a0 | a1] + bias) with plain K-major weight rows
-int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act* a0, const Act* a1, int H, int Kpad, int B, int BN,
-                       zrnn::ChainParams& p) {
+int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act* a0, const Act* a1, int H, int Kpad, int B,
+                       const zrnn::ChainPlan& plan, bool a1_early, zrnn::ChainParams& p) {
   const int epk = 128 / eng_eb(eng);
   std::memset(&p, 0, sizeof(p));
   p.a_rows = chain_a_rows(B);
   p.kb = (H + epk - 1) / epk;
-  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows);
+  const int BN = plan.BN;
+  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows, p.kb, plan.split);
+  if (a1 && a1_early) ZR_TRY(chain_source(p, *a1, eng, H, Kpad, B, Kpad));
+  p.n_early = p.nsrc;
   ZR_TRY(chain_source(p, *a0, eng, H, Kpad, B, 0));
-  if (a1) ZR_TRY(chain_source(p, *a1, eng, H, Kpad, B, Kpad));
+  if (a1 && !a1_early) ZR_TRY(chain_source(p, *a1, eng, H, Kpad, B, Kpad));
   const long long rows = (N + 127) / 128 * 128;
   if (!zrnn::make_rows_map(&p.w, w.hi, eng_eb(eng), ldw * eng_eb(eng), rows, eng_split(eng) ? 2 : 1, w.part_bytes(),
                            (int)(ldw / epk), BN, p.kbs))
@@ -509,45 +519,50 @@ int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act*
 }
 
 // One LSTM cell.  x / h_prev / htild and the output are activations in the form the layer's engine needs.
+// early: inputs that were complete before the launch ahead of this one began its work: the kernels multiply by them while that
+// launch runs (every kernel on the chain lets its successor start only after its own wait)
+enum { EARLY_X = 1, EARLY_H = 2 };
 int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
-                 int B, const Act& out, float* c_out, cudaStream_t st) {
+                 int B, const Act& out, float* c_out, cudaStream_t st, int early = 0) {
   if (L->eng == ENG_SIMT)
     return lstm_cell_simt(L, x.f32, mask, hp.f32, c_prev, q ? q->f32 : nullptr, B, out.f32, c_out, st);
   const int H = L->H, eng = L->eng;
-  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, H, B);
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, (early & 1) + (early >> 1), H, B);
   KScope ks(KC_LSTM, st);
   if (plan.skinny) {
     zrnn::SkinnyBatch sb;
-    skinny_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, sb.p[0]);
-    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_LSTM, false, st));
+    skinny_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, early, sb.p[0]);
+    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_LSTM, st));
     return ZRNN_OK;
   }
   zrnn::ChainBatch cb;
-  ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain.BN, cb.p[0]));
+  ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain, early, cb.p[0]));
   ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, st));
   return ZRNN_OK;
 }
 // out = act(W [a0 | a1] + bias) * mask for plain K-major weight rows, act = tanh on the first act_rows rows (0: all)
 int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, const Act* a1, const float* bias, const int* mask,
-               int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st) {
+               int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st, bool a1_early = false) {
   const int nsrc = a1 ? 2 : 1;
-  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, H, B);
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, a1 && a1_early, H, B);
   if (plan.skinny) {
     zrnn::SkinnyBatch sb;
     zrnn::SkinnyParams& sp = sb.p[0];
     std::memset(&sp, 0, sizeof(sp));
     skinny_weights(sp, w, 0, (long long)nsrc * Kpad);
-    skinny_source(sp, *a0, false, 0);
-    if (a1) skinny_source(sp, *a1, false, Kpad);
+    if (a1 && a1_early) skinny_source(sp, *a1, Kpad);
+    sp.n_early = sp.nsrc;
+    skinny_source(sp, *a0, 0);
+    if (a1 && !a1_early) skinny_source(sp, *a1, Kpad);
     sp.lda = Kpad; sp.K = H; sp.M = B; sp.N = N; sp.bias = bias; sp.mask = mask; sp.act = 1; sp.act_rows = act_rows;
     sp.C = C; sp.ldc = ldc;
     if (op) { sp.op_hi = op->hi; sp.op_lo = op->lo; sp.ld_op = Kpad; }
-    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_STORE, false, st));
+    ZR_CUDA(zrnn::launch_skinny(sb, 1, skinny_mode(eng), zrnn::SK_EPI_STORE, st));
     return ZRNN_OK;
   }
   zrnn::ChainBatch cb;
   zrnn::ChainParams& p = cb.p[0];
-  ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain.BN, p));
+  ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain, a1_early, p));
   p.bias = bias; p.mask = mask; p.act = 1; p.act_rows = act_rows; p.C = C; p.ldc = ldc;
   if (op) chain_operand_outputs(p, eng, *op, Kpad);
   ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, plan.chain.split, st));
@@ -603,7 +618,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
     g.M = H; g.N = B; g.C = out.f32; g.ldc = H; g.bias[0] = A->bias; g.mask = mask; g.act = 1;
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, 0, st));
   } else {
-    ZR_TRY(link_store(eng, A->Wc_op, H, H, Kpad, &ctx, &h_t, A->bias, mask, 0, B, out.f32, H, &out, st));
+    ZR_TRY(link_store(eng, A->Wc_op, H, H, Kpad, &ctx, &h_t, A->bias, mask, 0, B, out.f32, H, &out, st, true));
   }
   return ZRNN_OK;
 }
@@ -1608,7 +1623,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
   }();
   const zrnn_lstm_layer* L0 = layers[0];
   if (!by_layers && L >= 2 && L <= zrnn::ChainBatch::MAX && L0->eng != ENG_SIMT && B <= 128) {
-    const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, g.H, B, L);
+    const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, 0, g.H, B, L);
     KScope sweep(KC_LSTM, s, S * L, true);
     zrnn::SkinnyBatch sb;
     for (int d = 0; d < S + L - 1; ++d) {
@@ -1619,13 +1634,13 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         const Act hp = t == 0 ? h0[l] : act_at(seq[l], (size_t)(t - 1) * B, g);
         const Act out = act_at(seq[l], (size_t)t * B, g);
         const int cu = cur[l];
-        if (plan.skinny) skinny_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], sb.p[n]);
+        if (plan.skinny) skinny_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], 0, sb.p[n]);
         else ZR_TRY(chain_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l],
-                                      plan.chain.BN, m->diag.p[n]));
+                                      plan.chain, 0, m->diag.p[n]));
         cur[l] = cu ^ 1;
         ++n;
       }
-      if (plan.skinny) ZR_CUDA(zrnn::launch_skinny(sb, n, skinny_mode(L0->eng), zrnn::SK_EPI_LSTM, false, s));
+      if (plan.skinny) ZR_CUDA(zrnn::launch_skinny(sb, n, skinny_mode(L0->eng), zrnn::SK_EPI_LSTM, s));
       else ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, s));
     }
     return ZRNN_OK;
@@ -1639,7 +1654,8 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
       const Act hp = t == 0 ? h0[l] : act_at(seq[l], (size_t)(t - 1) * B, g);
       const Act out = act_at(seq[l], (size_t)t * B, g);
       const int cu = cur[l];
-      ZR_TRY(cell_forward(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], s));
+      ZR_TRY(cell_forward(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], s,
+                          t > 0 || (l > 0 && S > 1) ? EARLY_X : 0));  // (the gather of X0 is the launch ahead of the first cell)
       cur[l] = cu ^ 1;
     }
   }
@@ -1886,7 +1902,9 @@ static int score_batch_body(zrnn_model* m, const int* d_src_ids, int S_max, cons
         const Act feed = act_at(hts, (size_t)(t > 0 ? t - 1 : 0) * B, g);
         const bool use_feed = (l == 0 && t > 0);
         const int cu = cur[l];
-        ZR_TRY(cell_forward(m->tgt[l], x, hp, use_feed ? &feed : nullptr, mk, cst[cu][l], B, out, cst[cu ^ 1][l], s));
+        // (the first cell reads what the launches just ahead of it left)
+        const int early = l > 0 ? EARLY_H : (t > 0 ? EARLY_X | EARLY_H : 0);
+        ZR_TRY(cell_forward(m->tgt[l], x, hp, use_feed ? &feed : nullptr, mk, cst[cu][l], B, out, cst[cu ^ 1][l], s, early));
         cur[l] = cu ^ 1;
         x = out;
       }
@@ -2189,7 +2207,8 @@ struct BeamModel {
     Act xin = x;
     for (int l = 0; l < c.num_layers; ++l) {
       const bool use_feed = (l == 0 && c.feed_input && t > 0);
-      ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], cols, hn[l], cn[l], s));
+      ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], cols, hn[l], cn[l], s,
+                          l > 0 ? EARLY_H : 0));  // (layer 0 reads what the reorder launch just wrote)
       xin = hn[l];
     }
     *top = xin;
@@ -2862,9 +2881,9 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
     zrnn::ChainParams& p = cb.p[0];
     std::memset(&p, 0, sizeof(p));
     p.nsrc = 1; p.kb = (K + kb_elems - 1) / kb_elems;
-    const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, p.kb, m_cols);
+    const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, 1, p.kb, 0, m_cols);
     p.a_rows = chain_a_rows(m_cols);
-    p.kbs = zrnn::chain_kbs(tcm, plan.BN, p.a_rows);
+    p.kbs = zrnn::chain_kbs(tcm, plan.BN, p.a_rows, p.kb, plan.split);
     const int kbs_total = Kpad / kb_elems;
     if (!zrnn::make_rows_map(&p.a[0], a_hi, eb, (long long)Kpad * eb, m_cols, parts, (long long)a_part, kbs_total, p.a_rows, p.kbs) ||
         !zrnn::make_rows_map(&p.w, b_hi, eb, (long long)Kpad * eb, (long long)n_tiles * 128, parts, (long long)b_part, kbs_total,
