@@ -98,3 +98,28 @@ def test_ragged_batch_equals_single_sentences(beam):
         np.testing.assert_array_equal(ids[i], i1[0])
         np.testing.assert_array_equal(al[i], a1[0])
         np.testing.assert_allclose(sc[i], s1[0], rtol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [5, 1, 4, 2])
+@pytest.mark.parametrize("H,V,N", [(64, 130, 1), (72, 257, 15), (200, 1000, 16), (504, 1281, 17), (1000, 40000, 12), (512, 20001, 63),
+                                   (1000, 5000, 65), (264, 19001, 128), (264, 19001, 129)])
+def test_vocabulary_projection_edges(dtype, H, V, N):
+    """Best words, their log-probabilities and the target's, on both sides of the column count where the kernel changes."""
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(H + V + N)
+    D = (rng.standard_normal((H, V)) * 2 / np.sqrt(H)).astype(np.float32)  # (column-major V x H)
+    b = (rng.standard_normal(V) * 0.1).astype(np.float32)
+    h = rng.uniform(-1, 1, (N, H)).astype(np.float32)
+    layer = api.softmax_layer(V, H, dtype=dtype)
+    layer.load_weights(D.reshape(-1), b)
+    z = h.astype(np.float64) @ D.astype(np.float64) + b
+    logp = z - (z.max(1, keepdims=True) + np.log(np.exp(z - z.max(1, keepdims=True)).sum(1, keepdims=True)))
+    dh, k = torch.as_tensor(h.reshape(-1)).cuda(), 5
+    r, a = {5: (1e-5, 2e-5), 4: (1e-5, 2e-5), 1: (2e-2, 4e-2), 2: (5e-3, 5e-3)}[dtype]
+    val, idx = (t.cpu().numpy().reshape(N, k) for t in layer.topk(dh, k)[:2])
+    np.testing.assert_allclose(val, np.take_along_axis(logp, idx.astype(np.int64), 1), rtol=r, atol=a)
+    np.testing.assert_allclose(val, -np.sort(-logp, axis=1)[:, :k], rtol=r, atol=a)
+    tgt = rng.integers(0, V, N).astype(np.int32)
+    got = layer.compute_loss(dh, torch.as_tensor(tgt).cuda(), torch.ones(N, dtype=torch.int32, device="cuda"))
+    np.testing.assert_allclose(got.cpu().numpy().reshape(-1), logp[np.arange(N), tgt], rtol=r, atol=a)

@@ -350,9 +350,21 @@ cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
   const int total = m_tiles * n_tiles;
   if (total == 0) return cudaSuccess;
   const int grid = total < sm_count() ? total : sm_count();
-  tc_gemm_persistent_kernel<BN, MODE, EPI><<<grid, 320, smem, st>>>(p, m_tiles, n_tiles);
+  // (it may be launched while its predecessor drains; its successor starts when it has finished)
+  static const bool pdl = std::getenv("ZRNN_NO_PDL") == nullptr;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(320);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
   count_launch();
-  return cudaGetLastError();
+  return cudaLaunchKernelEx(&cfg, tc_gemm_persistent_kernel<BN, MODE, EPI>, p, m_tiles, n_tiles);
 }
 
 }  // namespace

@@ -20,6 +20,7 @@
 #include "model_file.hpp"
 #include "skinny_gemm.cuh"
 #include "tc_chain.cuh"
+#include "tc_vocab.cuh"
 #include "tc_decoder.cuh"
 #include "tc_gemm.cuh"
 
@@ -623,6 +624,23 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   return ZRNN_OK;
 }
 
+// the part of a VocabParams that scoring and decoding share
+int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams& p) {
+  const int eng = S->eng, mode = eng_tcmode(eng), eb = eng_eb(eng), parts = eng_split(eng) ? 2 : 1;
+  const long long row_bytes = (long long)S->Kpad * eb;
+  std::memset(&p, 0, sizeof(p));
+  p.M = N; p.N = S->hi - S->lo; p.nb = zrnn::vocab_columns(N);
+  p.kb = (S->H + 128 / eb - 1) / (128 / eb); p.kbs = zrnn::vocab_kbs(mode);
+  if (!h.hi) return fail(ZRNN_E_STATE, "internal: activation has no operand-form copy");
+  if (!zrnn::make_rows_map(&p.w, S->D_op.hi, eb, row_bytes, (long long)S->n_tiles * S->BN, parts, S->D_op.part_bytes(), p.kb, 128, p.kbs) ||
+      !zrnn::make_rows_map(&p.h, h.hi, eb, row_bytes, N, parts, (char*)h.lo - (char*)h.hi, p.kb, p.nb, p.kbs))
+    return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for the vocabulary projection");
+  p.bias = S->b;
+  p.part_max = S->parts.as<float>(); p.part_sum = p.part_max + (size_t)np * N;
+  p.part_rows = S->BN / zrnn::kPersistentParts; p.n_parts = np;
+  p.err = tc_error_word();
+  return ZRNN_OK;
+}
 // per-column (max, sum exp) partials over this layer's rows + target logit into S->parts / tgt
 int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, int N, int* n_parts, float** pm,
                             float** ps, float* tgt, cudaStream_t st) {
@@ -648,6 +666,15 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   }
   const int eng = S->eng, np = S->n_tiles * zrnn::kPersistentParts;
   ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
+  if (N <= zrnn::kVocabMaxCols) {
+    zrnn::VocabParams vp;
+    ZR_TRY(vocab_params(S, h, N, np, vp));
+    vp.target = targets; vp.target_offset = S->lo; vp.tgt_logit = tgt;
+    *n_parts = np; *pm = vp.part_max; *ps = vp.part_sum;
+    KScope ks(KC_SOFTMAX_GEMM, st);
+    ZR_CUDA(zrnn::launch_tc_vocab(vp, eng_tcmode(eng), zrnn::TC_EPI_LSE, st));
+    return ZRNN_OK;
+  }
   zrnn::TcParams tp;
   std::memset(&tp, 0, sizeof(tp));
   ZR_TRY(act_maps(h, eng, H, S->Kpad, N, &tp.a[0], &tp.a_lo[0]));
@@ -691,6 +718,17 @@ int softmax_logits_act(zrnn_softmax* S, const Act& h, int N, cudaStream_t st, co
     g.M = Vs; g.N = N; g.C = S->logits.as<float>(); g.ldc = Vs; g.bias[0] = S->b;
     KScope ks(KC_SOFTMAX_GEMM, st);
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, (N >= 96 && Vs >= 512) ? 1 : 0, st));
+  } else if (N <= zrnn::kVocabMaxCols) {
+    np = S->n_tiles * zrnn::kPersistentParts;
+    ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
+    zrnn::VocabParams vp;
+    ZR_TRY(vocab_params(S, h, N, np, vp));
+    vp.C = S->logits.as<float>(); vp.ldc = Vs;
+    if (!ps_out) vp.part_sum = nullptr;
+    pm = vp.part_max;
+    if (ps_out) *ps_out = vp.part_sum;
+    KScope ks(KC_SOFTMAX_GEMM, st);
+    ZR_CUDA(zrnn::launch_tc_vocab(vp, eng_tcmode(S->eng), zrnn::TC_EPI_STORE, st));
   } else {
     const int eng = S->eng;
     np = S->n_tiles * zrnn::kPersistentParts;
@@ -1607,7 +1645,8 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
       a.h_seq = seq[l].f32;
       a.xp = m->seq_xp.as<float>();
       a.ld_op = g.Kpad;
-      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm;  // the decoder's cells and the attention read these rows as operands
+      // the decoder's cells, the attention and the vocabulary projection of few columns read whole k-blocks of these rows
+      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm || S * B <= zrnn::kVocabMaxCols;
       if (g.eng == ENG_BF16) a.op_b16 = seq[l].hi;
       else if (g.eng == ENG_H2) { a.op_h_hi = seq[l].hi; a.op_h_lo = seq[l].lo; }
       else if (g.eng != ENG_SIMT) { a.op_hi = (float*)seq[l].hi; a.op_lo = g.eng == ENG_X3 ? seq[l].lo : nullptr; }
