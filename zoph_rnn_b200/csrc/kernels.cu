@@ -85,6 +85,7 @@ cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cuda
 // The first launch of a scoring pass: the id preparation of up to three id arrays (-1 -> 0 and a 0/1 mask,
 // src/custom_kernels.h:9-50) and the zero fills of the start states, which were one graph node each.
 __global__ void __launch_bounds__(256) score_prologue_kernel(const PrologueArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the successor waits for this launch before it reads anything
   const size_t gtid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, gsz = (size_t)gridDim.x * blockDim.x;
   for (int q = 0; q < 3; ++q) {
     const int* raw = a.raw[q];
@@ -1199,26 +1200,28 @@ cudaError_t launch_att_global(const AttArgs& a, cudaStream_t st) {
 // resident-weight LSTM sequence kernel (small layers)
 // ------------------------------------------------------------------------------------------
 // Input-side products of ALL steps: xp[n][j] = (M_i, M_f, M_g, M_o)[:, j] . x_n for every column n = (step, sentence).
-// A CTA takes 8 columns at a time (their x vectors staged in shared memory) and 128 hidden units; its 256 threads are
-// two halves of the k range, each thread accumulating 4 gates x 8 columns, so that a weight value fetched from L2 is
-// used 8 times and the loads of ten k values are in flight together (one column per CTA and one load per FMA made this
-// launch as long as the whole recurrent loop it prepares).
+// A CTA takes 8 columns at a time (their x vectors staged in shared memory, two warps each) and 128 hidden units; its 512
+// threads are four parts of the k range, each thread accumulating 4 gates x 8 columns, so that a weight value fetched from L2 is
+// used 8 times and the loads of several k values are in flight together (one column per CTA and one load per FMA made this
+// launch as long as the whole recurrent loop it prepares; with the columns fetched one after the other, id then row, and two
+// parts of the k range it took 15 us at H = 100 and 280 columns).
 constexpr int kSeqXpartMaxH = 320;
-__global__ void __launch_bounds__(256) lstm_seq_xpart_kernel(const SeqArgs a) {
+__global__ void __launch_bounds__(512) lstm_seq_xpart_kernel(const SeqArgs a) {
   __shared__ __align__(16) float xs[kSeqXpartMaxH * 8];
-  __shared__ __align__(16) float red[32 * 128];
-  // the sequence kernel that follows may start now: its set-up (weights into registers or shared memory, barriers)
-  // needs nothing from this launch, and it waits (griddepcontrol.wait) before it reads the first product
+  __shared__ __align__(16) float red[2][16 * 128];
+  // the sequence kernel that follows may start once the launches before this one are complete: its set-up reads the start
+  // states, and it waits for this launch before it reads the first product
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int H = a.H, N = a.S * a.B;
-  const int tid = threadIdx.x, jt = tid & 127, half = tid >> 7;
+  const int tid = threadIdx.x, jt = tid & 127, part = tid >> 7;
   const int j = blockIdx.x * 128 + jt;
   const size_t HH = (size_t)H * H;
-  const int k_lo = half ? H / 2 : 0, k_hi = half ? H : H / 2;
+  const int k_lo = part * H / 4, k_hi = (part + 1) * H / 4;
   for (int n0 = blockIdx.y * 8; n0 < N; n0 += gridDim.y * 8) {
     __syncthreads();  // the previous group's xs and red are free
-    for (int c = 0; c < 8; ++c) {
-      const int n = n0 + c;
+    {
+      const int c = tid >> 6, n = n0 + c;
       const float* x = nullptr;
       if (n < N) {
         if (a.x_seq) {
@@ -1228,12 +1231,16 @@ __global__ void __launch_bounds__(256) lstm_seq_xpart_kernel(const SeqArgs a) {
           if (id < 0) id = 0;
           if (a.V > 0 && id >= a.V) {
             id = 0;
-            if (a.err && tid == 0 && blockIdx.x == 0) atomicExch(a.err, kErrBadTokenId);
+            if (a.err && (tid & 63) == 0 && blockIdx.x == 0) atomicExch(a.err, kErrBadTokenId);
           }
           x = a.emb + (size_t)id * H;
         }
       }
-      for (int k = tid; k < H; k += 256) xs[k * 8 + c] = x ? __ldg(x + k) : 0.f;
+#pragma unroll
+      for (int i = 0; i < (kSeqXpartMaxH + 63) / 64; ++i) {
+        const int k = (tid & 63) + 64 * i;
+        if (k < H) xs[k * 8 + c] = x ? __ldg(x + k) : 0.f;
+      }
     }
     __syncthreads();
     float acc[4][8];
@@ -1242,7 +1249,7 @@ __global__ void __launch_bounds__(256) lstm_seq_xpart_kernel(const SeqArgs a) {
 #pragma unroll
       for (int c = 0; c < 8; ++c) acc[g][c] = 0.f;
     if (j < H) {
-#pragma unroll 10
+#pragma unroll 8
       for (int k = k_lo; k < k_hi; ++k) {
         const size_t at = (size_t)k * H + j;
         const float w0 = __ldg(a.Mx + at), w1 = __ldg(a.Mx + HH + at), w2 = __ldg(a.Mx + 2 * HH + at), w3 = __ldg(a.Mx + 3 * HH + at);
@@ -1257,21 +1264,29 @@ __global__ void __launch_bounds__(256) lstm_seq_xpart_kernel(const SeqArgs a) {
         }
       }
     }
-    if (half == 1) {
+    // parts 2, 3 -> 0, 1 and then 1 -> 0, two gates at a time (shared memory)
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
+    for (int step = 0; step < 2; ++step)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) red[(g * 8 + c) * 128 + jt] = acc[g][c];
-    }
-    __syncthreads();
-    if (half == 0 && j < H) {
+      for (int gp = 0; gp < 2; ++gp) {
+        const bool give = step == 0 ? part >= 2 : part == 1, take = step == 0 ? part < 2 : part == 0;
+        float* r = red[step == 0 ? part & 1 : 0];
+        if (give) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x) r[x * 128 + jt] = acc[gp * 2 + (x >> 3)][x & 7];
+        }
+        __syncthreads();
+        if (take) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x) acc[gp * 2 + (x >> 3)][x & 7] += r[x * 128 + jt];
+        }
+        __syncthreads();
+      }
+    if (part == 0 && j < H) {
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
         const int n = n0 + c;
-        if (n < N)
-          reinterpret_cast<float4*>(a.xp)[(size_t)n * H + j] =
-              make_float4(acc[0][c] + red[(0 * 8 + c) * 128 + jt], acc[1][c] + red[(1 * 8 + c) * 128 + jt],
-                          acc[2][c] + red[(2 * 8 + c) * 128 + jt], acc[3][c] + red[(3 * 8 + c) * 128 + jt]);
+        if (n < N) reinterpret_cast<float4*>(a.xp)[(size_t)n * H + j] = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
       }
     }
   }
@@ -1731,9 +1746,8 @@ cudaError_t launch_lstm_seq_resident(const SeqArgs& a, cudaStream_t st) {
   const int N = a.S * a.B, groups = (N + 7) / 8;
   if (a.H > kSeqXpartMaxH) return cudaErrorInvalidValue;
   dim3 grid((a.H + 127) / 128, groups > 1024 ? 1024 : groups);
-  lstm_seq_xpart_kernel<<<grid, 256, 0, st>>>(a);
   count_launch();
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chain(lstm_seq_xpart_kernel, grid, dim3(512), 0, st, a);
   if (e != cudaSuccess) return e;
   if (seq_reg_fits(a.H, a.B)) {
     // a cluster of 16 CTAs (non-portable size) where the device schedules one, else 8: half the warps per SM

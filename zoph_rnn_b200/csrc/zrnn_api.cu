@@ -345,13 +345,15 @@ void prof_attach(P& tp) {
   }
 }
 
-int* tc_error_word() {  // one word per device
+// One word per device, in page-locked host memory that the device can write: after a synchronised pass the host reads it
+// without a copy (a blocking 4-byte copy took 8 of the 127 us of the smallest scoring call).
+int* tc_error_word() {
   static int* p[64] = {nullptr};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!p[dev]) {
-    if (cudaMalloc((void**)&p[dev], sizeof(int)) != cudaSuccess) return nullptr;
-    cudaMemset(p[dev], 0, sizeof(int));
+    if (cudaHostAlloc((void**)&p[dev], sizeof(int), cudaHostAllocMapped) != cudaSuccess) return nullptr;
+    *p[dev] = 0;
   }
   return p[dev];
 }
@@ -642,10 +644,11 @@ int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams
   return ZRNN_OK;
 }
 // per-column (max, sum exp) partials over this layer's rows + target logit into S->parts / tgt
+// tgt_zeroed: the caller's first launch has zeroed tgt
 int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, int N, int* n_parts, float** pm,
-                            float** ps, float* tgt, cudaStream_t st) {
+                            float** ps, float* tgt, cudaStream_t st, bool tgt_zeroed = false) {
   const int Vs = S->hi - S->lo, H = S->H;
-  ZR_CUDA(cudaMemsetAsync(tgt, 0, sizeof(float) * (size_t)N, st));
+  if (!tgt_zeroed) ZR_CUDA(cudaMemsetAsync(tgt, 0, sizeof(float) * (size_t)N, st));
   if (S->eng == ENG_SIMT) {
     const int tile = (N >= 96 && Vs >= 512) ? 1 : 0;
     const int rows = zrnn::gemm_rows_per_tile(1, tile);
@@ -692,11 +695,11 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
 }
 
 int softmax_score_act(zrnn_softmax* S, const Act& h, const int* targets, const int* mask, int N, float* logp,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool tgt_zeroed = false) {
   ZR_CUDA(S->tgt.reserve(sizeof(float) * (size_t)N));
   int np = 0;
   float *pm, *ps;
-  ZR_TRY(softmax_partials_launch(S, h, targets, N, &np, &pm, &ps, S->tgt.as<float>(), st));
+  ZR_TRY(softmax_partials_launch(S, h, targets, N, &np, &pm, &ps, S->tgt.as<float>(), st, tgt_zeroed));
   KScope ks(KC_SOFTMAX_REDUCE, st);
   ZR_CUDA(zrnn::launch_lse_combine(pm, ps, S->tgt.as<float>(), np, N, mask, logp, st));
   return ZRNN_OK;
@@ -801,6 +804,24 @@ struct TensorSlot {
   int index;  // position in the owner's load list
 };
 
+// Page-locked host memory that kernels read and write in place (ids going in, results coming out)
+struct PinBuf {
+  void* p = nullptr;
+  size_t cap = 0;
+  cudaError_t reserve(size_t bytes) {
+    if (bytes <= cap) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaHostAlloc(&p, bytes, cudaHostAllocMapped);
+    if (e == cudaSuccess) cap = bytes;
+    return e;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
+
 struct zrnn_model {
   zrnn_model_config cfg;
   int eng = ENG_SIMT;
@@ -814,6 +835,7 @@ struct zrnn_model {
   bool finalized = false;
   cudaStream_t stream = nullptr;
   DevBuf ws, io;
+  PinBuf pin;               // ids and log-probabilities of the host-buffer entry points
   DevBuf dec_counter;       // phase counter of the persistent decoder kernel
   DevBuf seq_xp;            // input half of the pre-activations for the resident-weight sequence kernel
   int persist_state = 0;    // 0 untried, 1 works, -1 refused by the runtime (the per-launch path is used)
@@ -844,7 +866,7 @@ struct zrnn_model {
     for (auto* l : tgt) delete l;
     delete att;
     delete sm;
-    ws.release(); io.release(); dec_counter.release(); seq_xp.release();
+    ws.release(); io.release(); pin.release(); dec_counter.release(); seq_xp.release();
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -860,9 +882,17 @@ int check_ids(const int* ids, size_t n, int V, const char* what) {
                                   std::to_string(i) + " is outside the vocabulary of " + std::to_string(V) + " words");
   return ZRNN_OK;
 }
-// Reads and clears the device error word after a synchronised pass and turns it into a status.
+// Reads and clears the device error word after a synchronised pass (launches on the default stream report there, too) ...
+int take_error_code() {
+  volatile int* w = tc_error_word();
+  if (!w || cudaStreamSynchronize(nullptr) != cudaSuccess) return -1;
+  const int v = *w;
+  if (v) *w = 0;
+  return v;
+}
+// ... and turns it into a status.
 int device_error_status(const char* what) {
-  const int code = zrnn_tc_error();
+  const int code = take_error_code();
   if (code == 0) return ZRNN_OK;
   if (code == zrnn::kErrBadTokenId)
     return fail(ZRNN_E_ARG, std::string(what) + ": a token id on the device is outside the vocabulary (column 0 was read instead)");
@@ -931,12 +961,7 @@ int zrnn_debug_bounded_wait(long long limit_cycles, void* stream) {
 }
 
 int zrnn_tc_error(void) {
-  int* d = tc_error_word();
-  int v = 0;
-  if (!d) return -1;
-  if (cudaMemcpy(&v, d, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-  if (v) cudaMemset(d, 0, sizeof(int));
-  return v;
+  return take_error_code();
 }
 
 int zrnn_kernel_timing(int on) {
@@ -1909,6 +1934,10 @@ static int score_batch_body(zrnn_model* m, const int* d_src_ids, int S_max, cons
     zero_fill(zero.hi, (size_t)B * g.Kpad * eng_eb(g.eng));
     zero_fill(zero.lo, (size_t)B * g.Kpad * eng_eb(g.eng));
     for (int l = 0; l < L; ++l) zero_fill(cst[0][l], sizeof(float) * HB);
+    if (d_logp_out) {
+      ZR_CUDA(m->sm->tgt.reserve(sizeof(float) * nT));
+      zero_fill(m->sm->tgt.p, sizeof(float) * nT);
+    }
     ZR_CUDA(zrnn::launch_score_prologue(pa, s));
   }
   if (!c.lm) {
@@ -1955,7 +1984,7 @@ static int score_batch_body(zrnn_model* m, const int* d_src_ids, int S_max, cons
   m->last_top_act = top;
   m->last_top_cols = (int)nT;
   if (!d_logp_out) return ZRNN_OK;
-  return softmax_score_act(m->sm, top, tout_id, tout_mk, (int)nT, d_logp_out, s);
+  return softmax_score_act(m->sm, top, tout_id, tout_mk, (int)nT, d_logp_out, s, true);
 }
 
 int zrnn_forward_states_device(zrnn_model* m, const int* d_src_ids, int S_max, const int* d_tgt_in, int T, int B,
@@ -1984,19 +2013,22 @@ int zrnn_score_batch(zrnn_model* m, const int* src_ids, int S_max, const int* tg
   if (nS) ZR_TRY(check_ids(src_ids, nS, m->cfg.V_src, "score_batch (source)"));
   ZR_TRY(check_ids(tgt_in, nT, m->cfg.V_tgt, "score_batch (target input)"));
   ZR_TRY(check_ids(tgt_out, nT, m->cfg.V_tgt, "score_batch (target output)"));
-  ZR_CUDA(m->io.reserve(aligned(sizeof(int) * (nS + 1)) + 2 * aligned(sizeof(int) * nT) + aligned(sizeof(float) * nT)));
-  Carver cv(m->io.p);
-  int* d_src = cv.take<int>(nS + 1);
-  int* d_tin = cv.take<int>(nT);
-  int* d_tout = cv.take<int>(nT);
-  float* d_lp = cv.take<float>(nT);
+  // The first kernel reads the ids, and the last one writes the log-probabilities, straight from and to page-locked memory: a
+  // few KB over the bus inside launches that run anyway, instead of three copies in and two out, each several us of latency.
+  const size_t need = aligned(sizeof(int) * (nS + 1)) + 2 * aligned(sizeof(int) * nT) + aligned(sizeof(float) * nT);
+  ZR_CUDA(m->pin.reserve(need));
+  Carver cv(m->pin.p);
+  int* h_src = cv.take<int>(nS + 1);
+  int* h_tin = cv.take<int>(nT);
+  int* h_tout = cv.take<int>(nT);
+  float* h_lp = cv.take<float>(nT);
+  if (nS) std::memcpy(h_src, src_ids, sizeof(int) * nS);
+  std::memcpy(h_tin, tgt_in, sizeof(int) * nT);
+  std::memcpy(h_tout, tgt_out, sizeof(int) * nT);
   cudaStream_t s = m->stream;
-  if (nS) ZR_CUDA(cudaMemcpyAsync(d_src, src_ids, sizeof(int) * nS, cudaMemcpyHostToDevice, s));
-  ZR_CUDA(cudaMemcpyAsync(d_tin, tgt_in, sizeof(int) * nT, cudaMemcpyHostToDevice, s));
-  ZR_CUDA(cudaMemcpyAsync(d_tout, tgt_out, sizeof(int) * nT, cudaMemcpyHostToDevice, s));
-  ZR_TRY(zrnn_score_batch_device(m, nS ? d_src : nullptr, S_max, d_tin, d_tout, T, B, d_lp, s));
-  ZR_CUDA(cudaMemcpyAsync(logp_out, d_lp, sizeof(float) * nT, cudaMemcpyDeviceToHost, s));
+  ZR_TRY(zrnn_score_batch_device(m, nS ? h_src : nullptr, S_max, h_tin, h_tout, T, B, h_lp, s));
   ZR_CUDA(cudaStreamSynchronize(s));
+  std::memcpy(logp_out, h_lp, sizeof(float) * nT);
   ZR_TRY(device_error_status("score_batch"));
   if (total_logp) {
     double tot = 0;
@@ -2471,32 +2503,31 @@ static int beam_decode_host(zrnn_model* m, zrnn_comm* comm, const int* src_ids, 
   }
   ZR_TRY(check_ids(src_ids, n_ids, m->cfg.V_src, "beam_decode (source)"));
   const int Lmax = longest_sent + 4;
-  // pad on the host into the reference's minibatch layout: time-major, left-padded with -1
-  std::vector<int> padded((size_t)S_max * n_sent, -1);
+  const size_t nO = (size_t)n_sent * k_best, n_pad = (size_t)S_max * n_sent;
+  // device results in one block, so that one copy brings them back
+  const size_t o_len = nO * Lmax * (out_align ? 2 : 1), o_sc = o_len + nO, n_out = o_sc + nO;
+  ZR_CUDA(m->pin.reserve(aligned(sizeof(int) * n_pad) + sizeof(int) * n_out));
+  // pad into the reference's minibatch layout: time-major, left-padded with -1 (page-locked: the first kernel reads it there)
+  int* padded = (int*)m->pin.p;
+  std::fill(padded, padded + n_pad, -1);
   size_t pos = 0;
   for (int i = 0; i < n_sent; ++i) {
     for (int t = 0; t < src_len[i]; ++t) padded[(size_t)(S_max - src_len[i] + t) * n_sent + i] = src_ids[pos + t];
     pos += src_len[i];
   }
-  const size_t nO = (size_t)n_sent * k_best;
-  ZR_CUDA(m->io.reserve(aligned(sizeof(int) * padded.size()) + 2 * aligned(sizeof(int) * nO * Lmax) +
-                        aligned(sizeof(int) * nO) + aligned(sizeof(float) * nO)));
-  Carver cv(m->io.p);
-  int* d_src = cv.take<int>(padded.size());
-  int* d_ids = cv.take<int>(nO * Lmax);
-  int* d_len = cv.take<int>(nO);
-  float* d_sc = cv.take<float>(nO);
-  int* d_al = out_align ? cv.take<int>(nO * Lmax) : nullptr;
+  ZR_CUDA(m->io.reserve(sizeof(int) * n_out));
+  int* d_ids = m->io.as<int>();
+  int* h_ids = (int*)((char*)m->pin.p + aligned(sizeof(int) * n_pad));
   cudaStream_t s = m->stream;
-  ZR_CUDA(cudaMemcpyAsync(d_src, padded.data(), sizeof(int) * padded.size(), cudaMemcpyHostToDevice, s));
-  const int* d_src_c = d_src;
-  ZR_TRY(beam_decode_core(&m, 1, &d_src_c, src_len, &S_max, n_sent, beam, k_best, min_ratio, max_ratio, penalty,
-                          longest_sent, d_ids, d_len, d_sc, d_al, s, comm));
-  if (out_align) ZR_CUDA(cudaMemcpyAsync(out_align, d_al, sizeof(int) * nO * Lmax, cudaMemcpyDeviceToHost, s));
-  ZR_CUDA(cudaMemcpyAsync(out_ids, d_ids, sizeof(int) * nO * Lmax, cudaMemcpyDeviceToHost, s));
-  ZR_CUDA(cudaMemcpyAsync(out_len, d_len, sizeof(int) * nO, cudaMemcpyDeviceToHost, s));
-  ZR_CUDA(cudaMemcpyAsync(out_score, d_sc, sizeof(float) * nO, cudaMemcpyDeviceToHost, s));
+  const int* src_c = padded;
+  ZR_TRY(beam_decode_core(&m, 1, &src_c, src_len, &S_max, n_sent, beam, k_best, min_ratio, max_ratio, penalty,
+                          longest_sent, d_ids, d_ids + o_len, (float*)(d_ids + o_sc), out_align ? d_ids + nO * Lmax : nullptr, s, comm));
+  ZR_CUDA(cudaMemcpyAsync(h_ids, d_ids, sizeof(int) * n_out, cudaMemcpyDeviceToHost, s));
   ZR_CUDA(cudaStreamSynchronize(s));
+  std::memcpy(out_ids, h_ids, sizeof(int) * nO * Lmax);
+  if (out_align) std::memcpy(out_align, h_ids + nO * Lmax, sizeof(int) * nO * Lmax);
+  std::memcpy(out_len, h_ids + o_len, sizeof(int) * nO);
+  std::memcpy(out_score, h_ids + o_sc, sizeof(float) * nO);
   ZR_TRY(device_error_status("beam_decode"));
   return ZRNN_OK;
 }
