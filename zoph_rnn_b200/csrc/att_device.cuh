@@ -283,6 +283,86 @@ __device__ __forceinline__ void att_local_fast_body(const AttArgs& a, const int 
   }
 }
 
+// A masked column: zero context, zero weights.
+__device__ __forceinline__ void att_global_masked(const AttArgs& a, const int b, const int tid) {
+  float* c = a.c_t + (size_t)b * a.H;
+  for (int i = tid; i < a.H; i += kAttTeam) { c[i] = 0.f; att_store_op(a, b, i, 0.f); }
+  if (a.align_out)
+    for (int s = tid; s < a.S_max; s += kAttTeam) a.align_out[(size_t)s * a.B + b] = 0.f;
+  if (a.viterbi_out && tid == 0) a.viterbi_out[b] = -1;
+}
+// One source position into a warp's running (max m, sum l, context, best position): score sc, the lane's pieces rv of its vector.
+__device__ __forceinline__ void att_global_take(const AttArgs& a, const int b, const int lane, const int pos, const float sc,
+                                                const float4* rv, float& m, float& l, float& bsc, int& bpos, float4* ctx) {
+  if (a.align_out && lane == 0) a.align_out[(size_t)pos * a.B + b] = sc;  // raw score, normalised at the end
+  if (sc > bsc) { bsc = sc; bpos = pos; }
+  const float mn = fmaxf(m, sc);
+  const float scale = expf(m - mn), e = expf(sc - mn);
+  l = l * scale + e;
+  m = mn;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    ctx[i].x = ctx[i].x * scale + e * rv[i].x;
+    ctx[i].y = ctx[i].y * scale + e * rv[i].y;
+    ctx[i].z = ctx[i].z * scale + e * rv[i].z;
+    ctx[i].w = ctx[i].w * scale + e * rv[i].w;
+  }
+}
+// The eight warps' partial results -> context, weights, best position.
+template <class Sync>
+__device__ __forceinline__ void att_global_merge(const AttArgs& a, const int b, const int tid, const int len, unsigned char* scratch,
+                                                 const float m, const float l, const float bsc, const int bpos, const float4* ctx,
+                                                 Sync sync) {
+  float4(*s_ctx)[256] = reinterpret_cast<float4(*)[256]>(scratch);
+  float* s_m = reinterpret_cast<float*>(scratch + 8 * 256 * 16);
+  float* s_l = s_m + 8;
+  float* s_bsc = s_l + 8;
+  int* s_bpos = reinterpret_cast<int*>(s_bsc + 8);
+  const int lane = tid & 31, w = tid >> 5, H4 = a.H >> 2;
+  if (lane == 0) { s_m[w] = m; s_l[w] = l; s_bsc[w] = bsc; s_bpos[w] = bpos; }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s_ctx[w][lane + 32 * i] = ctx[i];
+  sync();
+  if (a.viterbi_out && tid == 0) {  // largest score = largest weight; the lowest position wins a tie
+    float best = -INFINITY;
+    int best_pos = -1;
+    for (int q = 0; q < 8; ++q)
+      if (s_bpos[q] >= 0 && (s_bsc[q] > best || (s_bsc[q] == best && s_bpos[q] < best_pos))) { best = s_bsc[q]; best_pos = s_bpos[q]; }
+    a.viterbi_out[b] = best_pos;
+  }
+  float M = -INFINITY;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) M = fmaxf(M, s_m[q]);
+  float Lsum = 0.f, wq[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    wq[q] = (s_m[q] == -INFINITY) ? 0.f : expf(s_m[q] - M);
+    Lsum += s_l[q] * wq[q];
+  }
+  const float inv = 1.0f / Lsum;
+  if (tid < H4) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 v = s_ctx[q][tid];
+      acc.x += wq[q] * v.x; acc.y += wq[q] * v.y; acc.z += wq[q] * v.z; acc.w += wq[q] * v.w;
+    }
+    acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
+    reinterpret_cast<float4*>(a.c_t + (size_t)b * a.H)[tid] = acc;
+    att_store_op(a, b, 4 * tid + 0, acc.x);
+    att_store_op(a, b, 4 * tid + 1, acc.y);
+    att_store_op(a, b, 4 * tid + 2, acc.z);
+    att_store_op(a, b, 4 * tid + 3, acc.w);
+  }
+  if (a.align_out) {
+    sync();
+    for (int pos = tid; pos < a.S_max; pos += kAttTeam) {
+      const size_t idx = (size_t)pos * a.B + b;
+      a.align_out[idx] = pos < len ? expf(a.align_out[idx] - M) * inv : 0.f;
+    }
+  }
+}
+
 // Global dot-product attention of target column b in a single pass: each of the team's 8 warps walks over every 8th
 // source position, keeps the position's vector in registers for both the score and the context (so the source memory
 // is read once, with 16-byte loads), and carries a running (max, sum, context); the 8 partial results are merged through
@@ -290,22 +370,10 @@ __device__ __forceinline__ void att_local_fast_body(const AttArgs& a, const int 
 template <class Sync>
 __device__ __forceinline__ void att_global_fast_body(const AttArgs& a, const int b, const int tid, unsigned char* scratch,
                                                      Sync sync) {
-  float4(*s_ctx)[256] = reinterpret_cast<float4(*)[256]>(scratch);
-  float* s_m = reinterpret_cast<float*>(scratch + 8 * 256 * 16);
-  float* s_l = s_m + 8;
-  float* s_bsc = s_l + 8;
-  int* s_bpos = reinterpret_cast<int*>(s_bsc + 8);
   const int lane = tid & 31, w = tid >> 5;
   const int H = a.H, H4 = H >> 2, sb = b / a.cols_per_sent;
-  float* c = a.c_t + (size_t)b * H;
   att_zero_pad(a, b, tid, kAttTeam);
-  if (a.mask && a.mask[b] != 1) {
-    for (int i = tid; i < H; i += kAttTeam) { c[i] = 0.f; att_store_op(a, b, i, 0.f); }
-    if (a.align_out)
-      for (int s = tid; s < a.S_max; s += kAttTeam) a.align_out[(size_t)s * a.B + b] = 0.f;
-    if (a.viterbi_out && tid == 0) a.viterbi_out[b] = -1;
-    return;
-  }
+  if (a.mask && a.mask[b] != 1) return att_global_masked(a, b, tid);
   const int len = a.len[sb], off = a.offset[sb];
   const float4* h4 = reinterpret_cast<const float4*>(a.h_t + (size_t)b * H);
   float4 hv[8], ctx[8];
@@ -339,79 +407,10 @@ __device__ __forceinline__ void att_global_fast_body(const AttArgs& a, const int
     }
     sc = warp_sum(sc);
     sc2 = warp_sum(sc2);
-    {
-      if (a.align_out && lane == 0) a.align_out[(size_t)pos * a.B + b] = sc;  // raw score, normalised below
-      if (sc > bsc) { bsc = sc; bpos = pos; }
-      const float mn = fmaxf(m, sc);
-      const float scale = expf(m - mn), e = expf(sc - mn);
-      l = l * scale + e;
-      m = mn;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        ctx[i].x = ctx[i].x * scale + e * rv[i].x;
-        ctx[i].y = ctx[i].y * scale + e * rv[i].y;
-        ctx[i].z = ctx[i].z * scale + e * rv[i].z;
-        ctx[i].w = ctx[i].w * scale + e * rv[i].w;
-      }
-    }
-    if (two) {
-      if (a.align_out && lane == 0) a.align_out[(size_t)pos2 * a.B + b] = sc2;
-      if (sc2 > bsc) { bsc = sc2; bpos = pos2; }
-      const float mn = fmaxf(m, sc2);
-      const float scale = expf(m - mn), e = expf(sc2 - mn);
-      l = l * scale + e;
-      m = mn;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        ctx[i].x = ctx[i].x * scale + e * sv[i].x;
-        ctx[i].y = ctx[i].y * scale + e * sv[i].y;
-        ctx[i].z = ctx[i].z * scale + e * sv[i].z;
-        ctx[i].w = ctx[i].w * scale + e * sv[i].w;
-      }
-    }
+    att_global_take(a, b, lane, pos, sc, rv, m, l, bsc, bpos, ctx);
+    if (two) att_global_take(a, b, lane, pos2, sc2, sv, m, l, bsc, bpos, ctx);
   }
-  if (lane == 0) { s_m[w] = m; s_l[w] = l; s_bsc[w] = bsc; s_bpos[w] = bpos; }
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s_ctx[w][lane + 32 * i] = ctx[i];
-  sync();
-  if (a.viterbi_out && tid == 0) {  // largest score = largest weight; the lowest position wins a tie
-    float best = -INFINITY;
-    int best_pos = -1;
-    for (int q = 0; q < 8; ++q)
-      if (s_bpos[q] >= 0 && (s_bsc[q] > best || (s_bsc[q] == best && s_bpos[q] < best_pos))) { best = s_bsc[q]; best_pos = s_bpos[q]; }
-    a.viterbi_out[b] = best_pos;
-  }
-  float M = -INFINITY;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) M = fmaxf(M, s_m[q]);
-  float Lsum = 0.f, wq[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    wq[q] = (s_m[q] == -INFINITY) ? 0.f : expf(s_m[q] - M);
-    Lsum += s_l[q] * wq[q];
-  }
-  const float inv = 1.0f / Lsum;
-  if (tid < H4) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float4 v = s_ctx[q][tid];
-      acc.x += wq[q] * v.x; acc.y += wq[q] * v.y; acc.z += wq[q] * v.z; acc.w += wq[q] * v.w;
-    }
-    acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
-    reinterpret_cast<float4*>(c)[tid] = acc;
-    att_store_op(a, b, 4 * tid + 0, acc.x);
-    att_store_op(a, b, 4 * tid + 1, acc.y);
-    att_store_op(a, b, 4 * tid + 2, acc.z);
-    att_store_op(a, b, 4 * tid + 3, acc.w);
-  }
-  if (a.align_out) {
-    sync();
-    for (int pos = tid; pos < a.S_max; pos += kAttTeam) {
-      const size_t idx = (size_t)pos * a.B + b;
-      a.align_out[idx] = pos < len ? expf(a.align_out[idx] - M) * inv : 0.f;
-    }
-  }
+  att_global_merge(a, b, tid, len, scratch, m, l, bsc, bpos, ctx, sync);
 }
 
 }  // namespace zrnn

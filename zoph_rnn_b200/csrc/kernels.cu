@@ -1178,17 +1178,81 @@ __global__ void __launch_bounds__(256) att_global_kernel(const AttArgs a) {
     att_store_op(a, b, i, acc);
   }
 }
-// att_global_fast_body (att_device.cuh): single pass for H % 4 == 0, H <= 1024, one CTA of 256 threads per column.
-__global__ void __launch_bounds__(256) att_global_fast_kernel(const AttArgs a) {
-  pdl_enter();
+// Single pass for H % 4 == 0, H <= 1024, one CTA of 8 warps per column: warp w walks over the positions w, w + 8, ... and streams
+// their vectors through a ring of its own in shared memory, every lane the 16-byte pieces that it will read itself (no barrier).
+// What bounds a scoring step's launch is latency: the source vectors do not depend on the predecessor, so the first kAttRing rows
+// of every warp (24 of a sentence's positions) are requested before griddepcontrol.wait, and the 96 KB of the ring leave room for
+// a CTA of the predecessor or successor on the SM.  us per launch at H = 1000, 50 positions, against rows held in registers (64 KB
+// in flight, requested after the wait): 128 columns 11.5 -> 7.4; a batch of 64 x 12 columns 22 -> 14.
+constexpr int kAttRing = 3;
+constexpr int kAttStreamBytes = 8 * kAttRing * 4096;
+static_assert(kAttStreamBytes >= kAttGlobalScratchBytes, "the merge reuses the ring");
+__global__ void __launch_bounds__(256, 2) att_global_stream_kernel(const AttArgs a) {
   extern __shared__ __align__(16) unsigned char att_dyn_scratch[];
-  att_global_fast_body(a, (int)blockIdx.x, (int)threadIdx.x, att_dyn_scratch, SyncCta());
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int H = a.H, H4 = H >> 2, sb = b / a.cols_per_sent;
+  const int len = __ldcg(a.len + sb), off = __ldcg(a.offset + sb);
+  float4* ring = reinterpret_cast<float4*>(att_dyn_scratch) + w * kAttRing * 256 + lane;
+  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+  auto request = [&](int k, int slot) {
+    const int pos = w + 8 * k;
+    if (pos < len) {
+      const float4* r4 = reinterpret_cast<const float4*>(a.hs + ((size_t)(len - 1 - pos + off) * a.B_src + sb) * H) + lane;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (lane + 32 * i < H4)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring_s + slot * 4096 + i * 512), "l"(r4 + 32 * i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < kAttRing; ++k) request(k, k);
+  pdl_enter();
+  att_zero_pad(a, b, tid, kAttTeam);
+  if (a.mask && a.mask[b] != 1) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return att_global_masked(a, b, tid);
+  }
+  const float4* h4 = reinterpret_cast<const float4*>(a.h_t + (size_t)b * H);
+  float4 hv[8], ctx[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int j = lane + 32 * i;
+    hv[i] = j < H4 ? h4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    ctx[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float m = -INFINITY, l = 0.f, bsc = -INFINITY;
+  int bpos = -1, slot = 0;
+  for (int k = 0; w + 8 * k < len; ++k) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kAttRing - 1) : "memory");
+    float4 rv[8];
+    float sc = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      rv[i] = lane + 32 * i < H4 ? ring[slot * 256 + 32 * i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      sc += rv[i].x * hv[i].x + rv[i].y * hv[i].y + rv[i].z * hv[i].z + rv[i].w * hv[i].w;
+    }
+    request(k + kAttRing, slot);
+    if (++slot == kAttRing) slot = 0;
+    att_global_take(a, b, lane, w + 8 * k, warp_sum(sc), rv, m, l, bsc, bpos, ctx);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();  // the merge reuses the ring
+  att_global_merge(a, b, tid, len, att_dyn_scratch, m, l, bsc, bpos, ctx, SyncCta());
 }
 cudaError_t launch_att_global(const AttArgs& a, cudaStream_t st) {
   if (a.B <= 0) return cudaSuccess;
   if ((a.H & 3) == 0 && a.H <= 1024) {
     count_launch();
-    return launch_chain(att_global_fast_kernel, dim3(a.B), dim3(256), (size_t)kAttGlobalScratchBytes, st, a);
+    static bool configured[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (!configured[dev]) {
+      const cudaError_t e = cudaFuncSetAttribute(att_global_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttStreamBytes);
+      if (e != cudaSuccess) return e;
+      configured[dev] = true;
+    }
+    return launch_chain(att_global_stream_kernel, dim3(a.B), dim3(256), (size_t)kAttStreamBytes, st, a);
   }
   const size_t smem = sizeof(float) * (size_t)(a.S_max > 0 ? a.S_max : 1);
   if (smem > 40 * 1024) return cudaErrorInvalidValue;
@@ -1452,12 +1516,12 @@ __global__ void __launch_bounds__(CPT >= 4 ? 256 : 1024, 1) lstm_seq_resident_ke
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
         if (cb + c < B) {
-          const float gi = sigmoidf_acc(ai[c] + xp[c].x + bi);
-          const float gf = sigmoidf_acc(af[c] + xp[c].y + bf);
-          const float gg = tanhf(ag[c] + xp[c].z + bg);
-          const float go = sigmoidf_acc(ao[c] + xp[c].w + bo);
+          const float gi = sigmoid_f32(ai[c] + xp[c].x + bi);
+          const float gf = sigmoid_f32(af[c] + xp[c].y + bf);
+          const float gg = tanh_f32(ag[c] + xp[c].z + bg);
+          const float go = sigmoid_f32(ao[c] + xp[c].w + bo);
           const float cn = gf * cst[c] + gi * gg;
-          const float hn = go * tanhf(cn) * mk[c];
+          const float hn = go * tanh_f32(cn) * mk[c];
           cst[c] = cn * mk[c];
           hnew[c] = hn;
           // the new h into every CTA's copy of the other buffer (nobody reads the last step's)
@@ -1636,12 +1700,12 @@ __global__ void __launch_bounds__(512, 1) lstm_seq_reg_kernel(const SeqArgs a, i
       const float si = __shfl_sync(0xffffffffu, v1, c8), sf = __shfl_sync(0xffffffffu, v1, 8 + c8);
       const float sg = __shfl_sync(0xffffffffu, v1, 16 + c8), so = __shfl_sync(0xffffffffu, v1, 24 + c8);
       if (col) {
-        const float gi = sigmoidf_acc(si + xp.x + bi);
-        const float gf = sigmoidf_acc(sf + xp.y + bf);
-        const float gg = tanhf(sg + xp.z + bg);
-        const float go = sigmoidf_acc(so + xp.w + bo);
+        const float gi = sigmoid_f32(si + xp.x + bi);
+        const float gf = sigmoid_f32(sf + xp.y + bf);
+        const float gg = tanh_f32(sg + xp.z + bg);
+        const float go = sigmoid_f32(so + xp.w + bo);
         const float cn = gf * cst + gi * gg;
-        const float hn = go * tanhf(cn) * mk;
+        const float hn = go * tanh_f32(cn) * mk;
         cst = cn * mk;
         if (t + 1 < a.S) {
           const uint32_t off = (uint32_t)((((size_t)((t + 1) & 1) * H + j) * Bp + s) * 4);
