@@ -2103,7 +2103,7 @@ __device__ void beam_insert_hyp(const BeamArgs& a, int s, const int* row, int la
 // NL: candidates per lane of the selecting warp: 8 covers beam * (beam + 1) <= 256 (beam <= 15), 33 covers beam <= 32
 template <int NL>
 __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
-  __shared__ float cv[32 * NL];
+  __shared__ __align__(16) float cv[32 * NL];
   __shared__ int ci[32 * NL];
   __shared__ int order[NL <= 8 ? 256 : 1];
   __shared__ int n_chg[ZR_BEAM_MAX], n_cur[ZR_BEAM_MAX];
@@ -2111,6 +2111,15 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
   pdl_enter();
   const int s = blockIdx.x, tid = threadIdx.x, beam = a.beam, kc = a.k_cand, t = a.step;
   const int base = s * beam;
+  // one candidate per thread, requested together with what decides whether it counts (a chain of three L2 latencies otherwise)
+  float lp0 = -INFINITY, sc0 = 0.f;
+  int wd0 = -1;
+  if (NL <= 8 && tid < beam * kc) {
+    lp0 = a.cand_val[(size_t)base * kc + tid];
+    wd0 = a.cand_idx[(size_t)base * kc + tid];
+    sc0 = a.scores[base + tid / kc];
+  }
+  const int cur = (tid & 31) < beam ? a.cur_ids[base + (tid & 31)] : 0;
   const int max_steps = a.max_steps[s];
   int* rows = a.top_sent + (size_t)base * a.Lmax;
   int* tmp = a.top_tmp + (size_t)base * a.Lmax;
@@ -2136,7 +2145,7 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
   int ncols = (t == 0) ? 1 : beam;
   {
     const int l = tid & 31;
-    const bool dead = l < ncols && a.cur_ids[base + l] == -1;
+    const bool dead = l < ncols && cur == -1;
     const unsigned db = __ballot_sync(0xffffffffu, dead);
     if (db) ncols = __ffs(db) - 1;
   }
@@ -2145,9 +2154,9 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
     float v = -INFINITY;
     int wd = -1;
     if (i < ncols) {
-      const float lp = a.cand_val[(size_t)(base + i) * kc + r];
-      wd = a.cand_idx[(size_t)(base + i) * kc + r];
-      if (wd >= 0 && lp != -INFINITY) v = lp + a.scores[base + i];
+      const float lp = NL <= 8 ? lp0 : a.cand_val[(size_t)(base + i) * kc + r];
+      wd = NL <= 8 ? wd0 : a.cand_idx[(size_t)(base + i) * kc + r];
+      if (wd >= 0 && lp != -INFINITY) v = lp + (NL <= 8 ? sc0 : a.scores[base + i]);
     }
     cv[c] = v;   // candidate c = beam column * kc + candidate rank
     ci[c] = wd;  // its word, kept on chip: the selection below reads one per pick
@@ -2161,9 +2170,12 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
     if (tid < n_cand) {
       const float v = cv[tid];
       int rank = 0;
-      for (int i = 0; i < n_cand; ++i) {
-        const float o = cv[i];
-        rank += (o > v || (o == v && i < tid)) ? 1 : 0;
+      for (int i = 0; i < n_cand; i += 4) {  // (entries beyond n_cand are -inf and come after every candidate)
+        const float4 o = *reinterpret_cast<const float4*>(cv + i);
+        rank += (o.x > v || (o.x == v && i < tid)) ? 1 : 0;
+        rank += (o.y > v || (o.y == v && i + 1 < tid)) ? 1 : 0;
+        rank += (o.z > v || (o.z == v && i + 2 < tid)) ? 1 : 0;
+        rank += (o.w > v || (o.w == v && i + 3 < tid)) ? 1 : 0;
       }
       order[rank] = tid;
     }
@@ -2242,6 +2254,22 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
   }
   __syncthreads();
   // the surviving hypotheses' rows go to the other row buffer, which the host makes the current one for the next step
+  if ((a.Lmax & 3) == 0) {  // whole rows of 16-byte pieces
+    const int q = a.Lmax >> 2;
+    for (int e = tid; e < beam * q; e += blockDim.x) {
+      const int f = e / q, i = 4 * (e - f * q), at = t + 1 - i;
+      const size_t from = (size_t)n_chg[f] * a.Lmax + i;
+      int4 v = *reinterpret_cast<const int4*>(rows + from), al = make_int4(0, 0, 0, 0);
+      if (vrows) al = *reinterpret_cast<const int4*>(vrows + from);
+      if (at >= 0 && at < 4) {
+        const int wd = n_cur[f] == -1 ? 0 : n_cur[f];
+        (at == 0 ? v.x : at == 1 ? v.y : at == 2 ? v.z : v.w) = wd;
+        if (vrows && n_cur[f] != -1) (at == 0 ? al.x : at == 1 ? al.y : at == 2 ? al.z : al.w) = a.viterbi[base + n_chg[f]];
+      }
+      reinterpret_cast<int4*>(tmp)[e] = v;
+      if (vrows) reinterpret_cast<int4*>(vtmp)[e] = al;
+    }
+  } else
   for (int e = tid; e < beam * a.Lmax; e += blockDim.x) {
     const int f = e / a.Lmax, i = e % a.Lmax;
     int v = rows[(size_t)n_chg[f] * a.Lmax + i];
