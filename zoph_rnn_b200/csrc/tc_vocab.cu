@@ -1,4 +1,4 @@
-// Vocabulary projection for up to 128 batch columns on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
+// Vocabulary projection for few batch columns (128, split modes 256) on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
 //
 // The weights are the M side of the MMA (128 vocabulary rows) and the columns its N side, padded to a multiple of 16 only: with
 // the columns as the M side (tc_gemm.cu) a step of 12 columns multiplied 128 padded rows, 19 us of MMAs for 160 MB of weights, and
@@ -6,9 +6,10 @@
 // h_hi.  An accumulator row is a vocabulary row, so a warp stores 32 consecutive logits of a column at once; maxima and sums
 // over the rows are reductions across the warp that halve the number of columns per lane as they go.
 //
-// Persistent CTAs walk over the vocabulary, the accumulators are double-buffered in TMEM and the loads run ahead across tiles.  Up
-// to 64 columns a CTA takes half an SM (113 KB, 256 TMEM columns), so that it is resident, and streams its first weights, while
-// the kernel before it runs.  us per launch, before -> now, f32: 12 columns x 40000 words x 1000: 48 -> 31 (HBM: 25).
+// Persistent CTAs walk over the vocabulary, the accumulators are double-buffered in TMEM (while 512 columns hold two) and the loads
+// run ahead across tiles.  Up to 64 columns a CTA takes half an SM (113 KB, 256 TMEM columns), so that it is resident, and streams
+// its first weights, while the kernel before it runs.  us per launch, before -> now, f32: 12 columns x 40000 words x 1000: 48 -> 31
+// (HBM: 25); 130 - 250 columns x 50000 words x 1000: 128 -> 84.  Marking the weights to leave the L2 first changes nothing.
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -28,9 +29,10 @@ struct VocabCtrl {
   uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort;
-  float red_max[4][kVocabMaxCols], red_sum[4][kVocabMaxCols];  // per lane quadrant and column
-  int target[kVocabMaxCols];
 };
+
+// behind it, per column: maxima and sums of the four lane quadrants, target
+__host__ __device__ constexpr int column_bytes(int nb) { return nb * (4 * 4 + 4 * 4 + 4); }
 
 // eight values per lane -> the reduction over the warp of value lane >> 2: each exchange halves the values that a lane carries
 template <class Op>
@@ -56,7 +58,7 @@ __device__ __forceinline__ float reduce8(const float* v, int lane, Op op) {
 
 template <int MODE, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_constant__ VocabParams p, int stages, int n_tiles,
-                                                               int tmem_cols) {
+                                                               int tmem_cols, int bufs) {
   constexpr bool SPLIT_MODE = mode_split(MODE);
   constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t vocab_smem[];
@@ -65,6 +67,9 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
   const int w_bytes = PARTS * KBS * 128 * 128, h_bytes = PARTS * KBS * hkb, stage_bytes = w_bytes + h_bytes;
   uint8_t* tiles = vocab_smem;
   VocabCtrl& ct = *reinterpret_cast<VocabCtrl*>(tiles + (size_t)stages * stage_bytes);
+  float* red_max = reinterpret_cast<float*>(&ct + 1);
+  float* red_sum = red_max + 4 * nb;
+  int* s_target = reinterpret_cast<int*>(red_sum + 4 * nb);
   const int k_its = (p.kb + KBS - 1) / KBS;
   const int acc_cols = PARTS * nb;  // columns of one accumulator buffer
   if (threadIdx.x == 0) {
@@ -121,13 +126,14 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0 && sound) {
-      const uint32_t idesc = make_idesc(mode_fmt(MODE), (uint32_t)nb), idesc2 = make_idesc(mode_fmt(MODE), (uint32_t)(PARTS * nb));
+      const bool stacked = PARTS * nb <= 256;  // the widest MMA
+      const uint32_t idesc = make_idesc(mode_fmt(MODE), (uint32_t)nb), idesc2 = make_idesc(mode_fmt(MODE), (uint32_t)(stacked ? PARTS * nb : nb));
       int st = 0, ti = 0;
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
-        const int buf = ti & 1;
-        if (!mbar_wait(&ct.acc_empty[buf], (uint32_t)(((ti >> 1) & 1) ^ 1), &ct.abort, p.err, 4)) { ok = false; break; }
+        const int buf = bufs == 2 ? ti & 1 : 0, use = bufs == 2 ? ti >> 1 : ti;
+        if (!mbar_wait(&ct.acc_empty[buf], (uint32_t)((use & 1) ^ 1), &ct.abort, p.err, 4)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(buf * acc_cols);
         for (int k = 0; k < k_its; ++k) {
@@ -136,10 +142,16 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
           const uint32_t w_addr = smem_u32(tiles + (size_t)st * stage_bytes), h_addr = w_addr + w_bytes;
           for (int b = 0; b < KBS; ++b) {
             const uint64_t dw = make_smem_desc(w_addr + b * PARTS * 16384), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * 16384);
-            const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb);
+            const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb), dhl = make_smem_desc(h_addr + (b * PARTS + 1) * hkb);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, (k > 0 || b > 0 || i > 0) ? 1u : 0u);
+              const uint32_t acc = (k > 0 || b > 0 || i > 0) ? 1u : 0u;
+              if (!SPLIT_MODE || stacked) {
+                umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
+              } else {
+                umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc, acc);
+                umma<mode_kind_tf32(MODE)>(d + nb, dw + 2 * i, dhl + 2 * i, idesc, acc);
+              }
               if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + nb, dwl + 2 * i, dh + 2 * i, idesc, 1u);
             }
           }
@@ -155,15 +167,15 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
     const bool want_max = p.part_max != nullptr, want_sum = want_max && p.part_sum != nullptr;
     pdl_wait();
     if (EPI == TC_EPI_LSE)
-      for (int m = threadIdx.x; m < p.M; m += kEpiWarps * 32) ct.target[m] = p.target[m] - p.target_offset;
+      for (int m = threadIdx.x; m < p.M; m += kEpiWarps * 32) s_target[m] = p.target[m] - p.target_offset;
     asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
     int ti = 0;
     bool ready = sound;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++ti) {  // (to the end even after a wait that gave up: barriers)
-      const int buf = ti & 1, v = tile * 128 + quad * 32 + lane;
+      const int buf = bufs == 2 ? ti & 1 : 0, use = bufs == 2 ? ti >> 1 : ti, v = tile * 128 + quad * 32 + lane;
       const bool in = v < p.N;
       const float bias = in && p.bias ? __ldg(p.bias + v) : 0.f;
-      ready = ready && __all_sync(0xffffffffu, mbar_wait(&ct.acc_full[buf], (uint32_t)((ti >> 1) & 1), &ct.abort, p.err, 3));
+      ready = ready && __all_sync(0xffffffffu, mbar_wait(&ct.acc_full[buf], (uint32_t)(use & 1), &ct.abort, p.err, 3));
       tc_fence_after();
       if (ready) {
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * acc_cols);
@@ -183,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
           } else {
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-              if (c0 + u < p.M && ct.target[c0 + u] == v && in) p.tgt_logit[c0 + u] = z[u];
+              if (c0 + u < p.M && s_target[c0 + u] == v && in) p.tgt_logit[c0 + u] = z[u];
           }
           if (want_max) {
             if (!in) {
@@ -202,8 +214,8 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
               sm = reduce8(e, lane, [](float a, float b) { return a + b; });
             }
             if ((lane & 3) == 0) {
-              ct.red_max[quad][c0 + (lane >> 2)] = mx;
-              ct.red_sum[quad][c0 + (lane >> 2)] = sm;
+              red_max[quad * nb + c0 + (lane >> 2)] = mx;
+              red_sum[quad * nb + c0 + (lane >> 2)] = sm;
             }
           }
         }
@@ -218,9 +230,9 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
           const int part = i / p.M, m = i - part * p.M, at = tile * per + part;
           if (at >= p.n_parts) continue;
           float M = -INFINITY, S = 0.f;
-          for (int q = part * qs; q < (part + 1) * qs; ++q) M = fmaxf(M, ct.red_max[q][m]);
+          for (int q = part * qs; q < (part + 1) * qs; ++q) M = fmaxf(M, red_max[q * nb + m]);
           if (want_sum && M != -INFINITY)
-            for (int q = part * qs; q < (part + 1) * qs; ++q) S += ct.red_sum[q][m] * expf(ct.red_max[q][m] - M);
+            for (int q = part * qs; q < (part + 1) * qs; ++q) S += red_sum[q * nb + m] * expf(red_max[q * nb + m] - M);
           p.part_max[(size_t)at * p.M + m] = M;
           if (want_sum) p.part_sum[(size_t)at * p.M + m] = S;
         }
@@ -249,11 +261,13 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   constexpr int PARTS = mode_split(MODE) ? 2 : 1;
   const int stage = PARTS * p.kbs * (128 + p.nb) * 128;
   const bool half = p.nb <= kHalfCols;
-  const int stages = std::min(((half ? kHalfSm : kWholeSm) - (int)sizeof(VocabCtrl)) / stage, (int)kMaxStages);
+  const int fixed = (int)sizeof(VocabCtrl) + column_bytes(p.nb);
+  const int stages = std::min(((half ? kHalfSm : kWholeSm) - fixed) / stage, (int)kMaxStages);
   if (stages < 2) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)stages * stage + sizeof(VocabCtrl);
+  const size_t smem = (size_t)stages * stage + fixed;
+  const int bufs = 2 * PARTS * p.nb <= 512 ? 2 : 1;
   int tmem = 32;
-  while (tmem < 2 * PARTS * p.nb) tmem *= 2;
+  while (tmem < bufs * PARTS * p.nb) tmem *= 2;
   static bool configured[64] = {false};
   static int sms[64] = {0};
   int dev = 0;
@@ -277,7 +291,7 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = g_pdl_on ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, tc_vocab_kernel<MODE, EPI>, p, stages, n_tiles, tmem);
+  return cudaLaunchKernelEx(&cfg, tc_vocab_kernel<MODE, EPI>, p, stages, n_tiles, tmem, bufs);
 }
 template <int MODE>
 cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
@@ -289,7 +303,7 @@ cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
 }  // namespace
 
 cudaError_t launch_tc_vocab(const VocabParams& p, int mode, int epi, cudaStream_t st) {
-  if (p.M < 1 || p.M > kVocabMaxCols || p.N < 1 || p.nb != vocab_columns(p.M) || p.kb < 1 || p.kbs != vocab_kbs(mode) ||
+  if (p.M < 1 || p.M > vocab_max_cols(mode, p.kb) || p.N < 1 || p.nb != vocab_columns(p.M) || p.kb < 1 || p.kbs != vocab_kbs(mode) ||
       (p.part_rows != 64 && p.part_rows != 128))
     return cudaErrorInvalidValue;
   switch (mode) {

@@ -5,7 +5,11 @@
 
 namespace zrnn {
 
-constexpr int kVocabMaxCols = 128;
+constexpr int kVocabMaxCols = 256;
+// Beyond 128 columns the split modes have room for one accumulator only, so a tile's epilogue is not hidden: that pays, against
+// fetching the weights twice, where K is long (kb k-blocks; us per launch, 130 - 200 columns: K = 1000 84 against 128, K = 500 33
+// against 28).
+inline int vocab_max_cols(int mode, int kb) { return (mode == TC_TF32X3 || mode == TC_F16X2) && kb >= 12 ? 256 : 128; }
 
 // z[v, m] = W[v] . h[m] + bias[v] for v < N, m < M
 struct VocabParams {

@@ -626,6 +626,10 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   return ZRNN_OK;
 }
 
+int vocab_cols_limit(const zrnn_softmax* S) {
+  const int epk = 128 / eng_eb(S->eng);
+  return zrnn::vocab_max_cols(eng_tcmode(S->eng), (S->H + epk - 1) / epk);
+}
 // the part of a VocabParams that scoring and decoding share
 int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams& p) {
   const int eng = S->eng, mode = eng_tcmode(eng), eb = eng_eb(eng), parts = eng_split(eng) ? 2 : 1;
@@ -669,7 +673,7 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   }
   const int eng = S->eng, np = S->n_tiles * zrnn::kPersistentParts;
   ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
-  if (N <= zrnn::kVocabMaxCols) {
+  if (N <= vocab_cols_limit(S)) {
     zrnn::VocabParams vp;
     ZR_TRY(vocab_params(S, h, N, np, vp));
     vp.target = targets; vp.target_offset = S->lo; vp.tgt_logit = tgt;
@@ -721,7 +725,7 @@ int softmax_logits_act(zrnn_softmax* S, const Act& h, int N, cudaStream_t st, co
     g.M = Vs; g.N = N; g.C = S->logits.as<float>(); g.ldc = Vs; g.bias[0] = S->b;
     KScope ks(KC_SOFTMAX_GEMM, st);
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, (N >= 96 && Vs >= 512) ? 1 : 0, st));
-  } else if (N <= zrnn::kVocabMaxCols) {
+  } else if (N <= vocab_cols_limit(S)) {
     np = S->n_tiles * zrnn::kPersistentParts;
     ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
     zrnn::VocabParams vp;
