@@ -412,7 +412,7 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   const int fixed = (128 - p.a_rows) * 128 + slot_bytes(BN, EPI, SPLIT) + (int)sizeof(LinkCtrl);
   const int its = (p.kb + p.kbs - 1) / p.kbs;
   if (its < SPLIT) return cudaErrorInvalidValue;
-  // (a launch of several cells fills the chip and has no early sources: it takes the whole SM)
+  // (a launch of several cells has no early sources: it takes the whole SM, 3 x 500, 50 columns 9.7 us a launch against 11)
   int stages = ((n > 1 ? kWholeSm : kHalfSm) - fixed) / stage;
   stages = std::min(std::min(stages, (int)kMaxStages), p.nsrc * ((its + SPLIT - 1) / SPLIT));
   if (stages < kMmaWarps) stages = kMmaWarps;  // (both MMA warps own a stage)

@@ -838,6 +838,7 @@ struct zrnn_model {
   std::set<size_t> group_loaded;   // first slot of every tensor group that is on the device
   bool finalized = false;
   cudaStream_t stream = nullptr;
+  cudaEvent_t ev = nullptr; // joins the streams of an ensemble's models
   DevBuf ws, io;
   PinBuf pin;               // ids and log-probabilities of the host-buffer entry points
   DevBuf dec_counter;       // phase counter of the persistent decoder kernel
@@ -871,6 +872,7 @@ struct zrnn_model {
     delete att;
     delete sm;
     ws.release(); io.release(); pin.release(); dec_counter.release(); seq_xp.release();
+    if (ev) cudaEventDestroy(ev);
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -1438,7 +1440,8 @@ static int model_create_impl(const zrnn_model_config* c, int shard_lo, int shard
     m->slots.push_back({"softmax.b_d", c->V_tgt, 1, 3, 0, 1});
     m->staged.resize(m->slots.size());
     m->have_host.assign(m->slots.size(), 0);
-    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming) != cudaSuccess)
       st = fail(ZRNN_E_CUDA, "model_create: cannot create stream");
   }
   if (st != ZRNN_OK) {
@@ -2406,7 +2409,28 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
   }
 
   ZR_CUDA(cudaMemcpyAsync(d_len_host, m0->h_tmp.data(), sizeof(int) * 3 * n, cudaMemcpyHostToDevice, s));
-  for (int k = 0; k < K; ++k) ZR_TRY(bm[k].encode(d_src[k], sorted ? nullptr : d_order, s));
+  // An ensemble's models run side by side, each on a stream of its own: their chains of small launches leave most of the chip idle.
+  // What they share (current words, column map) changes on `s` only, between a join of all streams and the next fork.
+  std::vector<cudaStream_t> lane(K, s);
+  if (!g_kt.on)
+    for (int k = 1; k < K; ++k) lane[k] = models[k]->stream;
+  auto fork = [&]() -> int {
+    if (K == 1) return ZRNN_OK;
+    ZR_CUDA(cudaEventRecord(m0->ev, s));
+    for (int k = 1; k < K; ++k)
+      if (lane[k] != s) ZR_CUDA(cudaStreamWaitEvent(lane[k], m0->ev, 0));
+    return ZRNN_OK;
+  };
+  auto join = [&]() -> int {
+    for (int k = 1; k < K; ++k)
+      if (lane[k] != s) {
+        ZR_CUDA(cudaEventRecord(models[k]->ev, lane[k]));
+        ZR_CUDA(cudaStreamWaitEvent(s, models[k]->ev, 0));
+      }
+    return ZRNN_OK;
+  };
+  ZR_TRY(fork());
+  for (int k = K - 1; k >= 0; --k) ZR_TRY(bm[k].encode(d_src[k], sorted ? nullptr : d_order, lane[k]));
 
   zrnn::BeamArgs ba;
   std::memset(&ba, 0, sizeof(ba));
@@ -2418,6 +2442,7 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
   ba.best_ids = d_out_ids; ba.best_len = d_out_len; ba.best_score = d_out_score;
   ba.viterbi = bm[0].vit; ba.vit_rows = vit_rows; ba.vit_tmp = vit_tmp; ba.best_align = d_out_align;
   ZR_CUDA(zrnn::launch_beam_init(ba, s));
+  ZR_TRY(fork());
 
   int n_act = n;  // sentences still running: the leading ones
   for (int t = 0; t <= Tmax; ++t) {
@@ -2434,14 +2459,15 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
       bool partials = true;
       for (int k = 0; k < K; ++k) {
         Act top;
-        ZR_TRY(bm[k].forward(t, cur_ids, cols, &top, s));
+        ZR_TRY(bm[k].forward(t, cur_ids, cols, &top, lane[k]));
         const float *pm = nullptr, *ps = nullptr;
         int np = 0;
-        ZR_TRY(softmax_logits_act(models[k]->sm, top, cols, s, &pm, &np, &ps));
+        ZR_TRY(softmax_logits_act(models[k]->sm, top, cols, lane[k], &pm, &np, &ps));
         ea.logits[k] = models[k]->sm->logits.as<float>();
         ea.part_max[k] = pm; ea.part_sum[k] = ps; ea.n_parts[k] = np; ea.part_width[k] = models[k]->sm->BN / zrnn::kPersistentParts;
         partials = partials && pm && ps && np == ea.n_parts[0] && ea.part_width[k] == ea.part_width[0];
       }
+      ZR_TRY(join());
       ea.K = K; ea.V = V; ea.N = cols; ea.out = mean_logits;
       if (vote) {  // ensembles_models: sum the models' weights per source position, take the largest
         zrnn::EnsembleVitArgs va;
@@ -2467,8 +2493,10 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
       std::swap(ba.top_sent, ba.top_tmp);
       std::swap(ba.vit_rows, ba.vit_tmp);
     }
-    if (t < Tmax)
-      for (int k = 0; k < K; ++k) ZR_TRY(bm[k].reorder(col_map, cur_ids, cols, s));
+    if (t < Tmax) {
+      ZR_TRY(fork());
+      for (int k = 0; k < K; ++k) ZR_TRY(bm[k].reorder(col_map, cur_ids, cols, lane[k]));
+    }
   }
   return ZRNN_OK;
 }
