@@ -1902,19 +1902,27 @@ __global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constan
   __shared__ float tmax[256], cval[ZR_TOPK_CAND];
   __shared__ int cidx[ZR_TOPK_CAND];
   __shared__ float red_m[ZR_ENSEMBLE_MAX][8], red_s[ZR_ENSEMBLE_MAX][8], s_M[ZR_ENSEMBLE_MAX], s_inv[ZR_ENSEMBLE_MAX];
+  __shared__ float s_part[ZR_ENSEMBLE_MAX][ZR_TOPK_TILES], s_eos[ZR_ENSEMBLE_MAX];
   __shared__ float s_thr;
   __shared__ int s_count, s_nsel;
   const int col = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_parts = a.n_parts[0], K = a.K;
+  // Everything that does not depend on anything is requested at once: the <EOF> logits and, model by model, the partials.  (A chain
+  // of L2 latencies otherwise: two models x 20000 words 13.6 us per step, 11 so.)
+  const float z_eos = logp_eos && tid >= 32 && tid < 32 + K ? a.logits[tid - 32][(size_t)col * a.V + 1] : 0.f;
   for (int m = 0; m < K; ++m) {
-    float mx = -INFINITY, sum = 0.f;
+    float mx = -INFINITY, sum = 0.f, pmv[4], psv[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int j = tid + 256 * q;
-      if (j < n_parts) {
-        const float pm = a.part_max[m][(size_t)j * a.N + col], ps = a.part_sum[m][(size_t)j * a.N + col];
-        if (pm > mx) { sum = sum * expf(mx - pm) + ps; mx = pm; }
-        else if (pm != -INFINITY) sum += ps * expf(pm - mx);
-      }
+      pmv[q] = j < n_parts ? a.part_max[m][(size_t)j * a.N + col] : -INFINITY;
+      psv[q] = j < n_parts ? a.part_sum[m][(size_t)j * a.N + col] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float pm = pmv[q], ps = psv[q];
+      if (tid + 256 * q < n_parts) s_part[m][tid + 256 * q] = pm;  // (this thread reads it again below)
+      if (pm > mx) { sum = sum * expf(mx - pm) + ps; mx = pm; }
+      else if (pm != -INFINITY) sum += ps * expf(pm - mx);
     }
     float wm = mx;
 #pragma unroll
@@ -1922,6 +1930,7 @@ __global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constan
     const float ws = warp_sum(mx == -INFINITY ? 0.f : sum * expf(mx - wm));
     if (lane == 0) { red_m[m][w] = wm; red_s[m][w] = ws; }
   }
+  if (tid >= 32 && tid < 32 + K) s_eos[tid - 32] = z_eos;
   if (tid == 0) { s_count = 0; s_nsel = 0; }
   __syncthreads();
   if (tid < K) {
@@ -1940,9 +1949,9 @@ __global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constan
     const int j = tid + 256 * q;
     if (j < n_parts)
       for (int m = 0; m < K; ++m) {
-        const float e = expf(a.part_max[m][(size_t)j * a.N + col] - s_M[m]) * s_inv[m];
+        const float e = __fmul_rn(expf(s_part[m][j] - s_M[m]), s_inv[m]);
         lb = fmaxf(lb, e);
-        ub[q] += e;
+        ub[q] = __fadd_rn(ub[q], e);
       }
   }
   tmax[tid] = lb;
@@ -1953,7 +1962,7 @@ __global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constan
   }
   if (tid == 32 && logp_eos) {
     float p = 0.f;
-    for (int m = 0; m < K; ++m) p += expf(a.logits[m][(size_t)col * a.V + 1] - s_M[m]) * s_inv[m];
+    for (int m = 0; m < K; ++m) p += expf(s_eos[m] - s_M[m]) * s_inv[m];
     logp_eos[col] = logf(p);
   }
   __syncthreads();
@@ -1966,15 +1975,35 @@ __global__ void __launch_bounds__(256) ensemble_topk_kernel(const __grid_constan
   const int width = a.part_width[0];
   for (int attempt = 0; attempt < 4; ++attempt) {
     const int tot = s_nsel * width;
-    for (int e = tid; e < tot; e += 256) {
-      const int i = sel[e / width] * width + e % width;
-      if (i >= a.V) continue;
-      float p = 0.f;
-      for (int m = 0; m < K; ++m) p += expf(a.logits[m][(size_t)col * a.V + i] - s_M[m]) * s_inv[m];
-      if (p >= thr && p > 0.f) {
-        const int at = atomicAdd(&s_count, 1);
-        if (at < ZR_TOPK_CAND) { cval[at] = p; cidx[at] = i; }
+    for (int e0 = tid; e0 < tot; e0 += 4 * 256) {  // four elements of two models in flight per thread
+      int at4[4];
+      float p4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e = e0 + 256 * u;
+        at4[u] = e < tot ? sel[e / width] * width + e % width : a.V;
       }
+      for (int m = 0; m < K; m += 2) {
+        const int m1 = m + 1 < K ? m + 1 : m;
+        float z0[4], z1[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const size_t at = (size_t)col * a.V + (at4[u] < a.V ? at4[u] : 0);
+          z0[u] = a.logits[m][at];
+          z1[u] = a.logits[m1][at];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          p4[u] = __fadd_rn(p4[u], __fmul_rn(expf(z0[u] - s_M[m]), s_inv[m]));
+          if (m1 != m) p4[u] = __fadd_rn(p4[u], __fmul_rn(expf(z1[u] - s_M[m1]), s_inv[m1]));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (at4[u] < a.V && p4[u] >= thr && p4[u] > 0.f) {
+          const int at = atomicAdd(&s_count, 1);
+          if (at < ZR_TOPK_CAND) { cval[at] = p4[u]; cidx[at] = at4[u]; }
+        }
     }
     __syncthreads();
     if (s_count <= ZR_TOPK_CAND) break;
