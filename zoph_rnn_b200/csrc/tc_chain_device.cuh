@@ -33,6 +33,12 @@ __device__ __forceinline__ void tmem_ldw(uint32_t taddr, float* v) {
   if constexpr (W == 4) tmem_ld4(taddr, v);
   else tmem_ld8(taddr, v);
 }
+// 16 bytes into the shared memory of another CTA of the cluster, counted on a transaction barrier there
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(addr), "r"(bar),
+               "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)), "r"(__float_as_uint(d))
+               : "memory");
+}
 // after a wait that gave up: copies in flight land before the CTA may retire
 __device__ __forceinline__ void settle_copies() {
   const long long t0 = clock64();

@@ -99,7 +99,11 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
       mbar_init(&ct.set_full[i], 1);
       mbar_init(&ct.set_empty[i], kEpiWarps);
     }
-    for (int i = 0; i < kEpiWarps; ++i) mbar_init(&ct.xchg[i], SPLIT > 1 ? SPLIT - 1 : 1);
+    if (SPLIT > 1)
+      for (int i = 0; i < kEpiWarps; ++i) {
+        mbar_init(&ct.xchg[i], 1);
+        mbar_expect_tx(&ct.xchg[i], (uint32_t)(slot_bytes(BN, EPI, SPLIT) / kEpiWarps));
+      }
     ct.abort = (smem_u32(link_smem) & 1023) ? 1 : 0;  // (the swizzled tiles need the alignment that the declaration asks for)
     if (ct.abort && p.err) atomicExch(p.err, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -319,11 +323,11 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
 #pragma unroll
               for (int u = 0; u < NF; ++u) fin[g][u] = f[g * NF + u];
           } else {
+            // the bytes themselves complete the receiver's barrier: no release, whose fence cost as much as the transfer
             const uint32_t peer = cluster_map(slot0 + (uint32_t)(rank < q ? rank : rank - 1) * SENDER, (uint32_t)q);
+            const uint32_t bar = cluster_map(smem_u32(&ct.xchg[warp]), (uint32_t)q);
 #pragma unroll
-            for (int i = 0; i < V4; ++i) st_cluster_v4(peer + i * 512, f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(&ct.xchg[warp], (uint32_t)q);  // releases the whole warp's stores
+            for (int i = 0; i < V4; ++i) st_async_v4(peer + i * 512, bar, f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
           }
         }
         ready = __all_sync(0xffffffffu, mbar_wait_cluster(&ct.xchg[warp], 0, &ct.abort, p.err, 6));
