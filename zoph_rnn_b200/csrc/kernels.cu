@@ -68,6 +68,7 @@ __device__ float block_sum(float v, float* red) {
 // ------------------------------------------------------------------------------------------
 __global__ void prep_ids_kernel(const int* __restrict__ raw, int n, int* __restrict__ nonm1, int* __restrict__ mask01,
                                 const int* __restrict__ order, int n_cols) {
+  pdl_enter();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int v = raw[order ? i - i % n_cols + order[i % n_cols] : i];
     if (nonm1) nonm1[i] = (v == -1) ? 0 : v;
@@ -77,9 +78,8 @@ __global__ void prep_ids_kernel(const int* __restrict__ raw, int n, int* __restr
 cudaError_t launch_prep_ids(const int* raw, int n, int* nonm1, int* mask01, cudaStream_t st, const int* order, int n_cols) {
   if (n <= 0) return cudaSuccess;
   const int blocks = (n + 255) / 256;
-  prep_ids_kernel<<<blocks > 1184 ? 1184 : blocks, 256, 0, st>>>(raw, n, nonm1, mask01, order, n_cols);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(prep_ids_kernel, dim3(blocks > 1184 ? 1184 : blocks), dim3(256), 0, st, raw, n, nonm1, mask01, order, n_cols);
 }
 
 // The first launch of a scoring pass: the id preparation of up to three id arrays (-1 -> 0 and a 0/1 mask,
@@ -123,28 +123,29 @@ __global__ void fill_int_kernel(int* p, int v, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
 }
 __global__ void src_len_kernel(const int* __restrict__ mask01, int T, int B, int* len, int* offset) {
+  pdl_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   int n = 0;
+#pragma unroll 8
   for (int t = 0; t < T; ++t) n += mask01[(size_t)t * B + b];
   len[b] = n;
   offset[b] = T - n;
 }
 cudaError_t launch_src_len(const int* mask01, int T, int B, int* len, int* offset, cudaStream_t st) {
   if (B <= 0) return cudaSuccess;
-  src_len_kernel<<<(B + 127) / 128, 128, 0, st>>>(mask01, T, B, len, offset);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(src_len_kernel, dim3((B + 127) / 128), dim3(128), 0, st, mask01, T, B, len, offset);
 }
 __global__ void div_map_kernel(int* map, int n, int div) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) map[i] = i / div;
 }
 cudaError_t launch_div_map(int* map, int n, int div, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  div_map_kernel<<<(n + 127) / 128, 128, 0, st>>>(map, n, div);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(div_map_kernel, dim3((n + 127) / 128), dim3(128), 0, st, map, n, div);
 }
 cudaError_t launch_fill_int(int* p, int v, size_t n, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
@@ -210,6 +211,7 @@ cudaError_t launch_pack_weights(const PackArgs& a, cudaStream_t st) {
 }
 __global__ void convert_rows_kernel(const float* __restrict__ src, long long rows, int K, long long ld_src, int mode,
                                     void* dst_hi, float* dst_lo, long long ld_dst) {
+  pdl_enter();
   const long long total = rows * ld_dst;  // the padding up to ld_dst is set to zero
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
     const long long r = e / ld_dst;
@@ -222,10 +224,9 @@ cudaError_t launch_convert_rows(const float* src, long long rows, int K, long lo
   const long long total = rows * ld_dst;
   if (total <= 0) return cudaSuccess;
   long long blocks = (total + 255) / 256;
-  convert_rows_kernel<<<(unsigned)(blocks > 148 * 32 ? 148 * 32 : blocks), 256, 0, st>>>(src, rows, K, ld_src, op_mode,
-                                                                                        dst_hi, dst_lo, ld_dst);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(convert_rows_kernel, dim3((unsigned)(blocks > 148 * 32 ? 148 * 32 : blocks)), dim3(256), 0, st, src, rows, K,
+                      ld_src, op_mode, dst_hi, dst_lo, ld_dst);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -234,6 +235,7 @@ cudaError_t launch_convert_rows(const float* src, long long rows, int K, long lo
 // ------------------------------------------------------------------------------------------
 __global__ void gather_columns_kernel(const float* __restrict__ W, int H, int V, const int* __restrict__ ids, int n_cols,
                                       float* __restrict__ x, int* err) {
+  pdl_enter();
   const int vec = ((H & 3) == 0);
   for (int col = blockIdx.x; col < n_cols; col += gridDim.x) {
     int id = ids[col];
@@ -257,13 +259,17 @@ cudaError_t launch_gather_columns(const float* W, int H, int V, const int* ids, 
                                   cudaStream_t st) {
   if (n_cols <= 0) return cudaSuccess;
   const int threads = H >= 512 ? 128 : 64;
-  gather_columns_kernel<<<n_cols > 148 * 16 ? 148 * 16 : n_cols, threads, 0, st>>>(W, H, V, ids, n_cols, x, err);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(gather_columns_kernel, dim3(n_cols > 148 * 16 ? 148 * 16 : n_cols), dim3(threads), 0, st, W, H, V, ids, n_cols, x, err);
 }
 
-__global__ void gather_rows16_kernel(const uint4* __restrict__ src, int vec_per_row, int n_src_rows,
-                                     const int* __restrict__ ids, int n_rows, uint4* __restrict__ dst, int* err) {
+// blockIdx.y: the hi or the lo part of split operands
+__global__ void gather_rows16_kernel(const uint4* __restrict__ src_hi, const uint4* __restrict__ src_lo, int vec_per_row, int n_src_rows,
+                                     const int* __restrict__ ids, int n_rows, uint4* __restrict__ dst_hi, uint4* __restrict__ dst_lo,
+                                     int* err) {
+  pdl_enter();
+  const uint4* src = blockIdx.y ? src_lo : src_hi;
+  uint4* dst = blockIdx.y ? dst_lo : dst_hi;
   for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
     int id = ids[r];
     if (id < 0) id = 0;
@@ -276,15 +282,14 @@ __global__ void gather_rows16_kernel(const uint4* __restrict__ src, int vec_per_
     for (int i = threadIdx.x; i < vec_per_row; i += blockDim.x) d[i] = __ldg(s + i);
   }
 }
-cudaError_t launch_gather_rows16(const void* src, size_t row_bytes, int n_src_rows, const int* ids, int n_rows,
-                                 void* dst, int* err, cudaStream_t st) {
+cudaError_t launch_gather_rows16(const void* src_hi, const void* src_lo, size_t row_bytes, int n_src_rows, const int* ids, int n_rows,
+                                 void* dst_hi, void* dst_lo, int* err, cudaStream_t st) {
   if (n_rows <= 0) return cudaSuccess;
   if (row_bytes % 16 != 0) return cudaErrorInvalidValue;
-  gather_rows16_kernel<<<n_rows > 148 * 16 ? 148 * 16 : n_rows, 128, 0, st>>>(
-      reinterpret_cast<const uint4*>(src), (int)(row_bytes / 16), n_src_rows, ids, n_rows,
-      reinterpret_cast<uint4*>(dst), err);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(gather_rows16_kernel, dim3(n_rows > 148 * 16 ? 148 * 16 : n_rows, src_lo ? 2 : 1), dim3(128), 0, st,
+                      reinterpret_cast<const uint4*>(src_hi), reinterpret_cast<const uint4*>(src_lo), (int)(row_bytes / 16), n_src_rows,
+                      ids, n_rows, reinterpret_cast<uint4*>(dst_hi), reinterpret_cast<uint4*>(dst_lo), err);
 }
 
 __global__ void __launch_bounds__(128) col_gather_kernel(const __grid_constant__ ColGatherArgs a) {
@@ -571,6 +576,7 @@ __global__ void __launch_bounds__(256) lse_combine_kernel(const float* __restric
                                                            const float* __restrict__ tgt, int n_parts, int n_tgt, int N,
                                                            size_t part_stride, const int* __restrict__ mask,
                                                            float* __restrict__ logp) {
+  pdl_enter();
   __shared__ float s_m[kLsePy * kLseCx];
   __shared__ double s_s[kLsePy * kLseCx];
   const int n = blockIdx.x * kLseCx + threadIdx.x;
@@ -588,6 +594,7 @@ __global__ void __launch_bounds__(256) lse_combine_kernel(const float* __restric
 __global__ void __launch_bounds__(256) lse_reduce_kernel(const float* __restrict__ pm, const float* __restrict__ ps,
                                                           int n_parts, int N, float* __restrict__ out_max,
                                                           float* __restrict__ out_sum) {
+  pdl_enter();
   __shared__ float s_m[kLsePy * kLseCx];
   __shared__ double s_s[kLsePy * kLseCx];
   const int n = blockIdx.x * kLseCx + threadIdx.x;
@@ -602,24 +609,22 @@ __global__ void __launch_bounds__(256) lse_reduce_kernel(const float* __restrict
 cudaError_t launch_lse_reduce(const float* pm, const float* ps, int n_parts, int N, float* out_max, float* out_sum,
                               cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
-  lse_reduce_kernel<<<(N + kLseCx - 1) / kLseCx, dim3(kLseCx, kLsePy), 0, st>>>(pm, ps, n_parts, N, out_max, out_sum);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(lse_reduce_kernel, dim3((N + kLseCx - 1) / kLseCx), dim3(kLseCx, kLsePy), 0, st, pm, ps, n_parts, N, out_max, out_sum);
 }
 cudaError_t launch_lse_combine_shards(const float* pm, const float* ps, const float* tgt, int G, int N, const int* mask,
                                       float* logp, cudaStream_t st, size_t shard_stride) {
   if (N <= 0) return cudaSuccess;
-  lse_combine_kernel<<<(N + kLseCx - 1) / kLseCx, dim3(kLseCx, kLsePy), 0, st>>>(pm, ps, tgt, G, G, N, shard_stride ? shard_stride : (size_t)N, mask,
-                                                            logp);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(lse_combine_kernel, dim3((N + kLseCx - 1) / kLseCx), dim3(kLseCx, kLsePy), 0, st, pm, ps, tgt, G, G, N,
+                      shard_stride ? shard_stride : (size_t)N, mask, logp);
 }
 cudaError_t launch_lse_combine(const float* pm, const float* ps, const float* tgt, int n_parts, int N, const int* mask,
                                float* logp, cudaStream_t st) {
   if (N <= 0) return cudaSuccess;
-  lse_combine_kernel<<<(N + kLseCx - 1) / kLseCx, dim3(kLseCx, kLsePy), 0, st>>>(pm, ps, tgt, n_parts, 1, N, (size_t)N, mask, logp);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(lse_combine_kernel, dim3((N + kLseCx - 1) / kLseCx), dim3(kLseCx, kLsePy), 0, st, pm, ps, tgt, n_parts, 1, N,
+                      (size_t)N, mask, logp);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2071,6 +2076,7 @@ cudaError_t launch_ensemble_logmean(const EnsembleArgs& a, cudaStream_t st) {
 // beam bookkeeping, one CTA per sentence
 // ------------------------------------------------------------------------------------------
 __global__ void beam_init_kernel(const BeamArgs a) {
+  pdl_enter();
   const int s = blockIdx.x, tid = threadIdx.x;  // (every sentence's results are cleared: the order does not matter here)
   const size_t rowbase = (size_t)s * a.beam * a.Lmax;
   for (int i = tid; i < a.beam * a.Lmax; i += blockDim.x) { a.top_sent[rowbase + i] = 0; a.top_tmp[rowbase + i] = 0; }
@@ -2088,9 +2094,8 @@ __global__ void beam_init_kernel(const BeamArgs a) {
 }
 cudaError_t launch_beam_init(const BeamArgs& a, cudaStream_t st) {
   if (a.n_sent <= 0) return cudaSuccess;
-  beam_init_kernel<<<a.n_sent, 128, 0, st>>>(a);
   count_launch();
-  return cudaGetLastError();
+  return launch_chain(beam_init_kernel, dim3(a.n_sent), dim3(128), 0, st, a);
 }
 
 // insert (prefix of `row` up to position last_pos, then <EOF>) with `score` into the sentence's k-best list; one whole warp

@@ -20,8 +20,8 @@ cudaError_t launch_gather_columns(const float* W, int H, int V, const int* ids, 
                                   cudaStream_t st);
 // same for rows of `row_bytes` bytes (a multiple of 16) of any element type: dst row n = src row ids[n]; n_src_rows > 0
 // bounds the ids the same way
-cudaError_t launch_gather_rows16(const void* src, size_t row_bytes, int n_src_rows, const int* ids, int n_rows,
-                                 void* dst, int* err, cudaStream_t st);
+cudaError_t launch_gather_rows16(const void* src_hi, const void* src_lo, size_t row_bytes, int n_src_rows, const int* ids, int n_rows,
+                                 void* dst_hi, void* dst_lo, int* err, cudaStream_t st);
 
 // ---- generic column gather over several H x ncols arrays at once: dst[a][:,c] = src[a][:,map[c]]
 // (replaces the per-column cudaMemcpy loops of swap_states_decoding / transfer_decoding_states_GPU,

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_s;
   pdl_wait();
+  pdl_trigger();
 
   if (warp == 8) {
     // ------------------------------------------------------------ TMA producer (runs ahead across tiles)
@@ -350,7 +351,6 @@ cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
   const int total = m_tiles * n_tiles;
   if (total == 0) return cudaSuccess;
   const int grid = total < sm_count() ? total : sm_count();
-  // (it may be launched while its predecessor drains; its successor starts when it has finished)
   static const bool pdl = std::getenv("ZRNN_NO_PDL") == nullptr;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));

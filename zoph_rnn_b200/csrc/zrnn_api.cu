@@ -1118,8 +1118,9 @@ static int gather_act(zrnn_lstm_layer* L, const int* ids, int n, const Act& x, c
     return ZRNN_OK;
   }
   const size_t rb = (size_t)L->Kpad * eng_eb(L->eng);
-  ZR_CUDA(zrnn::launch_gather_rows16(L->emb.hi, rb, L->V, ids, n, x.hi, tc_error_word(), st));
-  if (eng_split(L->eng)) ZR_CUDA(zrnn::launch_gather_rows16(L->emb.lo, rb, L->V, ids, n, x.lo, tc_error_word(), st));
+  const bool two = eng_split(L->eng);
+  ZR_CUDA(zrnn::launch_gather_rows16(L->emb.hi, two ? L->emb.lo : nullptr, rb, L->V, ids, n, x.hi, two ? x.lo : nullptr,
+                                     tc_error_word(), st));
   return ZRNN_OK;
 }
 
