@@ -119,9 +119,6 @@ cudaError_t launch_score_prologue(const PrologueArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-__global__ void fill_int_kernel(int* p, int v, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
-}
 __global__ void src_len_kernel(const int* __restrict__ mask01, int T, int B, int* len, int* offset) {
   pdl_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -146,13 +143,6 @@ cudaError_t launch_div_map(int* map, int n, int div, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   count_launch();
   return launch_chain(div_map_kernel, dim3((n + 127) / 128), dim3(128), 0, st, map, n, div);
-}
-cudaError_t launch_fill_int(int* p, int v, size_t n, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  size_t blocks = (n + 255) / 256;
-  fill_int_kernel<<<(unsigned)(blocks > 1184 ? 1184 : blocks), 256, 0, st>>>(p, v, n);
-  count_launch();
-  return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------
