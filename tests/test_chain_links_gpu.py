@@ -123,3 +123,18 @@ def test_vocabulary_projection_edges(dtype, H, V, N):
     tgt = rng.integers(0, V, N).astype(np.int32)
     got = layer.compute_loss(dh, torch.as_tensor(tgt).cuda(), torch.ones(N, dtype=torch.int32, device="cuda"))
     np.testing.assert_allclose(got.cpu().numpy().reshape(-1), logp[np.arange(N), tgt], rtol=r, atol=a)
+
+
+@pytest.mark.parametrize("mode,K,steps", [(4, 64, 4), (4, 320, 4), (4, 512, 4), (4, 1000, 8), (3, 64, 4), (3, 512, 4), (3, 1000, 8)])
+@pytest.mark.parametrize("n,m", [(512, 100), (1000, 12), (320, 200)])
+def test_products_of_one_sign_do_not_shrink(mode, K, steps, n, m):
+    """The tensor core truncates: at each k-step the products, as they are aligned, and the new accumulator, which positive terms show as a
+    shrinking sum.  Taken as one ulp per k-step (at most 2^-23 of a partial sum that grows linearly), an accumulator that absorbs `steps`
+    of them loses (steps + 1) 2^-24 of its sum.  Adding the accumulators up in fp32, and storing, rounds: below 2^-24 on average."""
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(n + m + K)
+    W, X = rng.uniform(0.05, 0.15, (K, n)).astype(np.float32), rng.uniform(0.5, 1.5, (m, K)).astype(np.float32)
+    C = api.gemm(torch.as_tensor(W).cuda().reshape(-1), torch.as_tensor(X).cuda().reshape(-1), n, m, K, mode).cpu().numpy().reshape(m, n)
+    want = X.astype(np.float64) @ W.astype(np.float64)
+    assert np.abs(C / want - 1).mean() < (steps + 2) * 2.0 ** -24

@@ -33,18 +33,22 @@ constexpr int kEpiWarps = 8, kAWarp = 8, kWWarp = 9, kMmaWarp = 10, kMmaWarps = 
 constexpr int kHalfSm = 113 * 1024;  // two CTAs per SM: (228 KB - 2 x 1 KB) / 2
 constexpr int kWholeSm = 224 * 1024;
 constexpr int kMaxStages = 8;
-// The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb many k-blocks in a row: the K axis
-// is walked in rounds of 8 k-blocks (4 in the 3xTF32 mode; half of them each MMA warp's), and the epilogue warps add each finished round to sums
-// of their own in registers (round to nearest).
-constexpr int round_kb(int mode) { return mode == TC_TF32X3 ? 4 : 8; }
-template <int MODE>
-__device__ __forceinline__ int round_stages(int kbs) { return round_kb(MODE) / kbs; }  // kbs: 1, 2 or 4
+// The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb many products in a row: the K axis
+// is walked in rounds of round_kb k-blocks (half of them each MMA warp's), and the epilogue warps add each finished round to sums
+// of their own in registers (round to nearest).  Up to 512 elements per source (8 k-blocks of fp16, 16 of tf32) an accumulator absorbs
+// 4 k-steps, beyond that 8.  Hidden states of a scoring pass against float64 (uniform weights +-0.08, fp16 split), 16 / 8 / 4 k-steps:
+// 2 layers x 512, 100 columns 5.5 / 3.2 / 2.1e-7, 1 x 1024, 30 columns 6.1 / 3.4 / 2.3e-7, 4 x 1000, 64 columns 15 / 9.6 / 7.5e-7.
+// A round more costs a commit, a wait and a drain: three cells of 500 units and 50 columns in a launch take 11.2 instead of 10.0 us,
+// cells of 1000 units in 8 k-steps what they took in 16 (+2 % of a step of 64 columns).
+__host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 2 : 4; }
 // Split modes multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the columns for two products (an MMA of 128 rows
 // takes 45 cycles up to 32 columns, 48 at 64, 64 at 128), and A_lo by W_hi: two MMAs per k-step instead of three.
 __host__ __device__ constexpr int set_cols(int BN, int mode) { return mode_split(mode) ? 2 * BN : BN; }  // one accumulator set per MMA warp
-__host__ __device__ constexpr int link_tmem(int BN, int mode) {
+// sets that an MMA warp takes in turn, one being added up while the next fills: where the CTA's columns hold them (half an SM: 256)
+__host__ __device__ constexpr int set_bufs(int BN, int mode, bool whole_sm) { return mode_split(mode) && (BN <= 32 || whole_sm) ? 2 : 1; }
+__host__ __device__ constexpr int link_tmem(int BN, int mode, bool whole_sm) {
   int c = 32;
-  while (c < kMmaWarps * set_cols(BN, mode)) c *= 2;
+  while (c < kMmaWarps * set_bufs(BN, mode, whole_sm) * set_cols(BN, mode)) c *= 2;
   return c;
 }
 // outputs per row and epilogue warp (LSTM: hidden units); a CTA finishes 1 / SPLIT of them
@@ -61,19 +65,19 @@ __device__ __forceinline__ int own_stages(int mw, int n, int stages) {
 struct LinkCtrl {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t accum;                               // everything accumulated (modes without rounds)
-  uint64_t set_full[kMmaWarps], set_empty[kMmaWarps];
+  uint64_t set_full[2 * kMmaWarps], set_empty[2 * kMmaWarps];
   uint64_t xchg[kEpiWarps];                     // the other CTAs' shares for this warp have arrived
   uint32_t tmem_base;
   int abort;
   float bias[64];
 };
 
-template <int BN, int MODE, int EPI, int SPLIT>
+template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
 __device__ __forceinline__ void link_body(const ChainParams& p, const int m_block, const int stages) {
   constexpr bool SPLIT_MODE = mode_split(MODE), ROUNDS = SPLIT_MODE;
   constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   constexpr int WKB = BN * 128;  // bytes of one k-block of one weight part
-  constexpr int SETC = set_cols(BN, MODE), TMEM_COLS = link_tmem(BN, MODE);
+  constexpr int SETC = set_cols(BN, MODE), NB = set_bufs(BN, MODE, WHOLE), TMEM_COLS = link_tmem(BN, MODE, WHOLE);
   constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN), IDESC2 = make_idesc(mode_fmt(MODE), SETC);
   extern __shared__ __align__(1024) uint8_t link_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -95,7 +99,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
       mbar_init(&ct.empty[s], 1);
     }
     mbar_init(&ct.accum, kMmaWarps);
-    for (int i = 0; i < kMmaWarps; ++i) {
+    for (int i = 0; i < kMmaWarps * NB; ++i) {
       mbar_init(&ct.set_full[i], 1);
       mbar_init(&ct.set_empty[i], kEpiWarps);
     }
@@ -166,14 +170,15 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   } else if (warp >= kMmaWarp) {
     // ------------------------------------------------------------ MMA issuers
     if (lane == 0 && sound) {
-      const int mw = warp - kMmaWarp, R = round_stages<MODE>(KBS);
-      const uint32_t d = tmem_base + (uint32_t)(mw * SETC);
+      const int mw = warp - kMmaWarp, R = round_kb(MODE, p.kb) / KBS;
+      int set = mw * NB;
       int st = mw, it = mw, round_end = 0, round = 0;
       uint32_t ph = 0;
       bool ok = true, fresh = true;
       while (it < n_it) {
         if (ROUNDS && it >= round_end) {  // first stage of this warp in a round
-          if (round > 0 && !mbar_wait(&ct.set_empty[mw], (uint32_t)(round & 1) ^ 1u, &ct.abort, p.err, 4)) { ok = false; break; }
+          set = mw * NB + round % NB;
+          if (round >= NB && !mbar_wait(&ct.set_empty[set], (uint32_t)(round / NB & 1) ^ 1u, &ct.abort, p.err, 4)) { ok = false; break; }
           tc_fence_after();
           fresh = true;
           round_end = (it / R + 1) * R;
@@ -182,6 +187,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
         if (!mbar_wait(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
+        const uint32_t d = tmem_base + (uint32_t)(set * SETC);
         for (int b = 0; b < KBS; ++b) {
           const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
           const uint64_t dw = make_smem_desc(w_addr + b * PARTS * WKB);
@@ -201,7 +207,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
           st = mw;
           ph ^= 1u;
         }
-        if (ROUNDS && (it >= round_end || it >= n_it)) umma_commit(&ct.set_full[mw]);
+        if (ROUNDS && (it >= round_end || it >= n_it)) umma_commit(&ct.set_full[set]);
       }
       if (ok && !ROUNDS) umma_commit(&ct.accum);
     }
@@ -270,7 +276,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
         }
     };
     if constexpr (ROUNDS) {
-      const int R = round_stages<MODE>(KBS);
+      const int R = round_kb(MODE, p.kb) / KBS;
       int seen[2] = {0, 0};  // rounds of each MMA warp so far (one in which it has no stage is none of its rounds)
       for (int lo = 0; ready && lo < n_it; lo += R) {
         if (lo + R > n_early) fetch_inputs();
@@ -278,13 +284,14 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
 #pragma unroll
         for (int mw = 0; mw < kMmaWarps; ++mw) {
           if (!ready || own_stages(mw, hi, stages) == own_stages(mw, lo, stages)) continue;
-          ready = __all_sync(0xffffffffu, mbar_wait(&ct.set_full[mw], (uint32_t)(seen[mw] & 1), &ct.abort, p.err, 3));
+          const int set = mw * NB + seen[mw] % NB;
+          ready = __all_sync(0xffffffffu, mbar_wait(&ct.set_full[set], (uint32_t)(seen[mw] / NB & 1), &ct.abort, p.err, 3));
           ++seen[mw];
           tc_fence_after();
-          if (ready && live) drain(mw);
+          if (ready && live) drain(set);
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&ct.set_empty[mw]);
+          if (lane == 0) mbar_arrive(&ct.set_empty[set]);
         }
       }
       fetch_inputs();
@@ -397,13 +404,13 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
 
 template <int BN, int MODE, int EPI, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 2) tc_link_kernel(const __grid_constant__ ChainParams p, int stages) {
-  link_body<BN, MODE, EPI, SPLIT>(p, (int)blockIdx.x, stages);
+  link_body<BN, MODE, EPI, SPLIT, false>(p, (int)blockIdx.x, stages);
 }
 // Several independent problems of one row block each (M <= 128): blockIdx.x selects the problem.  The cells of one
 // anti-diagonal of a stack (layer l at step t, layer l - 1 at step t + 1, ...) do not depend on one another.
 template <int BN, int MODE>
 __global__ void __launch_bounds__(kThreads, 2) tc_link_multi_kernel(const __grid_constant__ ChainBatch pb, int stages) {
-  link_body<BN, MODE, TC_EPI_LSTM, 1>(pb.p[blockIdx.x], 0, stages);
+  link_body<BN, MODE, TC_EPI_LSTM, 1, true>(pb.p[blockIdx.x], 0, stages);
 }
 
 const bool g_pdl_on = std::getenv("ZRNN_NO_PDL") == nullptr;
@@ -489,7 +496,9 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, int split, 
 
 int link_kbs(int mode, int BN, int a_rows, int kb, int split) {
   const int kb_bytes = (mode_split(mode) ? 2 : 1) * (a_rows + BN) * 128;
-  int k = 4;  // k-blocks per stage: as many as leave the ring four stages and every CTA two stages of a source
+  // k-blocks per stage: as many as leave the ring four stages and every CTA two stages of a source; a round has two stages at least,
+  // one for each MMA warp
+  int k = mode_split(mode) ? round_kb(mode, kb) / 2 : 4;
   while (k > 1 && (4 * k * kb_bytes > kHalfSm - 20 * 1024 - (128 - a_rows) * 128 || (kb + k - 1) / k < 2 * split)) k /= 2;
   return k;
 }
