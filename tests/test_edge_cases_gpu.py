@@ -138,6 +138,30 @@ def test_shape_sweep_against_the_oracle(api, oracle, att, lm, L, H, Vs, Vt, B, S
         assert abs(got16[msk].sum() - want[msk].sum()) < 5e-3 * abs(want[msk].sum())
 
 
+@pytest.mark.parametrize("beam", [1, 12, 15, 16, 20])
+@pytest.mark.parametrize("dtype", [3, 0, 1])
+def test_nan_scores_are_no_candidates(api, dtype, beam):
+    """A model with one NaN in the softmax bias has no finite log-probability: the search ends without a hypothesis, words and
+    alignments stay within range, and a sound model decodes the same before and after.  Both ways of picking a beam (one candidate
+    per thread up to beam 15, a warp-wide argmax beyond), and an ensemble with the diverged model."""
+    cfg = synth.make_cfg(1, 64, 60, 500, attention=1, feed_input=1, D=2)
+    w = synth.make_weights(cfg, seed=9, scale=0.3)
+    bad = [a.copy() for a in w]
+    bad[-1][7] = np.nan
+    good, diverged = build(api, cfg, w, dtype), build(api, cfg, bad, dtype)
+    rng = np.random.default_rng(4)
+    srcs = [rng.integers(2, 60, n).astype(np.int32) for n in (5, 2, 9)]
+    kw = dict(beam=beam, k_best=2, min_ratio=0.0, max_ratio=1.5, longest_sent=20, want_align=True)
+    want = good.decode(srcs, **kw)
+    for got in (diverged.decode(srcs, **kw), good.decode(srcs, penalty=float("nan"), **kw),
+                api.decode_ensemble([good, diverged], [srcs, srcs], **kw)):
+        ids, ln, _, al = got
+        assert ids.min() >= -1 and ids.max() < 500 and ln.min() >= 0 and ln.max() <= 24 and al.min() >= -1 and al.max() <= 9
+    assert not diverged.decode(srcs, **kw)[1].any()
+    for a, b in zip(good.decode(srcs, **kw), want):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_two_devices_in_one_process(api):
     """zrnn_set_device lets one process put models on several devices in turn: per-device state inside the library
     (kernel attributes, error word, scratch addresses) must not leak from one device to the other."""

@@ -2181,6 +2181,7 @@ __global__ void __launch_bounds__(256) beam_step_kernel(const BeamArgs a) {
       const float lp = NL <= 8 ? lp0 : a.cand_val[(size_t)(base + i) * kc + r];
       wd = NL <= 8 ? wd0 : a.cand_idx[(size_t)(base + i) * kc + r];
       if (wd >= 0 && lp != -INFINITY) v = lp + (NL <= 8 ? sc0 : a.scores[base + i]);
+      if (!(v > -INFINITY)) v = -INFINITY;  // NaN (a model that has diverged) is no candidate: the ranks below need an order
     }
     cv[c] = v;   // candidate c = beam column * kc + candidate rank
     ci[c] = wd;  // its word, kept on chip: the selection below reads one per pick
