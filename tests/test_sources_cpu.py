@@ -1,0 +1,26 @@
+"""Properties of kernel sources that no run on a sound machine shows."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "zoph_rnn_b200", "csrc")
+
+
+def body(name, start, end):
+    with open(os.path.join(CSRC, name)) as f:
+        s = re.sub(r"//[^\n]*", "", f.read())
+    i = s.index(start)
+    return s[i:s.index(end, i)]
+
+
+def test_a_split_link_that_gave_up_waits_for_its_partner():
+    """The halves of a split tile travel with asynchronous stores into another CTA's shared memory.  A CTA that ends in order has waited for
+    them; one whose wait gave up must not leave before the others' threads have ended or arrived: a cluster barrier at the end of the
+    kernel, by all threads, on the flag that every wait sets when it gives up."""
+    s = body("tc_link.cu", "void link_body(", "template <int BN, int MODE, int EPI, int SPLIT>\n__global__")
+    end = s[s.index("tcgen05.dealloc"):]
+    steps = [end.index(t) for t in ("if (SPLIT > 1 && ct.abort) {", "cluster_arrive();", "cluster_wait();", "settle_copies();")]
+    assert steps == sorted(steps)
+    # every bounded wait of the kernel reports through that flag, and no thread looks at it before all of them are over
+    waits = re.findall(r"mbar_wait(?:_cluster)?\(([^;]*?), p\.err, \d\)", s)
+    assert len(waits) == len(re.findall(r"\bmbar_wait(?:_cluster)?\(", s)) and all(w.endswith("&ct.abort") for w in waits)
+    assert s.rindex("__syncthreads()") > s.rindex("mbar_wait")
