@@ -271,3 +271,31 @@ def test_softmax_topk_matches_oracle(api, oracle, V, H, N, k):
         np.testing.assert_allclose(val, want, rtol=2e-5, atol=5e-5)
         np.testing.assert_allclose(eos, np.log(p[:, 1].astype(np.float64)), rtol=2e-5, atol=5e-5)
         assert np.all(np.diff(val, axis=1) <= 0)
+
+
+@pytest.mark.parametrize("dtype", [3, 0])
+def test_global_attention_right_behind_the_launch_that_writes_its_sources(api, dtype):
+    """The source states come from the launch just ahead on the stream, one that lets its successor start before it has written anything
+    (the embedding gather): the attention step must not read them earlier."""
+    import torch
+    H, S, B, V = 1000, 50, 128, 2000
+    rng = np.random.default_rng(8)
+    emb = api.Input_To_Hidden_Layer(H, V, dtype=dtype)
+    t = [np.zeros(n, np.float32) for n in [H * H, H] * 4] + [rng.uniform(-0.3, 0.3, H * V).astype(np.float32)] + [np.zeros(H * H, np.float32)] * 4
+    emb.load_weights(t)
+    att = api.attention_layer(H, 10, att_type=2, dtype=dtype)
+    att.load_weights([(rng.standard_normal(n) * 0.03).astype(np.float32) for n in (H * H, H * H, H, H, H * H, H * H)])
+    ids = [torch.as_tensor(rng.integers(0, V, S * B).astype(np.int32)).cuda() for _ in range(2)]
+    h = torch.as_tensor(rng.uniform(-0.5, 0.5, B * H).astype(np.float32)).cuda()
+    mask, lens, off = (torch.full((B,), v, dtype=torch.int32, device="cuda") for v in (1, S, 0))
+    hs = torch.empty(S * B * H, dtype=torch.float32, device="cuda")
+
+    def step(i, wait):
+        api.check(api.lib().zrnn_ih_gather(emb._h, api._ptr(ids[i]), S * B, api._ptr(hs), api._stream()))
+        if wait:
+            torch.cuda.synchronize()
+        att.prep_minibatch_info(hs, S, B, lens, off)
+        return att.forward_prop(h, mask).clone()
+    want = [step(i, True).cpu() for i in (0, 1)]
+    for k in range(6):
+        assert torch.equal(step(k % 2, False).cpu(), want[k % 2])

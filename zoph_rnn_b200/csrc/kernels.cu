@@ -1175,8 +1175,8 @@ __global__ void __launch_bounds__(256) att_global_kernel(const AttArgs a) {
 }
 // Single pass for H % 4 == 0, H <= 1024, one CTA of 8 warps per column: warp w walks over the positions w, w + 8, ... and streams
 // their vectors through a ring of its own in shared memory, every lane the 16-byte pieces that it will read itself (no barrier).
-// What bounds a scoring step's launch is latency: the source vectors do not depend on the predecessor, so the first kAttRing rows
-// of every warp (24 of a sentence's positions) are requested before griddepcontrol.wait, and the 96 KB of the ring leave room for
+// What bounds a scoring step's launch is latency: the source vectors do not depend on the predecessor (a.src_ready), so the first
+// kAttRing rows of every warp (24 of a sentence's positions) are requested before griddepcontrol.wait, and the 96 KB of the ring leave room for
 // a CTA of the predecessor or successor on the SM.  us per launch at H = 1000, 50 positions, against rows held in registers (64 KB
 // in flight, requested after the wait): 128 columns 11.5 -> 7.4; a batch of 64 x 12 columns 22 -> 14.
 constexpr int kAttRing = 3;
@@ -1186,6 +1186,7 @@ __global__ void __launch_bounds__(256, 2) att_global_stream_kernel(const AttArgs
   extern __shared__ __align__(16) unsigned char att_dyn_scratch[];
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int H = a.H, H4 = H >> 2, sb = b / a.cols_per_sent;
+  if (!a.src_ready) pdl_enter();  // the predecessor may have written them: a caller's own kernel
   const int len = __ldcg(a.len + sb), off = __ldcg(a.offset + sb);
   float4* ring = reinterpret_cast<float4*>(att_dyn_scratch) + w * kAttRing * 256 + lane;
   const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
@@ -1202,7 +1203,7 @@ __global__ void __launch_bounds__(256, 2) att_global_stream_kernel(const AttArgs
   };
 #pragma unroll
   for (int k = 0; k < kAttRing; ++k) request(k, k);
-  pdl_enter();
+  if (a.src_ready) pdl_enter();
   att_zero_pad(a, b, tid, kAttTeam);
   if (a.mask && a.mask[b] != 1) {
     asm volatile("cp.async.wait_all;" ::: "memory");

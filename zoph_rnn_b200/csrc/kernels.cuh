@@ -168,6 +168,7 @@ struct AttArgs {
   const float* hs;  // S_max slots of H x B_src
   const int* len;   // per source column
   const int* offset;
+  int src_ready;     // hs, len and offset were complete when the predecessor kernel passed its own wait (0: perhaps not)
   const int* mask;   // per target column
   const float* h_t;  // H x B
   // local-p only

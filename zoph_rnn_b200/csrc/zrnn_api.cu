@@ -572,8 +572,9 @@ int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, c
   return ZRNN_OK;
 }
 
-int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const Act& out, float* align,
-                cudaStream_t st, int* viterbi = nullptr, float viterbi_init = -1.f, bool align_by_pos = false) {
+// src_ready: a launch of this library lies between the ones that wrote the source states and lengths and the one ahead of this call
+int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const Act& out, float* align, cudaStream_t st,
+                int* viterbi = nullptr, float viterbi_init = -1.f, bool align_by_pos = false, bool src_ready = true) {
   const int H = A->H, eng = A->eng, Kpad = A->Kpad;
   ZR_CUDA(A->ctx.reserve(sizeof(float) * (size_t)H * B));
   KScope ks(KC_ATT, st);
@@ -583,6 +584,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   a.hs = A->hs; a.len = A->len; a.offset = A->off; a.mask = mask; a.h_t = h_t.f32;
   a.c_t = A->ctx.as<float>(); a.align_out = align; a.viterbi_out = viterbi; a.viterbi_init = viterbi_init;
   a.align_by_pos = align_by_pos ? 1 : 0;
+  a.src_ready = src_ready ? 1 : 0;
   Act ctx;
   ctx.f32 = A->ctx.as<float>();
   if (eng != ENG_SIMT) {
@@ -1266,7 +1268,8 @@ int zrnn_att_forward(zrnn_attention* A, const float* d_h_t, const int* d_mask, i
   h.f32 = const_cast<float*>(d_h_t);
   out.f32 = d_htild_out;
   if (A->eng != ENG_SIMT) ZR_TRY(to_operand(d_h_t, A->H, A->Kpad, B, A->eng, A->sc_h, &h, st));
-  return att_forward(A, h, d_mask, B, out, d_align_out, st, g_att_viterbi_out);
+  // (the exact engine has no conversion ahead of the attention kernel, which is then the call's first launch)
+  return att_forward(A, h, d_mask, B, out, d_align_out, st, g_att_viterbi_out, -1.f, false, A->eng != ENG_SIMT);
 }
 int zrnn_att_forward_viterbi(zrnn_attention* A, const float* d_h_t, const int* d_mask, int B, float* d_htild_out,
                              int* d_viterbi_out, void* stream) {
