@@ -30,6 +30,9 @@ int zrnn_debug_decoder_timeline(long long* d_buf, int cta);
  * synchronisation returns ZRNN_E_TIMEOUT once; the context stays usable. */
 int zrnn_debug_bounded_wait(long long limit_cycles, void* stream);
 
+/* The gate functions of the LSTM kernels, elementwise over n device values: sigmoid and tanh of x. */
+int zrnn_debug_gates(const float* d_x, int n, float* d_sigmoid, float* d_tanh, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -299,3 +299,23 @@ def test_global_attention_right_behind_the_launch_that_writes_its_sources(api, d
     want = [step(i, True).cpu() for i in (0, 1)]
     for k in range(6):
         assert torch.equal(step(k % 2, False).cpu(), want[k % 2])
+
+
+def test_gate_functions(api):
+    """sigmoid and tanh of the LSTM kernels against float64: the absolute error that their comment states, small arguments of tanh to a
+    rounding or two of their own, saturation, infinities and NaN."""
+    import torch
+    mag = np.concatenate([np.logspace(-30, 2, 200001), np.linspace(0, 30, 1000001), [0.4, np.nextafter(np.float32(0.4), 0), 87.5, 88.8, 104.0, 1e30]])
+    x = np.concatenate([mag, -mag, [np.inf, -np.inf, np.nan]]).astype(np.float32)
+    dx = torch.as_tensor(x).cuda()
+    sig, th = torch.empty_like(dx), torch.empty_like(dx)
+    api.check(api.lib().zrnn_debug_gates(api._ptr(dx), x.size, api._ptr(sig), api._ptr(th), api._stream()))
+    sig, th, x = (v.astype(np.float64) for v in (sig.cpu().numpy(), th.cpu().numpy(), x))
+    assert np.isnan(sig[-1]) and np.isnan(th[-1])
+    assert list(sig[-3:-1]) == [1, 0] and list(th[-3:-1]) == [1, -1]
+    sig, th, x = sig[:-3], th[:-3], x[:-3]
+    with np.errstate(over="ignore"):
+        assert np.abs(sig - 1 / (1 + np.exp(-x))).max() < 1.2e-7
+    assert np.abs(th - np.tanh(x)).max() < 1.2e-7
+    small = (np.abs(x) < 0.4) & (np.abs(x) > 1e-30)
+    assert np.abs(th[small] / np.tanh(x[small]) - 1).max() < 2.0 ** -23

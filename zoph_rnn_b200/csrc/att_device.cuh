@@ -17,9 +17,10 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// The gates of the fp32-accurate tensor-core engines: absolute error of a rounding or two (1.2e-7), in 4 and about 16 instructions.
-// With expf, an IEEE division and tanhf the epilogue of a launch of four 1000-unit cells (128 columns) spent 2.5 of its 5 us on
-// issuing them.
+// The gates of the fp32-accurate tensor-core engines and of the sequence kernels of small layers (the exact engine's, too): absolute
+// error of a rounding or two (1.2e-7; 1 / (1 + expf(-x)): 0.9e-7, tanhf: 1.1e-7), in 4 and about 16 instructions.  With expf, an
+// IEEE division and tanhf the epilogue of a launch of four 1000-unit cells (128 columns) spent 2.5 of its 5 us on issuing them.
+// Log-probabilities of small language models (40 - 300 units) are as far from float64 with either, 3.0 - 4.7e-8 relative.
 __device__ __forceinline__ float exp2_fast(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -134,6 +134,16 @@ cudaError_t launch_src_len(const int* mask01, int T, int B, int* len, int* offse
   count_launch();
   return launch_chain(src_len_kernel, dim3((B + 127) / 128), dim3(128), 0, st, mask01, T, B, len, offset);
 }
+__global__ void gates_kernel(const float* __restrict__ x, int n, float* __restrict__ sig, float* __restrict__ th) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) { sig[i] = sigmoid_f32(x[i]); th[i] = tanh_f32(x[i]); }
+}
+cudaError_t launch_gates(const float* x, int n, float* sig, float* th, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  gates_kernel<<<(n + 255) / 256, 256, 0, st>>>(x, n, sig, th);
+  count_launch();
+  return cudaGetLastError();
+}
 __global__ void div_map_kernel(int* map, int n, int div) {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -283,6 +283,8 @@ cudaError_t launch_convert_rows(const float* src, long long rows, int K, long lo
                                 float* dst_lo, long long ld_dst, cudaStream_t st);
 
 // misc
+// sigmoid_f32 / tanh_f32 (att_device.cuh) elementwise: developer entry point
+cudaError_t launch_gates(const float* x, int n, float* sig, float* th, cudaStream_t st);
 // len[b] = number of unmasked steps of column b in mask[T x B]; offset[b] = T - len[b]
 // (the reference's batch_info, src/fileHelper.h:480-496)
 cudaError_t launch_src_len(const int* mask01, int T, int B, int* len, int* offset, cudaStream_t st);

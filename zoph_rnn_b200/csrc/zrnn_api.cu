@@ -968,6 +968,12 @@ int zrnn_debug_bounded_wait(long long limit_cycles, void* stream) {
   return ZRNN_OK;
 }
 
+int zrnn_debug_gates(const float* d_x, int n, float* d_sigmoid, float* d_tanh, void* stream) {
+  ZR_CHECK(d_x && d_sigmoid && d_tanh && n >= 0, "debug_gates: bad arguments");
+  ZR_CUDA(zrnn::launch_gates(d_x, n, d_sigmoid, d_tanh, (cudaStream_t)stream));
+  return ZRNN_OK;
+}
+
 int zrnn_tc_error(void) {
   return take_error_code();
 }
