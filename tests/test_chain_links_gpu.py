@@ -102,7 +102,7 @@ def test_ragged_batch_equals_single_sentences(beam):
 
 @pytest.mark.parametrize("dtype", [5, 1, 4, 2])
 @pytest.mark.parametrize("H,V,N", [(64, 130, 1), (72, 257, 15), (200, 1000, 16), (504, 1281, 17), (1000, 40000, 12), (512, 20001, 63),
-                                   (1000, 5000, 65), (264, 19001, 128), (264, 19001, 129), (504, 20000, 200), (800, 5003, 256), (800, 5003, 257)])
+                                   (1000, 5000, 65), (264, 19001, 128), (264, 19001, 129), (504, 20000, 200), (800, 5003, 144), (800, 5003, 145), (800, 5003, 256), (800, 5003, 257)])
 def test_vocabulary_projection_edges(dtype, H, V, N):
     """Best words, their log-probabilities and the target's, on both sides of the column count where the kernel changes."""
     import torch

@@ -1,4 +1,4 @@
-// Vocabulary projection for few batch columns (128, split modes 256) on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
+// Vocabulary projection for few batch columns (128, split modes 144 where K is long) on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
 //
 // The weights are the M side of the MMA (128 vocabulary rows) and the columns its N side, padded to a multiple of 16 only: with
 // the columns as the M side (tc_gemm.cu) a step of 12 columns multiplied 128 padded rows, 19 us of MMAs for 160 MB of weights, and
@@ -9,7 +9,7 @@
 // Persistent CTAs walk over the vocabulary, the accumulators are double-buffered in TMEM (while 512 columns hold two) and the loads
 // run ahead across tiles.  Up to 64 columns a CTA takes half an SM (113 KB, 256 TMEM columns), so that it is resident, and streams
 // its first weights, while the kernel before it runs.  us per launch, before -> now, f32: 12 columns x 40000 words x 1000: 48 -> 31
-// (HBM: 25); 130 - 250 columns x 50000 words x 1000: 128 -> 84.  Marking the weights to leave the L2 first changes nothing.
+// (HBM: 25).  Marking the weights to leave the L2 first changes nothing.
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>

@@ -5,11 +5,14 @@
 
 namespace zrnn {
 
-constexpr int kVocabMaxCols = 256;
-// Beyond 128 columns the split modes have room for one accumulator only, so a tile's epilogue is not hidden: that pays, against
-// fetching the weights twice, where K is long (kb k-blocks; us per launch, 130 - 200 columns: K = 1000 84 against 128, K = 500 33
-// against 28).
-inline int vocab_max_cols(int mode, int kb) { return (mode == TC_TF32X3 || mode == TC_F16X2) && kb >= 12 ? 256 : 128; }
+constexpr int kVocabMaxCols = 144;
+// Beyond 128 columns the split modes have room for one accumulator only, so a tile's epilogue is not hidden.  Against the kernel of
+// many columns, which fetches the weights twice, that pays for one more group of 16 columns and from K = 768 on (kb k-blocks of 128
+// bytes).  us per beam step of a 2-layer model, here / there, at 144, 152 and 168 columns:
+//   fp16 split, K = 1000, 50000 words 173 / 178, 185 / 181, 189 / 182;  K = 768, 50000 words 143 / 146, 157 / 147, 159 / 147
+//   3xTF32,     K = 1000, 50000 words 278 / 297, 288 / 301, 303 / 304;  K = 640, 40000 words 191 / 190, 203 / 191, 213 / 192
+// (252 columns, K = 1000: 220 / 192 and 342 / 316.)
+inline int vocab_max_cols(int mode, int kb) { return (mode == TC_F16X2 && kb >= 12) || (mode == TC_TF32X3 && kb >= 24) ? 144 : 128; }
 
 // z[v, m] = W[v] . h[m] + bias[v] for v < N, m < M
 struct VocabParams {
