@@ -24,3 +24,10 @@ def test_a_split_link_that_gave_up_waits_for_its_partner():
     waits = re.findall(r"mbar_wait(?:_cluster)?\(([^;]*?), p\.err, \d\)", s)
     assert len(waits) == len(re.findall(r"\bmbar_wait(?:_cluster)?\(", s)) and all(w.endswith("&ct.abort") for w in waits)
     assert s.rindex("__syncthreads()") > s.rindex("mbar_wait")
+
+
+def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
+    """A link kernel requests its weights before it waits for the launch ahead of it.  In the stand-alone product the weights are packed by a
+    launch of the same call, so another launch, which waits for that one, has to lie between."""
+    s = body("zrnn_api.cu", "int zrnn_gemm(", "zrnn_tc_error()")
+    assert s.index("launch_pack_weights(") < s.index("launch_convert_rows(") < s.index("launch_tc_chain(")

@@ -2983,12 +2983,13 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
   char *a_hi = buf.as<char>(), *b_hi = a_hi + a_part * parts;
   auto run = [&]() -> int {
     ZR_CUDA(cudaMemsetAsync(b_hi, 0, b_part * parts, st));
-    ZR_CUDA(zrnn::launch_convert_rows(d_X, m_cols, K, ldx, op_mode, a_hi, (float*)(a_hi + a_part), Kpad, st));
     zrnn::PackArgs pk;
     std::memset(&pk, 0, sizeof(pk));
     pk.src[0] = d_W; pk.G = 1; pk.H = n_rows; pk.K = K; pk.lda = ldw; pk.TH = 128; pk.n_tiles = n_tiles;
     pk.dst_hi = b_hi; pk.dst_lo = (float*)(b_hi + b_part); pk.op_mode = op_mode; pk.ld_dst = Kpad; pk.koff = 0;
     ZR_CUDA(zrnn::launch_pack_weights(pk, st));
+    // second: the product requests its weights while the launch ahead of it runs, so that must not be the one that writes them
+    ZR_CUDA(zrnn::launch_convert_rows(d_X, m_cols, K, ldx, op_mode, a_hi, (float*)(a_hi + a_part), Kpad, st));
     zrnn::ChainBatch cb;
     zrnn::ChainParams& p = cb.p[0];
     std::memset(&p, 0, sizeof(p));
