@@ -162,6 +162,27 @@ def test_nan_scores_are_no_candidates(api, dtype, beam):
         np.testing.assert_array_equal(a, b)
 
 
+def test_ensemble_that_fails_midway_leaves_the_models_usable(api):
+    """The second model's source is longer than the attention layer takes, which shows when its encoder is on its way on a stream of its
+    own.  After the error both models, alone and together, give what they gave before."""
+    cfg = synth.make_cfg(1, 64, 60, 500, attention=2, feed_input=1)
+    models = [build(api, cfg, synth.make_weights(cfg, seed=s, scale=0.3), 0) for s in (1, 2)]
+    rng = np.random.default_rng(4)
+    srcs = [rng.integers(2, 60, n).astype(np.int32) for n in (5, 2, 9)]
+    long = [rng.integers(2, 60, 10001).astype(np.int32)] + srcs[1:]
+    kw = dict(beam=4, k_best=2, max_ratio=1.5, longest_sent=20)
+    calls = [lambda: models[0].decode(srcs, **kw), lambda: models[1].decode(srcs, **kw),
+             lambda: api.decode_ensemble(models, [srcs, srcs], **kw)]
+    want = [c() for c in calls]
+    for _ in range(2):
+        with pytest.raises(api.ZrnnError) as e:
+            api.decode_ensemble(models, [srcs, long], **kw)
+        assert e.value.status == 1 and "S_max" in str(e.value)
+        for c, w in zip(calls, want):
+            for a, b in zip(c(), w):
+                np.testing.assert_array_equal(a, b)
+
+
 def test_two_devices_in_one_process(api):
     """zrnn_set_device lets one process put models on several devices in turn: per-device state inside the library
     (kernel attributes, error word, scratch addresses) must not leak from one device to the other."""

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <set>
 #include <string>
 #include <vector>
@@ -2424,8 +2425,10 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
   std::vector<cudaStream_t> lane(K, s);
   if (!g_kt.on)
     for (int k = 1; k < K; ++k) lane[k] = models[k]->stream;
+  bool apart = false;  // between a fork and the next join
   auto fork = [&]() -> int {
     if (K == 1) return ZRNN_OK;
+    apart = true;
     ZR_CUDA(cudaEventRecord(m0->ev, s));
     for (int k = 1; k < K; ++k)
       if (lane[k] != s) ZR_CUDA(cudaStreamWaitEvent(lane[k], m0->ev, 0));
@@ -2437,8 +2440,17 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
         ZR_CUDA(cudaEventRecord(models[k]->ev, lane[k]));
         ZR_CUDA(cudaStreamWaitEvent(s, models[k]->ev, 0));
       }
+    apart = false;
     return ZRNN_OK;
   };
+  // a search that ends with an error leaves nothing running that the caller's stream does not wait for
+  struct OnExit {
+    std::function<void()> f;
+    ~OnExit() { f(); }
+  } join_at_exit{[&]() {
+    for (int k = 1; k < K && apart; ++k)
+      if (lane[k] != s && cudaEventRecord(models[k]->ev, lane[k]) == cudaSuccess) cudaStreamWaitEvent(s, models[k]->ev, 0);
+  }};
   ZR_TRY(fork());
   for (int k = K - 1; k >= 0; --k) ZR_TRY(bm[k].encode(d_src[k], sorted ? nullptr : d_order, lane[k]));
 
