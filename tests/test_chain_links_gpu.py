@@ -56,6 +56,26 @@ def test_cell_edges(dtype, H, B, feed):
     np.testing.assert_allclose(got_c.cpu().numpy().reshape(B, H), cn * mask[:, None], rtol=r, atol=a)
 
 
+@pytest.mark.parametrize("dtype", sorted(TOL))
+@pytest.mark.parametrize("H,B", [(72, 1), (104, 9), (264, 16), (500, 17), (504, 33), (520, 64), (1000, 8), (1000, 65), (1000, 127), (1000, 129), (324, 200)])
+def test_scoring_with_early_operands_edges(dtype, H, B):
+    """A scoring pass with feed-input at the same edges: there every cell but the first, and the combiner, multiplies by operands that were
+    complete earlier before it waits for its predecessor (the layer calls above have none).  Log-probabilities against the float64
+    witness; three target steps, ragged sentences."""
+    from oracle import ref_numpy
+    from zoph_rnn_b200 import api, synth
+    if dtype == 1 and H % 8:
+        pytest.skip("bf16 needs a multiple of 8")
+    cfg = synth.make_cfg(2, H, 60, 90, attention=2, feed_input=1)
+    w = synth.make_weights(cfg, seed=H + B, dist="normal", scale=1 / np.sqrt(H))
+    m = api.neuralMT_model(cfg, dtype=dtype)
+    m.load_weights(w)
+    src, tin, tout = synth.make_s2s_batch(60, 90, B, 1, 3, 2, 3, seed=B)
+    got, _ = m.get_error(src, tin, tout)
+    r, a = TOL[dtype]
+    np.testing.assert_allclose(got, ref_numpy.score_batch(cfg, w, src, tin, tout), rtol=r, atol=a)
+
+
 @pytest.mark.parametrize("dtype", [5, 1, 4])
 @pytest.mark.parametrize("H,B", [(72, 1), (200, 12), (504, 40), (1000, 64), (1000, 130)])
 @pytest.mark.parametrize("att", [1, 2])
