@@ -333,7 +333,9 @@ def measure(args, w, cfg, dtype, rank, world, steps=None, parity=False):
         step_device()
         torch.cuda.synchronize()
         tokens_per_step = int(np.maximum(d_len.cpu().numpy() - 1, 0).sum())  # emitted 1-best tokens incl. <EOF>
-        ncols = n * synth.beam_cap(w["beam"], w["Vt"])
+        # columns of a step's launches on average: a step covers the sentences that are still running
+        limits = np.minimum((w["max_ratio"] * lens).astype(int), Lmax - 2) + 1
+        ncols = synth.beam_cap(w["beam"], w["Vt"]) * float(limits.sum()) / int(limits.max())
     else:
         src, tin, tout = inp["src"], inp["tin"], inp["tout"]
         T, B = tin.shape
@@ -629,24 +631,16 @@ def summary(name, w, cfg, r, dtype, peaks, peak_src, full):
     return out
 
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch of the LSTM cell kernel on an 8-matrix
-# layer (no feed-input operand) from an ncu capture, keyed by (kernel class, dtype, H, B): a figure applies only to the
-# shape it was captured on; every other shape reports null.  The capture ran the c2s workload, whose layer shapes are
-# configuration 2's.
-NCU_TRAFFIC = {("lstm_cell", "f32", 1000, 128): 35.2e6, ("lstm_cell", "f32_f16x2", 1000, 128): 35.2e6,
-               ("lstm_cell", "f32_3xtf32", 1000, 128): 71.6e6, ("lstm_cell", "bf16", 1000, 128): 17.9e6}
-
-
 def roofline(w, cfg, ktime, peaks, peak_src, softmax_cols, dtype):
     """Roofline of the dominant kernel class.  Durations are CUDA-event pairs around every launch of the class in
     the instrumented pass (one pair per encoder layer sweep).  Algorithmic bytes per LSTM cell launch: the layer's
     H x H weight matrices as stored (4 or 2 bytes each) plus 5 H x B fp32 activations; flops of the softmax GEMM:
-    2 V H N."""
+    2 V H N (decoding: N averaged over the steps, whose launches cover the sentences that are still running)."""
     if not ktime:
         return None
     top = max(ktime, key=lambda k: ktime[k]["ms"])
     H = cfg["H"]
-    B = w["B"] * (w.get("beam", 1) if w["kind"] == "decode" else 1)
+    B = softmax_cols if w["kind"] == "decode" else w["B"]
     n = ktime[top]["launches"]
     avg_s = ktime[top]["ms"] / 1e3 / max(n, 1)
     wbytes = 2 if dtype == "bf16" else 4   # bytes per weight as the reference stores them (fp32) or bf16
@@ -670,12 +664,6 @@ def roofline(w, cfg, ktime, peaks, peak_src, softmax_cols, dtype):
         if cfg["feed_input"] and not cfg["lm"]:
             mats = (8.0 * (2 * L - 1) + 12.0) / (2 * L) if w["kind"] != "decode" else (8.0 * (L - 1) + 12.0) / L
         alg = mats * H * H * wbytes + (4 * H + 5.0 * H * B) * 4
-        cap = NCU_TRAFFIC.get((top, dtype, H, B))
-        if cap:  # captured on an 8-matrix launch; the average launch of this workload holds `mats` matrices
-            alg8 = 8.0 * H * H * wbytes + (4 * H + 5.0 * H * B) * 4
-            out["traffic"] = cap * alg / alg8
-            out["traffic_note"] = ("ncu capture of an 8-matrix cell launch of this shape, scaled by the algorithmic "
-                                   "bytes of the workload's average launch")
         out.update(bound="hbm", unit="GB/s", peak=float(peaks.get("hbm_gbs", 6650.0)), achieved=alg / avg_s / 1e9,
                    algorithmic_bytes_per_launch=alg,
                    note=f"avg {mats:.2f} HxH matrices of {wbytes}-byte weights + 5 HxB fp32 activations per launch")

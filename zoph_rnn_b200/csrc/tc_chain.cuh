@@ -6,7 +6,7 @@
 
 namespace zrnn {
 
-// acc[M x N] = sum_s A_s[M x K] * W[N x Kcat]^T as in tc_gemm.cuh; M: batch columns, N: weight rows
+// acc[M x N] = sum_s A_s[M x K] * W[N x Kcat]^T, both operands K-major; M: batch columns, N: weight rows
 struct ChainParams {
   CUtensorMap a[3];           // activation rows: make_rows_map with a_rows rows, all parts, kbs k-blocks
   CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units (BN == 256: 32 units,
@@ -24,7 +24,7 @@ struct ChainParams {
   float* C;                   // fp32 out, row m at C + m * ldc
   int ldc;
   int act, act_rows;          // STORE: tanh for n < act_rows (0 = all) when act == 1
-  __nv_bfloat16* op_b16;      // operand-form copies of the output (row m at + m * ld_op), as TcParams
+  __nv_bfloat16* op_b16;      // operand-form copies of the output for the next product (row m at + m * ld_op)
   float* op_hi;
   float* op_lo;
   __half* op_h_hi;

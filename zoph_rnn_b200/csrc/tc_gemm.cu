@@ -54,8 +54,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const int total_tiles = m_tiles * n_tiles;
   ZR_STAMP(0);
-  int kb_per_tile = 0;
-  for (int s = 0; s < p.nsrc; ++s) kb_per_tile += p.kblocks[s];
+  const int kb_per_tile = p.kblocks;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < ST; ++s) {
@@ -88,20 +87,18 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * 128, n0 = (tile / m_tiles) * BN;
-        for (int s = 0; s < p.nsrc && ok; ++s) {
-          for (int kb = 0; kb < p.kblocks[s]; ++kb, ++it) {
-            const int st = it % ST;
-            const uint32_t ph = (uint32_t)((it / ST) & 1);
-            if (!mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
-            uint8_t* base = tiles + (size_t)st * STAGE;
-            mbar_expect_tx(&full_bar[st], (uint32_t)STAGE);
-            const int kx = kb * mode_epk(MODE);
-            tma_load_2d(base, &p.a[s], &full_bar[st], kx, m0);
-            tma_load_2d(base + kABytes, &p.b, &full_bar[st], p.b_koff[s] + kx, n0);
-            if (mode_split(MODE)) {
-              tma_load_2d(base + kABytes + BBYTES, &p.a_lo[s], &full_bar[st], kx, m0);
-              tma_load_2d(base + 2 * kABytes + BBYTES, &p.b_lo, &full_bar[st], p.b_koff[s] + kx, n0);
-            }
+        for (int kb = 0; kb < kb_per_tile; ++kb, ++it) {
+          const int st = it % ST;
+          const uint32_t ph = (uint32_t)((it / ST) & 1);
+          if (!mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
+          uint8_t* base = tiles + (size_t)st * STAGE;
+          mbar_expect_tx(&full_bar[st], (uint32_t)STAGE);
+          const int kx = kb * mode_epk(MODE);
+          tma_load_2d(base, &p.a, &full_bar[st], kx, m0);
+          tma_load_2d(base + kABytes, &p.b, &full_bar[st], kx, n0);
+          if (mode_split(MODE)) {
+            tma_load_2d(base + kABytes + BBYTES, &p.a_lo, &full_bar[st], kx, m0);
+            tma_load_2d(base + 2 * kABytes + BBYTES, &p.b_lo, &full_bar[st], kx, n0);
           }
         }
       }
@@ -150,9 +147,9 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
     float* xp = reinterpret_cast<float*>(tiles + (size_t)ST * STAGE) + warp * 1024;
     // Stores go through the warp's transposition buffer so that every store instruction writes whole 128-byte lines
     // (a thread per output row would scatter 16-byte pieces over 32 lines).  That needs 16-byte aligned rows; any
-    // other layout, and launches that also emit operand copies, take the per-row path.
-    const bool fast_store = EPI == TC_EPI_STORE && p.C && (p.ldc & 3) == 0 && (p.N & 3) == 0 &&
-                            (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && !p.op_b16 && !p.op_hi && !p.op_h_hi;
+    // other layout takes the per-row path.
+    const bool fast_store = EPI == TC_EPI_STORE && (p.ldc & 3) == 0 && (p.N & 3) == 0 &&
+                            (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     int ti = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++ti) {
       const int buf = ti & 1;
@@ -168,7 +165,6 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
       tc_fence_after();
       asm volatile("bar.sync 1, 256;" ::: "memory");  // the new bias values are visible
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC_COLS + half * HC);
-      const float mk = (p.mask && row_ok) ? (float)p.mask[row] : 1.0f;
       const int n0 = n_tile * BN + half * HC;  // first output column of this warp
       const float* sb = s_bias + half * HC;
       const size_t pi = (size_t)(n_tile * kPersistentParts + half) * p.M + row;
@@ -196,11 +192,8 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
             const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              float t = v[u + e] + bb[e];
-              if (p.act == 1 && (p.act_rows == 0 || nb + u + e < p.act_rows)) t = act_tanh<MODE>(t);
-              t *= mk;
-              v[u + e] = t;
-              if (u + e < nvalid) cm = fmaxf(cm, t);
+              v[u + e] += bb[e];
+              if (u + e < nvalid) cm = fmaxf(cm, v[u + e]);
             }
           }
           if (want_lse) {
@@ -244,8 +237,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
                 float x8[8];  // a copy: the ragged tail indexes it dynamically, which must not push v out of registers
 #pragma unroll
                 for (int u = 0; u < 8; ++u) x8[u] = v[8 * g + u];
-                if (p.C) store8_f32(p.C, (size_t)row * p.ldc + nb + 8 * g, x8, nv);
-                store8_operand(p, (size_t)row * p.ld_op + nb + 8 * g, x8, nv);
+                store8_f32(p.C, (size_t)row * p.ldc + nb + 8 * g, x8, nv);
               }
             }
           }

@@ -1,8 +1,8 @@
 // Blackwell tensor-core GEMM family (tcgen05.mma with TMEM accumulators, TMA-fed shared-memory ring):
-//   acc[M x N] = sum_s A_s[M x K_s] * B[N x Kcat]^T        (both operands K-major)
+//   acc[M x N] = A[M x K] * B[N x K]^T        (both operands K-major)
 // M indexes batch columns (the reference's H x B activations are already "B rows of K contiguous values"),
 // N indexes weight rows, so every epilogue thread owns one batch column and sees all N outputs of its row: the softmax's
-// max / sum-exp and the bias + tanh + mask are thread-local.  The recurrent cells and the attention products are in tc_chain.cuh.
+// max / sum-exp and the bias are thread-local.  The recurrent cells and the attention products are in tc_chain.cuh.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -15,29 +15,17 @@ enum { TC_BF16 = 0, TC_TF32 = 1, TC_TF32X3 = 2, TC_F16X2 = 3 };
 enum { TC_EPI_STORE = 0, TC_EPI_LSTM = 1, TC_EPI_LSE = 2 };
 
 struct TcParams {
-  CUtensorMap a[3];     // A operand per source (bf16, or fp32 "hi" = values representable in tf32)
-  CUtensorMap a_lo[3];  // TC_TF32X3: fp32 residuals a - a_hi
-  CUtensorMap b;        // weights, rows = packed output rows, K = concatenated (padded) sources
-  CUtensorMap b_lo;     // TC_TF32X3
-  int nsrc;
-  int kblocks[3];  // 128-byte k-blocks per source
-  int b_koff[3];   // element offset of each source inside B's K axis
-  int M;           // batch columns
-  int N;           // output rows
+  CUtensorMap a;     // activations (split modes: their hi part)
+  CUtensorMap a_lo;  // split modes: the lo part
+  CUtensorMap b;     // weights, a row per output
+  CUtensorMap b_lo;
+  int kblocks;        // 128-byte k-blocks
+  int M;              // batch columns
+  int N;              // output rows
   const float* bias;  // [N]
-  const int* mask;    // [M] or null
-  // --- STORE: C[n + m*ldc] = act(acc + bias[n]) * mask[m]
+  // --- STORE: C[n + m*ldc] = acc + bias[n]
   float* C;
   int ldc;
-  int act;       // 0 none, 1 tanh
-  int act_rows;  // act applies to n < act_rows (0 = all)
-  // optional A-operand copies of the output for the next GEMM (row m at + m*ld_op)
-  __nv_bfloat16* op_b16;
-  float* op_hi;
-  float* op_lo;
-  __half* op_h_hi;  // TC_F16X2 consumers: fp16 hi part and scaled fp16 lo part
-  __half* op_h_lo;
-  int ld_op;
   // --- LSE: per (N tile, m) max and sum exp(z - max) of z = acc + bias, plus the logit of target[m]
   const int* target;
   int target_offset;

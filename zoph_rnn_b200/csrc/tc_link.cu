@@ -38,8 +38,8 @@ constexpr int kMaxStages = 8;
 // of their own in registers (round to nearest).  Up to 512 elements per source (8 k-blocks of fp16, 16 of tf32) an accumulator absorbs
 // 4 k-steps, beyond that 8.  Hidden states of a scoring pass against float64 (uniform weights +-0.08, fp16 split), 16 / 8 / 4 k-steps:
 // 2 layers x 512, 100 columns 5.5 / 3.2 / 2.1e-7, 1 x 1024, 30 columns 6.1 / 3.4 / 2.3e-7, 4 x 1000, 64 columns 15 / 9.6 / 7.5e-7.
-// A round more costs a commit, a wait and a drain: three cells of 500 units and 50 columns in a launch take 11.2 instead of 10.0 us,
-// cells of 1000 units in 8 k-steps what they took in 16 (+2 % of a step of 64 columns).
+// Every round costs a commit, a wait and a drain: a launch of three cells of 500 units and 50 columns takes 1.2 us longer in 4 k-steps
+// than in 16, a target step of 2 x 1000, 64 columns in 8 k-steps 2 % longer than in 16.
 __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 2 : 4; }
 // Split modes multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the columns for two products (an MMA of 128 rows
 // takes 45 cycles up to 32 columns, 48 at 64, 64 at 128), and A_lo by W_hi: two MMAs per k-step instead of three.

@@ -687,8 +687,8 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   }
   zrnn::TcParams tp;
   std::memset(&tp, 0, sizeof(tp));
-  ZR_TRY(act_maps(h, eng, H, S->Kpad, N, &tp.a[0], &tp.a_lo[0]));
-  tp.nsrc = 1; tp.kblocks[0] = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng)); tp.b_koff[0] = 0;
+  ZR_TRY(act_maps(h, eng, H, S->Kpad, N, &tp.a, &tp.a_lo));
+  tp.kblocks = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
   tp.b = S->dmap; tp.b_lo = S->dmap_lo;
   tp.M = N; tp.N = Vs; tp.bias = S->b;
   tp.target = targets; tp.target_offset = S->lo;
@@ -745,8 +745,8 @@ int softmax_logits_act(zrnn_softmax* S, const Act& h, int N, cudaStream_t st, co
     ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
     zrnn::TcParams tp;
     std::memset(&tp, 0, sizeof(tp));
-    ZR_TRY(act_maps(h, eng, S->H, S->Kpad, N, &tp.a[0], &tp.a_lo[0]));
-    tp.nsrc = 1; tp.kblocks[0] = (S->H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng)); tp.b_koff[0] = 0;
+    ZR_TRY(act_maps(h, eng, S->H, S->Kpad, N, &tp.a, &tp.a_lo));
+    tp.kblocks = (S->H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
     tp.b = S->dmap; tp.b_lo = S->dmap_lo;
     tp.M = N; tp.N = Vs; tp.bias = S->b; tp.C = S->logits.as<float>(); tp.ldc = Vs;
     // the epilogue also leaves each tile's maximum and exp-sum: the top-k kernel derives the normaliser and its
