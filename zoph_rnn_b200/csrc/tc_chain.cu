@@ -62,7 +62,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   __shared__ int abort_s;
   __shared__ float s_bias[BN];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const int m0 = m_block * 128, n_tile = blockIdx.y;
   const int akb = p.a_rows * 128;  // bytes of one k-block of one activation part
@@ -102,30 +102,34 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
 
   if (warp == kWWarp) {
     // ------------------------------------------------------------ weights: nothing here depends on the predecessor
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       bool ok = true;
       int it = 0, st = 0;
       uint32_t ph = 0;
       int s = 0, c = 0;
       for (; it < n_it; ++it) {
-        if (it >= stages && !mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
+        if (it >= stages && !mbar_wait_warp(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
         uint8_t* w = tiles + (size_t)st * stage_bytes + PARTS * KBS * akb;
-        mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * WKB));
         const int wkb = p.wkb0[s] + c * KBS;
-        if constexpr (EPI == TC_EPI_LSTM && BN <= 128) {
-          constexpr int TH = BN / 4;
-          tma_load_5d(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
-        } else if constexpr (EPI == TC_EPI_LSTM) {  // rows of several packed tiles side by side: one box per k-block, tile and part
-          constexpr int NP = BN / 128;
-          for (int b = 0; b < KBS; ++b)
-            for (int h = 0; h < NP; ++h)
-              for (int x = 0; x < PARTS; ++x) {
-                const int tile = min(n_tile * NP + h, p.w_tiles - 1);  // (the units of a tile beyond the last are dropped)
-                tma_load_5d(w + (b * PARTS + x) * WKB + h * (WKB / NP), &p.w, &full_bar[st], 0, x, tile * p.w_kbtot + wkb + b);
-              }
-        } else {
-          tma_load_4d(w, &p.w, &full_bar[st], n_tile * BN, wkb);
+        if (one) {
+          mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * WKB));
+          if constexpr (EPI == TC_EPI_LSTM && BN <= 128) {
+            constexpr int TH = BN / 4;
+            tma_load_5d(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
+          } else if constexpr (EPI == TC_EPI_LSTM) {  // rows of several packed tiles side by side: one box per k-block, tile and part
+            constexpr int NP = BN / 128;
+            for (int b = 0; b < KBS; ++b)
+              for (int h = 0; h < NP; ++h)
+                for (int x = 0; x < PARTS; ++x) {
+                  const int tile = min(n_tile * NP + h, p.w_tiles - 1);  // (the units of a tile beyond the last are dropped)
+                  tma_load_5d(w + (b * PARTS + x) * WKB + h * (WKB / NP), &p.w, &full_bar[st], 0, x, tile * p.w_kbtot + wkb + b);
+                }
+          } else {
+            tma_load_4d(w, &p.w, &full_bar[st], n_tile * BN, wkb);
+          }
         }
+        __syncwarp();
         if (++st == stages) { st = 0; ph ^= 1u; }
         if (++c == src_it) { c = 0; ++s; }
       }
@@ -137,17 +141,21 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
     pdl_wait();
     if (warp == kAWarp) {
       // ------------------------------------------------------------ activations
-      if (lane == 0) {
-        pdl_trigger();  // after the wait: the successor may read what this kernel's predecessor left (tc_link.cu)
+      {
+        const bool one = elect_one();
+        if (one) pdl_trigger();  // after the wait: the successor may read what this kernel's predecessor left (tc_link.cu)
         bool ok = true;
         int it = 0, st = 0;
         uint32_t ph = 0;
         int s = 0, c = 0;
         for (; it < n_it; ++it) {
-          if (it >= stages && !mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 7)) { ok = false; break; }
+          if (it >= stages && !mbar_wait_warp(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 7)) { ok = false; break; }
           uint8_t* a = tiles + (size_t)st * stage_bytes;
-          mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * akb));
-          tma_load_4d(a, &p.a[s], &full_bar[st], p.a_row0[s] + m0, c * KBS);
+          if (one) {
+            mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * akb));
+            tma_load_4d(a, &p.a[s], &full_bar[st], p.a_row0[s] + m0, c * KBS);
+          }
+          __syncwarp();
           if (++st == stages) { st = 0; ph ^= 1u; }
           if (++c == src_it) { c = 0; ++s; }
         }
@@ -155,7 +163,8 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       }
     } else if (warp >= kMmaWarp) {
       // ------------------------------------------------------------ MMA issuers
-      if (lane == 0) {
+      {
+        const bool one = elect_one();
         const int mw = warp - kMmaWarp;
         bool ok = true;
         const bool rounds = ROUNDS && !(BY_PRODUCT && mw == 1);
@@ -164,37 +173,40 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         for (int it = st; it < n_it; it += STEP) {
           if (rounds && in_round == 0) {
             set = BY_PRODUCT ? round % NBUF : mw + kMmaWarps * (round % NBUF);
-            if (round >= NBUF && !mbar_wait(&set_empty[set], (uint32_t)((round / NBUF) & 1) ^ 1u, &abort_s, p.err, 4)) { ok = false; break; }
+            if (round >= NBUF && !mbar_wait_warp(&set_empty[set], (uint32_t)((round / NBUF) & 1) ^ 1u, &abort_s, p.err, 4)) { ok = false; break; }
             tc_fence_after();
           }
-          if (!mbar_wait(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
           const uint32_t d = tmem_base + (uint32_t)(set * BN), d_cross = tmem_base + (uint32_t)(NSET * BN);
           const bool fresh = rounds ? in_round == 0 : it < STEP;  // the accumulator starts with this stage
-          for (int b = 0; b < KBS; ++b) {
-            const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
-            const uint64_t dw = make_smem_desc(w_addr + b * PARTS * WKB), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * WKB);
+          if (one) {
+            for (int b = 0; b < KBS; ++b) {
+              const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
+              const uint64_t dw = make_smem_desc(w_addr + b * PARTS * WKB), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * WKB);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint32_t acc = (!fresh || b > 0 || k > 0) ? 1u : 0u;
-              if (!BY_PRODUCT || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC, acc);
-              if (BY_PRODUCT && mw == 1) {
-                umma<mode_kind_tf32(MODE)>(d_cross, dal + 2 * k, dw + 2 * k, IDESC, acc);
-                umma<mode_kind_tf32(MODE)>(d_cross, da + 2 * k, dwl + 2 * k, IDESC, 1u);
+              for (int k = 0; k < 4; ++k) {
+                const uint32_t acc = (!fresh || b > 0 || k > 0) ? 1u : 0u;
+                if (!BY_PRODUCT || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC, acc);
+                if (BY_PRODUCT && mw == 1) {
+                  umma<mode_kind_tf32(MODE)>(d_cross, dal + 2 * k, dw + 2 * k, IDESC, acc);
+                  umma<mode_kind_tf32(MODE)>(d_cross, da + 2 * k, dwl + 2 * k, IDESC, 1u);
+                }
               }
             }
+            umma_commit(&empty_bar[st]);
           }
-          umma_commit(&empty_bar[st]);
+          __syncwarp();
           if (rounds && (++in_round == round_its || it + STEP >= n_it)) {
-            umma_commit(&set_full[set]);
+            if (one) umma_commit(&set_full[set]);
             in_round = 0;
             ++round;
           }
           st += STEP;
           if (st >= stages) { st -= stages; ph ^= 1u; }
         }
-        if (ok && !rounds) umma_commit(&accum_bar);
+        if (ok && !rounds && one) umma_commit(&accum_bar);
       }
     }
   }

@@ -56,6 +56,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
   return true;
 }
+// Roles of one warp (loads, MMA issue) run with all of its lanes and let one of them issue.  Their instructions take descriptors, barrier
+// and tensor-memory addresses from uniform registers; in a loop of a single thread every one of those is moved there anew: 62 cycles
+// per MMA and 400 per stage (bf16, 128 x 64 x 64: 648 cycles a stage against 415 with a whole warp; fp16 split, 128 x 64: 908 / 667).
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// mbar_wait by a whole warp
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code));
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

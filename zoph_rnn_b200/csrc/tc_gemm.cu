@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
   // bias values of the tile whose epilogue is running (two named barriers per tile order its refill)
   __shared__ __align__(16) float s_bias[BN];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const int total_tiles = m_tiles * n_tiles;
   ZR_STAMP(0);
@@ -82,24 +82,28 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
 
   if (warp == 8) {
     // ------------------------------------------------------------ TMA producer (runs ahead across tiles)
-    if (lane == 0 && kb_per_tile > 0) {
-      int it = 0;
+    if (kb_per_tile > 0) {
+      const bool one = elect_one();
+      int st = 0;
+      uint32_t ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % m_tiles) * 128, n0 = (tile / m_tiles) * BN;
-        for (int kb = 0; kb < kb_per_tile; ++kb, ++it) {
-          const int st = it % ST;
-          const uint32_t ph = (uint32_t)((it / ST) & 1);
-          if (!mbar_wait(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
+        for (int kb = 0; kb < kb_per_tile; ++kb) {
+          if (!mbar_wait_warp(&empty_bar[st], ph ^ 1u, &abort_s, p.err, 1)) { ok = false; break; }
           uint8_t* base = tiles + (size_t)st * STAGE;
-          mbar_expect_tx(&full_bar[st], (uint32_t)STAGE);
           const int kx = kb * mode_epk(MODE);
-          tma_load_2d(base, &p.a, &full_bar[st], kx, m0);
-          tma_load_2d(base + kABytes, &p.b, &full_bar[st], kx, n0);
-          if (mode_split(MODE)) {
-            tma_load_2d(base + kABytes + BBYTES, &p.a_lo, &full_bar[st], kx, m0);
-            tma_load_2d(base + 2 * kABytes + BBYTES, &p.b_lo, &full_bar[st], kx, n0);
+          if (one) {
+            mbar_expect_tx(&full_bar[st], (uint32_t)STAGE);
+            tma_load_2d(base, &p.a, &full_bar[st], kx, m0);
+            tma_load_2d(base + kABytes, &p.b, &full_bar[st], kx, n0);
+            if (mode_split(MODE)) {
+              tma_load_2d(base + kABytes + BBYTES, &p.a_lo, &full_bar[st], kx, m0);
+              tma_load_2d(base + 2 * kABytes + BBYTES, &p.b_lo, &full_bar[st], kx, n0);
+            }
           }
+          __syncwarp();
+          if (++st == ST) { st = 0; ph ^= 1u; }
         }
       }
       if (!ok) {
@@ -109,36 +113,40 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && kb_per_tile > 0) {
-      int it = 0, ti = 0;
+    if (kb_per_tile > 0) {
+      const bool one = elect_one();
+      int st = 0, ti = 0;
+      uint32_t ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++ti) {
         const int buf = ti & 1;
         // wait until the epilogue has drained this accumulator buffer (passes at once on its first use)
-        if (!mbar_wait(&acc_empty[buf], (uint32_t)(((ti >> 1) & 1) ^ 1), &abort_s, p.err, 4)) { ok = false; break; }
+        if (!mbar_wait_warp(&acc_empty[buf], (uint32_t)(((ti >> 1) & 1) ^ 1), &abort_s, p.err, 4)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_main = tmem_base + (uint32_t)(buf * ACC_COLS);
-        for (int kk = 0; kk < kb_per_tile; ++kk, ++it) {
-          const int st = it % ST;
-          const uint32_t ph = (uint32_t)((it / ST) & 1);
-          if (!mbar_wait(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
+        for (int kk = 0; kk < kb_per_tile; ++kk) {
+          if (!mbar_wait_warp(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)st * STAGE);
           const uint32_t b_addr = a_addr + kABytes;
           const uint64_t da = make_smem_desc(a_addr), db = make_smem_desc(b_addr);
+          if (one) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t acc = (kk > 0 || k > 0) ? 1u : 0u;
-            umma<mode_kind_tf32(MODE)>(d_main, da + 2 * k, db + 2 * k, IDESC, acc);
-            if (mode_split(MODE)) {
-              const uint64_t dal = make_smem_desc(b_addr + BBYTES), dbl = make_smem_desc(b_addr + BBYTES + kABytes);
-              umma<mode_kind_tf32(MODE)>(d_main + BN, dal + 2 * k, db + 2 * k, IDESC, acc);
-              umma<mode_kind_tf32(MODE)>(d_main + BN, da + 2 * k, dbl + 2 * k, IDESC, 1u);
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t acc = (kk > 0 || k > 0) ? 1u : 0u;
+              umma<mode_kind_tf32(MODE)>(d_main, da + 2 * k, db + 2 * k, IDESC, acc);
+              if (mode_split(MODE)) {
+                const uint64_t dal = make_smem_desc(b_addr + BBYTES), dbl = make_smem_desc(b_addr + BBYTES + kABytes);
+                umma<mode_kind_tf32(MODE)>(d_main + BN, dal + 2 * k, db + 2 * k, IDESC, acc);
+                umma<mode_kind_tf32(MODE)>(d_main + BN, da + 2 * k, dbl + 2 * k, IDESC, 1u);
+              }
             }
+            umma_commit(&empty_bar[st]);
           }
-          umma_commit(&empty_bar[st]);
+          __syncwarp();
+          if (++st == ST) { st = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        if (ok && one) umma_commit(&acc_full[buf]);
       }
     }
   } else if (kb_per_tile > 0) {

@@ -80,7 +80,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   constexpr int SETC = set_cols(BN, MODE), NB = set_bufs(BN, MODE, WHOLE), TMEM_COLS = link_tmem(BN, MODE, WHOLE);
   constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN), IDESC2 = make_idesc(mode_fmt(MODE), SETC);
   extern __shared__ __align__(1024) uint8_t link_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int m0 = m_block * 128, n_tile = blockIdx.y;
   const int akb = p.a_rows * 128;  // bytes of one k-block of one activation part
   const int KBS = p.kbs;
@@ -123,26 +123,30 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   tc_fence_after();
   if (SPLIT > 1) cluster_arrive();  // (the barriers above are ready; waited for before the first remote store)
   const uint32_t tmem_base = ct.tmem_base;
-  const bool sound = ct.abort == 0;
+  const bool sound = __all_sync(0xffffffffu, ct.abort == 0);
   ZR_STAMP(1);
 
   if (warp == kWWarp) {
     // ------------------------------------------------------------ weights: nothing here depends on the predecessor
-    if (lane == 0 && sound) {
+    if (sound) {
+      const bool one = elect_one();
       bool ok = true;
       int st = 0, s = 0, c = 0;
       uint32_t ph = 0;
       for (int it = 0; it < n_it; ++it) {
-        if (it >= stages && !mbar_wait(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 1)) { ok = false; break; }
+        if (it >= stages && !mbar_wait_warp(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 1)) { ok = false; break; }
         uint8_t* w = tiles + (size_t)st * stage_bytes + PARTS * KBS * akb;
-        mbar_expect_tx(&ct.full[st], (uint32_t)(PARTS * KBS * WKB));
         const int wkb = p.wkb0[s] + (c_lo + c) * KBS;
-        if constexpr (EPI == TC_EPI_LSTM) {
-          constexpr int TH = BN / 4;
-          tma_load_5d(w, &p.w, &ct.full[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
-        } else {
-          tma_load_4d(w, &p.w, &ct.full[st], n_tile * BN, wkb);
+        if (one) {
+          mbar_expect_tx(&ct.full[st], (uint32_t)(PARTS * KBS * WKB));
+          if constexpr (EPI == TC_EPI_LSTM) {
+            constexpr int TH = BN / 4;
+            tma_load_5d(w, &p.w, &ct.full[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
+          } else {
+            tma_load_4d(w, &p.w, &ct.full[st], n_tile * BN, wkb);
+          }
         }
+        __syncwarp();
         if (++st == stages) { st = 0; ph ^= 1u; }
         if (++c == n_src) { c = 0; ++s; }
       }
@@ -150,7 +154,8 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
     }
   } else if (warp == kAWarp) {
     // ------------------------------------------------------------ activations: the early sources before the predecessor's end
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       bool ok = sound;
       int st = 0, s = 0, c = 0;
       uint32_t ph = 0;
@@ -159,9 +164,12 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
           pdl_wait();
           pdl_trigger();
         }
-        if (it >= stages && !mbar_wait(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 7)) { ok = false; break; }
-        mbar_expect_tx(&ct.full[st], (uint32_t)(PARTS * KBS * akb));
-        tma_load_4d(tiles + (size_t)st * stage_bytes, &p.a[s], &ct.full[st], p.a_row0[s] + m0, (c_lo + c) * KBS);
+        if (it >= stages && !mbar_wait_warp(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 7)) { ok = false; break; }
+        if (one) {
+          mbar_expect_tx(&ct.full[st], (uint32_t)(PARTS * KBS * akb));
+          tma_load_4d(tiles + (size_t)st * stage_bytes, &p.a[s], &ct.full[st], p.a_row0[s] + m0, (c_lo + c) * KBS);
+        }
+        __syncwarp();
         if (++st == stages) { st = 0; ph ^= 1u; }
         if (++c == n_src) { c = 0; ++s; }
       }
@@ -169,7 +177,8 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
     }
   } else if (warp >= kMmaWarp) {
     // ------------------------------------------------------------ MMA issuers
-    if (lane == 0 && sound) {
+    if (sound) {
+      const bool one = elect_one();
       const int mw = warp - kMmaWarp, R = round_kb(MODE, p.kb) / KBS;
       int set = mw * NB;
       int st = mw, it = mw, round_end = 0, round = 0;
@@ -178,27 +187,30 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
       while (it < n_it) {
         if (ROUNDS && it >= round_end) {  // first stage of this warp in a round
           set = mw * NB + round % NB;
-          if (round >= NB && !mbar_wait(&ct.set_empty[set], (uint32_t)(round / NB & 1) ^ 1u, &ct.abort, p.err, 4)) { ok = false; break; }
+          if (round >= NB && !mbar_wait_warp(&ct.set_empty[set], (uint32_t)(round / NB & 1) ^ 1u, &ct.abort, p.err, 4)) { ok = false; break; }
           tc_fence_after();
           fresh = true;
           round_end = (it / R + 1) * R;
           ++round;
         }
-        if (!mbar_wait(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
+        if (!mbar_wait_warp(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
         const uint32_t d = tmem_base + (uint32_t)(set * SETC);
-        for (int b = 0; b < KBS; ++b) {
-          const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
-          const uint64_t dw = make_smem_desc(w_addr + b * PARTS * WKB);
+        if (one) {
+          for (int b = 0; b < KBS; ++b) {
+            const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
+            const uint64_t dw = make_smem_desc(w_addr + b * PARTS * WKB);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC2, (!fresh || b > 0 || k > 0) ? 1u : 0u);
-            if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + BN, dal + 2 * k, dw + 2 * k, IDESC, 1u);
+            for (int k = 0; k < 4; ++k) {
+              umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC2, (!fresh || b > 0 || k > 0) ? 1u : 0u);
+              if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + BN, dal + 2 * k, dw + 2 * k, IDESC, 1u);
+            }
           }
+          umma_commit(&ct.empty[st]);
         }
+        __syncwarp();
         fresh = false;
-        umma_commit(&ct.empty[st]);
         if (st + kMmaWarps < stages) {
           st += kMmaWarps;
           it += kMmaWarps;
@@ -207,9 +219,9 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
           st = mw;
           ph ^= 1u;
         }
-        if (ROUNDS && (it >= round_end || it >= n_it)) umma_commit(&ct.set_full[set]);
+        if (ROUNDS && (it >= round_end || it >= n_it) && one) umma_commit(&ct.set_full[set]);
       }
-      if (ok && !ROUNDS) umma_commit(&ct.accum);
+      if (ok && !ROUNDS && one) umma_commit(&ct.accum);
     }
   }
   __syncwarp();

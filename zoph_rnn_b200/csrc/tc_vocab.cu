@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
   constexpr bool SPLIT_MODE = mode_split(MODE);
   constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t vocab_smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int nb = p.nb, KBS = p.kbs, hkb = nb * 128;
   const int w_bytes = PARTS * KBS * 128 * 128, h_bytes = PARTS * KBS * hkb, stage_bytes = w_bytes + h_bytes;
   uint8_t* tiles = vocab_smem;
@@ -95,11 +95,12 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ct.tmem_base;
-  const bool sound = ct.abort == 0;
+  const bool sound = __all_sync(0xffffffffu, ct.abort == 0);
 
   if (warp == kWWarp || warp == kHWarp) {
     // ------------------------------------------------------------ loads; the weights do not depend on the predecessor
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       if (warp == kHWarp) {
         pdl_wait();
         pdl_trigger();
@@ -109,15 +110,18 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
       uint32_t ph = 0;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         for (int k = 0; k < k_its; ++k, ++it) {
-          if (it >= stages && !mbar_wait(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 1)) { ok = false; break; }
+          if (it >= stages && !mbar_wait_warp(&ct.empty[st], ph ^ 1u, &ct.abort, p.err, 1)) { ok = false; break; }
           uint8_t* dst = tiles + (size_t)st * stage_bytes;
-          if (warp == kWWarp) {
-            mbar_expect_tx(&ct.full[st], (uint32_t)w_bytes);
-            tma_load_4d(dst, &p.w, &ct.full[st], tile * 128, k * KBS);
-          } else {
-            mbar_expect_tx(&ct.full[st], (uint32_t)h_bytes);
-            tma_load_4d(dst + w_bytes, &p.h, &ct.full[st], 0, k * KBS);
+          if (one) {
+            if (warp == kWWarp) {
+              mbar_expect_tx(&ct.full[st], (uint32_t)w_bytes);
+              tma_load_4d(dst, &p.w, &ct.full[st], tile * 128, k * KBS);
+            } else {
+              mbar_expect_tx(&ct.full[st], (uint32_t)h_bytes);
+              tma_load_4d(dst + w_bytes, &p.h, &ct.full[st], 0, k * KBS);
+            }
           }
+          __syncwarp();
           if (++st == stages) { st = 0; ph ^= 1u; }
         }
       }
@@ -125,7 +129,8 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && sound) {
+    if (sound) {
+      const bool one = elect_one();
       const bool stacked = PARTS * nb <= 256;  // the widest MMA
       const uint32_t idesc = make_idesc(mode_fmt(MODE), (uint32_t)nb), idesc2 = make_idesc(mode_fmt(MODE), (uint32_t)(stacked ? PARTS * nb : nb));
       int st = 0, ti = 0;
@@ -133,32 +138,35 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
         const int buf = bufs == 2 ? ti & 1 : 0, use = bufs == 2 ? ti >> 1 : ti;
-        if (!mbar_wait(&ct.acc_empty[buf], (uint32_t)((use & 1) ^ 1), &ct.abort, p.err, 4)) { ok = false; break; }
+        if (!mbar_wait_warp(&ct.acc_empty[buf], (uint32_t)((use & 1) ^ 1), &ct.abort, p.err, 4)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(buf * acc_cols);
         for (int k = 0; k < k_its; ++k) {
-          if (!mbar_wait(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
+          if (!mbar_wait_warp(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t w_addr = smem_u32(tiles + (size_t)st * stage_bytes), h_addr = w_addr + w_bytes;
-          for (int b = 0; b < KBS; ++b) {
-            const uint64_t dw = make_smem_desc(w_addr + b * PARTS * 16384), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * 16384);
-            const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb), dhl = make_smem_desc(h_addr + (b * PARTS + 1) * hkb);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint32_t acc = (k > 0 || b > 0 || i > 0) ? 1u : 0u;
-              if (!SPLIT_MODE || stacked) {
-                umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
-              } else {
-                umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc, acc);
-                umma<mode_kind_tf32(MODE)>(d + nb, dw + 2 * i, dhl + 2 * i, idesc, acc);
+          if (one) {
+            for (int b = 0; b < KBS; ++b) {
+              const uint64_t dw = make_smem_desc(w_addr + b * PARTS * 16384), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * 16384);
+              const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb), dhl = make_smem_desc(h_addr + (b * PARTS + 1) * hkb);
+  #pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const uint32_t acc = (k > 0 || b > 0 || i > 0) ? 1u : 0u;
+                if (!SPLIT_MODE || stacked) {
+                  umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
+                } else {
+                  umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc, acc);
+                  umma<mode_kind_tf32(MODE)>(d + nb, dw + 2 * i, dhl + 2 * i, idesc, acc);
+                }
+                if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + nb, dwl + 2 * i, dh + 2 * i, idesc, 1u);
               }
-              if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + nb, dwl + 2 * i, dh + 2 * i, idesc, 1u);
             }
+            umma_commit(&ct.empty[st]);
           }
-          umma_commit(&ct.empty[st]);
+          __syncwarp();
           if (++st == stages) { st = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit(&ct.acc_full[buf]);
+        if (ok && one) umma_commit(&ct.acc_full[buf]);
       }
     }
   } else {
