@@ -145,6 +145,14 @@ def test_vocabulary_projection_edges(dtype, H, V, N):
     np.testing.assert_allclose(got.cpu().numpy().reshape(-1), logp[np.arange(N), tgt], rtol=r, atol=a)
 
 
+@pytest.mark.parametrize("dtype,H,V,N", [(5, 336, 129, 65), (5, 336, 256, 96), (5, 324, 257, 97), (5, 320, 513, 513), (5, 1000, 3001, 700), (5, 600, 20000, 1025),
+                                         (4, 104, 385, 160), (4, 324, 19001, 321), (1, 1024, 511, 160), (1, 1032, 2050, 289), (2, 544, 700, 255)])
+def test_vocabulary_projection_pairs_of_ctas(dtype, H, V, N):
+    """One and several column tiles, full and broken; a pair whose second CTA has no vocabulary row at all; both sides of the K where short
+    log-sum-exp products leave the pairs; tiles of one and of two accumulator buffers."""
+    test_vocabulary_projection_edges(dtype, H, V, N)
+
+
 @pytest.mark.parametrize("mode,K,steps", [(4, 64, 4), (4, 320, 4), (4, 512, 4), (4, 1000, 8), (3, 64, 4), (3, 512, 4), (3, 1000, 8)])
 @pytest.mark.parametrize("n,m", [(512, 100), (1000, 12), (320, 200)])
 def test_products_of_one_sign_do_not_shrink(mode, K, steps, n, m):

@@ -1,4 +1,4 @@
-// tcgen05 / TMEM / TMA GEMM for large products (the vocabulary projection) and the tensor-map helpers.  See tc_gemm.cuh for the
+// tcgen05 / TMEM / TMA product of the scoring softmax for short K (others: tc_vocab_pair.cu) and the tensor-map helpers.  See tc_gemm.cuh for the
 // operand convention.  A ring of shared-memory stages is guarded by full/empty mbarriers; every wait is bounded (about a
 // second of SM clock) and reports through p.err instead of spinning forever.
 #include "tc_gemm.cuh"
@@ -21,12 +21,11 @@ namespace {
 // Warp roles: warps 0-7 run the epilogue (warp w reads TMEM lanes 32 (w % 4) .. +31, the only ones it may access, and
 // the column half w / 4 of the tile), warp 8 is the TMA producer, warp 9 issues the MMAs and owns the TMEM allocation.
 // Every tile therefore leaves kPersistentParts = 2 (max, sum) partials per output row, one per column half.
-constexpr int kXposeBytes = 8 * 32 * 32 * 4;  // one 32 x 32 fp32 transposition buffer per epilogue warp
 __host__ __device__ constexpr int persistent_stages(int BN, int mode) {
-  return (225 * 1024 - 1024 - kXposeBytes) / stage_bytes(BN, mode);
+  return 192 * 1024 / stage_bytes(BN, mode);
 }
 
-template <int BN, int MODE, int EPI>
+template <int BN, int MODE>
 __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid_constant__ TcParams p, int m_tiles,
                                                                      int n_tiles) {
   constexpr int ST = persistent_stages(BN, MODE);
@@ -39,7 +38,6 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
   static_assert(ST >= 2, "need at least a double-buffered ring");
   static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "TMEM budget");
   static_assert(HC % 32 == 0, "the epilogue works on chunks of 32 columns");
-  static_assert(EPI != TC_EPI_LSTM, "the persistent variant has store and log-sum-exp epilogues only");
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[ST];
   __shared__ __align__(8) uint64_t empty_bar[ST];
@@ -152,12 +150,6 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
   } else if (kb_per_tile > 0) {
     // ------------------------------------------------------------ epilogue warps 0-7
     const int q = warp & 3, half = warp >> 2;
-    float* xp = reinterpret_cast<float*>(tiles + (size_t)ST * STAGE) + warp * 1024;
-    // Stores go through the warp's transposition buffer so that every store instruction writes whole 128-byte lines
-    // (a thread per output row would scatter 16-byte pieces over 32 lines).  That needs 16-byte aligned rows; any
-    // other layout takes the per-row path.
-    const bool fast_store = EPI == TC_EPI_STORE && (p.ldc & 3) == 0 && (p.N & 3) == 0 &&
-                            (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     int ti = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++ti) {
       const int buf = ti & 1;
@@ -167,7 +159,7 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
       asm volatile("bar.sync 1, 256;" ::: "memory");  // all epilogue threads have finished with the previous bias
       for (int i = threadIdx.x; i < BN; i += 256) {
         const int n = n_tile * BN + i;
-        s_bias[i] = n < p.N ? (p.bias ? __ldg(p.bias + n) : 0.f) : (EPI == TC_EPI_LSE ? -INFINITY : 0.f);
+        s_bias[i] = n < p.N ? (p.bias ? __ldg(p.bias + n) : 0.f) : -INFINITY;
       }
       if (!mbar_wait(&acc_full[buf], (uint32_t)((ti >> 1) & 1), &abort_s, p.err, 3)) break;
       tc_fence_after();
@@ -176,130 +168,50 @@ __global__ void __launch_bounds__(320, 1) tc_gemm_persistent_kernel(const __grid
       const int n0 = n_tile * BN + half * HC;  // first output column of this warp
       const float* sb = s_bias + half * HC;
       const size_t pi = (size_t)(n_tile * kPersistentParts + half) * p.M + row;
-      if constexpr (EPI == TC_EPI_STORE) {
-        const bool want_max = p.part_max != nullptr;  // also emit the maximum of this warp's stored values per row
-        const bool want_lse = want_max && p.part_sum != nullptr;  // ... and sum exp(x - max)
-        float mx = -INFINITY, sm = 0.f;
-        for (int c0 = 0; c0 < HC; c0 += 32) {
-          float v[32];
-          tmem_ld32(taddr + c0, v);
-          if (mode_split(MODE)) {
-            float t[32];
-            tmem_ld32(taddr + BN + c0, t);
-            tmem_wait_ld();
-#pragma unroll
-            for (int u = 0; u < 32; ++u) v[u] = fmaf(t[u], mode_cross_scale(MODE), v[u]);
-          }
+      const int tg = (p.target && row_ok) ? p.target[row] - p.target_offset : -1;
+      float mx = -INFINITY, sm = 0.f;
+      for (int c0 = 0; c0 < HC; c0 += 32) {
+        float v[32];
+        tmem_ld32(taddr + c0, v);
+        if (mode_split(MODE)) {
+          float t[32];
+          tmem_ld32(taddr + BN + c0, t);
           tmem_wait_ld();
-          const int nb = n0 + c0;
-          const int nvalid = p.N - nb >= 32 ? 32 : (p.N - nb > 0 ? p.N - nb : 0);
-          float cm = -INFINITY;
+#pragma unroll
+          for (int u = 0; u < 32; ++u) v[u] = fmaf(t[u], mode_cross_scale(MODE), v[u]);
+        }
+        tmem_wait_ld();
+        float cm = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 32; u += 4) {
+          const float4 b4 = *reinterpret_cast<const float4*>(sb + c0 + u);
+          v[u] += b4.x; v[u + 1] += b4.y; v[u + 2] += b4.z; v[u + 3] += b4.w;
+          cm = fmaxf(fmaxf(cm, fmaxf(v[u], v[u + 1])), fmaxf(v[u + 2], v[u + 3]));
+        }
+        const int rel = tg - (n0 + c0);
+        if ((unsigned)rel < 32u && tg < p.N) {  // the target's logit lies in this chunk (once per row at most)
+          float t = 0.f;
+#pragma unroll
+          for (int u = 0; u < 32; ++u)
+            if (u == rel) t = v[u];
+          p.tgt_logit[row] = t;
+        }
+        if (cm > mx) {
+          sm *= expf(mx - cm);
+          mx = cm;
+        }
+        if (mx != -INFINITY) {
+          float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
           for (int u = 0; u < 32; u += 4) {
-            const float4 b4 = *reinterpret_cast<const float4*>(sb + c0 + u);
-            const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              v[u + e] += bb[e];
-              if (u + e < nvalid) cm = fmaxf(cm, v[u + e]);
-            }
+            s0 += expf(v[u] - mx); s1 += expf(v[u + 1] - mx); s2 += expf(v[u + 2] - mx); s3 += expf(v[u + 3] - mx);
           }
-          if (want_lse) {
-            if (cm > mx) { sm *= expf(mx - cm); mx = cm; }
-            if (mx != -INFINITY) {
-              float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-              for (int u = 0; u < 32; u += 4) {
-                s0 += u < nvalid ? expf(v[u] - mx) : 0.f;
-                s1 += u + 1 < nvalid ? expf(v[u + 1] - mx) : 0.f;
-                s2 += u + 2 < nvalid ? expf(v[u + 2] - mx) : 0.f;
-                s3 += u + 3 < nvalid ? expf(v[u + 3] - mx) : 0.f;
-              }
-              sm += (s0 + s1) + (s2 + s3);
-            }
-          } else if (want_max) {
-            mx = fmaxf(mx, cm);
-          }
-          if (fast_store) {
-            // row `lane` of the 32 x 32 chunk, its eight 16-byte pieces XOR-swizzled by the row so that neither
-            // these writes nor the transposed reads below collide on a bank
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              *reinterpret_cast<float4*>(xp + lane * 32 + ((j ^ (lane & 7)) << 2)) =
-                  make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {  // eight lanes per row, four rows per instruction
-              const int r = 4 * i + (lane >> 3), j = lane & 7;
-              const float4 o = *reinterpret_cast<const float4*>(xp + r * 32 + ((j ^ (r & 7)) << 2));
-              const int grow = m_tile * 128 + q * 32 + r, n = nb + 4 * j;
-              // streaming stores: the consumer reads a few tiles of the logits once, the weights should stay in L2
-              if (grow < p.M && n < p.N) __stcs(reinterpret_cast<float4*>(p.C + (size_t)grow * p.ldc + n), o);
-            }
-            __syncwarp();
-          } else if (row_ok) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              const int nv = nvalid - 8 * g >= 8 ? 8 : (nvalid - 8 * g > 0 ? nvalid - 8 * g : 0);
-              if (nv > 0) {
-                float x8[8];  // a copy: the ragged tail indexes it dynamically, which must not push v out of registers
-#pragma unroll
-                for (int u = 0; u < 8; ++u) x8[u] = v[8 * g + u];
-                store8_f32(p.C, (size_t)row * p.ldc + nb + 8 * g, x8, nv);
-              }
-            }
-          }
+          sm += (s0 + s1) + (s2 + s3);
         }
-        if (want_max && row_ok) {
-          p.part_max[pi] = mx;
-          if (want_lse) p.part_sum[pi] = sm;
-        }
-      } else {  // TC_EPI_LSE
-        const int tg = (p.target && row_ok) ? p.target[row] - p.target_offset : -1;
-        float mx = -INFINITY, sm = 0.f;
-        for (int c0 = 0; c0 < HC; c0 += 32) {
-          float v[32];
-          tmem_ld32(taddr + c0, v);
-          if (mode_split(MODE)) {
-            float t[32];
-            tmem_ld32(taddr + BN + c0, t);
-            tmem_wait_ld();
-#pragma unroll
-            for (int u = 0; u < 32; ++u) v[u] = fmaf(t[u], mode_cross_scale(MODE), v[u]);
-          }
-          tmem_wait_ld();
-          float cm = -INFINITY;
-#pragma unroll
-          for (int u = 0; u < 32; u += 4) {
-            const float4 b4 = *reinterpret_cast<const float4*>(sb + c0 + u);
-            v[u] += b4.x; v[u + 1] += b4.y; v[u + 2] += b4.z; v[u + 3] += b4.w;
-            cm = fmaxf(fmaxf(cm, fmaxf(v[u], v[u + 1])), fmaxf(v[u + 2], v[u + 3]));
-          }
-          const int rel = tg - (n0 + c0);
-          if ((unsigned)rel < 32u && tg < p.N) {  // the target's logit lies in this chunk (once per row at most)
-            float t = 0.f;
-#pragma unroll
-            for (int u = 0; u < 32; ++u)
-              if (u == rel) t = v[u];
-            p.tgt_logit[row] = t;
-          }
-          if (cm > mx) {
-            sm *= expf(mx - cm);
-            mx = cm;
-          }
-          if (mx != -INFINITY) {
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-            for (int u = 0; u < 32; u += 4) {
-              s0 += expf(v[u] - mx); s1 += expf(v[u + 1] - mx); s2 += expf(v[u + 2] - mx); s3 += expf(v[u + 3] - mx);
-            }
-            sm += (s0 + s1) + (s2 + s3);
-          }
-        }
-        if (row_ok) {
-          p.part_max[pi] = mx;
-          p.part_sum[pi] = sm;
-        }
+      }
+      if (row_ok) {
+        p.part_max[pi] = mx;
+        p.part_sum[pi] = sm;
       }
       // this warp's TMEM reads are complete: hand the buffer back to the MMA warp
       tc_fence_before();
@@ -335,13 +247,13 @@ static int sm_count() {
   return n;
 }
 
-template <int BN, int MODE, int EPI>
+template <int BN, int MODE>
 cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
-  const size_t smem = (size_t)persistent_stages(BN, MODE) * stage_bytes(BN, MODE) + 1024 + kXposeBytes;
+  const size_t smem = (size_t)persistent_stages(BN, MODE) * stage_bytes(BN, MODE) + 1024;
   static bool configured[kMaxDevices] = {false};  // the attribute is per device
   const int dev = current_device();
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_persistent_kernel<BN, MODE, EPI>,
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_persistent_kernel<BN, MODE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
@@ -363,24 +275,17 @@ cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, tc_gemm_persistent_kernel<BN, MODE, EPI>, p, m_tiles, n_tiles);
+  return cudaLaunchKernelEx(&cfg, tc_gemm_persistent_kernel<BN, MODE>, p, m_tiles, n_tiles);
 }
 
 }  // namespace
 
-cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, int epi, cudaStream_t st) {
-  // tile widths: 256 columns for bf16 / tf32, 128 for 3xTF32 (its second, cross-term accumulator doubles the TMEM need)
-  if (epi == TC_EPI_LSE) {
-    if (mode == TC_BF16) return launch_persistent_t<256, TC_BF16, TC_EPI_LSE>(p, st);
-    if (mode == TC_TF32) return launch_persistent_t<256, TC_TF32, TC_EPI_LSE>(p, st);
-    if (mode == TC_TF32X3) return launch_persistent_t<128, TC_TF32X3, TC_EPI_LSE>(p, st);
-    if (mode == TC_F16X2) return launch_persistent_t<128, TC_F16X2, TC_EPI_LSE>(p, st);
-  } else if (epi == TC_EPI_STORE) {
-    if (mode == TC_BF16) return launch_persistent_t<256, TC_BF16, TC_EPI_STORE>(p, st);
-    if (mode == TC_TF32) return launch_persistent_t<256, TC_TF32, TC_EPI_STORE>(p, st);
-    if (mode == TC_TF32X3) return launch_persistent_t<128, TC_TF32X3, TC_EPI_STORE>(p, st);
-    if (mode == TC_F16X2) return launch_persistent_t<128, TC_F16X2, TC_EPI_STORE>(p, st);
-  }
+cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, cudaStream_t st) {
+  // tile widths: 256 columns for bf16 / tf32, 128 for the split modes (their second, cross-term accumulator doubles the TMEM need)
+  if (mode == TC_BF16) return launch_persistent_t<256, TC_BF16>(p, st);
+  if (mode == TC_TF32) return launch_persistent_t<256, TC_TF32>(p, st);
+  if (mode == TC_TF32X3) return launch_persistent_t<128, TC_TF32X3>(p, st);
+  if (mode == TC_F16X2) return launch_persistent_t<128, TC_F16X2>(p, st);
   return cudaErrorInvalidValue;
 }
 

@@ -23,10 +23,7 @@ struct TcParams {
   int M;              // batch columns
   int N;              // output rows
   const float* bias;  // [N]
-  // --- STORE: C[n + m*ldc] = acc + bias[n]
-  float* C;
-  int ldc;
-  // --- LSE: per (N tile, m) max and sum exp(z - max) of z = acc + bias, plus the logit of target[m]
+  // per (N tile, m) max and sum exp(z - max) of z = acc + bias, plus the logit of target[m]
   const int* target;
   int target_offset;
   float* part_max;  // [n_tiles x M]
@@ -37,12 +34,12 @@ struct TcParams {
   int prof_slot;     // >= 0: only CTA (0,0,0) stamps, into prof[prof_slot*8 ..] (timeline of many launches)
 };
 
-// Persistent one-CTA-per-SM variant for large problems (store and log-sum-exp epilogues).  The B tensor map must use
+// One CTA per SM walks over the tiles, log-sum-exp epilogue.  The B tensor map must use
 // 256-row boxes for TC_BF16 / TC_TF32 and 128-row boxes for the split modes.  Two epilogue warps share each output
 // row of a tile, one per half of its columns, so the (max, sum) partials are indexed
 // [(n_tile * kPersistentParts + half) x M] and each covers tile width / kPersistentParts consecutive columns.
 constexpr int kPersistentParts = 2;
-cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, int epi, cudaStream_t st);
+cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, cudaStream_t st);
 // One warp waits (bounded by limit_cycles SM cycles) on a barrier that never completes and reports `code` in *err.
 cudaError_t launch_wait_probe(int* err, long long limit_cycles, int code, cudaStream_t st);
 

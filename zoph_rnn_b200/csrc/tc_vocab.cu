@@ -1,4 +1,4 @@
-// Vocabulary projection for few batch columns (128, split modes 144 where K is long) on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
+// Vocabulary projection for up to 64 batch columns on tcgen05, bound by the stream of the weights from HBM (f32: 4 bytes a value).
 //
 // The weights are the M side of the MMA (128 vocabulary rows) and the columns its N side, padded to a multiple of 16 only: with
 // the columns as the M side (tc_gemm.cu) a step of 12 columns multiplied 128 padded rows, 19 us of MMAs for 160 MB of weights, and
@@ -6,10 +6,10 @@
 // h_hi.  An accumulator row is a vocabulary row, so a warp stores 32 consecutive logits of a column at once; maxima and sums
 // over the rows are reductions across the warp that halve the number of columns per lane as they go.
 //
-// Persistent CTAs walk over the vocabulary, the accumulators are double-buffered in TMEM (while 512 columns hold two) and the loads
-// run ahead across tiles.  Up to 64 columns a CTA takes half an SM (113 KB, 256 TMEM columns), so that it is resident, and streams
-// its first weights, while the kernel before it runs.  us per launch, before -> now, f32: 12 columns x 40000 words x 1000: 48 -> 31
-// (HBM: 25).  Marking the weights to leave the L2 first changes nothing.
+// Persistent CTAs walk over the vocabulary, the accumulators are double-buffered in TMEM and the loads run ahead across tiles.  A CTA
+// takes half an SM (113 KB, 256 TMEM columns), so that it is resident, and streams its first weights, while the kernel before it
+// runs.  us per launch, with the columns as the M side -> now, f32: 12 columns x 40000 words x 1000: 48 -> 31 (HBM: 25).  Marking the
+// weights to leave the L2 first changes nothing.
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -23,7 +23,7 @@ namespace zrnn {
 namespace {
 
 constexpr int kEpiWarps = 8, kHWarp = 8, kWWarp = 9, kMmaWarp = 10, kThreads = 352;
-constexpr int kHalfSm = 113 * 1024, kWholeSm = 224 * 1024, kMaxStages = 8, kHalfCols = 64;
+constexpr int kHalfSm = 113 * 1024, kMaxStages = 8;
 struct VocabCtrl {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], acc_empty[2];
@@ -58,7 +58,7 @@ __device__ __forceinline__ float reduce8(const float* v, int lane, Op op) {
 
 template <int MODE, int EPI>
 __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_constant__ VocabParams p, int stages, int n_tiles,
-                                                               int tmem_cols, int bufs) {
+                                                               int tmem_cols) {
   constexpr bool SPLIT_MODE = mode_split(MODE);
   constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   extern __shared__ __align__(1024) uint8_t vocab_smem[];
@@ -131,13 +131,12 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
     // ------------------------------------------------------------ MMA issuer
     if (sound) {
       const bool one = elect_one();
-      const bool stacked = PARTS * nb <= 256;  // the widest MMA
-      const uint32_t idesc = make_idesc(mode_fmt(MODE), (uint32_t)nb), idesc2 = make_idesc(mode_fmt(MODE), (uint32_t)(stacked ? PARTS * nb : nb));
+      const uint32_t idesc = make_idesc(mode_fmt(MODE), (uint32_t)nb), idesc2 = make_idesc(mode_fmt(MODE), (uint32_t)(PARTS * nb));
       int st = 0, ti = 0;
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++ti) {
-        const int buf = bufs == 2 ? ti & 1 : 0, use = bufs == 2 ? ti >> 1 : ti;
+        const int buf = ti & 1, use = ti >> 1;
         if (!mbar_wait_warp(&ct.acc_empty[buf], (uint32_t)((use & 1) ^ 1), &ct.abort, p.err, 4)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)(buf * acc_cols);
@@ -148,16 +147,11 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
           if (one) {
             for (int b = 0; b < KBS; ++b) {
               const uint64_t dw = make_smem_desc(w_addr + b * PARTS * 16384), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * 16384);
-              const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb), dhl = make_smem_desc(h_addr + (b * PARTS + 1) * hkb);
+              const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb);
   #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const uint32_t acc = (k > 0 || b > 0 || i > 0) ? 1u : 0u;
-                if (!SPLIT_MODE || stacked) {
                   umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
-                } else {
-                  umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc, acc);
-                  umma<mode_kind_tf32(MODE)>(d + nb, dw + 2 * i, dhl + 2 * i, idesc, acc);
-                }
                 if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + nb, dwl + 2 * i, dh + 2 * i, idesc, 1u);
               }
             }
@@ -180,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
     int ti = 0;
     bool ready = sound;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++ti) {  // (to the end even after a wait that gave up: barriers)
-      const int buf = bufs == 2 ? ti & 1 : 0, use = bufs == 2 ? ti >> 1 : ti, v = tile * 128 + quad * 32 + lane;
+      const int buf = ti & 1, use = ti >> 1, v = tile * 128 + quad * 32 + lane;
       const bool in = v < p.N;
       const float bias = in && p.bias ? __ldg(p.bias + v) : 0.f;
       ready = ready && __all_sync(0xffffffffu, mbar_wait(&ct.acc_full[buf], (uint32_t)(use & 1), &ct.abort, p.err, 3));
@@ -268,20 +262,18 @@ template <int MODE, int EPI>
 cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   constexpr int PARTS = mode_split(MODE) ? 2 : 1;
   const int stage = PARTS * p.kbs * (128 + p.nb) * 128;
-  const bool half = p.nb <= kHalfCols;
   const int fixed = (int)sizeof(VocabCtrl) + column_bytes(p.nb);
-  const int stages = std::min(((half ? kHalfSm : kWholeSm) - fixed) / stage, (int)kMaxStages);
+  const int stages = std::min((kHalfSm - fixed) / stage, (int)kMaxStages);
   if (stages < 2) return cudaErrorInvalidValue;
   const size_t smem = (size_t)stages * stage + fixed;
-  const int bufs = 2 * PARTS * p.nb <= 512 ? 2 : 1;
   int tmem = 32;
-  while (tmem < bufs * PARTS * p.nb) tmem *= 2;
+  while (tmem < 2 * PARTS * p.nb) tmem *= 2;
   static bool configured[64] = {false};
   static int sms[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_vocab_kernel<MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaError_t e = cudaFuncSetAttribute(tc_vocab_kernel<MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfSm);
     if (e != cudaSuccess) return e;
     cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
     configured[dev] = true;
@@ -289,7 +281,7 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   const int n_tiles = (p.N + 127) / 128;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(std::min(n_tiles, (half ? 2 : 1) * sms[dev]));
+  cfg.gridDim = dim3(std::min(n_tiles, 2 * sms[dev]));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -299,7 +291,7 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = g_pdl_on ? 1 : 0;
   count_launch();
-  return cudaLaunchKernelEx(&cfg, tc_vocab_kernel<MODE, EPI>, p, stages, n_tiles, tmem, bufs);
+  return cudaLaunchKernelEx(&cfg, tc_vocab_kernel<MODE, EPI>, p, stages, n_tiles, tmem);
 }
 template <int MODE>
 cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
@@ -311,7 +303,7 @@ cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
 }  // namespace
 
 cudaError_t launch_tc_vocab(const VocabParams& p, int mode, int epi, cudaStream_t st) {
-  if (p.M < 1 || p.M > vocab_max_cols(mode, p.kb) || p.N < 1 || p.nb != vocab_columns(p.M) || p.kb < 1 || p.kbs != vocab_kbs(mode) ||
+  if (p.M < 1 || p.M > kVocabFewCols || p.N < 1 || p.nb != vocab_columns(p.M) || p.kb < 1 || p.kbs != vocab_kbs(mode) ||
       (p.part_rows != 64 && p.part_rows != 128))
     return cudaErrorInvalidValue;
   switch (mode) {

@@ -1,24 +1,22 @@
-// The vocabulary projection for few batch columns (a beam step, a short sentence): a stream of the weights past a handful of
-// columns.  See tc_vocab.cu; for more columns launch_tc_gemm_persistent (tc_gemm.cuh).
+// The vocabulary projection.  Few batch columns (a beam step of a sentence or two): a stream of the weights past a handful of columns,
+// tc_vocab.cu.  More columns: pairs of CTAs, tc_vocab_pair.cu.
 #pragma once
 #include "tc_gemm.cuh"
 
 namespace zrnn {
 
-constexpr int kVocabMaxCols = 144;
-// Beyond 128 columns the split modes have room for one accumulator only, so a tile's epilogue is not hidden.  Against the kernel of
-// many columns, which fetches the weights twice, that pays for one more group of 16 columns and from K = 768 on (kb k-blocks of 128
-// bytes).  us per beam step of a 2-layer model, here / there, at 144, 152 and 168 columns:
-//   fp16 split, K = 1000, 50000 words 173 / 178, 185 / 181, 189 / 182;  K = 768, 50000 words 143 / 146, 157 / 147, 159 / 147
-//   3xTF32,     K = 1000, 50000 words 278 / 297, 288 / 301, 303 / 304;  K = 640, 40000 words 191 / 190, 203 / 191, 213 / 192
-// (252 columns, K = 1000: 220 / 192 and 342 / 316.)
-inline int vocab_max_cols(int mode, int kb) { return (mode == TC_F16X2 && kb >= 12) || (mode == TC_TF32X3 && kb >= 24) ? 144 : 128; }
+// Up to here a CTA of the few-columns kernel fits half an SM and asks for its first weights while the kernel before it runs; beyond, pairs
+// of CTAs are faster.  us, few columns / pairs, fp16 split, K = 1000, 50000 words: 64 columns 43.5 / 40.2 (14.0 / 14.8 at K = 512,
+// 20000 words; without the overlap, which a beam step has), 96 columns 45.7 / 42.3 (20.6 / 17.9), 128 columns 49.7 / 44.0 (25.2 / 16.8);
+// bf16, 128 columns 37.3 / 25.3.
+constexpr int kVocabFewCols = 64;
 
 // z[v, m] = W[v] . h[m] + bias[v] for v < N, m < M
 struct VocabParams {
   CUtensorMap w;       // make_rows_map: 128 weight rows, all parts, kbs k-blocks
   CUtensorMap h;       // make_rows_map: nb rows, all parts, kbs k-blocks
-  int M, N, nb;        // columns, vocabulary rows, columns rounded up to a multiple of 16
+  int M, N, nb;        // columns, vocabulary rows, columns rounded up to a multiple of 16 (pairs: columns of a tile, a multiple of 32)
+  int n_ct;            // pairs: column tiles
   int kb, kbs;         // k-blocks, k-blocks per ring stage: vocab_kbs(mode)
   const float* bias;
   float* C;            // STORE: z[v, m] at C + m * ldc + v
@@ -35,5 +33,12 @@ struct VocabParams {
 inline int vocab_columns(int M) { return (M + 15) / 16 * 16; }
 inline int vocab_kbs(int mode) { return mode == TC_TF32X3 || mode == TC_F16X2 ? 1 : 2; }
 cudaError_t launch_tc_vocab(const VocabParams& p, int mode, int epi, cudaStream_t st);
+
+// Pairs of CTAs: n_ct column tiles of nb columns; the box of h has nb / 2 rows.
+struct VocabTiles {
+  int n_ct, nb;
+};
+VocabTiles vocab_pair_tiles(int M, int N);
+cudaError_t launch_tc_vocab_pair(const VocabParams& p, int mode, int epi, cudaStream_t st);
 
 }  // namespace zrnn

@@ -629,26 +629,36 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   return ZRNN_OK;
 }
 
-int vocab_cols_limit(const zrnn_softmax* S) {
-  const int epk = 128 / eng_eb(S->eng);
-  return zrnn::vocab_max_cols(eng_tcmode(S->eng), (S->H + epk - 1) / epk);
+// Tiles of one CTA (tc_gemm.cu) are still faster for the log-sum-exp epilogue of short products, which takes longer than their MMAs: it
+// has a column per lane, so no value changes hands.  us, single CTAs / pairs, 160, 512 and 6400 columns: fp16 split, K = 100, 10000
+// words 9.2 / 10.0, 11.5 / 14.3, 69 / 86; K = 512, 20000 words 19.1 / 18.8, 30.5 / 30.1, 277 / 246; bf16, 50000 words, K = 1000 31.6 /
+// 29.2, 50.5 / 50.9, 405 / 420; K = 1536 41.5 / 36.6, 67 / 64, 598 / 582.
+bool short_lse(const zrnn_softmax* S) {
+  const int epk = 128 / eng_eb(S->eng), products = eng_split(S->eng) ? 3 : 1;
+  return (S->H + epk - 1) / epk * products <= 16;
 }
 // the part of a VocabParams that scoring and decoding share
 int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams& p) {
   const int eng = S->eng, mode = eng_tcmode(eng), eb = eng_eb(eng), parts = eng_split(eng) ? 2 : 1;
   const long long row_bytes = (long long)S->Kpad * eb;
   std::memset(&p, 0, sizeof(p));
-  p.M = N; p.N = S->hi - S->lo; p.nb = zrnn::vocab_columns(N);
+  const bool pair = N > zrnn::kVocabFewCols;
+  p.M = N; p.N = S->hi - S->lo;
+  const zrnn::VocabTiles t = pair ? zrnn::vocab_pair_tiles(N, p.N) : zrnn::VocabTiles{1, zrnn::vocab_columns(N)};
+  p.nb = t.nb; p.n_ct = t.n_ct;
   p.kb = (S->H + 128 / eb - 1) / (128 / eb); p.kbs = zrnn::vocab_kbs(mode);
   if (!h.hi) return fail(ZRNN_E_STATE, "internal: activation has no operand-form copy");
   if (!zrnn::make_rows_map(&p.w, S->D_op.hi, eb, row_bytes, (long long)S->n_tiles * S->BN, parts, S->D_op.part_bytes(), p.kb, 128, p.kbs) ||
-      !zrnn::make_rows_map(&p.h, h.hi, eb, row_bytes, N, parts, (char*)h.lo - (char*)h.hi, p.kb, p.nb, p.kbs))
+      !zrnn::make_rows_map(&p.h, h.hi, eb, row_bytes, N, parts, (char*)h.lo - (char*)h.hi, p.kb, pair ? p.nb / 2 : p.nb, p.kbs))
     return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for the vocabulary projection");
   p.bias = S->b;
   p.part_max = S->parts.as<float>(); p.part_sum = p.part_max + (size_t)np * N;
   p.part_rows = S->BN / zrnn::kPersistentParts; p.n_parts = np;
   p.err = tc_error_word();
   return ZRNN_OK;
+}
+cudaError_t vocab_launch(const zrnn::VocabParams& p, int eng, int epi, cudaStream_t st) {
+  return p.M <= zrnn::kVocabFewCols ? zrnn::launch_tc_vocab(p, eng_tcmode(eng), epi, st) : zrnn::launch_tc_vocab_pair(p, eng_tcmode(eng), epi, st);
 }
 // per-column (max, sum exp) partials over this layer's rows + target logit into S->parts / tgt
 // tgt_zeroed: the caller's first launch has zeroed tgt
@@ -676,13 +686,13 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   }
   const int eng = S->eng, np = S->n_tiles * zrnn::kPersistentParts;
   ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
-  if (N <= vocab_cols_limit(S)) {
+  if (N <= zrnn::kVocabFewCols || !short_lse(S)) {
     zrnn::VocabParams vp;
     ZR_TRY(vocab_params(S, h, N, np, vp));
     vp.target = targets; vp.target_offset = S->lo; vp.tgt_logit = tgt;
     *n_parts = np; *pm = vp.part_max; *ps = vp.part_sum;
     KScope ks(KC_SOFTMAX_GEMM, st);
-    ZR_CUDA(zrnn::launch_tc_vocab(vp, eng_tcmode(eng), zrnn::TC_EPI_LSE, st));
+    ZR_CUDA(vocab_launch(vp, eng, zrnn::TC_EPI_LSE, st));
     return ZRNN_OK;
   }
   zrnn::TcParams tp;
@@ -697,7 +707,7 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   if (g_tc_prof_slot >= 0) prof_attach(tp);
   *n_parts = np; *pm = tp.part_max; *ps = tp.part_sum;
   KScope ks(KC_SOFTMAX_GEMM, st);
-  ZR_CUDA(zrnn::launch_tc_gemm_persistent(tp, eng_tcmode(eng), zrnn::TC_EPI_LSE, st));
+  ZR_CUDA(zrnn::launch_tc_gemm_persistent(tp, eng_tcmode(eng), st));
   return ZRNN_OK;
 }
 
@@ -728,35 +738,19 @@ int softmax_logits_act(zrnn_softmax* S, const Act& h, int N, cudaStream_t st, co
     g.M = Vs; g.N = N; g.C = S->logits.as<float>(); g.ldc = Vs; g.bias[0] = S->b;
     KScope ks(KC_SOFTMAX_GEMM, st);
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, (N >= 96 && Vs >= 512) ? 1 : 0, st));
-  } else if (N <= vocab_cols_limit(S)) {
+  } else {
     np = S->n_tiles * zrnn::kPersistentParts;
     ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
     zrnn::VocabParams vp;
     ZR_TRY(vocab_params(S, h, N, np, vp));
     vp.C = S->logits.as<float>(); vp.ldc = Vs;
+    // the epilogue also leaves each part's maximum and exp-sum: the top-k kernel derives the normaliser and its
+    // selection bound from them and then reads only the few parts that reach the bound
     if (!ps_out) vp.part_sum = nullptr;
     pm = vp.part_max;
     if (ps_out) *ps_out = vp.part_sum;
     KScope ks(KC_SOFTMAX_GEMM, st);
-    ZR_CUDA(zrnn::launch_tc_vocab(vp, eng_tcmode(S->eng), zrnn::TC_EPI_STORE, st));
-  } else {
-    const int eng = S->eng;
-    np = S->n_tiles * zrnn::kPersistentParts;
-    ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
-    zrnn::TcParams tp;
-    std::memset(&tp, 0, sizeof(tp));
-    ZR_TRY(act_maps(h, eng, S->H, S->Kpad, N, &tp.a, &tp.a_lo));
-    tp.kblocks = (S->H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
-    tp.b = S->dmap; tp.b_lo = S->dmap_lo;
-    tp.M = N; tp.N = Vs; tp.bias = S->b; tp.C = S->logits.as<float>(); tp.ldc = Vs;
-    // the epilogue also leaves each tile's maximum and exp-sum: the top-k kernel derives the normaliser and its
-    // selection bound from them and then reads only the few tiles that reach the bound
-    tp.part_max = S->parts.as<float>(); tp.part_sum = ps_out ? tp.part_max + (size_t)np * N : nullptr;
-    pm = tp.part_max;
-    if (ps_out) *ps_out = tp.part_sum;
-    tp.err = tc_error_word();
-    KScope ks(KC_SOFTMAX_GEMM, st);
-    ZR_CUDA(zrnn::launch_tc_gemm_persistent(tp, eng_tcmode(eng), zrnn::TC_EPI_STORE, st));
+    ZR_CUDA(vocab_launch(vp, S->eng, zrnn::TC_EPI_STORE, st));
   }
   *pm_out = pm;
   *np_out = np;
@@ -1688,8 +1682,8 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
       a.h_seq = seq[l].f32;
       a.xp = m->seq_xp.as<float>();
       a.ld_op = g.Kpad;
-      // the decoder's cells, the attention and the vocabulary projection of few columns read whole k-blocks of these rows
-      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm || S * B <= zrnn::kVocabMaxCols;
+      // the decoder's cells, the attention and the vocabulary projections but one read whole k-blocks of these rows
+      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm || S * B <= zrnn::kVocabFewCols || !short_lse(m->sm);
       if (g.eng == ENG_BF16) a.op_b16 = seq[l].hi;
       else if (g.eng == ENG_H2) { a.op_h_hi = seq[l].hi; a.op_h_lo = seq[l].lo; }
       else if (g.eng != ENG_SIMT) { a.op_hi = (float*)seq[l].hi; a.op_lo = g.eng == ENG_X3 ? seq[l].lo : nullptr; }
