@@ -145,6 +145,27 @@ def test_vocabulary_projection_edges(dtype, H, V, N):
     np.testing.assert_allclose(got.cpu().numpy().reshape(-1), logp[np.arange(N), tgt], rtol=r, atol=a)
 
 
+@pytest.mark.parametrize("H,n_sent,beam", [(504, 5, 9), (520, 9, 8), (1000, 2, 12)])
+def test_ensemble_of_one_model_twice(H, n_sent, beam):
+    """The models of an ensemble run side by side and their cells take half an SM, a lone model's take all of it: a model beside its copy finds
+    the hypotheses that it finds alone (the mean of two equal distributions), scores within the rounding of log(mean(exp))."""
+    from zoph_rnn_b200 import api, synth
+    cfg = synth.make_cfg(2, H, 200, 1500, attention=2, feed_input=1)
+    w = synth.make_weights(cfg, seed=H, dist="normal", scale=2 / np.sqrt(H))
+    ms = []
+    for _ in range(2):
+        m = api.neuralMT_model(cfg, dtype=5)
+        m.load_weights(w)
+        ms.append(m)
+    rng = np.random.default_rng(H + beam)
+    srcs = [rng.integers(2, 200, n).astype(np.int32) for n in rng.integers(1, 9, n_sent)]
+    kw = dict(beam=beam, k_best=1, min_ratio=0.5, max_ratio=1.5, longest_sent=30)
+    one, two = ms[0].decode(srcs, **kw), api.decode_ensemble(ms, [srcs, srcs], **kw)
+    np.testing.assert_array_equal(two[1], one[1])
+    np.testing.assert_array_equal(two[0], one[0])
+    np.testing.assert_allclose(two[2], one[2], rtol=1e-5)
+
+
 @pytest.mark.parametrize("dtype,H,V,N", [(5, 336, 129, 65), (5, 336, 256, 96), (5, 324, 257, 97), (5, 320, 513, 513), (5, 1000, 3001, 700), (5, 600, 20000, 1025),
                                          (4, 104, 385, 160), (4, 324, 19001, 321), (1, 1024, 511, 160), (1, 1032, 2050, 289), (2, 544, 700, 255)])
 def test_vocabulary_projection_pairs_of_ctas(dtype, H, V, N):

@@ -456,17 +456,18 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_
 
 }  // namespace
 
-// Which tile: a launch takes, per wave of CTAs, the longest of (a) the bytes a CTA fetches, at the 77 KB/us that an SM takes in from
-// L2 while all of them load, (b) the MMAs, (c) the shared-memory traffic of both, 128 bytes per cycle; then a fixed part, the
-// exchange of a K split and an epilogue that grows with the outputs per CTA.  Of a narrow tile's early sources half is counted: the
-// other half runs beside the predecessor.
-ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M) {
+// Which tile: a launch takes, per wave of CTAs, the longest of (a) the bytes a CTA fetches, at the 77 KB/us that its loop of loads and
+// MMAs takes in, (b) the MMAs, (c) the shared-memory traffic of both, 128 bytes per cycle; then a fixed part, the exchange of a K
+// split and an epilogue that grows with the outputs per CTA.  Of a narrow tile's early sources half is counted: the other half runs
+// beside the predecessor.
+ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside) {
   const bool two = mode_split(mode);
   const int parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
-  ChainPlan best{0, 1, 1e30f};
+  ChainPlan best{0, 1, 1e30f, false};
   for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 256; BN *= 2) {
     if (BN == 256 && (cells > 1 || mode == TC_TF32X3)) continue;  // (one accumulator over all of K: not for the most exact mode)
-    for (int split = 1; split <= 2; ++split) {
+    for (int split = 1; split <= 4; split *= 2) {
+      if (split == 4 && (epi == TC_EPI_LSTM || BN != 32)) continue;
       if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
       const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + 147) / 148;
       const float n_mma = BN <= 64 || !two ? 45.f : 64.f, cyc_n = BN <= 64 ? 48.f : BN / 2.f;
@@ -475,8 +476,8 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
       const float writes = parts * 128.f * (a_rows + BN);
       const float kb_us = std::max(writes / 77e3f, std::max(mma, (reads + writes) / 128.f) / 1900.f);
       const float kbs = kb * (nsrc - (BN <= 64 ? 0.5f * n_early : 0.f)) / split;
-      const float us = 3.2f + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : 0.f);
-      if (us < best.us) best = ChainPlan{BN, split, us};
+      const float us = 3.2f + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : split == 4 ? 1.8f : 0.f);
+      if (us < best.us) best = ChainPlan{BN, split, us, two && epi == TC_EPI_LSTM && BN <= 64 && !beside};
     }
   }
   return best;
@@ -490,7 +491,7 @@ int chain_kbs(int mode, int BN, int a_rows, int kb, int split) {
   return k;
 }
 
-cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st) {
+cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st) {
   if (n < 1 || n > ChainBatch::MAX) return cudaErrorInvalidValue;
   for (int i = 0; i < n; ++i) {
     const ChainParams& p = b.p[i];
@@ -500,7 +501,7 @@ cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int ep
         p.n_early < 0 || p.n_early >= p.nsrc)
       return cudaErrorInvalidValue;
   }
-  if (BN <= 64) return launch_tc_link(b, n, BN, mode, epi, split, st);
+  if (BN <= 64) return launch_tc_link(b, n, BN, mode, epi, split, whole, st);
   if (split != 1) return cudaErrorInvalidValue;
   switch (mode) {
     case TC_BF16: return launch_mode<TC_BF16>(b, n, BN, epi, st);

@@ -42,9 +42,10 @@ struct ChainBatch {
 };
 // n independent problems (same BN, mode, epilogue, N; M <= 128 each when n > 1) in one launch.
 // BN: 32, 64, 128, 256 for LSTM (256: tiles of two packed 128-row tiles); 16, 32, 64, 128, 256 for STORE.
-// split == 2 (n == 1, BN <= 64): two CTAs per tile, each over half of the K axis.
-cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st);
-cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st);
+// split == 2 (n == 1, BN <= 64) or 4 (n == 1, BN == 32, STORE): CTAs per tile, each over its part of the K axis.
+// whole (BN <= 64, LSTM, split modes): a CTA takes an SM, not half of one.
+cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
+cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
 // k-blocks per ring stage and TMA box: a TMA instruction costs its issuing thread about 200 cycles and a stage's hand-over 300
 int chain_kbs(int mode, int BN, int a_rows, int kb, int split);
 int link_kbs(int mode, int BN, int a_rows, int kb, int split);
@@ -52,9 +53,11 @@ int link_kbs(int mode, int BN, int a_rows, int kb, int split);
 struct ChainPlan {
   int BN, split;
   float us;
+  bool whole;
 };
-// rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks per source; M: columns
-ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M);
+// rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks per source; M: columns; beside: links of other
+// streams run at the same time
+ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside);
 
 // K-major rows as 4-D boxes (k within a 128-byte block, row, part, k-block): box_rows rows of all parts of box_kb k-blocks.
 // parts == 2: the lo rows lie part_bytes behind the hi rows.

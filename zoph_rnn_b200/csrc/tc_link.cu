@@ -1,22 +1,29 @@
 // tcgen05 kernel for the links of the recurrent chain whose tiles are narrow: 128 batch rows x BN = 16 .. 64 weight rows, the K
-// axis over SPLIT = 1 or 2 CTAs of a cluster (LSTM cells, attention projections, combiner; wide tiles: tc_chain.cu).
+// axis over SPLIT = 1, 2 or 4 CTAs of a cluster (LSTM cells, attention projections, combiner; wide tiles: tc_chain.cu).
 //
-// A link spends 4 - 5 us on launch, barrier and TMEM set-up, the first loads, exchange and epilogue, and the rest on bringing
-// operands into the SMs (about 77 KB/us each when all of them load).  A CTA is therefore kept to half of an SM - 113 KB of shared
-// memory, 256 TMEM columns, 384 threads x 80 registers - so that the next link's CTAs are resident while this one runs, and a
-// link multiplies what it already can before its predecessor has finished: the weights against the sources that were complete
-// earlier (n_early: the recurrent input of a cell, the hidden state in the combiner), which are half of the work.  Only the rest,
-// the exchange and the epilogue are left for the time after the predecessor's end.  Kernels on the chain let their successor
-// start only after their own griddepcontrol.wait has returned: everything up to the predecessor's predecessor is then complete.
+// A link spends 4 - 5 us on launch, barrier and TMEM set-up, the first loads, exchange and epilogue, and the rest on its MMAs: one
+// takes some 60 cycles to issue and to run, however few its rows, so a k-block of 128 x 64 in the split modes (8 MMAs) 512 at best.
+//
+// Half an SM per CTA - 113 KB of shared memory, 256 TMEM columns, 384 threads x 80 registers: the next link's CTAs are resident while
+// this one runs, and a link multiplies what it already can before its predecessor has finished: the weights against the sources
+// that were complete earlier (n_early: the recurrent input of a cell, the hidden state in the combiner), which are half of the work.
+// Only the rest, the exchange and the epilogue are left for the time after the predecessor's end.  Kernels on the chain let their
+// successor start only after their own griddepcontrol.wait has returned: everything up to the predecessor's predecessor is then complete.
+//
+// A whole SM per CTA (WHOLE: cells of the split modes, and launches of several cells): with all 512 TMEM columns each MMA warp has two
+// accumulator sets, so that it need not wait for a round to be added up, and a CTA's MMAs have the tensor core to themselves: 0.36 us
+// per k-block against 0.51.  That is worth more than the overlap (us per link in a scoring pass, 2 x 1000 units, 64 columns 13.7 ->
+// 10.2; 4 x 1000, 128 columns 13.4 -> 11.2; a pass 4693 -> 4378 and 6921 -> 6662), unless other streams' links run beside (two models
+// of an ensemble: a search 3806 -> 4008), and it is worth nothing in bf16, which adds up no rounds (3138 / 3150).
 //
 // Warps: 0 - 7 epilogue (warp w reads TMEM lane quadrant w % 4 and takes column group w / 4 of the tile), 8 activation loads,
 // 9 weight loads, 10 and 11 issue MMAs, each into accumulators of its own, so that the wait for a stage and the commit (300
 // cycles in one thread, as long as a k-block's MMAs) of one overlap the other's MMAs.
 //
-// Us per link inside a scoring pass, with a CTA per SM and everything after the wait -> now: 4 x 1000 units, 128 columns, bf16:
-// cells 2 - 4 of a step 9.0 -> 6.4 - 8.0, combiner 8.3 -> 6.5; f32 15.1 -> 10.5 - 15 (there the loads bound it: 75 % of them are
-// activations, which every row tile reads again).  Not better: four CTAs per tile; the successor's start put off to the end of
-// this link's loads (f32 cells 13.9 -> 16.5).
+// Not better: the successor's start put off to the end of this link's loads (f32 cells 13.9 -> 16.5); one MMA warp with two sets in turn
+// (3 x 500, 50 columns 1036 -> 1336 us a pass).  Four CTAs per tile (STORE): half the k-blocks of the narrower tile that two CTAs
+// would need for as many CTAs, for an exchange of 12 KB instead of 4 KB; combiner of 1000 units, 64 columns 6.6 -> 5.2 us, 128 columns
+// 8.3 -> 7.1.
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -423,20 +430,20 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   }
 }
 
-template <int BN, int MODE, int EPI, int SPLIT>
-__global__ void __launch_bounds__(kThreads, 2) tc_link_kernel(const __grid_constant__ ChainParams p, int stages) {
-  link_body<BN, MODE, EPI, SPLIT, false>(p, (int)blockIdx.x, stages);
+template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
+__global__ void __launch_bounds__(kThreads, WHOLE ? 1 : 2) tc_link_kernel(const __grid_constant__ ChainParams p, int stages) {
+  link_body<BN, MODE, EPI, SPLIT, WHOLE>(p, (int)blockIdx.x, stages);
 }
 // Several independent problems of one row block each (M <= 128): blockIdx.x selects the problem.  The cells of one
 // anti-diagonal of a stack (layer l at step t, layer l - 1 at step t + 1, ...) do not depend on one another.
 template <int BN, int MODE>
-__global__ void __launch_bounds__(kThreads, 2) tc_link_multi_kernel(const __grid_constant__ ChainBatch pb, int stages) {
+__global__ void __launch_bounds__(kThreads, 1) tc_link_multi_kernel(const __grid_constant__ ChainBatch pb, int stages) {
   link_body<BN, MODE, TC_EPI_LSTM, 1, true>(pb.p[blockIdx.x], 0, stages);
 }
 
 const bool g_pdl_on = std::getenv("ZRNN_NO_PDL") == nullptr;
 
-template <int BN, int MODE, int EPI, int SPLIT>
+template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
 cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   const ChainParams& p = b.p[0];
   const int stage = (mode_split(MODE) ? 2 : 1) * p.kbs * (p.a_rows + BN) * 128;
@@ -445,7 +452,7 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   const int its = (p.kb + p.kbs - 1) / p.kbs;
   if (its < SPLIT) return cudaErrorInvalidValue;
   // (a launch of several cells has no early sources: it takes the whole SM, 3 x 500, 50 columns 9.7 us a launch against 11)
-  int stages = ((n > 1 ? kWholeSm : kHalfSm) - fixed) / stage;
+  int stages = ((WHOLE ? kWholeSm : kHalfSm) - fixed) / stage;
   stages = std::min(std::min(stages, (int)kMaxStages), p.nsrc * ((its + SPLIT - 1) / SPLIT));
   if (stages < kMmaWarps) stages = kMmaWarps;  // (both MMA warps own a stage)
   const size_t smem = (size_t)stages * stage + fixed;
@@ -454,9 +461,9 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_link_kernel<BN, MODE, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaError_t e = cudaFuncSetAttribute(tc_link_kernel<BN, MODE, EPI, SPLIT, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
     if (e != cudaSuccess) return e;
-    if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1) {
+    if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1 && WHOLE) {
       e = cudaFuncSetAttribute(tc_link_multi_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
       if (e != cudaSuccess) return e;
     }
@@ -486,29 +493,37 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = na;
   count_launch();
-  if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1) {
+  if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1 && WHOLE) {
     if (n > 1) return cudaLaunchKernelEx(&cfg, tc_link_multi_kernel<BN, MODE>, b, stages);
   }
-  return cudaLaunchKernelEx(&cfg, tc_link_kernel<BN, MODE, EPI, SPLIT>, p, stages);
+  return cudaLaunchKernelEx(&cfg, tc_link_kernel<BN, MODE, EPI, SPLIT, WHOLE>, p, stages);
 }
 template <int MODE, int EPI, int SPLIT>
-cudaError_t launch_bn(const ChainBatch& b, int n, int BN, cudaStream_t st) {
-  if (BN == 32) return launch_t<32, MODE, EPI, SPLIT>(b, n, st);
-  if (BN == 64) return launch_t<64, MODE, EPI, SPLIT>(b, n, st);
+cudaError_t launch_bn(const ChainBatch& b, int n, int BN, bool whole, cudaStream_t st) {
+  if constexpr (EPI == TC_EPI_LSTM && (SPLIT == 1 || mode_split(MODE))) {
+    if (n > 1 || whole) {
+      if (BN == 32) return launch_t<32, MODE, EPI, SPLIT, true>(b, n, st);
+      if (BN == 64) return launch_t<64, MODE, EPI, SPLIT, true>(b, n, st);
+      return cudaErrorInvalidValue;
+    }
+  }
+  if (BN == 32) return launch_t<32, MODE, EPI, SPLIT, false>(b, n, st);
+  if (BN == 64) return launch_t<64, MODE, EPI, SPLIT, false>(b, n, st);
   if constexpr (EPI == TC_EPI_STORE) {
-    if (BN == 16) return launch_t<16, MODE, EPI, SPLIT>(b, n, st);
+    if constexpr (SPLIT < 4) if (BN == 16) return launch_t<16, MODE, EPI, SPLIT, false>(b, n, st);
   }
   return cudaErrorInvalidValue;
 }
 template <int MODE>
-cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, int split, cudaStream_t st) {
+cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, int split, bool whole, cudaStream_t st) {
   if (n > 1 && split > 1) return cudaErrorInvalidValue;
   if (epi == TC_EPI_LSTM) {
-    if (split == 1) return launch_bn<MODE, TC_EPI_LSTM, 1>(b, n, BN, st);
-    if (split == 2) return launch_bn<MODE, TC_EPI_LSTM, 2>(b, n, BN, st);
+    if (split == 1) return launch_bn<MODE, TC_EPI_LSTM, 1>(b, n, BN, whole, st);
+    if (split == 2) return launch_bn<MODE, TC_EPI_LSTM, 2>(b, n, BN, whole, st);
   } else if (n == 1) {
-    if (split == 1) return launch_bn<MODE, TC_EPI_STORE, 1>(b, n, BN, st);
-    if (split == 2) return launch_bn<MODE, TC_EPI_STORE, 2>(b, n, BN, st);
+    if (split == 1) return launch_bn<MODE, TC_EPI_STORE, 1>(b, n, BN, whole, st);
+    if (split == 2) return launch_bn<MODE, TC_EPI_STORE, 2>(b, n, BN, whole, st);
+    if (split == 4) return launch_bn<MODE, TC_EPI_STORE, 4>(b, n, BN, whole, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -524,12 +539,12 @@ int link_kbs(int mode, int BN, int a_rows, int kb, int split) {
   return k;
 }
 
-cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, cudaStream_t st) {
+cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st) {
   switch (mode) {
-    case TC_BF16: return launch_mode<TC_BF16>(b, n, BN, epi, split, st);
-    case TC_TF32: return launch_mode<TC_TF32>(b, n, BN, epi, split, st);
-    case TC_TF32X3: return launch_mode<TC_TF32X3>(b, n, BN, epi, split, st);
-    case TC_F16X2: return launch_mode<TC_F16X2>(b, n, BN, epi, split, st);
+    case TC_BF16: return launch_mode<TC_BF16>(b, n, BN, epi, split, whole, st);
+    case TC_TF32: return launch_mode<TC_TF32>(b, n, BN, epi, split, whole, st);
+    case TC_TF32X3: return launch_mode<TC_TF32X3>(b, n, BN, epi, split, whole, st);
+    case TC_F16X2: return launch_mode<TC_F16X2>(b, n, BN, epi, split, whole, st);
   }
   return cudaErrorInvalidValue;
 }

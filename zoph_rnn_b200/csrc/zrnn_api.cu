@@ -413,10 +413,10 @@ struct LinkPlan {
   bool skinny;
   zrnn::ChainPlan chain;
 };
-LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int cols, int n = 1) {
+LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int cols, int n = 1, bool beside = false) {
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
-  p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols);
+  p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols, beside);
   p.skinny = skinny_engine(eng) && cols <= 64 && zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) < p.chain.us;
   return p;
 }
@@ -525,13 +525,14 @@ int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act*
 // One LSTM cell.  x / h_prev / htild and the output are activations in the form the layer's engine needs.
 // early: inputs that were complete before the launch ahead of this one began its work: the kernels multiply by them while that
 // launch runs (every kernel on the chain lets its successor start only after its own wait)
-enum { EARLY_X = 1, EARLY_H = 2 };
+// BESIDE: launches of other streams run at the same time (the models of an ensemble)
+enum { EARLY_X = 1, EARLY_H = 2, BESIDE = 4 };
 int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
                  int B, const Act& out, float* c_out, cudaStream_t st, int early = 0) {
   if (L->eng == ENG_SIMT)
     return lstm_cell_simt(L, x.f32, mask, hp.f32, c_prev, q ? q->f32 : nullptr, B, out.f32, c_out, st);
   const int H = L->H, eng = L->eng;
-  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, (early & 1) + (early >> 1), H, B);
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, (early & 1) + (early >> 1 & 1), H, B, 1, (early & BESIDE) != 0);
   KScope ks(KC_LSTM, st);
   if (plan.skinny) {
     zrnn::SkinnyBatch sb;
@@ -541,7 +542,7 @@ int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, 
   }
   zrnn::ChainBatch cb;
   ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain, early, cb.p[0]));
-  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, st));
+  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, plan.chain.whole, st));
   return ZRNN_OK;
 }
 // out = act(W [a0 | a1] + bias) * mask for plain K-major weight rows, act = tanh on the first act_rows rows (0: all)
@@ -569,7 +570,7 @@ int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, c
   ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain, a1_early, p));
   p.bias = bias; p.mask = mask; p.act = 1; p.act_rows = act_rows; p.C = C; p.ldc = ldc;
   if (op) chain_operand_outputs(p, eng, *op, Kpad);
-  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, plan.chain.split, st));
+  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, plan.chain.split, plan.chain.whole, st));
   return ZRNN_OK;
 }
 
@@ -1717,7 +1718,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         ++n;
       }
       if (plan.skinny) ZR_CUDA(zrnn::launch_skinny(sb, n, skinny_mode(L0->eng), zrnn::SK_EPI_LSTM, s));
-      else ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, s));
+      else ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, true, s));
     }
     return ZRNN_OK;
   }
@@ -2190,6 +2191,7 @@ struct BeamModel {
   Geom g{0, 0, 0};
   bool tc = false;
   int S_max = 0, n = 0, NB = 0, beam = 0;
+  bool beside = false;  // other models' searches run on streams of their own at the same time
   int *src_id = nullptr, *src_mk = nullptr, *len = nullptr, *off = nullptr, *rep_map = nullptr;
   Act X0, zero, x, htild_new, htild_feed;
   std::vector<Act> sseq, hp, hn;
@@ -2291,7 +2293,7 @@ struct BeamModel {
     for (int l = 0; l < c.num_layers; ++l) {
       const bool use_feed = (l == 0 && c.feed_input && t > 0);
       ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], cols, hn[l], cn[l], s,
-                          l > 0 ? EARLY_H : 0));  // (layer 0 reads what the reorder launch just wrote)
+                          (l > 0 ? EARLY_H : 0) | (beside ? BESIDE : 0)));  // (layer 0 reads what the reorder launch just wrote)
       xin = hn[l];
     }
     *top = xin;
@@ -2383,7 +2385,7 @@ int beam_decode_core(zrnn_model* const* models, int K, const int* const* d_src, 
     b.m = models[k];
     b.g = Geom{models[k]->cfg.H, round64(models[k]->cfg.H), models[k]->eng};
     b.tc = models[k]->eng != ENG_SIMT;
-    b.S_max = S_max[k]; b.n = n; b.NB = NB; b.beam = beam;
+    b.S_max = S_max[k]; b.n = n; b.NB = NB; b.beam = beam; b.beside = K > 1;
     size_t bytes = b.bytes(track && k == 0, vote);
     if (k == 0) {  // shared bookkeeping lives in model 0's workspace
       bytes += aligned(sizeof(int) * 3 * n) + 2 * aligned(sizeof(int) * NB) + 2 * aligned(sizeof(int) * (size_t)NB * Lmax);
@@ -3000,7 +3002,7 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
     zrnn::ChainParams& p = cb.p[0];
     std::memset(&p, 0, sizeof(p));
     p.nsrc = 1; p.kb = (K + kb_elems - 1) / kb_elems;
-    const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, 1, p.kb, 0, m_cols);
+    const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, 1, p.kb, 0, m_cols, false);
     p.a_rows = chain_a_rows(m_cols);
     p.kbs = zrnn::chain_kbs(tcm, plan.BN, p.a_rows, p.kb, plan.split);
     const int kbs_total = Kpad / kb_elems;
@@ -3009,7 +3011,7 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
                              plan.BN, p.kbs))
       return fail(ZRNN_E_CUDA, "gemm: cannot encode TMA tensor maps");
     p.M = m_cols; p.N = n_rows; p.C = d_C; p.ldc = ldc; p.err = tc_error_word();
-    ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.BN, tcm, zrnn::TC_EPI_STORE, plan.split, st));
+    ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.BN, tcm, zrnn::TC_EPI_STORE, plan.split, plan.whole, st));
     return ZRNN_OK;
   };
   const int status = run();
