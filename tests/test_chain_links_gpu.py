@@ -56,6 +56,25 @@ def test_cell_edges(dtype, H, B, feed):
     np.testing.assert_allclose(got_c.cpu().numpy().reshape(B, H), cn * mask[:, None], rtol=r, atol=a)
 
 
+@pytest.mark.parametrize("dtype,H,B,feed", [(5, 1000, 257, 1), (5, 1000, 456, 0), (5, 968, 700, 1), (5, 1024, 900, 0), (5, 1000, 1100, 1), (4, 1000, 300, 1),
+                                            (4, 640, 1500, 0), (1, 1000, 700, 1), (1, 2048, 321, 0), (1, 1000, 900, 0), (2, 1000, 600, 0)])
+def test_cells_on_pairs_of_ctas(dtype, H, B, feed):
+    """Many columns: tiles of three, two and one accumulators, full and broken column tiles, an odd number of packed weight tiles."""
+    test_cell_edges(dtype, H, B, feed)
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,m,k", [(2000, 700, 1000), (2100, 513, 1000), (4000, 300, 1500)])
+def test_products_on_pairs_of_ctas(mode, n, m, k):
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(n + m + k)
+    W, X = (rng.standard_normal((k, n)) * 0.1).astype(np.float32), rng.standard_normal((m, k)).astype(np.float32)
+    C = api.gemm(torch.as_tensor(W).cuda().reshape(-1), torch.as_tensor(X).cuda().reshape(-1), n, m, k, mode).cpu().numpy().reshape(m, n)
+    scale = np.linalg.norm(X.astype(np.float64), axis=1)[:, None] * np.linalg.norm(W.astype(np.float64), axis=0)[None, :]
+    assert (np.abs(C - X.astype(np.float64) @ W.astype(np.float64)) / scale).max() < {1: 8e-3, 2: 1.5e-3, 3: 4e-6, 4: 4e-6}[mode]  # as the smaller products
+
+
 @pytest.mark.parametrize("dtype", sorted(TOL))
 @pytest.mark.parametrize("H,B", [(72, 1), (104, 9), (264, 16), (500, 17), (504, 33), (520, 64), (1000, 8), (1000, 65), (1000, 127), (1000, 129), (324, 200)])
 def test_scoring_with_early_operands_edges(dtype, H, B):

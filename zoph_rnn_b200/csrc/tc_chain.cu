@@ -1,8 +1,8 @@
-// tcgen05 kernel for the links of the recurrent chain with wide tiles (many columns, or several cells in a launch) and the rule
-// that picks a link's tile.  Narrow tiles: tc_link.cu.
+// tcgen05 kernel for the links of the recurrent chain with tiles of 128 batch rows x 128 weight rows (a few hundred columns, or several
+// cells in a launch), and the rule that picks a link's kernel and tile.  Narrow tiles: tc_link.cu; many columns: tc_cell_pair.cu.
 //
-// A CTA computes 128 batch rows x BN = 128 or 256 weight rows over the WHOLE K axis: no CTA waits for another one's partial
-// tile, so a launch is: activations in (one TMA latency), K loop, epilogue.
+// A CTA works over the WHOLE K axis: no CTA waits for another one's partial tile, so a launch is: activations in (one TMA latency),
+// K loop, epilogue.
 //
 // Warps: 16 epilogue warps (warp w reads TMEM lane quadrant w % 4 and takes column group w / 4 of the tile), one for the
 // activation loads, one for the weight loads, two that issue MMAs.  The weights do not depend on the predecessor kernel, so
@@ -21,9 +21,9 @@ namespace zrnn {
 namespace {
 
 constexpr int kEpiWarps = 16;
-// Two warps issue MMAs, so that the wait for a stage and the commit (300 cycles in one thread, as long as a k-block's MMAs) of
-// one overlap the other's MMAs.  They take alternate stages, each into accumulators of its own; wide tiles of the split modes
-// have no room for that, there one warp issues the hi * hi products of every stage and the other the two cross products.
+// Two warps issue MMAs, so that the wait for a stage and the commit of one overlap the other's MMAs.  They take alternate stages, each
+// into accumulators of its own; in the split modes there is no room for that: one warp issues the hi * hi products of every stage and
+// the other the two cross products.
 constexpr int kMmaWarps = 2;
 constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
 // The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb more than round_kb k-blocks
@@ -33,11 +33,11 @@ constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
 // Mean log-prob error against the oracle at H = 1000, 4 layers: 5.8e-7; with four accumulators over the whole K axis 13e-7.  Hidden
 // states of 4 x 640 units in 3xTF32 against float64: 5.8e-7 in rounds of 16 k-steps, 3.5e-7 at most in rounds of 8.
 __host__ __device__ constexpr int round_kb(int mode) { return mode == TC_TF32X3 ? 2 : 4; }
-__host__ __device__ constexpr bool chain_rounds(int BN, int mode) { return mode_split(mode) && BN <= 128; }
+__host__ __device__ constexpr bool chain_rounds(int mode) { return mode_split(mode); }
 // accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  Other modes: one per MMA warp.
-__host__ __device__ constexpr int chain_sets(int BN, int mode) { return !mode_split(mode) ? kMmaWarps : (BN <= 128 ? 3 : 1); }
+__host__ __device__ constexpr int chain_sets(int mode) { return mode_split(mode) ? 3 : kMmaWarps; }
 __host__ __device__ constexpr int chain_tmem(int BN, int mode) {
-  const int need = (chain_sets(BN, mode) + (mode_split(mode) ? 1 : 0)) * BN;
+  const int need = (chain_sets(mode) + (mode_split(mode) ? 1 : 0)) * BN;
   int c = 32;
   while (c < need) c *= 2;
   return c;
@@ -47,17 +47,17 @@ constexpr int kChainRingBytes = 224 * 1024, kMaxStages = 8;
 template <int BN, int MODE, int EPI>
 __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_block, const int stages) {
   constexpr int EW = kEpiWarps, kAWarp = EW, kWWarp = EW + 1, kMmaWarp = EW + 2;
-  constexpr bool BY_PRODUCT = mode_split(MODE), ROUNDS = chain_rounds(BN, MODE);
+  constexpr bool BY_PRODUCT = mode_split(MODE), ROUNDS = chain_rounds(MODE);
   constexpr int STEP = BY_PRODUCT ? 1 : kMmaWarps;  // stages from one of an MMA warp to its next
   constexpr int PARTS = mode_split(MODE) ? 2 : 1;
   constexpr int WKB = BN * 128;  // bytes of one k-block of one weight part
   constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN);
-  constexpr int NSET = chain_sets(BN, MODE), TMEM_COLS = chain_tmem(BN, MODE);
+  constexpr int NSET = chain_sets(MODE), TMEM_COLS = chain_tmem(BN, MODE);
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
   __shared__ __align__(8) uint64_t accum_bar;  // everything accumulated (rounds: the cross products of wide tiles)
-  __shared__ __align__(8) uint64_t set_full[chain_sets(BN, MODE)], set_empty[chain_sets(BN, MODE)];
+  __shared__ __align__(8) uint64_t set_full[chain_sets(MODE)], set_empty[chain_sets(MODE)];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   __shared__ float s_bias[BN];
@@ -80,7 +80,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
       mbar_init(&full_bar[s], 2);  // the activation and the weight producer
       mbar_init(&empty_bar[s], BY_PRODUCT ? kMmaWarps : 1);
     }
-    mbar_init(&accum_bar, BY_PRODUCT && ROUNDS ? 1 : kMmaWarps);
+    mbar_init(&accum_bar, BY_PRODUCT ? 1 : kMmaWarps);
     for (int i = 0; i < NSET; ++i) {
       mbar_init(&set_full[i], 1);
       mbar_init(&set_empty[i], EW);
@@ -114,17 +114,9 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         const int wkb = p.wkb0[s] + c * KBS;
         if (one) {
           mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * WKB));
-          if constexpr (EPI == TC_EPI_LSTM && BN <= 128) {
+          if constexpr (EPI == TC_EPI_LSTM) {
             constexpr int TH = BN / 4;
             tma_load_5d(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
-          } else if constexpr (EPI == TC_EPI_LSTM) {  // rows of several packed tiles side by side: one box per k-block, tile and part
-            constexpr int NP = BN / 128;
-            for (int b = 0; b < KBS; ++b)
-              for (int h = 0; h < NP; ++h)
-                for (int x = 0; x < PARTS; ++x) {
-                  const int tile = min(n_tile * NP + h, p.w_tiles - 1);  // (the units of a tile beyond the last are dropped)
-                  tma_load_5d(w + (b * PARTS + x) * WKB + h * (WKB / NP), &p.w, &full_bar[st], 0, x, tile * p.w_kbtot + wkb + b);
-                }
           } else {
             tma_load_4d(w, &p.w, &full_bar[st], n_tile * BN, wkb);
           }
@@ -298,11 +290,10 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         for (int u = 0; u < W; ++u) v[u] = fmaf(x[u], mode_cross_scale(MODE), v[u]);
       }
     } else {
-      float t[NSET][W], x[W];
+      float t[NSET][W];
 #pragma unroll
       for (int a = 0; a < NSET; ++a)
         if (a == 0 || a < n_sets) tmem_ldw<W>(taddr + a * BN + col, t[a]);
-      if (PARTS == 2) tmem_ldw<W>(taddr + NSET * BN + col, x);
       tmem_wait_ld();
 #pragma unroll
       for (int u = 0; u < W; ++u) v[u] = t[0][u];
@@ -312,10 +303,6 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
 #pragma unroll
           for (int u = 0; u < W; ++u) v[u] += t[a][u];
         }
-      if (PARTS == 2) {
-#pragma unroll
-        for (int u = 0; u < W; ++u) v[u] = fmaf(x[u], mode_cross_scale(MODE), v[u]);
-      }
     }
   };
   if (ready && live) {
@@ -448,37 +435,46 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
 template <int MODE>
 cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_t st) {
   if (epi == TC_EPI_LSTM && BN == 128) return launch_t<128, MODE, TC_EPI_LSTM>(b, n, st);
-  if (epi == TC_EPI_LSTM && BN == 256) return launch_t<256, MODE, TC_EPI_LSTM>(b, n, st);
   if (epi == TC_EPI_STORE && n == 1 && BN == 128) return launch_t<128, MODE, TC_EPI_STORE>(b, n, st);
-  if (epi == TC_EPI_STORE && n == 1 && BN == 256) return launch_t<256, MODE, TC_EPI_STORE>(b, n, st);
   return cudaErrorInvalidValue;
 }
 
 }  // namespace
 
-// Which tile: a launch takes, per wave of CTAs, the longest of (a) the bytes a CTA fetches, at the 77 KB/us that its loop of loads and
-// MMAs takes in, (b) the MMAs, (c) the shared-memory traffic of both, 128 bytes per cycle; then a fixed part, the exchange of a K
-// split and an epilogue that grows with the outputs per CTA.  Of a narrow tile's early sources half is counted: the other half runs
-// beside the predecessor.
+// Which tile: a launch takes, per wave of CTAs and k-block, the longer of the bytes a CTA fetches, at the 130 KB/us that an SM takes in
+// from L2, and the MMAs, of which each takes 60 cycles at least (the split modes at 128 rows, a warp per product and one cross
+// accumulator: 1.6 times their cycles; rounds with one accumulator set, on half an SM: 0.15 us more); then a fixed part per wave, the exchange of a K split and an epilogue that grows with the outputs per
+// CTA.  Of the early sources of links on half an SM half is counted: the other half runs beside the predecessor.  us, estimated /
+// measured, fp16 split: 1000 units, 128 columns 10.7 / 10.9, 200 columns 15.7 / 16.1, 384 in tiles of 128 rows 25.6 / 25.6; 500 units, 768
+// columns 15.1 / 15.9; bf16: 1000 units, 128 columns 7.7 / 7.8, 384 11.7 / 11.4.
 ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside) {
   const bool two = mode_split(mode);
   const int parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
-  ChainPlan best{0, 1, 1e30f, false};
-  for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 256; BN *= 2) {
-    if (BN == 256 && (cells > 1 || mode == TC_TF32X3)) continue;  // (one accumulator over all of K: not for the most exact mode)
+  ChainPlan best{0, 1, 1e30f, false, 0};
+  for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 128; BN *= 2) {
     for (int split = 1; split <= 4; split *= 2) {
       if (split == 4 && (epi == TC_EPI_LSTM || BN != 32)) continue;
       if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
       const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + 147) / 148;
-      const float n_mma = BN <= 64 || !two ? 45.f : 64.f, cyc_n = BN <= 64 ? 48.f : BN / 2.f;
-      const float mma = 4.f * (!two ? std::max(45.f, cyc_n) : (BN <= 64 ? std::max(45.f, (float)BN) + n_mma : 3.f * cyc_n));
-      const float reads = 4.f * (!two ? 4096.f + 32.f * BN : (BN <= 64 ? 8192.f + 96.f * BN : 3.f * (4096.f + 32.f * BN)));
-      const float writes = parts * 128.f * (a_rows + BN);
-      const float kb_us = std::max(writes / 77e3f, std::max(mma, (reads + writes) / 128.f) / 1900.f);
-      const float kbs = kb * (nsrc - (BN <= 64 ? 0.5f * n_early : 0.f)) / split;
-      const float us = 3.2f + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : split == 4 ? 1.8f : 0.f);
-      if (us < best.us) best = ChainPlan{BN, split, us, two && epi == TC_EPI_LSTM && BN <= 64 && !beside};
+      const bool whole = two && BN <= 64 && BN >= 32 && !beside;
+      const float cyc = 4.f * (!two ? std::max(60.f, BN / 2.f) : (BN <= 64 ? std::max(60.f, (float)BN) + 60.f : 1.6f * 3.f * BN / 2.f));
+      const float kb_us = std::max(parts * 128.f * (a_rows + BN) / 130e3f, cyc / 1850.f) + (two && epi == TC_EPI_STORE && BN <= 64 && !whole ? 0.15f : 0.f);
+      const float kbs = kb * (nsrc - (BN <= 64 && !whole ? 0.5f * n_early : 0.f)) / split;
+      const float us = (whole ? 3.6f : 3.2f) + 3.f * (waves - 1) + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : split == 4 ? 1.8f : 0.f);
+      if (us < best.us) best = ChainPlan{BN, split, us, whole, 0};
     }
+  }
+  // Pairs of CTAs, 148 SMs: a k-block's twelve MMAs (four) take 64 cycles each at least, half a cycle per column; set-up, first loads
+  // and end 8 us, all of an SM being needed.  More than 160 columns per tile have one accumulator for the whole K axis in the split
+  // modes: only where tiles of 128 rows and columns would not fit one wave.
+  const int row_tiles = (rows + 255) / 256;
+  for (int n_ct = (M + 255) / 256; M > 256 && cells == 1 && n_ct <= (M + 31) / 32; ++n_ct) {
+    const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
+    if (two && nb > 160 && (mode == TC_TF32X3 || (M + 127) / 128 * ((rows + 127) / 128) <= 148)) continue;
+    const int waves = (row_tiles * n_ct + 73) / 74;
+    const float cyc = two ? std::max(800.f, 6.5f * nb) : std::max(330.f, 2.2f * nb);
+    const float us = 8.f + waves * (nsrc * kb * cyc / 1850.f + (two ? 0.015f : 0.01f) * nb);
+    if (us < best.us) best = ChainPlan{128, 1, us, false, nb};
   }
   return best;
 }

@@ -9,8 +9,7 @@ namespace zrnn {
 // acc[M x N] = sum_s A_s[M x K] * W[N x Kcat]^T, both operands K-major; M: batch columns, N: weight rows
 struct ChainParams {
   CUtensorMap a[3];           // activation rows: make_rows_map with a_rows rows, all parts, kbs k-blocks
-  CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units (BN == 256: 32 units,
-                              // one part and one k-block per box)
+  CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units
   int w_kbtot, w_tiles;       // LSTM: k-blocks per packed tile, packed tiles
   int nsrc, kb;               // sources, k-blocks per source
   int n_early;                // leading sources that were complete when the predecessor kernel passed its own wait
@@ -41,19 +40,23 @@ struct ChainBatch {
   ChainParams p[MAX];
 };
 // n independent problems (same BN, mode, epilogue, N; M <= 128 each when n > 1) in one launch.
-// BN: 32, 64, 128, 256 for LSTM (256: tiles of two packed 128-row tiles); 16, 32, 64, 128, 256 for STORE.
+// BN: 32, 64, 128 for LSTM; 16, 32, 64, 128 for STORE.
 // split == 2 (n == 1, BN <= 64) or 4 (n == 1, BN == 32, STORE): CTAs per tile, each over its part of the K axis.
-// whole (BN <= 64, LSTM, split modes): a CTA takes an SM, not half of one.
+// whole (BN == 32 or 64, split modes): a CTA takes an SM, not half of one.
 cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
 cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
 // k-blocks per ring stage and TMA box: a TMA instruction costs its issuing thread about 200 cycles and a stage's hand-over 300
 int chain_kbs(int mode, int BN, int a_rows, int kb, int split);
 int link_kbs(int mode, int BN, int a_rows, int kb, int split);
+// Pairs of CTAs (tc_cell_pair.cu): a_rows = nb / 2, kbs = cell_pair_kbs; weight boxes of 128 rows (STORE) or 32 units (LSTM).
+cudaError_t launch_tc_cell_pair(const ChainBatch& b, int n, int mode, int epi, cudaStream_t st);
+int cell_pair_kbs(int mode);
 // Tile width and K split of a launch, and about how long it takes.
 struct ChainPlan {
   int BN, split;
   float us;
   bool whole;
+  int nb;  // > 0: pairs of CTAs with tiles of nb columns; the other fields do not count
 };
 // rows: weight rows (LSTM: 4 H); cells: problems in the launch; kb: 128-byte k-blocks per source; M: columns; beside: links of other
 // streams run at the same time

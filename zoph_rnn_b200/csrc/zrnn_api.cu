@@ -279,7 +279,7 @@ struct zrnn_lstm_layer {
   int kbtot = 0;  // > 0: weights stored tile-contiguously with this many k-blocks per row tile
   OpMem Wcat, emb;
   CUtensorMap wmap, wmap_lo;
-  CUtensorMap gmap[4][3];  // boxes of 8 / 16 / 32 hidden units x 4 gates (tc_chain.cu)
+  CUtensorMap gmap[3][3];  // boxes of 8 / 16 / 32 hidden units x 4 gates, 1 / 2 / 4 k-blocks
   DevBuf sc_x, sc_h, sc_q;  // operand scratch for the fp32 layer-level entry points
   ~zrnn_lstm_layer() {
     cudaFree(W); cudaFree(Wh); cudaFree(Mx); cudaFree(Q); cudaFree(b);
@@ -417,7 +417,9 @@ LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
   p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols, beside);
-  p.skinny = skinny_engine(eng) && cols <= 64 && zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) < p.chain.us;
+  // (a warp-level kernel with early operands starts beside its predecessor, but then holds up the next one's start: skinny_gemm.cu)
+  p.skinny = skinny_engine(eng) && cols <= 64 &&
+             zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) + (epi == zrnn::TC_EPI_LSTM && n_early && !beside ? 1.f : 0.f) < p.chain.us;
   return p;
 }
 // weights stored in packed 128-row tiles: tile-contiguous k-blocks (kbtot > 0) or plain rows of ld elements
@@ -454,6 +456,14 @@ void skinny_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const A
 
 // ---- one link of the recurrent chain on tcgen05 without splitting K (tc_chain.cu)
 int chain_a_rows(int B) { return B >= 128 ? 128 : (B + 7) / 8 * 8; }
+// activation rows and k-blocks per box
+void chain_tile(zrnn::ChainParams& p, int mode, const zrnn::ChainPlan& plan, int B) {
+  p.a_rows = plan.nb ? plan.nb / 2 : chain_a_rows(B);
+  p.kbs = plan.nb ? zrnn::cell_pair_kbs(mode) : zrnn::chain_kbs(mode, plan.BN, p.a_rows, p.kb, plan.split);
+}
+cudaError_t chain_launch(const zrnn::ChainBatch& b, int n, const zrnn::ChainPlan& plan, int mode, int epi, cudaStream_t st) {
+  return plan.nb ? zrnn::launch_tc_cell_pair(b, n, mode, epi, st) : zrnn::launch_tc_chain(b, n, plan.BN, mode, epi, plan.split, plan.whole, st);
+}
 // where the epilogue leaves the operand-form copy of its output for the next product
 void chain_operand_outputs(zrnn::ChainParams& tp, int eng, const Act& out, int Kpad) {
   tp.ld_op = Kpad;
@@ -481,17 +491,16 @@ int chain_cell_params(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act
                       int B, const Act& out, float* c_out, const zrnn::ChainPlan& plan, int early, zrnn::ChainParams& p) {
   const int H = L->H, Kpad = L->Kpad, eng = L->eng, epk = 128 / eng_eb(eng);
   std::memset(&p, 0, sizeof(p));
-  p.a_rows = chain_a_rows(B);
   p.kb = (H + epk - 1) / epk;
+  chain_tile(p, eng_tcmode(eng), plan, B);
   const int BN = plan.BN;
-  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows, p.kb, plan.split);
   const Act* src[3] = {&x, &hp, q};
   for (int pass = 0; pass < 2; ++pass) {  // the early sources first
     for (int i = 0; i < (q ? 3 : 2); ++i)
       if ((early >> i & 1) == 1 - pass) ZR_TRY(chain_source(p, *src[i], eng, H, Kpad, B, i * Kpad));
     if (pass == 0) p.n_early = p.nsrc;
   }
-  p.w = L->gmap[BN == 32 ? 0 : (BN == 64 ? 1 : (BN == 128 ? 2 : 3))][p.kbs == 1 ? 0 : (p.kbs == 2 ? 1 : 2)];
+  p.w = L->gmap[BN == 32 ? 0 : (BN == 64 ? 1 : 2)][p.kbs == 1 ? 0 : (p.kbs == 2 ? 1 : 2)];
   p.w_kbtot = L->kbtot; p.w_tiles = L->n_tiles;
   p.M = B; p.N = H; p.bias = L->b; p.mask = mask;
   p.C = out.f32; p.ldc = H;
@@ -505,10 +514,9 @@ int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act*
                        const zrnn::ChainPlan& plan, bool a1_early, zrnn::ChainParams& p) {
   const int epk = 128 / eng_eb(eng);
   std::memset(&p, 0, sizeof(p));
-  p.a_rows = chain_a_rows(B);
   p.kb = (H + epk - 1) / epk;
+  chain_tile(p, eng_tcmode(eng), plan, B);
   const int BN = plan.BN;
-  p.kbs = zrnn::chain_kbs(eng_tcmode(eng), BN, p.a_rows, p.kb, plan.split);
   if (a1 && a1_early) ZR_TRY(chain_source(p, *a1, eng, H, Kpad, B, Kpad));
   p.n_early = p.nsrc;
   ZR_TRY(chain_source(p, *a0, eng, H, Kpad, B, 0));
@@ -542,14 +550,14 @@ int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, 
   }
   zrnn::ChainBatch cb;
   ZR_TRY(chain_cell_params(L, x, hp, q, mask, c_prev, B, out, c_out, plan.chain, early, cb.p[0]));
-  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_LSTM, plan.chain.split, plan.chain.whole, st));
+  ZR_CUDA(chain_launch(cb, 1, plan.chain, eng_tcmode(eng), zrnn::TC_EPI_LSTM, st));
   return ZRNN_OK;
 }
 // out = act(W [a0 | a1] + bias) * mask for plain K-major weight rows, act = tanh on the first act_rows rows (0: all)
 int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, const Act* a1, const float* bias, const int* mask,
-               int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st, bool a1_early = false) {
+               int act_rows, int B, float* C, int ldc, const Act* op, cudaStream_t st, bool a1_early, bool beside) {
   const int nsrc = a1 ? 2 : 1;
-  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, a1 && a1_early, H, B);
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_STORE, N, nsrc, a1 && a1_early, H, B, 1, beside);
   if (plan.skinny) {
     zrnn::SkinnyBatch sb;
     zrnn::SkinnyParams& sp = sb.p[0];
@@ -570,13 +578,13 @@ int link_store(int eng, const OpMem& w, int N, int H, int Kpad, const Act* a0, c
   ZR_TRY(chain_store_params(eng, w, N, (long long)nsrc * Kpad, a0, a1, H, Kpad, B, plan.chain, a1_early, p));
   p.bias = bias; p.mask = mask; p.act = 1; p.act_rows = act_rows; p.C = C; p.ldc = ldc;
   if (op) chain_operand_outputs(p, eng, *op, Kpad);
-  ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.chain.BN, eng_tcmode(eng), zrnn::TC_EPI_STORE, plan.chain.split, plan.chain.whole, st));
+  ZR_CUDA(chain_launch(cb, 1, plan.chain, eng_tcmode(eng), zrnn::TC_EPI_STORE, st));
   return ZRNN_OK;
 }
 
 // src_ready: a launch of this library lies between the ones that wrote the source states and lengths and the one ahead of this call
 int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const Act& out, float* align, cudaStream_t st,
-                int* viterbi = nullptr, float viterbi_init = -1.f, bool align_by_pos = false, bool src_ready = true) {
+                int* viterbi = nullptr, float viterbi_init = -1.f, bool align_by_pos = false, bool src_ready = true, bool beside = false) {
   const int H = A->H, eng = A->eng, Kpad = A->Kpad;
   ZR_CUDA(A->ctx.reserve(sizeof(float) * (size_t)H * B));
   KScope ks(KC_ATT, st);
@@ -609,7 +617,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
       g.M = 2 * H; g.N = B; g.C = A->tq.as<float>(); g.ldc = 2 * H; g.act = 1; g.act_rows = H;
       ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, 0, st));
     } else {
-      ZR_TRY(link_store(eng, A->WpWaT_op, 2 * H, H, Kpad, &h_t, nullptr, nullptr, nullptr, H, B, A->tq.as<float>(), 2 * H, nullptr, st));
+      ZR_TRY(link_store(eng, A->WpWaT_op, 2 * H, H, Kpad, &h_t, nullptr, nullptr, nullptr, H, B, A->tq.as<float>(), 2 * H, nullptr, st, false, beside));
     }
     a.tanh1 = A->tq.as<float>(); a.q = A->tq.as<float>() + H; a.ld_tq = 2 * H; a.v_p = A->v_p;
     ZR_CUDA(zrnn::launch_att_local(a, st));
@@ -625,7 +633,7 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
     g.M = H; g.N = B; g.C = out.f32; g.ldc = H; g.bias[0] = A->bias; g.mask = mask; g.act = 1;
     ZR_CUDA(zrnn::launch_fused_gemm(g, 1, zrnn::EPI_STORE, 0, st));
   } else {
-    ZR_TRY(link_store(eng, A->Wc_op, H, H, Kpad, &ctx, &h_t, A->bias, mask, 0, B, out.f32, H, &out, st, true));
+    ZR_TRY(link_store(eng, A->Wc_op, H, H, Kpad, &ctx, &h_t, A->bias, mask, 0, B, out.f32, H, &out, st, true, beside));
   }
   return ZRNN_OK;
 }
@@ -1091,10 +1099,9 @@ int zrnn_lstm_load(zrnn_lstm_layer* L, const float* const* t, int n) {
     }
     ZR_TRY(weight_maps(L->Wcat, L->eng, epk, rows * L->kbtot, L->BN, &L->wmap, &L->wmap_lo));
     const int parts = eng_split(L->eng) ? 2 : 1;
-    for (int i = 0; i < 4; ++i)    // boxes of 8, 16 and 32 units with all parts, and of 32 units of one part
-      for (int k = 0; k < 3; ++k)  // of 1, 2 and 4 k-blocks
-        if (!zrnn::make_gate_map(&L->gmap[i][k], L->Wcat.hi, eng_eb(L->eng), parts, L->Wcat.part_bytes(), L->n_tiles * L->kbtot,
-                                 i < 3 ? 8 << i : 32, i < 3 ? parts : 1, i < 3 ? 1 << k : 1))
+    for (int i = 0; i < 3; ++i)
+      for (int k = 0; k < 3; ++k)
+        if (!zrnn::make_gate_map(&L->gmap[i][k], L->Wcat.hi, eng_eb(L->eng), parts, L->Wcat.part_bytes(), L->n_tiles * L->kbtot, 8 << i, parts, 1 << k))
           return fail(ZRNN_E_CUDA, "cannot encode a TMA tensor map for the gate weights");
     if (L->is_ih) {
       ZR_TRY(L->emb.alloc((size_t)L->V * Kpad, L->eng));
@@ -1718,7 +1725,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         ++n;
       }
       if (plan.skinny) ZR_CUDA(zrnn::launch_skinny(sb, n, skinny_mode(L0->eng), zrnn::SK_EPI_LSTM, s));
-      else ZR_CUDA(zrnn::launch_tc_chain(m->diag, n, plan.chain.BN, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, 1, true, s));
+      else ZR_CUDA(chain_launch(m->diag, n, plan.chain, eng_tcmode(L0->eng), zrnn::TC_EPI_LSTM, s));
     }
     return ZRNN_OK;
   }
@@ -2298,7 +2305,7 @@ struct BeamModel {
     }
     *top = xin;
     if (c.attention) {
-      ZR_TRY(att_forward(m->att, xin, nullptr, cols, htild_new, align_pos, s, vit, 0.f, align_pos != nullptr));
+      ZR_TRY(att_forward(m->att, xin, nullptr, cols, htild_new, align_pos, s, vit, 0.f, align_pos != nullptr, true, beside));
       *top = htild_new;
     }
     return ZRNN_OK;
@@ -3003,15 +3010,14 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
     std::memset(&p, 0, sizeof(p));
     p.nsrc = 1; p.kb = (K + kb_elems - 1) / kb_elems;
     const zrnn::ChainPlan plan = zrnn::plan_chain(tcm, zrnn::TC_EPI_STORE, n_rows, 1, 1, p.kb, 0, m_cols, false);
-    p.a_rows = chain_a_rows(m_cols);
-    p.kbs = zrnn::chain_kbs(tcm, plan.BN, p.a_rows, p.kb, plan.split);
+    chain_tile(p, tcm, plan, m_cols);
     const int kbs_total = Kpad / kb_elems;
     if (!zrnn::make_rows_map(&p.a[0], a_hi, eb, (long long)Kpad * eb, m_cols, parts, (long long)a_part, kbs_total, p.a_rows, p.kbs) ||
         !zrnn::make_rows_map(&p.w, b_hi, eb, (long long)Kpad * eb, (long long)n_tiles * 128, parts, (long long)b_part, kbs_total,
                              plan.BN, p.kbs))
       return fail(ZRNN_E_CUDA, "gemm: cannot encode TMA tensor maps");
     p.M = m_cols; p.N = n_rows; p.C = d_C; p.ldc = ldc; p.err = tc_error_word();
-    ZR_CUDA(zrnn::launch_tc_chain(cb, 1, plan.BN, tcm, zrnn::TC_EPI_STORE, plan.split, plan.whole, st));
+    ZR_CUDA(chain_launch(cb, 1, plan, tcm, zrnn::TC_EPI_STORE, st));
     return ZRNN_OK;
   };
   const int status = run();
