@@ -116,7 +116,9 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
           mbar_expect_tx(&full_bar[st], (uint32_t)(PARTS * KBS * WKB));
           if constexpr (EPI == TC_EPI_LSTM) {
             constexpr int TH = BN / 4;
-            tma_load_5d(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, (n_tile * TH / 32) * p.w_kbtot + wkb);
+            const int chunk = (n_tile * TH / 32) * p.w_kbtot + wkb;
+            if (p.w_first) tma_load_5d_first(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, chunk);
+            else tma_load_5d(w, &p.w, &full_bar[st], n_tile * TH % 32, 0, chunk);
           } else {
             tma_load_4d(w, &p.w, &full_bar[st], n_tile * BN, wkb);
           }

@@ -10,6 +10,7 @@ namespace zrnn {
 struct ChainParams {
   CUtensorMap a[3];           // activation rows: make_rows_map with a_rows rows, all parts, kbs k-blocks
   CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units
+  int w_first;                // LSTM, tiles of 128 rows: the weights' lines leave the L2 first
   int w_kbtot, w_tiles;       // LSTM: k-blocks per packed tile, packed tiles
   int nsrc, kb;               // sources, k-blocks per source
   int n_early;                // leading sources that were complete when the predecessor kernel passed its own wait

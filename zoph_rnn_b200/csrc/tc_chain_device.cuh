@@ -21,6 +21,15 @@ __device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* m
       : "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(part), "r"(kb)
       : "memory");
 }
+// ... whose lines leave the L2 first
+__device__ __forceinline__ void tma_load_5d_first(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int y, int part, int kb) {
+  asm volatile(
+      "{\n\t.reg .b64 pol;\n\tcreatepolicy.fractional.L2::evict_first.b64 pol, 1.0;\n\t"
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %3, %5, %6}], [%2], pol;\n\t}"
+      :
+      : "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(0), "r"(y), "r"(part), "r"(kb)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
   uint32_t r0, r1, r2, r3;
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"

@@ -1709,6 +1709,9 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
   if (!by_layers && L >= 2 && L <= zrnn::ChainBatch::MAX && L0->eng != ENG_SIMT && B <= 128) {
     const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, 0, g.H, B, L);
     KScope sweep(KC_LSTM, s, S * L, true);
+    // Weights that together exceed the L2 (126 MB), read launch after launch in the same order, would never be found there: the upper half
+    // of the layers gives way to the lower one (4 x 1000 units, 128 columns, 128 MB: 30.7 -> 28.2 us a launch)
+    const bool over_l2 = (size_t)L * layers[0]->n_tiles * layers[0]->kbtot * 128 * 128 * (eng_split(g.eng) ? 2 : 1) > ((size_t)110 << 20);
     zrnn::SkinnyBatch sb;
     for (int d = 0; d < S + L - 1; ++d) {
       int n = 0;
@@ -1721,6 +1724,7 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
         if (plan.skinny) skinny_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l], 0, sb.p[n]);
         else ZR_TRY(chain_cell_params(layers[l], x, hp, nullptr, mask + (size_t)t * B, cst[cu][l], B, out, cst[cu ^ 1][l],
                                       plan.chain, 0, m->diag.p[n]));
+        if (!plan.skinny) m->diag.p[n].w_first = over_l2 && l >= (L + 1) / 2;
         cur[l] = cu ^ 1;
         ++n;
       }
