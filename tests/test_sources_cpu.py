@@ -31,3 +31,16 @@ def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
     launch of the same call, so another launch, which waits for that one, has to lie between."""
     s = body("zrnn_api.cu", "int zrnn_gemm(", "zrnn_tc_error()")
     assert s.index("launch_pack_weights(") < s.index("launch_convert_rows(") < s.index("launch_tc_chain(")
+
+
+def test_a_cta_with_all_of_the_tensor_memory_and_a_partner_has_its_sm_for_itself():
+    """Two kernels of different streams whose CTAs wait for their cluster partners must not hold the tensor memory that the other one's
+    partner waits for: a kernel that allocates all 512 columns and has partners asks for (nearly) all of an SM's shared memory."""
+    s = body("tc_link.cu", "cudaError_t launch_t(", "cudaLaunchKernelEx")
+    assert "const size_t smem = WHOLE && SPLIT > 1 ? (size_t)kWholeSm :" in s and "cfg.dynamicSmemBytes = smem;" in s
+    with open(os.path.join(CSRC, "tc_link.cu")) as f:
+        assert "kWholeSm = 224 * 1024" in f.read()
+    for name in ("tc_vocab_pair.cu", "tc_cell_pair.cu"):
+        with open(os.path.join(CSRC, name)) as f:
+            assert "kSmem = 227 * 1024" in f.read()
+        assert "cfg.dynamicSmemBytes = kSmem;" in body(name, "cudaError_t launch_t(", "cudaLaunchKernelEx")

@@ -430,9 +430,13 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   }
 }
 
-template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
-__global__ void __launch_bounds__(kThreads, WHOLE ? 1 : 2) tc_link_kernel(const __grid_constant__ ChainParams p, int stages) {
-  link_body<BN, MODE, EPI, SPLIT, WHOLE>(p, (int)blockIdx.x, stages);
+template <int BN, int MODE, int EPI, int SPLIT>
+__global__ void __launch_bounds__(kThreads, 2) tc_link_kernel(const __grid_constant__ ChainParams p, int stages) {
+  link_body<BN, MODE, EPI, SPLIT, false>(p, (int)blockIdx.x, stages);
+}
+template <int BN, int MODE, int EPI, int SPLIT>
+__global__ void __launch_bounds__(kThreads, 1) tc_link_whole_kernel(const __grid_constant__ ChainParams p, int stages) {
+  link_body<BN, MODE, EPI, SPLIT, true>(p, (int)blockIdx.x, stages);
 }
 // Several independent problems of one row block each (M <= 128): blockIdx.x selects the problem.  The cells of one
 // anti-diagonal of a stack (layer l at step t, layer l - 1 at step t + 1, ...) do not depend on one another.
@@ -443,6 +447,11 @@ __global__ void __launch_bounds__(kThreads, 1) tc_link_multi_kernel(const __grid
 
 const bool g_pdl_on = std::getenv("ZRNN_NO_PDL") == nullptr;
 
+template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
+auto link_kernel() {
+  if constexpr (WHOLE) return &tc_link_whole_kernel<BN, MODE, EPI, SPLIT>;
+  else return &tc_link_kernel<BN, MODE, EPI, SPLIT>;
+}
 template <int BN, int MODE, int EPI, int SPLIT, bool WHOLE>
 cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   const ChainParams& p = b.p[0];
@@ -458,13 +467,16 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   // an even ring gives the MMA warps stages in turn: in an odd one a round's k-blocks may all fall to one of them, whose accumulator then
   // absorbs twice as many (500 units, 128 columns: 1.44e-7 from float64 against 1.35e-7)
   if (WHOLE && mode_split(MODE)) stages &= ~1;
-  const size_t smem = (size_t)stages * stage + fixed;
-  if (smem > kWholeSm) return cudaErrorInvalidValue;
+  // On a whole SM a CTA of a split tile holds all of the tensor memory while it waits for its cluster partner: it asks for all of the shared
+  // memory too, so that no CTA of another stream is there that holds tensor memory, and waits for some, in its turn.  (Without partners
+  // it takes what it needs: the next launch's set-up beside it is worth 1.4 % of a pass of 3 x 500 units, 50 columns.)
+  if ((size_t)stages * stage + fixed > kWholeSm) return cudaErrorInvalidValue;
+  const size_t smem = WHOLE && SPLIT > 1 ? (size_t)kWholeSm : (size_t)stages * stage + fixed;
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(tc_link_kernel<BN, MODE, EPI, SPLIT, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaError_t e = cudaFuncSetAttribute(link_kernel<BN, MODE, EPI, SPLIT, WHOLE>(), cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
     if (e != cudaSuccess) return e;
     if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1 && WHOLE) {
       e = cudaFuncSetAttribute(tc_link_multi_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
@@ -499,7 +511,7 @@ cudaError_t launch_t(const ChainBatch& b, int n, cudaStream_t st) {
   if constexpr (EPI == TC_EPI_LSTM && SPLIT == 1 && WHOLE) {
     if (n > 1) return cudaLaunchKernelEx(&cfg, tc_link_multi_kernel<BN, MODE>, b, stages);
   }
-  return cudaLaunchKernelEx(&cfg, tc_link_kernel<BN, MODE, EPI, SPLIT, WHOLE>, p, stages);
+  return cudaLaunchKernelEx(&cfg, link_kernel<BN, MODE, EPI, SPLIT, WHOLE>(), p, stages);
 }
 template <int MODE, int EPI, int SPLIT>
 cudaError_t launch_bn(const ChainBatch& b, int n, int BN, bool whole, cudaStream_t st) {

@@ -3021,7 +3021,8 @@ int zrnn_gemm(int mode, int n_rows, int m_cols, int K, const float* d_W, int ldw
                              plan.BN, p.kbs))
       return fail(ZRNN_E_CUDA, "gemm: cannot encode TMA tensor maps");
     p.M = m_cols; p.N = n_rows; p.C = d_C; p.ldc = ldc; p.err = tc_error_word();
-    ZR_CUDA(chain_launch(cb, 1, plan, tcm, zrnn::TC_EPI_STORE, st));
+    ZR_CUDA(plan.nb ? zrnn::launch_tc_cell_pair(cb, 1, tcm, zrnn::TC_EPI_STORE, st)
+                    : zrnn::launch_tc_chain(cb, 1, plan.BN, tcm, zrnn::TC_EPI_STORE, plan.split, plan.whole, st));
     return ZRNN_OK;
   };
   const int status = run();
