@@ -185,6 +185,39 @@ def test_ensemble_of_one_model_twice(H, n_sent, beam):
     np.testing.assert_allclose(two[2], one[2], rtol=1e-5)
 
 
+def test_two_models_on_two_threads():
+    """Models on streams of their own, worked on at the same time: small ones, whose cells' CTAs would fit an SM together, a large one, and
+    a search whose cells and projection run on pairs.  Every result is the one of working alone."""
+    import threading
+    from zoph_rnn_b200 import api, synth
+    jobs = []
+    for k, (H, B, att) in enumerate([(128, 24, 2), (192, 40, 1), (1000, 100, 2)]):
+        cfg = synth.make_cfg(2, H, 300, 900, attention=att, feed_input=1, D=3)
+        m = api.neuralMT_model(cfg, dtype=5)
+        m.load_weights(synth.make_weights(cfg, seed=H, dist="normal", scale=1 / np.sqrt(H)))
+        batch = synth.make_s2s_batch(300, 900, B, 2, 6, 2, 6, seed=k)
+        srcs = synth.make_decode_sources(300, 30, 2, 6, seed=k)
+        jobs.append(lambda m=m, b=batch: m.get_error(*b)[0])
+        if H == 1000:
+            jobs.append(lambda m=m, s=srcs: m.decode(s, beam=12, k_best=1, min_ratio=0.5, max_ratio=1.5, longest_sent=20)[2])
+    alone = [j() for j in jobs]
+    got = [[] for _ in jobs]
+
+    def work(i, members):
+        for _ in range(10):
+            for j in members:
+                got[j].append(jobs[j]())
+    threads = [threading.Thread(target=work, args=(i, mem)) for i, mem in enumerate([[0], [1], [2, 3]])]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for j, a in enumerate(alone):
+        assert len(got[j]) == 10
+        for g in got[j]:
+            np.testing.assert_array_equal(g, a)
+
+
 @pytest.mark.parametrize("dtype,H,V,N", [(5, 336, 129, 65), (5, 336, 256, 96), (5, 324, 257, 97), (5, 320, 513, 513), (5, 1000, 3001, 700), (5, 600, 20000, 1025),
                                          (4, 104, 385, 160), (4, 324, 19001, 321), (1, 1024, 511, 160), (1, 1032, 2050, 289), (2, 544, 700, 255)])
 def test_vocabulary_projection_pairs_of_ctas(dtype, H, V, N):
