@@ -26,6 +26,24 @@ def test_a_split_link_that_gave_up_waits_for_its_partner():
     assert s.rindex("__syncthreads()") > s.rindex("mbar_wait")
 
 
+def test_no_early_mask_can_name_the_fed_back_attention_output():
+    """Bit s of a cell's early mask lets its kernel read source s before the launch ahead has ended.  Source 2, the fed-back attention output,
+    is what that launch writes, so no flag that travels in such a mask may have its bit (nor a higher one: the mask's users count bits),
+    and a mask that has one all the same is refused before anything is launched."""
+    with open(os.path.join(CSRC, "zrnn_api.cu")) as f:
+        s = re.sub(r"//[^\n]*", "", f.read())
+    flags = {}
+    for enum in re.findall(r"enum \{([^{}]*\bEARLY_X\b[^{}]*)\}", s):
+        for name, value in re.findall(r"(\w+) = ([^,]+)", enum):
+            flags[name] = eval(value, {}, flags)
+    assert {"EARLY_X": 1, "EARLY_H": 2}.items() <= flags.items()
+    assert all(v & ~3 == 0 for v in flags.values()), flags
+    # every mask of a caller is made of these flags, and cell_forward looks at it before it does anything
+    cell = body("zrnn_api.cu", "int cell_forward(", "\n}")
+    assert re.search(r"\{\s*if \(early & ~EARLY_ANY\) return fail\(", cell)
+    assert flags["EARLY_ANY"] == 3
+
+
 def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
     """A link kernel requests its weights before it waits for the launch ahead of it.  In the stand-alone product the weights are packed by a
     launch of the same call, so another launch, which waits for that one, has to lie between."""

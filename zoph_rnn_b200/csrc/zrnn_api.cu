@@ -405,6 +405,10 @@ int lstm_cell_simt(zrnn_lstm_layer* L, const float* x, const int* mask, const fl
   return ZRNN_OK;
 }
 
+// The inputs of a cell are its sources 0 (x), 1 (the recurrent state) and 2 (the fed-back attention output).  Bit s of an `early` mask:
+// source s was complete before the launch ahead began.  The fed-back output never is: the launch that writes it comes directly before.
+enum { EARLY_X = 1, EARLY_H = 2, EARLY_ANY = EARLY_X | EARLY_H };
+
 // ---- few columns: the warp-level kernels of skinny_gemm.cu
 bool skinny_engine(int eng) { return eng == ENG_BF16 || eng == ENG_H2; }
 int skinny_mode(int eng) { return eng == ENG_BF16 ? zrnn::SK_BF16 : zrnn::SK_F16X2; }
@@ -533,14 +537,14 @@ int chain_store_params(int eng, const OpMem& w, int N, long long ldw, const Act*
 // One LSTM cell.  x / h_prev / htild and the output are activations in the form the layer's engine needs.
 // early: inputs that were complete before the launch ahead of this one began its work: the kernels multiply by them while that
 // launch runs (every kernel on the chain lets its successor start only after its own wait)
-// BESIDE: launches of other streams run at the same time (the models of an ensemble)
-enum { EARLY_X = 1, EARLY_H = 2, BESIDE = 4 };
+// beside: launches of other streams run at the same time (the models of an ensemble)
 int cell_forward(zrnn_lstm_layer* L, const Act& x, const Act& hp, const Act* q, const int* mask, const float* c_prev,
-                 int B, const Act& out, float* c_out, cudaStream_t st, int early = 0) {
+                 int B, const Act& out, float* c_out, cudaStream_t st, int early = 0, bool beside = false) {
+  if (early & ~EARLY_ANY) return fail(ZRNN_E_STATE, "internal: an input of a cell that cannot be early");
   if (L->eng == ENG_SIMT)
     return lstm_cell_simt(L, x.f32, mask, hp.f32, c_prev, q ? q->f32 : nullptr, B, out.f32, c_out, st);
   const int H = L->H, eng = L->eng;
-  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, (early & 1) + (early >> 1 & 1), H, B, 1, (early & BESIDE) != 0);
+  const LinkPlan plan = plan_link(eng, zrnn::TC_EPI_LSTM, 4 * H, q ? 3 : 2, (early & 1) + (early >> 1), H, B, 1, beside);
   KScope ks(KC_LSTM, st);
   if (plan.skinny) {
     zrnn::SkinnyBatch sb;
@@ -2304,7 +2308,7 @@ struct BeamModel {
     for (int l = 0; l < c.num_layers; ++l) {
       const bool use_feed = (l == 0 && c.feed_input && t > 0);
       ZR_TRY(cell_forward(m->tgt[l], xin, hp[l], use_feed ? &htild_feed : nullptr, nullptr, cp[l], cols, hn[l], cn[l], s,
-                          (l > 0 ? EARLY_H : 0) | (beside ? BESIDE : 0)));  // (layer 0 reads what the reorder launch just wrote)
+                          l > 0 ? EARLY_H : 0, beside));  // (layer 0 reads what the reorder launch just wrote)
       xin = hn[l];
     }
     *top = xin;
