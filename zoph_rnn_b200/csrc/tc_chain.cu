@@ -449,13 +449,16 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_
 // CTA.  Of the early sources of links on half an SM half is counted: the other half runs beside the predecessor.  us, estimated /
 // measured, fp16 split: 1000 units, 128 columns 10.7 / 10.9, 200 columns 15.7 / 16.1, 384 in tiles of 128 rows 25.6 / 25.6; 500 units, 768
 // columns 15.1 / 15.9; bf16: 1000 units, 128 columns 7.7 / 7.8, 384 11.7 / 11.4.
+// Four CTAs per tile in the split modes only: in bf16 they are worth 0.4 % of a scoring pass (4 x 1000 units, 128 columns 3108 -> 3097 us),
+// and the other order of the sums turns results that are rounded to bf16 at every step (6e-4 between the log-probabilities, 1.08e-3 from
+// float64 either way).
 ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside) {
   const bool two = mode_split(mode);
   const int parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
   ChainPlan best{0, 1, 1e30f, false, 0};
   for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 128; BN *= 2) {
     for (int split = 1; split <= 4; split *= 2) {
-      if (split == 4 && (epi == TC_EPI_LSTM || BN != 32)) continue;
+      if (split == 4 && (!two || epi == TC_EPI_LSTM || BN != 32)) continue;
       if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
       const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + 147) / 148;
       const bool whole = two && BN <= 64 && BN >= 32 && !beside;

@@ -42,7 +42,7 @@ struct ChainBatch {
 };
 // n independent problems (same BN, mode, epilogue, N; M <= 128 each when n > 1) in one launch.
 // BN: 32, 64, 128 for LSTM; 16, 32, 64, 128 for STORE.
-// split == 2 (n == 1, BN <= 64) or 4 (n == 1, BN == 32, STORE): CTAs per tile, each over its part of the K axis.
+// split == 2 (n == 1, BN <= 64) or 4 (n == 1, BN == 32, STORE, split modes): CTAs per tile, each over its part of the K axis.
 // whole (BN == 32 or 64, split modes): a CTA takes an SM, not half of one.
 cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
 cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);

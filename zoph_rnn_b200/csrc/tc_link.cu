@@ -1,5 +1,5 @@
 // tcgen05 kernel for the links of the recurrent chain whose tiles are narrow: 128 batch rows x BN = 16 .. 64 weight rows, the K
-// axis over SPLIT = 1, 2 or 4 CTAs of a cluster (LSTM cells, attention projections, combiner; wide tiles: tc_chain.cu).
+// axis over SPLIT = 1, 2 or (attention products of the split modes) 4 CTAs of a cluster (LSTM cells, attention projections, combiner; wide tiles: tc_chain.cu).
 //
 // A link spends 4 - 5 us on launch, barrier and TMEM set-up, the first loads, exchange and epilogue, and the rest on its MMAs: one
 // takes some 60 cycles to issue and to run, however few its rows, so a k-block of 128 x 64 in the split modes (8 MMAs) 512 at best.
@@ -538,7 +538,8 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, int split, 
   } else if (n == 1) {
     if (split == 1) return launch_bn<MODE, TC_EPI_STORE, 1>(b, n, BN, whole, st);
     if (split == 2) return launch_bn<MODE, TC_EPI_STORE, 2>(b, n, BN, whole, st);
-    if (split == 4) return launch_bn<MODE, TC_EPI_STORE, 4>(b, n, BN, whole, st);
+    if constexpr (mode_split(MODE))
+      if (split == 4) return launch_bn<MODE, TC_EPI_STORE, 4>(b, n, BN, whole, st);
   }
   return cudaErrorInvalidValue;
 }
