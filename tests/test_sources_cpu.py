@@ -44,6 +44,18 @@ def test_no_early_mask_can_name_the_fed_back_attention_output():
     assert flags["EARLY_ANY"] == 3
 
 
+def test_softmax_sums_use_full_precision_exponentials():
+    """The sums of the vocabulary softmax are fp32 in every mode, whatever its operands are rounded to: expf, no faster function of a larger
+    error.  (One unit of the last place of a sum of at least 1 hides the difference, so no output shows it.)"""
+    for name in ("tc_vocab.cu", "tc_vocab_pair.cu", "tc_gemm.cu"):
+        with open(os.path.join(CSRC, name)) as f:
+            s = re.sub(r"//[^\n]*", "", f.read())
+        assert "expf(" in s
+        assert not re.search(r"__expf|__exp10f|exp2f|ex2\.approx|__powf|use_fast_math", s), name
+    with open(os.path.join(os.path.dirname(CSRC), "build.py")) as f:
+        assert "use_fast_math" not in f.read()
+
+
 def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
     """A link kernel requests its weights before it waits for the launch ahead of it.  In the stand-alone product the weights are packed by a
     launch of the same call, so another launch, which waits for that one, has to lie between."""

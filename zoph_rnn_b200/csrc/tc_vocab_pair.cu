@@ -43,9 +43,6 @@ struct alignas(16) PairCtrl {
 __host__ __device__ constexpr int column_bytes(int nb) { return nb * (4 * 4 + 4 * 4 + 4); }
 constexpr int kXposeLd = 36, kXposeBytes = kEpiWarps * 8 * kXposeLd * 4;  // 8 columns x 32 rows per epilogue warp, rows spread over the banks
 
-template <int MODE>
-__device__ __forceinline__ float expo(float x) { return mode_exact_math(MODE) ? expf(x) : __expf(x); }
-
 template <int MODE, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     tc_vocab_pair_kernel(const __grid_constant__ VocabParams p, int stages, int v_tiles, int bufs) {
@@ -267,8 +264,8 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
               float sm = 0.f;
               if (want_sum) {
                 const float ref = mx == -INFINITY ? 0.f : mx;  // (rows beyond the vocabulary: exp(-inf) = 0)
-                sm = ((expo<MODE>(y[0] - ref) + expo<MODE>(y[1] - ref)) + (expo<MODE>(y[2] - ref) + expo<MODE>(y[3] - ref))) +
-                     ((expo<MODE>(y[4] - ref) + expo<MODE>(y[5] - ref)) + (expo<MODE>(y[6] - ref) + expo<MODE>(y[7] - ref)));
+                sm = ((expf(y[0] - ref) + expf(y[1] - ref)) + (expf(y[2] - ref) + expf(y[3] - ref))) +
+                     ((expf(y[4] - ref) + expf(y[5] - ref)) + (expf(y[6] - ref) + expf(y[7] - ref)));
                 sm += __shfl_xor_sync(0xffffffffu, sm, 1);
                 sm += __shfl_xor_sync(0xffffffffu, sm, 2);
               }
