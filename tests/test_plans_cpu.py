@@ -64,3 +64,24 @@ def test_single_pass_products_are_summed_over_two_parts_at_most(plans):
          for rows, nsrc in ((H, 2), (2 * H, 1)) for M in (1, 12, 64, 100, 128, 200, 256, 400, 768) for beside in (0, 1)]
     assert max(p[1] for p in plans(q)) == 2
     assert any(p[1] == 4 for p in plans([(F16X2, STORE, 1000, 2, 16, M, 0) for M in (64, 128)]))
+
+
+def waves(M, rows, width):
+    return -(-(-(-M // 128) * -(-rows // width)) // 148)
+
+
+def test_one_accumulator_over_the_whole_k_axis_only_where_it_halves_the_waves(plans):
+    """Tiles of more than 160 columns on pairs of CTAs give each split-mode product one truncating accumulator for the whole K axis, several
+    times as far from float64 as rounds.  Never in 3xTF32; in the fp16 split where, and only where, tiles of 256 weight rows on single CTAs, which
+    had such an accumulator too, took that much fewer waves of CTAs that they were chosen: 1000 units at 768 columns, not at 1500."""
+    q = [(mode, epi, (4 if epi == LSTM else 2 if nsrc == 1 else 1) * H, nsrc, kblocks(mode, H), M, 0) for mode in (TF32X3, F16X2) for epi in (STORE, LSTM)
+         for H in (256, 320, 400, 500, 512, 640, 768, 900, 1000, 1024, 1536, 2048) for nsrc in (1, 2, 3) for M in range(257, 4100, 31)]
+    seen = set()
+    for (mode, epi, rows, nsrc, kb, M, _), (_, _, nb, _) in zip(q, plans(q)):
+        if nb > 160:
+            assert mode == F16X2 and waves(M, rows, 128) > 1.6 * waves(M, rows, 256), (mode, epi, rows, nsrc, M, nb)
+            seen.add(rows)
+    assert 4000 in seen  # (the rule is reached)
+    cell = [(F16X2, LSTM, 4000, 2, 16, M, 0) for M in (600, 768, 1024, 1440, 1500, 1640)]
+    nb = [p[2] for p in plans(cell)]
+    assert nb[1] > 160 and nb[2] > 160 and all(0 < n <= 160 for n in nb[3:]), nb

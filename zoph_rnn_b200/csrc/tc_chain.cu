@@ -471,11 +471,15 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
   }
   // Pairs of CTAs, 148 SMs: a k-block's twelve MMAs (four) take 64 cycles each at least, half a cycle per column; set-up, first loads
   // and end 8 us, all of an SM being needed.  More than 160 columns per tile have one accumulator for the whole K axis in the split
-  // modes: only where tiles of 128 rows and columns would not fit one wave.
+  // modes, whose error is several times that of rounds (1000 units 1.74e-6 from float64 against 1.8e-7).  That is paid only where it buys most: in fp16,
+  // where tiles of 128 rows and columns take more than 1.6 times the waves of CTAs that tiles of 256 rows would (1000 units 513 - 1152 columns: two
+  // waves against one).
+  const auto waves_of = [&](int w) { return ((long long)mt * ((rows + w - 1) / w) + 147) / 148; };
+  const bool one_acc = !two || (mode == TC_F16X2 && 8 * waves_of(256) < 5 * waves_of(128));
   const int row_tiles = (rows + 255) / 256;
   for (int n_ct = (M + 255) / 256; M > 256 && cells == 1 && n_ct <= (M + 31) / 32; ++n_ct) {
     const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
-    if (two && nb > 160 && (mode == TC_TF32X3 || (M + 127) / 128 * ((rows + 127) / 128) <= 148)) continue;
+    if (nb > 160 && !one_acc) continue;
     const int waves = (row_tiles * n_ct + 73) / 74;
     const float cyc = two ? std::max(800.f, 6.5f * nb) : std::max(330.f, 2.2f * nb);
     const float us = 8.f + waves * (nsrc * kb * cyc / 1850.f + (two ? 0.015f : 0.01f) * nb);
