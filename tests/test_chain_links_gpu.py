@@ -239,3 +239,21 @@ def test_products_of_one_sign_do_not_shrink(mode, K, steps, n, m):
     C = api.gemm(torch.as_tensor(W).cuda().reshape(-1), torch.as_tensor(X).cuda().reshape(-1), n, m, K, mode).cpu().numpy().reshape(m, n)
     want = X.astype(np.float64) @ W.astype(np.float64)
     assert np.abs(C / want - 1).mean() < (steps + 2) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("mode,K", [(1, 1000), (1, 2000), (2, 500), (2, 1000), (2, 2000)])
+@pytest.mark.parametrize("n,m", [(4000, 700), (4000, 1100)])
+def test_single_pass_products_on_pairs_keep_two_accumulators(mode, K, n, m):
+    """Operands that the mode holds exactly, all positive, of magnitudes that make no sum exact: what is missing from a result is what the tensor core has truncated, in proportion
+    to the k-steps that an accumulator absorbs.  The first 200 columns alone take tiles of one CTA, whose two MMA warps have an
+    accumulator each: a product of many columns, on pairs, loses no more (with one accumulator twice as much; 1.25 is for the other order of the k-steps)."""
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(n + m + K)
+    W, X = [(np.exp2(rng.uniform(-6, 0, s)).astype(np.float32).view(np.uint32) & (0xffff0000 if mode == 1 else 0xffffe000)).astype(np.uint32).view(np.float32)
+            for s in ((K, n), (m, K))]
+    want = X.astype(np.float64) @ W.astype(np.float64)
+    dW, dX = torch.as_tensor(W).cuda().reshape(-1), torch.as_tensor(X).cuda().reshape(-1)
+    many, few = [1 - (api.gemm(dW, dX[:c * K], n, c, K, mode).cpu().numpy().reshape(c, n) / want[:c]).mean() for c in (m, 200)]
+    assert few > 3 * 2.0 ** -24  # (it is seen at all)
+    assert many < 1.25 * few
