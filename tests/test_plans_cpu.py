@@ -14,15 +14,15 @@ PROBE = r"""
 #include <chrono>
 #include <cstdio>
 #include "tc_chain.cuh"
-// lines of "mode epi rows nsrc kb columns beside" -> "BN split nb microseconds"; one call takes that long at least of three
+// lines of "mode epi rows nsrc kb n_early columns beside" -> "BN split nb microseconds"; one call takes that long at least of three
 int main() {
-  int mode, epi, rows, nsrc, kb, M, beside;
-  while (std::scanf("%d %d %d %d %d %d %d", &mode, &epi, &rows, &nsrc, &kb, &M, &beside) == 7) {
+  int mode, epi, rows, nsrc, kb, early, M, beside;
+  while (std::scanf("%d %d %d %d %d %d %d %d", &mode, &epi, &rows, &nsrc, &kb, &early, &M, &beside) == 8) {
     zrnn::ChainPlan p;
     double best = 1e30;
     for (int i = 0; i < 3; ++i) {
       const auto t0 = std::chrono::steady_clock::now();
-      p = zrnn::plan_chain(mode, epi, rows, 1, nsrc, kb, 0, M, beside != 0);
+      p = zrnn::plan_chain(mode, epi, rows, 1, nsrc, kb, early, M, beside != 0);
       const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
       if (us < best) best = us;
     }
@@ -50,7 +50,7 @@ def plans(tmp_path_factory):
                            "-o", exe, lib, "-Wl,-rpath," + PKG])
 
     def ask(questions):
-        out = subprocess.run([exe], input="".join("%d %d %d %d %d %d %d\n" % q for q in questions), stdout=subprocess.PIPE, text=True, check=True)
+        out = subprocess.run([exe], input="".join("%d %d %d %d %d %d %d %d\n" % q for q in questions), stdout=subprocess.PIPE, text=True, check=True)
         rows = [(int(a), int(b), int(c), float(t)) for a, b, c, t in (line.split() for line in out.stdout.splitlines())]
         assert len(rows) == len(questions)
         return rows
@@ -60,28 +60,33 @@ def plans(tmp_path_factory):
 def test_single_pass_products_are_summed_over_two_parts_at_most(plans):
     """A product of the single-pass modes is rounded to 10 or 7 bits at its end, so another order of its sums turns some of its results by a
     unit there: four parts of the K axis gave a bf16 scoring pass other values for 0.4 % of its time, and are for the split modes."""
-    q = [(mode, STORE, rows, nsrc, kblocks(mode, H), M, beside) for mode in (BF16, TF32) for H in (256, 500, 1000, 1024, 2048)
+    q = [(mode, STORE, rows, nsrc, kblocks(mode, H), 0, M, beside) for mode in (BF16, TF32) for H in (256, 500, 1000, 1024, 2048)
          for rows, nsrc in ((H, 2), (2 * H, 1)) for M in (1, 12, 64, 100, 128, 200, 256, 400, 768) for beside in (0, 1)]
     assert max(p[1] for p in plans(q)) == 2
-    assert any(p[1] == 4 for p in plans([(F16X2, STORE, 1000, 2, 16, M, 0) for M in (64, 128)]))
+    assert any(p[1] == 4 for p in plans([(F16X2, STORE, 1000, 2, 16, 0, M, 0) for M in (64, 128)]))
 
 
-def waves(M, rows, width):
-    return -(-(-(-M // 128) * -(-rows // width)) // 148)
+def waves(M, rows, width, split=1):
+    return -(-(-(-M // 128) * -(-rows // width) * split) // 148)
 
 
 def test_one_accumulator_over_the_whole_k_axis_only_where_it_halves_the_waves(plans):
     """Tiles of more than 160 columns on pairs of CTAs give each split-mode product one truncating accumulator for the whole K axis, several
     times as far from float64 as rounds.  Never in 3xTF32; in the fp16 split where, and only where, tiles of 256 weight rows on single CTAs, which
-    had such an accumulator too, took that much fewer waves of CTAs that they were chosen: 1000 units at 768 columns, not at 1500."""
-    q = [(mode, epi, (4 if epi == LSTM else 2 if nsrc == 1 else 1) * H, nsrc, kblocks(mode, H), M, 0) for mode in (TF32X3, F16X2) for epi in (STORE, LSTM)
-         for H in (256, 320, 400, 500, 512, 640, 768, 900, 1000, 1024, 1536, 2048) for nsrc in (1, 2, 3) for M in range(257, 4100, 31)]
+    had such an accumulator too, took so much less than tiles of 128 rows, and of 64 rows that have early sources, that they were chosen:
+    1000 units at 768 columns, not at 1500, and not where two of three sources are early."""
+    q = [(mode, epi, (4 if epi == LSTM else 2 if nsrc == 1 else 1) * H, nsrc, kblocks(mode, H), early, M, 0) for mode in (TF32X3, F16X2) for epi in (STORE, LSTM)
+         for H in (256, 320, 400, 500, 512, 640, 768, 900, 1000, 1024, 1536, 2048) for nsrc in (1, 2, 3) for early in range(nsrc) for M in range(257, 4100, 31)]
     seen = set()
-    for (mode, epi, rows, nsrc, kb, M, _), (_, _, nb, _) in zip(q, plans(q)):
+    for (mode, epi, rows, nsrc, kb, early, M, _), (_, _, nb, _) in zip(q, plans(q)):
         if nb > 160:
-            assert mode == F16X2 and waves(M, rows, 128) > 1.6 * waves(M, rows, 256), (mode, epi, rows, nsrc, M, nb)
-            seen.add(rows)
-    assert 4000 in seen  # (the rule is reached)
-    cell = [(F16X2, LSTM, 4000, 2, 16, M, 0) for M in (600, 768, 1024, 1440, 1500, 1640)]
+            w = waves(M, rows, 256)
+            assert mode == F16X2 and waves(M, rows, 128) > 1.6 * w, (mode, epi, rows, nsrc, M, nb)
+            assert (nsrc - early / 2) * min(waves(M, rows, 64), waves(M, rows, 64, 2) / 2) > 2 * nsrc * w, (mode, epi, rows, nsrc, early, M, nb)
+            seen.add((rows, early))
+    assert (4000, 0) in seen and (4000, 1) in seen  # (the rule is reached)
+    cell = [(F16X2, LSTM, 4000, 2, 16, 0, M, 0) for M in (600, 768, 1024, 1440, 1500, 1640)]
     nb = [p[2] for p in plans(cell)]
     assert nb[1] > 160 and nb[2] > 160 and all(0 < n <= 160 for n in nb[3:]), nb
+    feed = [(F16X2, LSTM, 4 * H, 3, kblocks(F16X2, H), 2, M, 0) for H, M in ((1000, 700), (1000, 890), (768, 1000), (900, 700), (2048, 350))]
+    assert all(p[2] <= 160 for p in plans(feed))

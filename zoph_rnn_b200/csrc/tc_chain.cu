@@ -473,9 +473,11 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
   // and end 8 us, all of an SM being needed.  More than 160 columns per tile have one accumulator for the whole K axis in the split
   // modes, whose error is several times that of rounds (1000 units 1.74e-6 from float64 against 1.8e-7).  That is paid only where it buys most: in fp16,
   // where tiles of 128 rows and columns take more than 1.6 times the waves of CTAs that tiles of 256 rows would (1000 units 513 - 1152 columns: two
-  // waves against one).
-  const auto waves_of = [&](int w) { return ((long long)mt * ((rows + w - 1) / w) + 147) / 148; };
-  const bool one_acc = !two || (mode == TC_F16X2 && 8 * waves_of(256) < 5 * waves_of(128));
+  // waves against one), and tiles of 64 rows, over all or half of the K axis, more than twice the time even if half of the early sources is
+  // free to them (1000 units, three sources, two of them early: 6 of 6 k-axes at 513 - 896 columns, 6 of 8 beyond).
+  const auto waves_of = [&](int w, int split) { return ((long long)mt * ((rows + w - 1) / w) * split + 147) / 148; };
+  const float narrow = (nsrc - 0.5f * n_early) * std::min((float)waves_of(64, 1), 0.5f * waves_of(64, 2));
+  const bool one_acc = !two || (mode == TC_F16X2 && 8 * waves_of(256, 1) < 5 * waves_of(128, 1) && 2.f * nsrc * waves_of(256, 1) < narrow);
   const int row_tiles = (rows + 255) / 256;
   for (int n_ct = (M + 255) / 256; M > 256 && cells == 1 && n_ct <= (M + 31) / 32; ++n_ct) {
     const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
