@@ -241,6 +241,13 @@ def test_products_of_one_sign_do_not_shrink(mode, K, steps, n, m):
     assert np.abs(C / want - 1).mean() < (steps + 2) * 2.0 ** -24
 
 
+@pytest.mark.parametrize("mode,K,steps", [(4, 320, 4), (4, 512, 4), (4, 1000, 8), (3, 320, 4), (3, 512, 4), (3, 1000, 8)])
+@pytest.mark.parametrize("n,m", [(2000, 520), (3000, 400), (6000, 200)])
+def test_products_of_one_sign_do_not_shrink_in_tiles_of_128_rows(mode, K, steps, n, m):
+    """Which tile takes a product is a question of time: accumulators of the tiles of 128 x 128 absorb what those of the narrow ones do."""
+    test_products_of_one_sign_do_not_shrink(mode, K, steps, n, m)
+
+
 @pytest.mark.parametrize("mode,K", [(1, 1000), (1, 2000), (2, 500), (2, 1000), (2, 2000)])
 @pytest.mark.parametrize("n,m", [(4000, 700), (4000, 1100)])
 def test_single_pass_products_on_pairs_keep_two_accumulators(mode, K, n, m):

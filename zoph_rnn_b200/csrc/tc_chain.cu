@@ -26,13 +26,12 @@ constexpr int kEpiWarps = 16;
 // the other the two cross products.
 constexpr int kMmaWarps = 2;
 constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
-// The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb more than round_kb k-blocks
-// (16 k-steps of fp16, 8 of the more exact 3xTF32) in a row: the K axis is walked in rounds, each into a fresh accumulator set, and
-// the epilogue warps, idle until the end otherwise, add every finished round to sums of their own in registers (round to nearest)
-// while the next round runs.
-// Mean log-prob error against the oracle at H = 1000, 4 layers: 5.8e-7; with four accumulators over the whole K axis 13e-7.  Hidden
-// states of 4 x 640 units in 3xTF32 against float64: 5.8e-7 in rounds of 16 k-steps, 3.5e-7 at most in rounds of 8.
-__host__ __device__ constexpr int round_kb(int mode) { return mode == TC_TF32X3 ? 2 : 4; }
+// The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb more than round_kb k-blocks in a row:
+// the K axis is walked in rounds, each into a fresh accumulator set, and the epilogue warps, idle until the end otherwise, add every
+// finished round to sums of their own in registers (round to nearest) while the next round runs.  As many k-steps per round as the
+// accumulators of the narrow tiles absorb (tc_link.cu: 4 up to 512 elements per source, else 8), so that the choice of a tile
+// is none of precision.
+__host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 1 : 2; }
 __host__ __device__ constexpr bool chain_rounds(int mode) { return mode_split(mode); }
 // accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  Other modes: one per MMA warp.
 __host__ __device__ constexpr int chain_sets(int mode) { return mode_split(mode) ? 3 : kMmaWarps; }
@@ -72,7 +71,7 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   // KBS x [A hi][A lo], KBS x [W hi][W lo]; every piece is a multiple of 1024 bytes
   const int stage_bytes = PARTS * KBS * (akb + WKB);
   const int src_it = (p.kb + KBS - 1) / KBS, n_it = p.nsrc * src_it;
-  const int round_its = KBS < round_kb(MODE) ? round_kb(MODE) / KBS : 1;  // stages per round
+  const int round_its = KBS < round_kb(MODE, p.kb) ? round_kb(MODE, p.kb) / KBS : 1;  // stages per round
   constexpr int NBUF = BY_PRODUCT ? NSET : NSET / kMmaWarps;  // accumulator sets an MMA warp takes in turn
   ZR_STAMP(0);
   if (threadIdx.x == 0) {
