@@ -264,3 +264,20 @@ def test_single_pass_products_on_pairs_keep_two_accumulators(mode, K, n, m):
     many, few = [1 - (api.gemm(dW, dX[:c * K], n, c, K, mode).cpu().numpy().reshape(c, n) / want[:c]).mean() for c in (m, 200)]
     assert few > 3 * 2.0 ** -24  # (it is seen at all)
     assert many < 1.25 * few
+
+
+@pytest.mark.parametrize("K", [1000, 2000])
+@pytest.mark.parametrize("m", [250, 400, 700, 900])
+def test_tf32_products_absorb_a_quarter_of_the_k_axis_in_every_tile(K, m):
+    """As above: 128 columns take tiles split over two CTAs with two accumulators each.  Tiles of 64 and of 128 rows on one CTA and pairs of CTAs
+    (250, 400, 700 and 900 columns) lose no more."""
+    import torch
+    from zoph_rnn_b200 import api
+    rng = np.random.default_rng(m + K)
+    n = 4000
+    W, X = [(np.exp2(rng.uniform(-6, 0, s)).astype(np.float32).view(np.uint32) & 0xffffe000).astype(np.uint32).view(np.float32) for s in ((K, n), (m, K))]
+    want = X.astype(np.float64) @ W.astype(np.float64)
+    dW, dX = torch.as_tensor(W).cuda().reshape(-1), torch.as_tensor(X).cuda().reshape(-1)
+    many, few = [1 - (api.gemm(dW, dX[:c * K], n, c, K, 2).cpu().numpy().reshape(c, n) / want[:c]).mean() for c in (m, 128)]
+    assert few > 3 * 2.0 ** -24  # (it is seen at all)
+    assert many < 1.25 * few

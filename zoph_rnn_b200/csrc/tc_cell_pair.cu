@@ -10,9 +10,9 @@
 // place of the operand tiles, and a warp finishes 32 units of a column at a time: loads and stores of whole lines.
 //
 // Split modes, up to 160 columns: the K axis is walked in rounds into fresh accumulators, which the epilogue warps add up in
-// registers (tc_link.cu); three accumulators take turns up to 128 columns, two up to 160, and beyond there is room for one only.  The other
-// modes take two accumulators in turn, stage by stage, and add them up at the end: the tensor core truncates as it accumulates (tf32, 1000
-// and 2048 units: 0.2 - 0.3 % farther from float64 with one).
+// registers (tc_link.cu); three accumulators take turns up to 128 columns, two up to 160, and beyond there is room for one only.  bf16
+// takes two accumulators in turn, stage by stage, and adds them up at the end; tf32 walks the K axis in four rounds with two: the tensor core
+// truncates as it accumulates (tf32, 1000 and 2048 units: 0.2 - 0.3 % farther from float64 with one for all of it).
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -72,8 +72,8 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
   PairCtrl& ct = *reinterpret_cast<PairCtrl*>(tiles + (size_t)stages * stage_bytes);
   const int src_it = (p.kb + KBS - 1) / KBS, n_it = p.nsrc * src_it;
   const int nsets = SPLIT_MODE ? acc_sets(nb) : 2;
-  const bool rounds = SPLIT_MODE && nsets > 1;
-  const int R = round_kb(MODE, p.kb);  // (split modes: a k-block per stage)
+  const bool rounds = MODE == TC_TF32 || (SPLIT_MODE && nsets > 1);
+  const int R = MODE == TC_TF32 ? (n_it + 3) / 4 : round_kb(MODE, p.kb);  // stages per round (split modes: a k-block per stage)
   ZR_STAMP(0);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
         if (!mbar_wait_warp(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t w_addr = smem_u32(tiles + (size_t)st * stage_bytes), a_addr = w_addr + w_bytes;
-        if (!SPLIT_MODE) set = it & 1;
+        if (MODE == TC_BF16) set = it & 1;
         const uint32_t d = tmem_base + (uint32_t)(set * nb);
         const bool fresh = rounds ? in_round == 0 : it < (SPLIT_MODE ? 1 : 2);
         if (one) {
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) __cluster_dims__(2, 1, 1)
     ZR_STAMP(2);
     if (ready && live) {
       if (!rounds) drain(taddr, 1.0f);
-      if (!SPLIT_MODE && n_it > 1) drain(taddr + (uint32_t)nb, 1.0f);
+      if (MODE == TC_BF16 && n_it > 1) drain(taddr + (uint32_t)nb, 1.0f);
       if (SPLIT_MODE) drain(taddr + (uint32_t)(nsets * nb), mode_cross_scale(MODE));
     }
     pdl_wait();

@@ -33,8 +33,8 @@ constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
 // is none of precision.
 __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 1 : 2; }
 __host__ __device__ constexpr bool chain_rounds(int mode) { return mode_split(mode); }
-// accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  Other modes: one per MMA warp.
-__host__ __device__ constexpr int chain_sets(int mode) { return mode_split(mode) ? 3 : kMmaWarps; }
+// accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  bf16: one per MMA warp, tf32: two (tc_link.cu).
+__host__ __device__ constexpr int chain_sets(int mode) { return mode_split(mode) ? 3 : (mode == TC_TF32 ? 2 : 1) * kMmaWarps; }
 __host__ __device__ constexpr int chain_tmem(int BN, int mode) {
   const int need = (chain_sets(mode) + (mode_split(mode) ? 1 : 0)) * BN;
   int c = 32;
@@ -169,11 +169,12 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
             if (round >= NBUF && !mbar_wait_warp(&set_empty[set], (uint32_t)((round / NBUF) & 1) ^ 1u, &abort_s, p.err, 4)) { ok = false; break; }
             tc_fence_after();
           }
+          if (!BY_PRODUCT) set = it % NSET;
           if (!mbar_wait_warp(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
           const uint32_t d = tmem_base + (uint32_t)(set * BN), d_cross = tmem_base + (uint32_t)(NSET * BN);
-          const bool fresh = rounds ? in_round == 0 : it < STEP;  // the accumulator starts with this stage
+          const bool fresh = rounds ? in_round == 0 : it < (BY_PRODUCT ? STEP : NSET);  // the accumulator starts with this stage
           if (one) {
             for (int b = 0; b < KBS; ++b) {
               const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);

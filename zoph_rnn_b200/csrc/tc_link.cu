@@ -51,11 +51,15 @@ __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mod
 // Split modes multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the columns for two products (an MMA of 128 rows
 // takes 45 cycles up to 32 columns, 48 at 64, 64 at 128), and A_lo by W_hi: two MMAs per k-step instead of three.
 __host__ __device__ constexpr int set_cols(int BN, int mode) { return mode_split(mode) ? 2 * BN : BN; }  // one accumulator set per MMA warp
-// sets that an MMA warp takes in turn, one being added up while the next fills: where the CTA's columns hold them (half an SM: 256)
-__host__ __device__ constexpr int set_bufs(int BN, int mode, bool whole_sm) { return mode_split(mode) && (BN <= 32 || whole_sm) ? 2 : 1; }
-__host__ __device__ constexpr int link_tmem(int BN, int mode, bool whole_sm) {
+// sets that an MMA warp takes in turn, one being added up while the next fills: where the CTA's columns hold them (half an SM: 256).  tf32 adds up
+// no rounds, but a tile of one CTA has four accumulators, a quarter of the K axis each, like the two CTAs of a split one (256 and 320
+// units, 64 - 500 columns: with two 0.03 % farther from float64; in bf16 the sixth digit of that distance is the same).
+__host__ __device__ constexpr int set_bufs(int BN, int mode, bool whole_sm, int split) {
+  return (mode_split(mode) && (BN <= 32 || whole_sm)) || (mode == TC_TF32 && split == 1) ? 2 : 1;
+}
+__host__ __device__ constexpr int link_tmem(int BN, int mode, bool whole_sm, int split) {
   int c = 32;
-  while (c < kMmaWarps * set_bufs(BN, mode, whole_sm) * set_cols(BN, mode)) c *= 2;
+  while (c < kMmaWarps * set_bufs(BN, mode, whole_sm, split) * set_cols(BN, mode)) c *= 2;
   return c;
 }
 // outputs per row and epilogue warp (LSTM: hidden units); a CTA finishes 1 / SPLIT of them
@@ -84,7 +88,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
   constexpr bool SPLIT_MODE = mode_split(MODE), ROUNDS = SPLIT_MODE;
   constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   constexpr int WKB = BN * 128;  // bytes of one k-block of one weight part
-  constexpr int SETC = set_cols(BN, MODE), NB = set_bufs(BN, MODE, WHOLE), TMEM_COLS = link_tmem(BN, MODE, WHOLE);
+  constexpr int SETC = set_cols(BN, MODE), NB = set_bufs(BN, MODE, WHOLE, SPLIT), TMEM_COLS = link_tmem(BN, MODE, WHOLE, SPLIT);
   constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN), IDESC2 = make_idesc(mode_fmt(MODE), SETC);
   extern __shared__ __align__(1024) uint8_t link_smem[];
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -188,7 +192,7 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
       const bool one = elect_one();
       const int mw = warp - kMmaWarp, R = round_kb(MODE, p.kb) / KBS;
       int set = mw * NB;
-      int st = mw, it = mw, round_end = 0, round = 0;
+      int st = mw, it = mw, round_end = 0, round = 0, own = 0;
       uint32_t ph = 0;
       bool ok = true, fresh = true;
       while (it < n_it) {
@@ -199,6 +203,10 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
           fresh = true;
           round_end = (it / R + 1) * R;
           ++round;
+        }
+        if (!ROUNDS && NB > 1) {
+          set = mw * NB + own % NB;
+          fresh = own++ < NB;
         }
         if (!mbar_wait_warp(&ct.full[st], ph, &ct.abort, p.err, 2)) { ok = false; break; }
         tc_fence_after();
@@ -320,8 +328,11 @@ __device__ __forceinline__ void link_body(const ChainParams& p, const int m_bloc
         ready = __all_sync(0xffffffffu, mbar_wait(&ct.accum, 0, &ct.abort, p.err, 3));
         tc_fence_after();
         if (ready && live) {
-          drain(0);
-          if (own_stages(1, n_it, stages) > 0) drain(1);
+#pragma unroll
+          for (int mw = 0; mw < kMmaWarps; ++mw)
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+              if (own_stages(mw, n_it, stages) > b) drain(mw * NB + b);
         }
       }
     }
@@ -551,7 +562,8 @@ int link_kbs(int mode, int BN, int a_rows, int kb, int split) {
   // k-blocks per stage: as many as leave the ring four stages and every CTA two stages of a source; a round has two stages at least,
   // one for each MMA warp
   int k = mode_split(mode) ? round_kb(mode, kb) / 2 : 4;
-  while (k > 1 && (4 * k * kb_bytes > kHalfSm - 20 * 1024 - (128 - a_rows) * 128 || (kb + k - 1) / k < 2 * split)) k /= 2;
+  const int least = mode == TC_TF32 ? 4 : 2 * split;  // (tf32: a stage for each of the four accumulators)
+  while (k > 1 && (4 * k * kb_bytes > kHalfSm - 20 * 1024 - (128 - a_rows) * 128 || (kb + k - 1) / k < least)) k /= 2;
   return k;
 }
 
