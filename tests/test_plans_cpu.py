@@ -90,3 +90,13 @@ def test_one_accumulator_over_the_whole_k_axis_only_where_it_halves_the_waves(pl
     assert nb[1] > 160 and nb[2] > 160 and all(0 < n <= 160 for n in nb[3:]), nb
     feed = [(F16X2, LSTM, 4 * H, 3, kblocks(F16X2, H), 2, M, 0) for H, M in ((1000, 700), (1000, 890), (768, 1000), (900, 700), (2048, 350))]
     assert all(p[2] <= 160 for p in plans(feed))
+
+
+def test_very_many_columns_are_planned_in_no_time_and_fit_a_grid(plans):
+    """A plan is made at every launch, so it must not look at every way to cut millions of columns into tiles; and the column tiles of pairs of
+    CTAs are the second axis of a grid, which ends at 65535: beyond, the tiles of single CTAs, whose columns are the first axis, take them."""
+    q = [(mode, STORE, rows, 1, kb, 0, M, 0) for mode in (BF16, TF32, TF32X3, F16X2) for rows in (64, 256, 2000) for kb in (1, 4, 16)
+         for M in (70000, 1 << 20, 10_500_000, 17_000_000, 30_000_000)]
+    for (mode, _, rows, _, _, _, M, _), (BN, split, nb, us) in zip(q, plans(q)):
+        assert nb == 0 or -(-M // nb) <= 65535, (mode, rows, M, nb)
+        assert us < 20, (M, us)

@@ -479,10 +479,10 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
   const float narrow = (nsrc - 0.5f * n_early) * std::min((float)waves_of(64, 1), 0.5f * waves_of(64, 2));
   const bool one_acc = !two || (mode == TC_F16X2 && 8 * waves_of(256, 1) < 5 * waves_of(128, 1) && 2.f * nsrc * waves_of(256, 1) < narrow);
   const int row_tiles = (rows + 255) / 256;
-  for (int n_ct = (M + 255) / 256; M > 256 && cells == 1 && n_ct <= (M + 31) / 32; ++n_ct) {
-    const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
-    if (nb > 160 && !one_acc) continue;
-    const int waves = (row_tiles * n_ct + 73) / 74;
+  for (int w = one_acc ? 256 : 160; M > 256 && cells == 1 && w >= 32; w -= 32) {  // (a width's time grows with the number of column tiles)
+    const int n_ct = (M - 1) / w + 1, nb = ((M - 1) / n_ct + 32) / 32 * 32;
+    if (n_ct > 65535) break;  // (a grid's second axis)
+    const long long waves = ((long long)row_tiles * n_ct + 73) / 74;
     const float cyc = two ? std::max(800.f, 6.5f * nb) : std::max(330.f, 2.2f * nb);
     const float us = 8.f + waves * (nsrc * kb * cyc / 1850.f + (two ? 0.015f : 0.01f) * nb);
     if (us < best.us) best = ChainPlan{128, 1, us, false, nb};
