@@ -56,6 +56,20 @@ def test_softmax_sums_use_full_precision_exponentials():
         assert "use_fast_math" not in f.read()
 
 
+def test_launch_rules_ask_the_current_device_for_its_multiprocessors():
+    """One function keeps the count, per device and safe for several threads; no rule has a count of its own or the first device's."""
+    asks = {}
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                s = re.sub(r"//[^\n]*", "", f.read())
+            asks[name] = s.count("cudaDevAttrMultiProcessorCount")
+            if name in ("tc_chain.cu", "tc_vocab.cu", "tc_vocab_pair.cu", "tc_cell_pair.cu"):
+                assert not re.search(r"\b(147|148|73|74)\b", s), name
+    assert {k: v for k, v in asks.items() if v} == {"tc_gemm.cu": 1}
+    assert "std::atomic<int> count[kMaxDevices]" in body("tc_gemm.cu", "int device_sms()", "\n}")
+
+
 def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
     """A link kernel requests its weights before it waits for the launch ahead of it.  In the stand-alone product the weights are packed by a
     launch of the same call, so another launch, which waits for that one, has to lie between."""

@@ -454,13 +454,13 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_
 // float64 either way).
 ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside) {
   const bool two = mode_split(mode);
-  const int parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
+  const int sms = device_sms(), parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
   ChainPlan best{0, 1, 1e30f, false, 0};
   for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 128; BN *= 2) {
     for (int split = 1; split <= 4; split *= 2) {
       if (split == 4 && (!two || epi == TC_EPI_LSTM || BN != 32)) continue;
       if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
-      const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + 147) / 148;
+      const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + sms - 1) / sms;
       const bool whole = two && BN <= 64 && BN >= 32 && !beside;
       const float cyc = 4.f * (!two ? std::max(60.f, BN / 2.f) : (BN <= 64 ? std::max(60.f, (float)BN) + 60.f : 1.6f * 3.f * BN / 2.f));
       const float kb_us = std::max(parts * 128.f * (a_rows + BN) / 130e3f, cyc / 1850.f) + (two && epi == TC_EPI_STORE && BN <= 64 && !whole ? 0.15f : 0.f);
@@ -469,20 +469,20 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
       if (us < best.us) best = ChainPlan{BN, split, us, whole, 0};
     }
   }
-  // Pairs of CTAs, 148 SMs: a k-block's twelve MMAs (four) take 64 cycles each at least, half a cycle per column; set-up, first loads
+  // Pairs of CTAs: a k-block's twelve MMAs (four) take 64 cycles each at least, half a cycle per column; set-up, first loads
   // and end 8 us, all of an SM being needed.  More than 160 columns per tile have one accumulator for the whole K axis in the split
   // modes, whose error is several times that of rounds (1000 units 1.74e-6 from float64 against 1.8e-7).  That is paid only where it buys most: in fp16,
   // where tiles of 128 rows and columns take more than 1.6 times the waves of CTAs that tiles of 256 rows would (1000 units 513 - 1152 columns: two
   // waves against one), and tiles of 64 rows, over all or half of the K axis, more than twice the time even if half of the early sources is
   // free to them (1000 units, three sources, two of them early: 6 of 6 k-axes at 513 - 896 columns, 6 of 8 beyond).
-  const auto waves_of = [&](int w, int split) { return ((long long)mt * ((rows + w - 1) / w) * split + 147) / 148; };
+  const auto waves_of = [&](int w, int split) { return ((long long)mt * ((rows + w - 1) / w) * split + sms - 1) / sms; };
   const float narrow = (nsrc - 0.5f * n_early) * std::min((float)waves_of(64, 1), 0.5f * waves_of(64, 2));
   const bool one_acc = !two || (mode == TC_F16X2 && 8 * waves_of(256, 1) < 5 * waves_of(128, 1) && 2.f * nsrc * waves_of(256, 1) < narrow);
   const int row_tiles = (rows + 255) / 256;
   for (int w = one_acc ? 256 : 160; M > 256 && cells == 1 && w >= 32; w -= 32) {  // (a width's time grows with the number of column tiles)
     const int n_ct = (M - 1) / w + 1, nb = ((M - 1) / n_ct + 32) / 32 * 32;
     if (n_ct > 65535) break;  // (a grid's second axis)
-    const long long waves = ((long long)row_tiles * n_ct + 73) / 74;
+    const long long waves = ((long long)row_tiles * n_ct + sms / 2 - 1) / (sms / 2);
     const float cyc = two ? std::max(800.f, 6.5f * nb) : std::max(330.f, 2.2f * nb);
     const float us = 8.f + waves * (nsrc * kb * cyc / 1850.f + (two ? 0.015f : 0.01f) * nb);
     if (us < best.us) best = ChainPlan{128, 1, us, false, nb};

@@ -3,6 +3,7 @@
 // second of SM clock) and reports through p.err instead of spinning forever.
 #include "tc_gemm.cuh"
 
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
@@ -236,17 +237,6 @@ static int current_device() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) dev = 0;
   return dev;
 }
-static int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 template <int BN, int MODE>
 cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
   const size_t smem = (size_t)persistent_stages(BN, MODE) * stage_bytes(BN, MODE) + 1024;
@@ -261,7 +251,7 @@ cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
   const int m_tiles = (p.M + 127) / 128, n_tiles = (p.N + BN - 1) / BN;
   const int total = m_tiles * n_tiles;
   if (total == 0) return cudaSuccess;
-  const int grid = total < sm_count() ? total : sm_count();
+  const int grid = total < device_sms() ? total : device_sms();
   static const bool pdl = std::getenv("ZRNN_NO_PDL") == nullptr;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
@@ -279,6 +269,17 @@ cudaError_t launch_persistent_t(const TcParams& p, cudaStream_t st) {
 }
 
 }  // namespace
+
+int device_sms() {
+  static std::atomic<int> count[kMaxDevices];  // (asked by several threads at a time)
+  std::atomic<int>& c = count[current_device()];
+  int n = c.load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, current_device()) != cudaSuccess || n < 2) n = 148;
+    c.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 
 cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, cudaStream_t st) {
   // tile widths: 256 columns for bf16 / tf32, 128 for the split modes (their second, cross-term accumulator doubles the TMEM need)

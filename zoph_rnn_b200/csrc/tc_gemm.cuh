@@ -44,6 +44,8 @@ cudaError_t launch_tc_gemm_persistent(const TcParams& p, int mode, cudaStream_t 
 cudaError_t launch_wait_probe(int* err, long long limit_cycles, int code, cudaStream_t st);
 
 // Host helpers -------------------------------------------------------------------------------------------
+// multiprocessors of the current device (148 where there is none to ask)
+int device_sms();
 // 2-D K-major tensor map: `rows` rows of `k` elements, row stride ld (elements); box = (128-byte k-block) x box_rows
 // elem_bytes 2 (bf16) or 4 (fp32).  Returns false when the driver entry point is unavailable or arguments are
 // not encodable (base not 16-byte aligned, ld*elem_bytes not a multiple of 16).

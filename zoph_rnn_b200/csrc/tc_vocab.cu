@@ -269,19 +269,17 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   int tmem = 32;
   while (tmem < 2 * PARTS * p.nb) tmem *= 2;
   static bool configured[64] = {false};
-  static int sms[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(tc_vocab_kernel<MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfSm);
     if (e != cudaSuccess) return e;
-    cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
     configured[dev] = true;
   }
   const int n_tiles = (p.N + 127) / 128;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(std::min(n_tiles, 2 * sms[dev]));
+  cfg.gridDim = dim3(std::min(n_tiles, 2 * device_sms()));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

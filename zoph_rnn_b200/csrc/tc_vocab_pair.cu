@@ -314,19 +314,17 @@ cudaError_t launch_t(const VocabParams& p, cudaStream_t st) {
   if (stages < 2) return cudaErrorInvalidValue;
   const int bufs = 2 * PARTS * p.nb <= 512 ? 2 : 1;
   static bool configured[64] = {false};
-  static int sms[64] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
   if (!configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(tc_vocab_pair_kernel<MODE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (e != cudaSuccess) return e;
-    cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
     configured[dev] = true;
   }
   const int v_tiles = (p.N + 255) / 256;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * std::min(v_tiles * p.n_ct, sms[dev] / 2));
+  cfg.gridDim = dim3(2 * std::min(v_tiles * p.n_ct, device_sms() / 2));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmem;
   cfg.stream = st;
@@ -350,19 +348,14 @@ cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
 // The time of a launch is the tiles of the busiest pair times the columns of a tile; a tile's fixed part counts as 16 more (K = 1000,
 // fp16 split: 9.5 us a tile of 128 columns, 12 of 160, 17.5 of 256).
 VocabTiles vocab_pair_tiles(int M, int N) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 2) sms = 148;
-  }
+  const int pairs = device_sms() / 2;
   VocabTiles best{0, 0};
   long long best_cost = 0;
   const int v_tiles = (N + 255) / 256, least = (M + 255) / 256;
   for (int n_ct = least; n_ct <= least + 3; ++n_ct) {
     const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
     if (nb * (n_ct - 1) >= M) continue;  // the last tile would be empty
-    const long long waves = ((long long)v_tiles * n_ct + sms / 2 - 1) / (sms / 2);
+    const long long waves = ((long long)v_tiles * n_ct + pairs - 1) / pairs;
     const long long cost = waves * (nb + 16);
     if (best.n_ct == 0 || cost < best_cost) {
       best = VocabTiles{n_ct, nb};
