@@ -70,6 +70,17 @@ def test_launch_rules_ask_the_current_device_for_its_multiprocessors():
     assert "std::atomic<int> count[kMaxDevices]" in body("tc_gemm.cu", "int device_sms()", "\n}")
 
 
+def test_the_persistent_decoder_requests_the_weights_of_its_last_k_blocks():
+    """Its activation ring may hold more k-blocks than its weight ring.  A producer that left with the last activation requested would, if the
+    MMAs had not freed a weight stage by then, leave the last k-blocks without weights, and the kernel would wait for them until its bounded
+    waits give up."""
+    s = body("tc_decoder.cu", "if (warp == 8) {", "else if (warp == 9)")
+    loop = s[s.index("while ("):]
+    assert loop.startswith("while (!ac.end || !wc.end) {")
+    weights, acts = loop.index("!wc.end && w_it < a_it + NW"), loop.index("if (!ac.end) {")
+    assert weights < acts < loop.index("ac.pl")  # (and no activation is looked at beyond the last)
+
+
 def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
     """A link kernel requests its weights before it waits for the launch ahead of it.  In the stand-alone product the weights are packed by a
     launch of the same call, so another launch, which waits for that one, has to lie between."""

@@ -398,7 +398,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_decoder_kernel(const __grid_co
       long long t_progress = clock64();
       int idle = 0;
       bool ok = true;
-      while (!ac.end) {
+      // To the end of both: the activation ring can hold more k-blocks than the weight ring, so the last activations may be requested while
+      // the weights of the last k-blocks still wait for a stage.
+      while (!ac.end || !wc.end) {
         bool progressed = false;
         const bool hold = p.hold_loads && *reinterpret_cast<volatile int*>(&in_exchange) != 0;
         // weights: as far ahead as the ring allows
@@ -422,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_decoder_kernel(const __grid_co
           }
         }
         // activations: the next k-block, once its data exists and its stage is free
-        {
+        if (!ac.end) {
           bool can = !hold;
           Item it;
           make_item(p, ac.pl, ac.s, ac.pl.lo[ac.s] + ac.k, ac.tile, gr.b0, EPK, it);
