@@ -13,20 +13,25 @@ STORE, LSTM = range(2)
 PROBE = r"""
 #include <chrono>
 #include <cstdio>
+#include "skinny_gemm.cuh"
 #include "tc_chain.cuh"
-// lines of "mode epi rows nsrc kb n_early columns beside" -> "BN split nb microseconds"; one call takes that long at least of three
+// lines of "mode epi rows nsrc kb n_early columns beside cells H" -> "BN split nb microseconds skinny"; one call takes that long at least of
+// three; skinny: the warp-level kernel's estimate is the shorter one
 int main() {
-  int mode, epi, rows, nsrc, kb, early, M, beside;
-  while (std::scanf("%d %d %d %d %d %d %d %d", &mode, &epi, &rows, &nsrc, &kb, &early, &M, &beside) == 8) {
+  int mode, epi, rows, nsrc, kb, early, M, beside, cells, H;
+  while (std::scanf("%d %d %d %d %d %d %d %d %d %d", &mode, &epi, &rows, &nsrc, &kb, &early, &M, &beside, &cells, &H) == 10) {
     zrnn::ChainPlan p;
     double best = 1e30;
     for (int i = 0; i < 3; ++i) {
       const auto t0 = std::chrono::steady_clock::now();
-      p = zrnn::plan_chain(mode, epi, rows, 1, nsrc, kb, early, M, beside != 0);
+      p = zrnn::plan_chain(mode, epi, rows, cells, nsrc, kb, early, M, beside != 0);
       const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
       if (us < best) best = us;
     }
-    std::printf("%d %d %d %g\n", p.BN, p.split, p.nb, best);
+    const bool skinny = M <= 64 && (mode == zrnn::TC_BF16 || mode == zrnn::TC_F16X2) &&
+                        zrnn::skinny_us(mode == zrnn::TC_BF16 ? zrnn::SK_BF16 : zrnn::SK_F16X2, epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE,
+                                        rows, nsrc * H, M, cells, early > 0 && !beside) < p.us;
+    std::printf("%d %d %d %g %d\n", p.BN, p.split, p.nb, best, (int)skinny);
   }
 }
 """
@@ -50,8 +55,9 @@ def plans(tmp_path_factory):
                            "-o", exe, lib, "-Wl,-rpath," + PKG])
 
     def ask(questions):
-        out = subprocess.run([exe], input="".join("%d %d %d %d %d %d %d %d\n" % q for q in questions), stdout=subprocess.PIPE, text=True, check=True)
-        rows = [(int(a), int(b), int(c), float(t)) for a, b, c, t in (line.split() for line in out.stdout.splitlines())]
+        lines = "".join("%d %d %d %d %d %d %d %d %d %d\n" % (q if len(q) == 10 else q + (1, 1)) for q in questions)
+        out = subprocess.run([exe], input=lines, stdout=subprocess.PIPE, text=True, check=True)
+        rows = [(int(a), int(b), int(c), float(t), int(k)) for a, b, c, t, k in (line.split() for line in out.stdout.splitlines())]
         assert len(rows) == len(questions)
         return rows
     return ask
@@ -78,7 +84,7 @@ def test_one_accumulator_over_the_whole_k_axis_only_where_it_halves_the_waves(pl
     q = [(mode, epi, (4 if epi == LSTM else 2 if nsrc == 1 else 1) * H, nsrc, kblocks(mode, H), early, M, 0) for mode in (TF32X3, F16X2) for epi in (STORE, LSTM)
          for H in (256, 320, 400, 500, 512, 640, 768, 900, 1000, 1024, 1536, 2048) for nsrc in (1, 2, 3) for early in range(nsrc) for M in range(257, 4100, 31)]
     seen = set()
-    for (mode, epi, rows, nsrc, kb, early, M, _), (_, _, nb, _) in zip(q, plans(q)):
+    for (mode, epi, rows, nsrc, kb, early, M, _), (_, _, nb, _, _) in zip(q, plans(q)):
         if nb > 160:
             w = waves(M, rows, 256)
             assert mode == F16X2 and waves(M, rows, 128) > 1.6 * w, (mode, epi, rows, nsrc, M, nb)
@@ -97,6 +103,28 @@ def test_very_many_columns_are_planned_in_no_time_and_fit_a_grid(plans):
     CTAs are the second axis of a grid, which ends at 65535: beyond, the tiles of single CTAs, whose columns are the first axis, take them."""
     q = [(mode, STORE, rows, 1, kb, 0, M, 0) for mode in (BF16, TF32, TF32X3, F16X2) for rows in (64, 256, 2000) for kb in (1, 4, 16)
          for M in (70000, 1 << 20, 10_500_000, 17_000_000, 30_000_000)]
-    for (mode, _, rows, _, _, _, M, _), (BN, split, nb, us) in zip(q, plans(q)):
+    for (mode, _, rows, _, _, _, M, _), (BN, split, nb, us, _) in zip(q, plans(q)):
         assert nb == 0 or -(-M // nb) <= 65535, (mode, rows, M, nb)
         assert us < 20, (M, us)
+
+
+# kind of link (epilogue, weight rows per H, sources, early ones), cells in the launch, mode, H, columns -> the kernels (warp-level: "skinny", else
+# tile rows / CTAs per tile) within 3 % of the best pass; with the next best one a pass took 2 - 28 % longer
+MEASURED = [("cell", 1, BF16, 320, 1, "skinny"), ("cell", 1, BF16, 320, 8, "skinny"), ("cell", 1, BF16, 320, 16, "skinny"), ("cell", 1, BF16, 504, 16, "skinny"),
+            ("cell", 1, BF16, 400, 24, "skinny"), ("cell", 1, BF16, 400, 128, "32/2"), ("cell", 1, BF16, 1000, 128, "64/2"), ("cell", 1, F16X2, 256, 100, "32/2"),
+            ("cell", 1, F16X2, 504, 64, "64/2"), ("cell", 1, F16X2, 256, 200, "32/1 64/2"), ("cell", 1, F16X2, 1000, 1, "skinny"), ("cell", 1, F16X2, 1000, 16, "skinny"),
+            ("cell", 1, TF32X3, 504, 4, "64/2"), ("stack", 2, BF16, 1000, 1, "skinny"), ("stack", 2, BF16, 1000, 8, "skinny"), ("stack", 4, BF16, 256, 40, "32/1"),
+            ("stack", 2, F16X2, 1000, 12, "skinny"), ("stack", 2, F16X2, 1000, 16, "skinny"), ("stack", 3, F16X2, 640, 12, "skinny"), ("stack", 3, F16X2, 640, 16, "skinny"),
+            ("stack", 4, F16X2, 400, 24, "skinny"), ("stack", 4, F16X2, 640, 32, "64/1 128/1"), ("stack", 3, F16X2, 1000, 24, "64/1 128/1"), ("stack", 4, F16X2, 1000, 56, "128/1"),
+            ("stack", 4, F16X2, 1000, 128, "128/1"), ("stack", 4, BF16, 1000, 128, "128/1"), ("projection", 1, F16X2, 400, 100, "32/4 32/2"), ("projection", 1, F16X2, 504, 80, "32/4 32/2")]
+
+
+def test_links_take_the_kernel_that_was_measured_to_be_faster(plans):
+    """Shapes at which the refitted rule of the links had left the faster kernel, and some at which it had not: passes of 10 + 10 steps, 1000 words."""
+    kinds = {"cell": (LSTM, 4, 2, 1), "stack": (LSTM, 4, 2, 0), "projection": (STORE, 2, 1, 0)}
+    q = []
+    for kind, cells, mode, H, M, _ in MEASURED:
+        epi, per, nsrc, early = kinds[kind]
+        q.append((mode, epi, per * H, nsrc, kblocks(mode, H), early, M, 0, cells, H))
+    got = ["skinny" if sk else "%d/%d" % (BN, split) for BN, split, _, _, sk in plans(q)]
+    assert [(m, g) for m, g in zip(MEASURED, got) if g not in m[5].split()] == []

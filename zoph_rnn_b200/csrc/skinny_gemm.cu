@@ -380,11 +380,15 @@ cudaError_t launch_nt(const SkinnyBatch& b, int n, int mt, int nt, cudaStream_t 
 
 }  // namespace
 
-// Fitted to measurements (us per launch; f32 / bf16): 4 M weights 5.8 / 4.2 at 8 columns, 8.7 / 5.1 at 32; 16 M weights 11 / 7.9 at
-// 8 columns, 17 / 10 at 24; 2 M weights at 64 columns 10 / -.  (From two column groups on every weight is read twice: not offered.)
-float skinny_us(int mode, int rows, int K, int cols, int n) {
+// Fitted, with the constants of plan_chain, to scoring passes in which every kernel and tile was taken for one kind of link after the other
+// (1 - 4 x 256 - 1000 units, 1 - 256 columns, f32, bf16 and 3xTF32): the choices cost 0.15 us per launch more than the best ones.
+// A cell with early operands starts beside its predecessor, but then holds up the next one's start (1.65 and 0.5 us); products of the attention
+// take 0.9 and 0.5 us more.  (From two column groups on every weight is read twice: not offered.)
+float skinny_us(int mode, int epi, int rows, int K, int cols, int n, bool early) {
   const float mw = (float)rows * K * n * 1e-6f, nt = (float)((cols + 7) / 8);
-  return mode == SK_F16X2 ? 4.0f + mw * (0.285f + nt * (0.144f + 0.0114f * nt)) : 3.2f + mw * (0.22f + 0.07f * nt);
+  const bool cell = epi == SK_EPI_LSTM;
+  if (mode == SK_F16X2) return 3.1f + (cell ? (early ? 1.65f : 0.f) : 0.9f) + mw * (0.105f + nt * (0.195f + 0.025f * nt));
+  return 3.15f + (cell ? (early ? 0.5f : 0.f) : 0.5f) + mw * (0.09f + 0.105f * nt);
 }
 
 cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st) {

@@ -41,8 +41,9 @@ struct SkinnyBatch {
   enum { MAX = 8 };
   SkinnyParams p[MAX];
 };
-// about how long launch_skinny takes for n problems of `rows` weight rows x K elements (all sources) and `cols` columns
-float skinny_us(int mode, int rows, int K, int cols, int n);
+// about how long launch_skinny takes for n problems of `rows` weight rows x K elements (all sources) and `cols` columns, on the scale of
+// plan_chain's estimate; early: some sources are early and no other stream's launches run beside
+float skinny_us(int mode, int epi, int rows, int K, int cols, int n, bool early);
 // n independent problems of the same shape class (mode, epilogue, N, K, M) in one launch
 cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st);
 

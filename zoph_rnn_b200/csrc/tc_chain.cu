@@ -445,16 +445,19 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_
 
 // Which tile: a launch takes, per wave of CTAs and k-block, the longer of the bytes a CTA fetches, at the 130 KB/us that an SM takes in
 // from L2, and the MMAs, of which each takes 60 cycles at least (the split modes at 128 rows, a warp per product and one cross
-// accumulator: 1.6 times their cycles; rounds with one accumulator set, on half an SM: 0.15 us more); then a fixed part per wave, the exchange of a K split and an epilogue that grows with the outputs per
-// CTA.  Of the early sources of links on half an SM half is counted: the other half runs beside the predecessor.  us, estimated /
-// measured, fp16 split: 1000 units, 128 columns 10.7 / 10.9, 200 columns 15.7 / 16.1, 384 in tiles of 128 rows 25.6 / 25.6; 500 units, 768
-// columns 15.1 / 15.9; bf16: 1000 units, 128 columns 7.7 / 7.8, 384 11.7 / 11.4.
+// accumulator: 1.6 times their cycles, 1.4 times in a launch of several cells; rounds with one accumulator set, on half an SM: 0.15 us
+// more); then a fixed part per wave, the exchange of a K split and an epilogue that grows with the outputs per CTA.  Of the early sources
+// of links on half an SM a half (bf16, tf32: a third) is counted off: that much runs beside the predecessor.  Cells on whole SMs that leave
+// the next launch no room beside them take up to 0.5 us more.  The exchange, these two and the factor of several cells are fitted to passes up to 256 columns (skinny_us, skinny_gemm.cu), the rest to launches: us, estimated / measured,
+// fp16 split, 1000 units, 384 columns in tiles of 128 rows 25.6 / 25.6; 500 units, 768 columns 15.1 / 15.9; bf16, 1000 units, 384 columns
+// 11.7 / 11.4.
 // Four CTAs per tile in the split modes only: in bf16 they are worth 0.4 % of a scoring pass (4 x 1000 units, 128 columns 3108 -> 3097 us),
 // and the other order of the sums turns results that are rounded to bf16 at every step (6e-4 between the log-probabilities, 1.08e-3 from
 // float64 either way).
 ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, int n_early, int M, bool beside) {
   const bool two = mode_split(mode);
   const int sms = device_sms(), parts = two ? 2 : 1, mt = cells * ((M + 127) / 128), a_rows = M >= 128 ? 128 : (M + 7) / 8 * 8;
+  const float two_ctas = epi == TC_EPI_LSTM ? (two ? 1.08f : 0.62f) : (two ? 0.4f : 1.0f);
   ChainPlan best{0, 1, 1e30f, false, 0};
   for (int BN = epi == TC_EPI_LSTM ? 32 : 16; BN <= 128; BN *= 2) {
     for (int split = 1; split <= 4; split *= 2) {
@@ -462,10 +465,11 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
       if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
       const int ctas = mt * ((rows + BN - 1) / BN) * split, waves = (ctas + sms - 1) / sms;
       const bool whole = two && BN <= 64 && BN >= 32 && !beside;
-      const float cyc = 4.f * (!two ? std::max(60.f, BN / 2.f) : (BN <= 64 ? std::max(60.f, (float)BN) + 60.f : 1.6f * 3.f * BN / 2.f));
+      const float crowd = whole && epi == TC_EPI_LSTM ? 0.5f * std::min(1.f, std::max(0.f, 2.f * ctas / sms - 1.f)) : 0.f;
+      const float cyc = 4.f * (!two ? std::max(60.f, BN / 2.f) : (BN <= 64 ? std::max(60.f, (float)BN) + 60.f : (cells > 1 ? 1.38f : 1.6f) * 3.f * BN / 2.f));
       const float kb_us = std::max(parts * 128.f * (a_rows + BN) / 130e3f, cyc / 1850.f) + (two && epi == TC_EPI_STORE && BN <= 64 && !whole ? 0.15f : 0.f);
-      const float kbs = kb * (nsrc - (BN <= 64 && !whole ? 0.5f * n_early : 0.f)) / split;
-      const float us = (whole ? 3.6f : 3.2f) + 3.f * (waves - 1) + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? 1.3f : split == 4 ? 1.8f : 0.f);
+      const float kbs = kb * (nsrc - (BN <= 64 && !whole ? (two ? 0.5f : 0.33f) * n_early : 0.f)) / split;
+      const float us = (whole ? 3.6f : 3.2f) + 3.f * (waves - 1) + waves * (kb_us * kbs + (two ? 0.01f : 0.005f) * BN / split) + (split == 2 ? two_ctas : split == 4 ? 0.9f : 0.f) + crowd;
       if (us < best.us) best = ChainPlan{BN, split, us, whole, 0};
     }
   }

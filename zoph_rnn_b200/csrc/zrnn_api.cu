@@ -421,9 +421,9 @@ LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
   p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols, beside);
-  // (a warp-level kernel with early operands starts beside its predecessor, but then holds up the next one's start: skinny_gemm.cu)
   p.skinny = skinny_engine(eng) && cols <= 64 &&
-             zrnn::skinny_us(skinny_mode(eng), rows, nsrc * H, cols, n) + (epi == zrnn::TC_EPI_LSTM && n_early && !beside ? 1.f : 0.f) < p.chain.us;
+             zrnn::skinny_us(skinny_mode(eng), epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE, rows, nsrc * H, cols, n,
+                             n_early > 0 && !beside) < p.chain.us;
   return p;
 }
 // weights stored in packed 128-row tiles: tile-contiguous k-blocks (kbtot > 0) or plain rows of ld elements
