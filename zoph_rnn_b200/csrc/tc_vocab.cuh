@@ -39,6 +39,10 @@ struct VocabTiles {
   int n_ct, nb;
 };
 VocabTiles vocab_pair_tiles(int M, int N);
+// short products (k-blocks times products per k-step): their log-sum-exp always runs in tiles of one CTA, which read no padding of the rows
+inline bool vocab_short(int mode, int kb) { return kb * (mode == TC_TF32X3 || mode == TC_F16X2 ? 3 : 1) <= 16; }
+// the log-sum-exp of M columns (more than kVocabFewCols) over N words takes less time in tiles of one CTA (launch_tc_gemm_persistent)
+bool vocab_lse_single(int mode, int kb, int M, int N);
 cudaError_t launch_tc_vocab_pair(const VocabParams& p, int mode, int epi, cudaStream_t st);
 
 }  // namespace zrnn

@@ -345,24 +345,42 @@ cudaError_t launch_mode(const VocabParams& p, int epi, cudaStream_t st) {
 
 }  // namespace
 
-// The time of a launch is the tiles of the busiest pair times the columns of a tile; a tile's fixed part counts as 16 more (K = 1000,
-// fp16 split: 9.5 us a tile of 128 columns, 12 of 160, 17.5 of 256).
+// The time of a launch is the tiles of the busiest pair times the columns of a tile, a tile's fixed part counting as 48 more: 0.3 % more than
+// the best tiles take (700 - 40000 words, K = 64 - 1000, 65 - 2400 columns, all widths forced).  Few words are cut into many
+// narrow tiles: 700 words, K = 1000, 1200 columns, fp16 split 18.5 us in tiles of 160 columns, 12.8 of 64.
 VocabTiles vocab_pair_tiles(int M, int N) {
-  const int pairs = device_sms() / 2;
+  const int pairs = device_sms() / 2, v_tiles = (N + 255) / 256;
   VocabTiles best{0, 0};
   long long best_cost = 0;
-  const int v_tiles = (N + 255) / 256, least = (M + 255) / 256;
-  for (int n_ct = least; n_ct <= least + 3; ++n_ct) {
-    const int nb = ((M + n_ct - 1) / n_ct + 31) / 32 * 32;
-    if (nb * (n_ct - 1) >= M) continue;  // the last tile would be empty
-    const long long waves = ((long long)v_tiles * n_ct + pairs - 1) / pairs;
-    const long long cost = waves * (nb + 16);
+  for (int w = 256; w >= 32; w -= 32) {
+    const int n_ct = (M - 1) / w + 1, nb = ((M - 1) / n_ct + 32) / 32 * 32;
+    if ((long long)nb * (n_ct - 1) >= M) continue;  // the last tile would be empty
+    const long long cost = (((long long)v_tiles * n_ct + pairs - 1) / pairs) * (nb + 48);
     if (best.n_ct == 0 || cost < best_cost) {
       best = VocabTiles{n_ct, nb};
       best_cost = cost;
     }
   }
   return best;
+}
+
+// Tiles of one CTA (tc_gemm.cu) are faster for the log-sum-exp epilogue of short products, which takes longer than their MMAs: it has a column
+// per lane, so no value changes hands.  us, single CTAs / pairs, 160, 512 and 6400 columns: fp16 split, K = 100, 10000 words 9.2 / 10.0,
+// 11.5 / 14.3, 69 / 86; K = 512, 20000 words 19.1 / 18.8, 30.5 / 30.1, 277 / 246; bf16, 50000 words, K = 1000 26.0 / 22.0 at 160
+// columns, 43.6 / 49.7, 405 / 420; K = 1536 41.5 / 36.6, 67 / 64, 598 / 582.  (65 - 144 columns of K = 100 - 1024: 6 - 22 us, the few-columns
+// kernel 10 - 41.)  In the split modes they are faster for longer products, too, where these have few tiles for 74 pairs (K = 504, 3000 words,
+// 768 columns 9.8 / 12.1): the estimates are fitted to products of 700 - 40000 words, K = 64 - 1000, 65 - 2400 columns (6.5 % rms).
+bool vocab_lse_single(int mode, int kb, int M, int N) {
+  if (vocab_short(mode, kb)) return true;
+  if (!mode_split(mode)) return false;
+  const int pairs = device_sms() / 2;
+  const VocabTiles t = vocab_pair_tiles(M, N);
+  const long long waves = ((long long)((N + 255) / 256) * t.n_ct + pairs - 1) / pairs;
+  if (waves > 3) return false;
+  const long long waves1 = ((long long)((N + 127) / 128) * ((M + 127) / 128) + 2 * pairs - 1) / (2 * pairs);
+  const float loop = 0.0042f * kb * std::max(75, t.nb), epi = 0.8f + 0.0177f * t.nb, loop1 = 0.62f * kb, epi1 = 2.35f;
+  return 2.6f + waves1 * std::max(loop1, epi1) + 0.77f * std::min(loop1, epi1) <
+         5.2f + waves * std::max(loop, epi) + 0.38f * std::min(loop, epi) * (t.nb > 128 ? waves : 1);
 }
 
 cudaError_t launch_tc_vocab_pair(const VocabParams& p, int mode, int epi, cudaStream_t st) {

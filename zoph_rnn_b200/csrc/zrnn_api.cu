@@ -642,13 +642,10 @@ int att_forward(zrnn_attention* A, const Act& h_t, const int* mask, int B, const
   return ZRNN_OK;
 }
 
-// Tiles of one CTA (tc_gemm.cu) are still faster for the log-sum-exp epilogue of short products, which takes longer than their MMAs: it
-// has a column per lane, so no value changes hands.  us, single CTAs / pairs, 160, 512 and 6400 columns: fp16 split, K = 100, 10000
-// words 9.2 / 10.0, 11.5 / 14.3, 69 / 86; K = 512, 20000 words 19.1 / 18.8, 30.5 / 30.1, 277 / 246; bf16, 50000 words, K = 1000 31.6 /
-// 29.2, 50.5 / 50.9, 405 / 420; K = 1536 41.5 / 36.6, 67 / 64, 598 / 582.
-bool short_lse(const zrnn_softmax* S) {
-  const int epk = 128 / eng_eb(S->eng), products = eng_split(S->eng) ? 3 : 1;
-  return (S->H + epk - 1) / epk * products <= 16;
+// k-blocks of the vocabulary projection
+int vocab_kb(const zrnn_softmax* S) {
+  const int epk = 128 / eng_eb(S->eng);
+  return (S->H + epk - 1) / epk;
 }
 // the part of a VocabParams that scoring and decoding share
 int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams& p) {
@@ -659,7 +656,7 @@ int vocab_params(zrnn_softmax* S, const Act& h, int N, int np, zrnn::VocabParams
   p.M = N; p.N = S->hi - S->lo;
   const zrnn::VocabTiles t = pair ? zrnn::vocab_pair_tiles(N, p.N) : zrnn::VocabTiles{1, zrnn::vocab_columns(N)};
   p.nb = t.nb; p.n_ct = t.n_ct;
-  p.kb = (S->H + 128 / eb - 1) / (128 / eb); p.kbs = zrnn::vocab_kbs(mode);
+  p.kb = vocab_kb(S); p.kbs = zrnn::vocab_kbs(mode);
   if (!h.hi) return fail(ZRNN_E_STATE, "internal: activation has no operand-form copy");
   if (!zrnn::make_rows_map(&p.w, S->D_op.hi, eb, row_bytes, (long long)S->n_tiles * S->BN, parts, S->D_op.part_bytes(), p.kb, 128, p.kbs) ||
       !zrnn::make_rows_map(&p.h, h.hi, eb, row_bytes, N, parts, (char*)h.lo - (char*)h.hi, p.kb, pair ? p.nb / 2 : p.nb, p.kbs))
@@ -699,7 +696,7 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   }
   const int eng = S->eng, np = S->n_tiles * zrnn::kPersistentParts;
   ZR_CUDA(S->parts.reserve(sizeof(float) * 2 * (size_t)np * N));
-  if (N <= zrnn::kVocabFewCols || !short_lse(S)) {
+  if (N <= zrnn::kVocabFewCols || !zrnn::vocab_lse_single(eng_tcmode(eng), vocab_kb(S), N, Vs)) {
     zrnn::VocabParams vp;
     ZR_TRY(vocab_params(S, h, N, np, vp));
     vp.target = targets; vp.target_offset = S->lo; vp.tgt_logit = tgt;
@@ -711,7 +708,7 @@ int softmax_partials_launch(zrnn_softmax* S, const Act& h, const int* targets, i
   zrnn::TcParams tp;
   std::memset(&tp, 0, sizeof(tp));
   ZR_TRY(act_maps(h, eng, H, S->Kpad, N, &tp.a, &tp.a_lo));
-  tp.kblocks = (H + 128 / eng_eb(eng) - 1) / (128 / eng_eb(eng));
+  tp.kblocks = vocab_kb(S);
   tp.b = S->dmap; tp.b_lo = S->dmap_lo;
   tp.M = N; tp.N = Vs; tp.bias = S->b;
   tp.target = targets; tp.target_offset = S->lo;
@@ -1694,8 +1691,9 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
       a.h_seq = seq[l].f32;
       a.xp = m->seq_xp.as<float>();
       a.ld_op = g.Kpad;
-      // the decoder's cells, the attention and the vocabulary projections but one read whole k-blocks of these rows
-      a.zero_pad = m->cfg.attention != 0 || !m->cfg.lm || S * B <= zrnn::kVocabFewCols || !short_lse(m->sm);
+      // the decoder's cells, the attention and the vocabulary projections but that of short products read whole k-blocks of these rows
+      a.zero_pad = g.eng != ENG_SIMT && (m->cfg.attention != 0 || !m->cfg.lm || S * B <= zrnn::kVocabFewCols ||
+                                         !zrnn::vocab_short(eng_tcmode(m->sm->eng), vocab_kb(m->sm)));
       if (g.eng == ENG_BF16) a.op_b16 = seq[l].hi;
       else if (g.eng == ENG_H2) { a.op_h_hi = seq[l].hi; a.op_h_lo = seq[l].lo; }
       else if (g.eng != ENG_SIMT) { a.op_hi = (float*)seq[l].hi; a.op_lo = g.eng == ENG_X3 ? seq[l].lo : nullptr; }
