@@ -159,3 +159,12 @@ MEASURED_VOCAB = [(F16X2, 1000, 700, 1200, 64, False), (F16X2, 504, 700, 500, 32
 def test_vocabulary_projection_takes_the_tiles_that_were_measured_to_be_faster(plans):
     got = plans([(mode, kblocks(mode, K), M, N) for mode, K, N, M, _, _ in MEASURED_VOCAB], vocab=True)
     assert [(m, g) for m, g in zip(MEASURED_VOCAB, got) if (m[4] and g[1] != m[4]) or bool(g[2]) != m[5]] == []
+
+
+def test_many_columns_take_pairs_of_ctas_only_where_they_are_faster(plans):
+    """Every wave of pairs pays its set-up and its end anew, so tiles of 128 x 128 on single CTAs, of which twice as many run at a time, can be
+    faster: us per cell, pairs / single CTAs, bf16, 504 units, 2100 columns 18.8 / 16.7, 1000 units, 900 columns 23.9 / 23.4; fp16 split, 504 units, 3000 columns
+    61.8 / 47.3; but 1000 units, 768 columns in bf16 19.8 / 22.6."""
+    q = [(BF16, 504, 2100, False), (BF16, 1000, 900, False), (BF16, 1000, 1024, False), (F16X2, 504, 3000, False), (F16X2, 1000, 1300, True), (BF16, 1000, 768, True), (F16X2, 2048, 600, True)]
+    got = plans([(mode, LSTM, 4 * H, 2, kblocks(mode, H), 0, M, 0) for mode, H, M, _ in q])
+    assert [(a, p[2]) for a, p in zip(q, got) if (p[2] > 0) != a[3]] == []

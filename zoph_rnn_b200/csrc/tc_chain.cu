@@ -473,8 +473,9 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
       if (us < best.us) best = ChainPlan{BN, split, us, whole, 0};
     }
   }
-  // Pairs of CTAs: a k-block's twelve MMAs (four) take 64 cycles each at least, half a cycle per column; set-up, first loads
-  // and end 8 us, all of an SM being needed.  More than 160 columns per tile have one accumulator for the whole K axis in the split
+  // Pairs of CTAs: a k-block's twelve MMAs (four) take 64 cycles each at least, and half a cycle per column and more; a wave's
+  // set-up, first loads and end 7 us (5), all of an SM being needed.  (Fitted to cells of 256 - 2048 units, 300 - 3000 columns, tiles of 96 - 256
+  // columns forced: 6 % rms; the choices cost 0.4 % more than the best ones.)  More than 160 columns per tile have one accumulator for the whole K axis in the split
   // modes, whose error is several times that of rounds (1000 units 1.74e-6 from float64 against 1.8e-7).  That is paid only where it buys most: in fp16,
   // where tiles of 128 rows and columns take more than 1.6 times the waves of CTAs that tiles of 256 rows would (1000 units 513 - 1152 columns: two
   // waves against one), and tiles of 64 rows, over all or half of the K axis, more than twice the time even if half of the early sources is
@@ -487,8 +488,8 @@ ChainPlan plan_chain(int mode, int epi, int rows, int cells, int nsrc, int kb, i
     const int n_ct = (M - 1) / w + 1, nb = ((M - 1) / n_ct + 32) / 32 * 32;
     if (n_ct > 65535) break;  // (a grid's second axis)
     const long long waves = ((long long)row_tiles * n_ct + sms / 2 - 1) / (sms / 2);
-    const float cyc = two ? std::max(800.f, 6.5f * nb) : std::max(330.f, 2.2f * nb);
-    const float us = 8.f + waves * (nsrc * kb * cyc / 1850.f + (two ? 0.015f : 0.01f) * nb);
+    const float cyc = two ? std::max(919.f, 7.94f * nb) : std::max(317.f, 2.92f * nb);
+    const float us = (two ? 2.7f : 2.05f) + waves * ((two ? 6.9f + 0.01f * nb : 4.9f + 0.016f * nb) + nsrc * kb * cyc / 1850.f);
     if (us < best.us) best = ChainPlan{128, 1, us, false, nb};
   }
   return best;
