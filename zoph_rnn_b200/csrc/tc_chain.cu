@@ -32,7 +32,6 @@ constexpr int kThreads = (kEpiWarps + 2 + kMmaWarps) * 32;
 // accumulators of the narrow tiles absorb (tc_link.cu: 4 up to 512 elements per source, else 8), so that the choice of a tile
 // is none of precision.
 __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 1 : 2; }
-__host__ __device__ constexpr bool chain_rounds(int mode) { return mode_split(mode); }
 // accumulator sets.  Split modes: main accumulators, with one cross accumulator behind them.  bf16: one per MMA warp, tf32: two (tc_link.cu).
 __host__ __device__ constexpr int chain_sets(int mode) { return mode_split(mode) ? 3 : (mode == TC_TF32 ? 2 : 1) * kMmaWarps; }
 __host__ __device__ constexpr int chain_tmem(int BN, int mode) {
@@ -46,16 +45,17 @@ constexpr int kChainRingBytes = 224 * 1024, kMaxStages = 8;
 template <int BN, int MODE, int EPI>
 __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_block, const int stages) {
   constexpr int EW = kEpiWarps, kAWarp = EW, kWWarp = EW + 1, kMmaWarp = EW + 2;
-  constexpr bool BY_PRODUCT = mode_split(MODE), ROUNDS = chain_rounds(MODE);
-  constexpr int STEP = BY_PRODUCT ? 1 : kMmaWarps;  // stages from one of an MMA warp to its next
-  constexpr int PARTS = mode_split(MODE) ? 2 : 1;
+  // (the modes that walk in rounds are those whose MMA warps share the work by product)
+  constexpr bool SPLIT_MODE = mode_split(MODE);
+  constexpr int STEP = SPLIT_MODE ? 1 : kMmaWarps;  // stages from one of an MMA warp to its next
+  constexpr int PARTS = SPLIT_MODE ? 2 : 1;
   constexpr int WKB = BN * 128;  // bytes of one k-block of one weight part
   constexpr uint32_t IDESC = make_idesc(mode_fmt(MODE), BN);
   constexpr int NSET = chain_sets(MODE), TMEM_COLS = chain_tmem(BN, MODE);
   extern __shared__ uint8_t smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
   __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
-  __shared__ __align__(8) uint64_t accum_bar;  // everything accumulated (rounds: the cross products of wide tiles)
+  __shared__ __align__(8) uint64_t accum_bar;  // everything accumulated (rounds: the cross products)
   __shared__ __align__(8) uint64_t set_full[chain_sets(MODE)], set_empty[chain_sets(MODE)];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
@@ -65,21 +65,20 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const int m0 = m_block * 128, n_tile = blockIdx.y;
   const int akb = p.a_rows * 128;  // bytes of one k-block of one activation part
-  // k-blocks per ring stage: a TMA instruction costs its issuing thread about 200 cycles and a stage's hand-over 300, so one
-  // instruction fetches the activations (the weights) of several blocks where the ring still holds a few stages
+  // k-blocks per ring stage: one TMA instruction and one hand-over for the activations (the weights) of several blocks where the ring
+  // still holds a few stages
   const int KBS = p.kbs;
   // KBS x [A hi][A lo], KBS x [W hi][W lo]; every piece is a multiple of 1024 bytes
   const int stage_bytes = PARTS * KBS * (akb + WKB);
   const int src_it = (p.kb + KBS - 1) / KBS, n_it = p.nsrc * src_it;
   const int round_its = KBS < round_kb(MODE, p.kb) ? round_kb(MODE, p.kb) / KBS : 1;  // stages per round
-  constexpr int NBUF = BY_PRODUCT ? NSET : NSET / kMmaWarps;  // accumulator sets an MMA warp takes in turn
   ZR_STAMP(0);
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(&full_bar[s], 2);  // the activation and the weight producer
-      mbar_init(&empty_bar[s], BY_PRODUCT ? kMmaWarps : 1);
+      mbar_init(&empty_bar[s], SPLIT_MODE ? kMmaWarps : 1);
     }
-    mbar_init(&accum_bar, BY_PRODUCT ? 1 : kMmaWarps);
+    mbar_init(&accum_bar, SPLIT_MODE ? 1 : kMmaWarps);
     for (int i = 0; i < NSET; ++i) {
       mbar_init(&set_full[i], 1);
       mbar_init(&set_empty[i], EW);
@@ -160,21 +159,21 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
         const bool one = elect_one();
         const int mw = warp - kMmaWarp;
         bool ok = true;
-        const bool rounds = ROUNDS && !(BY_PRODUCT && mw == 1);
-        int st = BY_PRODUCT ? 0 : mw, set = st, in_round = 0, round = 0;
+        const bool rounds = SPLIT_MODE && mw == 0;
+        int st = SPLIT_MODE ? 0 : mw, set = st, in_round = 0, round = 0;
         uint32_t ph = 0;
         for (int it = st; it < n_it; it += STEP) {
           if (rounds && in_round == 0) {
-            set = BY_PRODUCT ? round % NBUF : mw + kMmaWarps * (round % NBUF);
-            if (round >= NBUF && !mbar_wait_warp(&set_empty[set], (uint32_t)((round / NBUF) & 1) ^ 1u, &abort_s, p.err, 4)) { ok = false; break; }
+            set = round % NSET;
+            if (round >= NSET && !mbar_wait_warp(&set_empty[set], (uint32_t)((round / NSET) & 1) ^ 1u, &abort_s, p.err, 4)) { ok = false; break; }
             tc_fence_after();
           }
-          if (!BY_PRODUCT) set = it % NSET;
+          if (!SPLIT_MODE) set = it % NSET;
           if (!mbar_wait_warp(&full_bar[st], ph, &abort_s, p.err, 2)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(tiles + (size_t)st * stage_bytes), w_addr = a_addr + PARTS * KBS * akb;
           const uint32_t d = tmem_base + (uint32_t)(set * BN), d_cross = tmem_base + (uint32_t)(NSET * BN);
-          const bool fresh = rounds ? in_round == 0 : it < (BY_PRODUCT ? STEP : NSET);  // the accumulator starts with this stage
+          const bool fresh = rounds ? in_round == 0 : it < (SPLIT_MODE ? STEP : NSET);  // the accumulator starts with this stage
           if (one) {
             for (int b = 0; b < KBS; ++b) {
               const uint64_t da = make_smem_desc(a_addr + b * PARTS * akb), dal = make_smem_desc(a_addr + (b * PARTS + 1) * akb);
@@ -182,8 +181,8 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const uint32_t acc = (!fresh || b > 0 || k > 0) ? 1u : 0u;
-                if (!BY_PRODUCT || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC, acc);
-                if (BY_PRODUCT && mw == 1) {
+                if (!SPLIT_MODE || mw == 0) umma<mode_kind_tf32(MODE)>(d, da + 2 * k, dw + 2 * k, IDESC, acc);
+                if (SPLIT_MODE && mw == 1) {
                   umma<mode_kind_tf32(MODE)>(d_cross, dal + 2 * k, dw + 2 * k, IDESC, acc);
                   umma<mode_kind_tf32(MODE)>(d_cross, da + 2 * k, dwl + 2 * k, IDESC, 1u);
                 }
@@ -241,56 +240,49 @@ __device__ __forceinline__ void chain_body(const ChainParams& p, const int m_blo
   }
   const bool live = m0 + quad * 32 < p.M;  // whole warps: the TMEM loads are warp-wide
   bool ready = epi_warp;
-  // running sums (ROUNDS): chunk ch of W outputs; LSTM: one chunk per gate
+  // running sums (rounds): chunk ch of W outputs; LSTM: one chunk per gate
   constexpr int NCH = EPI == TC_EPI_LSTM ? 4 : PER / W;
   auto chunk_col = [&](int ch) { return EPI == TC_EPI_LSTM ? ch * (BN / 4) + cg * PER : cg * PER + ch * W; };
-  float sum[ROUNDS ? NCH : 1][W];
-  if constexpr (ROUNDS) {
+  float sum[SPLIT_MODE ? NCH : 1][W];
+  if constexpr (SPLIT_MODE) {
     static_assert(EPI != TC_EPI_LSTM || PER == W, "one chunk per gate");
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch)
 #pragma unroll
       for (int u = 0; u < W; ++u) sum[ch][u] = 0.f;
-    const int streams = BY_PRODUCT ? 1 : kMmaWarps;
-    for (int r = 0; ready && r * round_its * streams < n_it; ++r)
-      for (int mw = 0; ready && mw < streams; ++mw) {
-        if (r * round_its * streams + mw >= n_it) break;  // this MMA warp has fewer rounds
-        const int set = BY_PRODUCT ? r % NBUF : mw + kMmaWarps * (r % NBUF);
-        ready = __all_sync(0xffffffffu, mbar_wait(&set_full[set], (uint32_t)((r / NBUF) & 1), &abort_s, p.err, 3));
-        tc_fence_after();
-        if (ready && live) {
-          float t[NCH][W];
+    for (int r = 0; ready && r * round_its < n_it; ++r) {
+      const int set = r % NSET;
+      ready = __all_sync(0xffffffffu, mbar_wait(&set_full[set], (uint32_t)((r / NSET) & 1), &abort_s, p.err, 3));
+      tc_fence_after();
+      if (ready && live) {
+        float t[NCH][W];
 #pragma unroll
-          for (int ch = 0; ch < NCH; ++ch) tmem_ldw<W>(taddr + set * BN + chunk_col(ch), t[ch]);
-          tmem_wait_ld();
+        for (int ch = 0; ch < NCH; ++ch) tmem_ldw<W>(taddr + set * BN + chunk_col(ch), t[ch]);
+        tmem_wait_ld();
 #pragma unroll
-          for (int ch = 0; ch < NCH; ++ch)
+        for (int ch = 0; ch < NCH; ++ch)
 #pragma unroll
-            for (int u = 0; u < W; ++u) sum[ch][u] += t[ch][u];
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&set_empty[set]);
+          for (int u = 0; u < W; ++u) sum[ch][u] += t[ch][u];
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&set_empty[set]);
+    }
   }
-  if (ready && (!ROUNDS || BY_PRODUCT)) {
+  if (ready) {
     ready = __all_sync(0xffffffffu, mbar_wait(&accum_bar, 0, &abort_s, p.err, 3));
     tc_fence_after();
   }
   ZR_STAMP(2);
-  const int n_sets = n_it < NSET ? n_it : NSET;  // sets that were written (not ROUNDS)
+  const int n_sets = n_it < NSET ? n_it : NSET;  // sets that were written (without rounds)
   // the W finished accumulator columns of chunk ch, which start at tile column `col`
   auto load_acc = [&](int ch, int col, float* v) {
-    if constexpr (ROUNDS) {
+    if constexpr (SPLIT_MODE) {
+      float x[W];
+      tmem_ldw<W>(taddr + NSET * BN + col, x);
+      tmem_wait_ld();
 #pragma unroll
-      for (int u = 0; u < W; ++u) v[u] = sum[ch][u];
-      if constexpr (BY_PRODUCT) {
-        float x[W];
-        tmem_ldw<W>(taddr + NSET * BN + col, x);
-        tmem_wait_ld();
-#pragma unroll
-        for (int u = 0; u < W; ++u) v[u] = fmaf(x[u], mode_cross_scale(MODE), v[u]);
-      }
+      for (int u = 0; u < W; ++u) v[u] = fmaf(x[u], mode_cross_scale(MODE), sum[ch][u]);
     } else {
       float t[NSET][W];
 #pragma unroll
@@ -445,8 +437,8 @@ cudaError_t launch_mode(const ChainBatch& b, int n, int BN, int epi, cudaStream_
 
 // Which tile: a launch takes, per wave of CTAs and k-block, the longer of the bytes a CTA fetches, at the 130 KB/us that an SM takes in
 // from L2, and the MMAs, of which each takes 60 cycles at least (the split modes at 128 rows, a warp per product and one cross
-// accumulator: 1.6 times their cycles, 1.4 times in a launch of several cells; rounds with one accumulator set, on half an SM: 0.15 us
-// more); then a fixed part per wave, the exchange of a K split and an epilogue that grows with the outputs per CTA.  Of the early sources
+// accumulator: 1.6 times their cycles, 1.4 times in a launch of several cells; products in rounds with one accumulator set, on half an SM: 0.15
+// us more); then a fixed part per wave, the exchange of a K split and an epilogue that grows with the outputs per CTA.  Of the early sources
 // of links on half an SM a half (bf16, tf32: a third) is counted off: that much runs beside the predecessor.  Cells on whole SMs that leave
 // the next launch no room beside them take up to 0.5 us more.  The exchange, these two and the factor of several cells are fitted to passes up to 256 columns (skinny_us, skinny_gemm.cu), the rest to launches: us, estimated / measured,
 // fp16 split, 1000 units, 384 columns in tiles of 128 rows 25.6 / 25.6; 500 units, 768 columns 15.1 / 15.9; bf16, 1000 units, 384 columns

@@ -10,7 +10,7 @@ namespace zrnn {
 struct ChainParams {
   CUtensorMap a[3];           // activation rows: make_rows_map with a_rows rows, all parts, kbs k-blocks
   CUtensorMap w;              // STORE: make_rows_map with BN rows; LSTM: make_gate_map with BN / 4 units
-  int w_first;                // LSTM, tiles of 128 rows: the weights' lines leave the L2 first
+  int w_first;                // LSTM: the weights' lines leave the L2 first (tiles of 128 rows; the other kernels do not look at it)
   int w_kbtot, w_tiles;       // LSTM: k-blocks per packed tile, packed tiles
   int nsrc, kb;               // sources, k-blocks per source
   int n_early;                // leading sources that were complete when the predecessor kernel passed its own wait
@@ -46,7 +46,7 @@ struct ChainBatch {
 // whole (BN == 32 or 64, split modes): a CTA takes an SM, not half of one.
 cudaError_t launch_tc_chain(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
 cudaError_t launch_tc_link(const ChainBatch& b, int n, int BN, int mode, int epi, int split, bool whole, cudaStream_t st);
-// k-blocks per ring stage and TMA box: a TMA instruction costs its issuing thread about 200 cycles and a stage's hand-over 300
+// k-blocks per ring stage and TMA box: one instruction and one hand-over for several where the ring still holds a few stages
 int chain_kbs(int mode, int BN, int a_rows, int kb, int split);
 int link_kbs(int mode, int BN, int a_rows, int kb, int split);
 // Pairs of CTAs (tc_cell_pair.cu): a_rows = nb / 2, kbs = cell_pair_kbs; weight boxes of 128 rows (STORE) or 32 units (LSTM).

@@ -17,8 +17,8 @@
 // of an ensemble: a search 3806 -> 4008), and it is worth nothing in bf16, which adds up no rounds (3138 / 3150).
 //
 // Warps: 0 - 7 epilogue (warp w reads TMEM lane quadrant w % 4 and takes column group w / 4 of the tile), 8 activation loads,
-// 9 weight loads, 10 and 11 issue MMAs, each into accumulators of its own, so that the wait for a stage and the commit (300
-// cycles in one thread, as long as a k-block's MMAs) of one overlap the other's MMAs.
+// 9 weight loads, 10 and 11 issue MMAs, each into accumulators of its own, so that the wait for a stage and the commit of one overlap
+// the other's MMAs.
 //
 // Not better: the successor's start put off to the end of this link's loads (f32 cells 13.9 -> 16.5); one MMA warp with two sets in turn
 // (3 x 500, 50 columns 1036 -> 1336 us a pass).  Four CTAs per tile (STORE): half the k-blocks of the narrower tile that two CTAs
@@ -48,8 +48,8 @@ constexpr int kMaxStages = 8;
 // Every round costs a commit, a wait and a drain: a launch of three cells of 500 units and 50 columns takes 1.2 us longer in 4 k-steps
 // than in 16, a target step of 2 x 1000, 64 columns in 8 k-steps 2 % longer than in 16.
 __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 2 : 4; }
-// Split modes multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the columns for two products (an MMA of 128 rows
-// takes 45 cycles up to 32 columns, 48 at 64, 64 at 128), and A_lo by W_hi: two MMAs per k-step instead of three.
+// Split modes multiply A_hi by the stacked [W_hi ; W_lo] rows, one MMA of twice the columns for two products (an MMA of 128 rows takes some 60
+// cycles to issue and to run up to 64 columns, 64 at 128), and A_lo by W_hi: two MMAs per k-step instead of three.
 __host__ __device__ constexpr int set_cols(int BN, int mode) { return mode_split(mode) ? 2 * BN : BN; }  // one accumulator set per MMA warp
 // sets that an MMA warp takes in turn, one being added up while the next fills: where the CTA's columns hold them (half an SM: 256).  tf32 adds up
 // no rounds, but a tile of one CTA has four accumulators, a quarter of the K axis each, like the two CTAs of a split one (256 and 320

@@ -148,10 +148,10 @@ __global__ void __launch_bounds__(kThreads, 2) tc_vocab_kernel(const __grid_cons
             for (int b = 0; b < KBS; ++b) {
               const uint64_t dw = make_smem_desc(w_addr + b * PARTS * 16384), dwl = make_smem_desc(w_addr + (b * PARTS + 1) * 16384);
               const uint64_t dh = make_smem_desc(h_addr + b * PARTS * hkb);
-  #pragma unroll
+#pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const uint32_t acc = (k > 0 || b > 0 || i > 0) ? 1u : 0u;
-                  umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
+                umma<mode_kind_tf32(MODE)>(d, dw + 2 * i, dh + 2 * i, idesc2, acc);
                 if (SPLIT_MODE) umma<mode_kind_tf32(MODE)>(d + nb, dwl + 2 * i, dh + 2 * i, idesc, 1u);
               }
             }

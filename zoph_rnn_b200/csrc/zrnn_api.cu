@@ -1712,7 +1712,9 @@ static int run_stack(zrnn_model* m, const std::vector<zrnn_lstm_layer*>& layers,
     const LinkPlan plan = plan_link(L0->eng, zrnn::TC_EPI_LSTM, 4 * g.H, 2, 0, g.H, B, L);
     KScope sweep(KC_LSTM, s, S * L, true);
     // Weights that together exceed the L2 (126 MB), read launch after launch in the same order, would never be found there: the upper half
-    // of the layers gives way to the lower one (4 x 1000 units, 128 columns, 128 MB: 30.7 -> 28.2 us a launch)
+    // of the layers gives way to the lower one, in the tiles of 128 rows (tc_chain.cu; the narrow tiles of smaller launches do not look at
+    // it).  us a pass of 30 steps, 128 columns, without -> with: 4 x 1000 units (128 MB) 1034 -> 971, 8 x 1000 in bf16 1012 -> 935, 5 x 1000
+    // (160 MB) 1685 -> 1666, 8 x 1000 (256 MB) 2035 -> 2023, 3 x 2048 (403 MB) 3008 / 3013: half of it no longer fits either, and it is worth nothing.
     const bool over_l2 = (size_t)L * layers[0]->n_tiles * layers[0]->kbtot * 128 * 128 * (eng_split(g.eng) ? 2 : 1) > ((size_t)110 << 20);
     zrnn::SkinnyBatch sb;
     for (int d = 0; d < S + L - 1; ++d) {
