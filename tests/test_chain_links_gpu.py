@@ -281,3 +281,45 @@ def test_tf32_products_absorb_a_quarter_of_the_k_axis_in_every_tile(K, m):
     many, few = [1 - (api.gemm(dW, dX[:c * K], n, c, K, 2).cpu().numpy().reshape(c, n) / want[:c]).mean() for c in (m, 128)]
     assert few > 3 * 2.0 ** -24  # (it is seen at all)
     assert many < 1.25 * few
+
+
+@pytest.mark.parametrize("dtype", [5, 4, 1])
+@pytest.mark.parametrize("H,V", [(504, 3000), (1000, 700), (104, 9000)])
+def test_vocabulary_projection_with_values_that_are_not_finite(dtype, H, V):
+    """Logits of -inf (words that are masked out by their bias), NaN and infinite hidden states, in launches of many columns on pairs of CTAs
+    and on single ones: a column shows what its own states and the biases make of it, as in a launch of few columns, whatever the others hold."""
+    import torch
+    from zoph_rnn_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(H + V)
+    D = ((torch.rand(V * H, generator=g, device="cuda") - .5) * .4).cpu().numpy()
+    bias = ((torch.rand(V, generator=g, device="cuda") - .5) * .4).cpu().numpy()
+    bias[[0, 5, 64, V - 1]] = -np.inf
+    bias[128:192] = -np.inf  # (whole parts)
+    h = torch.tanh(torch.randn(1200 * H, generator=g, device="cuda")).view(1200, H)
+    targets = torch.randint(200, V - 1, (1200,), generator=g, device="cuda", dtype=torch.int32)
+    targets[3] = 5
+    for nan_word in (None, 300):
+        b = bias.copy()
+        if nan_word is not None:
+            b[nan_word] = np.nan
+        s = api.softmax_layer(V, H, dtype=dtype)
+        s.load_weights(D, b)
+        for N in (100, 300, 1200):
+            x, t = h[:N].clone(), targets[:N].contiguous()
+            mask = torch.ones(N, dtype=torch.int32, device="cuda")
+            clean = [s.compute_loss(x.reshape(-1), t, mask).cpu().numpy().reshape(-1)] + [a.cpu().numpy().reshape(N, -1) for a in s.topk(x.reshape(-1), 13)[:2]]
+            few = [s.compute_loss(x[:40].reshape(-1), t[:40], mask[:40]).cpu().numpy().reshape(-1)] + [a.cpu().numpy().reshape(40, -1) for a in s.topk(x[:40].reshape(-1), 13)[:2]]
+            # the kernels add in another order
+            np.testing.assert_allclose(clean[0][:40], few[0], rtol=2e-6, atol=2e-6)
+            np.testing.assert_allclose(clean[1][:40], few[1], rtol=2e-6, atol=2e-6)
+            if nan_word is None:
+                assert clean[0][3] == -np.inf and np.isfinite(clean[0][np.arange(N) != 3]).all() and np.isfinite(clean[1]).all()
+                assert not np.isin(clean[2], np.r_[[0, 5, 64, V - 1], 128:192]).any()
+            else:
+                assert np.isnan(clean[0][np.arange(N) != 3]).all()
+            x[7, 1], x[33, 2], x[N - 1, :] = float("nan"), float("inf"), float("nan")
+            bad, rest = [7, 33, N - 1], np.setdiff1d(np.arange(N), [7, 33, N - 1])
+            got = [s.compute_loss(x.reshape(-1), t, mask).cpu().numpy().reshape(-1)] + [a.cpu().numpy().reshape(N, -1) for a in s.topk(x.reshape(-1), 13)[:2]]
+            for a, c in zip(got, clean):
+                np.testing.assert_array_equal(a[rest], c[rest])
+            assert not np.isfinite(got[0][bad]).any()
