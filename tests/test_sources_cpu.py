@@ -90,12 +90,20 @@ def test_gemm_packs_its_weights_before_the_launch_ahead_of_the_product():
 
 def test_a_cta_with_all_of_the_tensor_memory_and_a_partner_has_its_sm_for_itself():
     """Two kernels of different streams whose CTAs wait for their cluster partners must not hold the tensor memory that the other one's
-    partner waits for: a kernel that allocates all 512 columns and has partners asks for (nearly) all of an SM's shared memory."""
-    s = body("tc_link.cu", "cudaError_t launch_t(", "cudaLaunchKernelEx")
-    assert "const size_t smem = WHOLE && SPLIT > 1 ? (size_t)kWholeSm :" in s and "cfg.dynamicSmemBytes = smem;" in s
-    with open(os.path.join(CSRC, "tc_link.cu")) as f:
-        assert "kWholeSm = 224 * 1024" in f.read()
-    for name in ("tc_vocab_pair.cu", "tc_cell_pair.cu"):
+    partner waits for: a kernel that allocates all 512 columns and has partners asks for (nearly) all of an SM's shared memory.  That the
+    constant is large enough is a static_assert beside it; here: that it is what these launches ask for, and that no other kernel with
+    cluster partners allocates all columns."""
+    for name, constant, when in (("tc_link.cu", "kWholeSm", r"WHOLE && SPLIT > 1 \? \(size_t\)kWholeSm :"), ("tc_vocab_pair.cu", "kSmem", None), ("tc_cell_pair.cu", "kSmem", None)):
         with open(os.path.join(CSRC, name)) as f:
-            assert "kSmem = 227 * 1024" in f.read()
-        assert "cfg.dynamicSmemBytes = kSmem;" in body(name, "cudaError_t launch_t(", "cudaLaunchKernelEx")
+            whole = re.sub(r"\s+", " ", re.sub(r"//[^\n]*", "", f.read()))
+        assert "static_assert(fills_sm(%s)," % constant in whole
+        launch = re.sub(r"\s+", " ", body(name, "cudaError_t launch_t(", "cudaLaunchKernelEx"))
+        asked = re.search(r"cfg\.dynamicSmemBytes = (\w+);", launch).group(1)
+        if when:
+            assert re.search(r"const size_t %s = %s" % (asked, when), launch)
+        else:
+            assert asked == constant
+    with_partners = {n for n in os.listdir(CSRC) if n.endswith(".cu") and "tcgen05.alloc" in open(os.path.join(CSRC, n)).read() + "\n"
+                     and re.search(r"__cluster_dims__|ClusterDimension", open(os.path.join(CSRC, n)).read())}
+    assert with_partners == {"tc_link.cu", "tc_decoder.cu"}  # (the pair kernels allocate through tc_pair_device.cuh)
+    assert "static_assert(fills_sm(dec_smem(TC_BF16))" in open(os.path.join(CSRC, "tc_decoder.cu")).read()

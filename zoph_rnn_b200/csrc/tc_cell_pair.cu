@@ -30,6 +30,7 @@ constexpr int kSmem = 227 * 1024, kMaxStages = 8, kGroups = 8;  // kGroups: grou
 // k-blocks per round: as many k-steps as an accumulator of the links absorbs (tc_link.cu)
 __host__ __device__ constexpr int round_kb(int mode, int kb) { return kb <= (mode == TC_TF32X3 ? 16 : 8) ? 1 : 2; }
 __host__ __device__ constexpr int acc_sets(int nb) { return nb <= 128 ? 3 : (nb <= 160 ? 2 : 1); }  // (split modes: and one for the cross products)
+static_assert(fills_sm(kSmem), "both CTAs of a pair hold all of the tensor memory");
 struct alignas(16) PairCtrl {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t set_full[3], set_empty[3], accum;

@@ -56,6 +56,9 @@ __host__ __device__ constexpr int dec_smem(int mode) {
   return dec_nw(mode) * dec_wstage(mode) + kARingBytes + kSlotBytes + 1024;
 }
 
+static_assert(fills_sm(dec_smem(TC_BF16)) && fills_sm(dec_smem(TC_TF32)) && fills_sm(dec_smem(TC_TF32X3)) && fills_sm(dec_smem(TC_F16X2)),
+              "CTAs that wait for all others are alone on their SMs");
+
 enum { PH_CELL = 0, PH_PGEMM = 1, PH_ATT = 2, PH_COMB = 3 };
 // developer timeline: CTA `detail_cta` leaves 8 %globaltimer stamps per phase in p.detail[ph * 8 ..]
 #define ZD_STAMP(k)                                                                                        \

@@ -56,6 +56,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
   return true;
 }
+// A CTA that holds all 512 columns of tensor memory while it waits for its cluster partners must be alone on its SM, or a CTA of another
+// stream could be there that holds columns and waits, in its turn, for a partner that this one's partner keeps out.  Dynamic shared memory that
+// leaves, of 228 KB and with 1 KB taken for every CTA, less than any kernel with tensor memory asks for (16 KB at the least: a stage and
+// the rows that an MMA reads beyond it).
+constexpr bool fills_sm(int dynamic_bytes) { return dynamic_bytes + 2 * 1024 + 16 * 1024 > 228 * 1024; }
 // Roles of one warp (loads, MMA issue) run with all of its lanes and let one of them issue.  Their instructions take descriptors, barrier
 // and tensor-memory addresses from uniform registers; in a loop of a single thread every one of those is moved there anew: 62 cycles
 // per MMA and 400 per stage (bf16, 128 x 64 x 64: 648 cycles a stage against 415 with a whole warp; fp16 split, 128 x 64: 908 / 667).

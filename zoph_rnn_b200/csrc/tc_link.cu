@@ -39,6 +39,7 @@ namespace {
 constexpr int kEpiWarps = 8, kAWarp = 8, kWWarp = 9, kMmaWarp = 10, kMmaWarps = 2, kThreads = 384;
 constexpr int kHalfSm = 113 * 1024;  // two CTAs per SM: (228 KB - 2 x 1 KB) / 2
 constexpr int kWholeSm = 224 * 1024;
+static_assert(fills_sm(kWholeSm), "CTAs of split tiles with all of the tensor memory are alone on their SMs");
 constexpr int kMaxStages = 8;
 // The tensor core's fp32 accumulator truncates, so in the split modes it is not asked to absorb many products in a row: the K axis
 // is walked in rounds of round_kb k-blocks (half of them each MMA warp's), and the epilogue warps add each finished round to sums

@@ -33,6 +33,7 @@ namespace {
 
 constexpr int kEpiWarps = 16, kHWarp = 16, kWWarp = 17, kMmaWarp = 18, kThreads = 608;
 constexpr int kSmem = 227 * 1024, kMaxStages = 8, kGroups = 8;  // kGroups: groups of 8 columns per epilogue warp
+static_assert(fills_sm(kSmem), "both CTAs of a pair hold all of the tensor memory");
 struct alignas(16) PairCtrl {
   uint64_t full[kMaxStages], empty[kMaxStages];
   uint64_t acc_full[2], main_empty[2], cross_empty[2];
