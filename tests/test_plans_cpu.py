@@ -37,9 +37,10 @@ int main(int argc, char**) {
       const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
       if (us < best) best = us;
     }
+    const int sk = epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE;
     const bool skinny = M <= 64 && (mode == zrnn::TC_BF16 || mode == zrnn::TC_F16X2) &&
-                        zrnn::skinny_us(mode == zrnn::TC_BF16 ? zrnn::SK_BF16 : zrnn::SK_F16X2, epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE,
-                                        rows, nsrc * H, M, cells, early > 0 && !beside) < p.us;
+                        (zrnn::skinny_us(mode == zrnn::TC_BF16 ? zrnn::SK_BF16 : zrnn::SK_F16X2, sk, rows, nsrc * H, M, cells, early > 0 && !beside) < p.us ||
+                         (mode == zrnn::TC_F16X2 && zrnn::skinny_more_exact(sk, rows, cells, nsrc, H, early, M)));
     std::printf("%d %d %d %g %d\n", p.BN, p.split, p.nb, best, (int)skinny);
   }
 }
@@ -168,3 +169,14 @@ def test_many_columns_take_pairs_of_ctas_only_where_they_are_faster(plans):
     q = [(BF16, 504, 2100, False), (BF16, 1000, 900, False), (BF16, 1000, 1024, False), (F16X2, 504, 3000, False), (F16X2, 1000, 1300, True), (BF16, 1000, 768, True), (F16X2, 2048, 600, True)]
     got = plans([(mode, LSTM, 4 * H, 2, kblocks(mode, H), 0, M, 0) for mode, H, M, _ in q])
     assert [(a, p[2]) for a, p in zip(q, got) if (p[2] > 0) != a[3]] == []
+
+
+def test_the_more_exact_kernel_keeps_its_shapes(plans):
+    """Accumulators of the warp-level kernel absorb fewer products than those of the links, so in the fp16 split the refitted estimates do not take
+    shapes from it: the largest numbers of columns at which it was chosen when links were issued by one thread (kind, H -> columns)."""
+    kept = [("cell", 500, 32), ("cell", 640, 24), ("cell", 320, 64), ("product", 500, 64), ("product", 768, 64), ("product", 1000, 48), ("product", 1024, 48),
+            ("stacked", 640, 64), ("stacked", 1000, 40), ("stacked", 1200, 40)]
+    kinds = {"cell": (LSTM, 4, 2, 1), "product": (STORE, 1, 2, 1), "stacked": (STORE, 2, 1, 0)}
+    q = [(kinds[k][0], kinds[k][1] * H, kinds[k][2], kinds[k][3], H, M) for k, H, top in kept for M in (1, top // 2, top)]
+    got = plans([(F16X2, epi, rows, nsrc, kblocks(F16X2, H), early, M, 0, 1, H) for epi, rows, nsrc, early, H, M in q])
+    assert [(a, g) for a, g in zip(q, got) if not g[4]] == []

@@ -19,12 +19,14 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
 
 #include "att_device.cuh"
 #include "kernels.cuh"
+#include "tc_gemm.cuh"
 
 namespace zrnn {
 namespace {
@@ -389,6 +391,26 @@ float skinny_us(int mode, int epi, int rows, int K, int cols, int n, bool early)
   const bool cell = epi == SK_EPI_LSTM;
   if (mode == SK_F16X2) return 3.1f + (cell ? (early ? 1.65f : 0.f) : 0.9f) + mw * (0.105f + nt * (0.195f + 0.025f * nt));
   return 3.15f + (cell ? (early ? 0.5f : 0.f) : 0.5f) + mw * (0.09f + 0.105f * nt);
+}
+
+// An accumulator of this kernel absorbs 2 k-steps, one of the links 4 or 8, and a cell of 600 units is 1.30e-7 from float64 here and 1.65e-7 there;
+// log-probabilities of 1 x 1024 units, 30 columns 1.36e-6 with the combiner here and 1.54e-6 with it there.  Time alone does not decide, then: the
+// links take over from the number of columns on at which this kernel's time reaches what a link took while one thread issued its MMAs
+// (this estimate), up to 2 us more than one takes now.
+bool skinny_more_exact(int epi, int rows, int cells, int nsrc, int H, int n_early, int cols) {
+  const float mw = (float)rows * H * nsrc * cells * 1e-6f, nt = (float)((cols + 7) / 8);
+  const float here = 4.0f + mw * (0.285f + nt * (0.144f + 0.0114f * nt));
+  const int kb = (H + 63) / 64, a_rows = (cols + 7) / 8 * 8, sms = device_sms();
+  for (int BN = epi == SK_EPI_LSTM ? 32 : 16; BN <= 128; BN *= 2)
+    for (int split = 1; split <= 2; ++split) {
+      if (split > 1 && (cells > 1 || BN > 64 || kb < 2 * split)) continue;
+      const int waves = (cells * ((rows + BN - 1) / BN) * split + sms - 1) / sms;
+      const float mma = BN <= 64 ? 4.f * (std::max(45, BN) + 45) : 6.f * BN, reads = BN <= 64 ? 4.f * (8192 + 96 * BN) : 12.f * (4096 + 32 * BN);
+      const float writes = 256.f * (a_rows + BN), kb_us = std::max(writes / 77e3f, std::max(mma, (reads + writes) / 128.f) / 1900.f);
+      const float kbs = kb * (nsrc - (BN <= 64 ? 0.5f * n_early : 0.f)) / split;
+      if (here >= 3.2f + waves * (kb_us * kbs + 0.01f * BN / split) + (split == 2 ? 1.3f : 0.f)) return false;
+    }
+  return true;
 }
 
 cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st) {

@@ -44,6 +44,8 @@ struct SkinnyBatch {
 // about how long launch_skinny takes for n problems of `rows` weight rows x K elements (all sources) and `cols` columns, on the scale of
 // plan_chain's estimate; early: some sources are early and no other stream's launches run beside
 float skinny_us(int mode, int epi, int rows, int K, int cols, int n, bool early);
+// the fp16 split takes this kernel up to here in any case, because its accumulators absorb fewer products (skinny_gemm.cu)
+bool skinny_more_exact(int epi, int rows, int cells, int nsrc, int H, int n_early, int cols);
 // n independent problems of the same shape class (mode, epilogue, N, K, M) in one launch
 cudaError_t launch_skinny(const SkinnyBatch& b, int n, int mode, int epi, cudaStream_t st);
 

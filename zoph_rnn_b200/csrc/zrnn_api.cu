@@ -421,9 +421,10 @@ LinkPlan plan_link(int eng, int epi, int rows, int nsrc, int n_early, int H, int
   const int epk = 128 / eng_eb(eng);
   LinkPlan p;
   p.chain = zrnn::plan_chain(eng_tcmode(eng), epi, rows, n, nsrc, (H + epk - 1) / epk, n_early, cols, beside);
+  const int sk_epi = epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE;
   p.skinny = skinny_engine(eng) && cols <= 64 &&
-             zrnn::skinny_us(skinny_mode(eng), epi == zrnn::TC_EPI_LSTM ? zrnn::SK_EPI_LSTM : zrnn::SK_EPI_STORE, rows, nsrc * H, cols, n,
-                             n_early > 0 && !beside) < p.chain.us;
+             (zrnn::skinny_us(skinny_mode(eng), sk_epi, rows, nsrc * H, cols, n, n_early > 0 && !beside) < p.chain.us ||
+              (eng == ENG_H2 && zrnn::skinny_more_exact(sk_epi, rows, n, nsrc, H, n_early, cols)));
   return p;
 }
 // weights stored in packed 128-row tiles: tile-contiguous k-blocks (kbtot > 0) or plain rows of ld elements
